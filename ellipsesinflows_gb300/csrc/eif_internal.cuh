@@ -209,6 +209,8 @@ struct eif_ctx {
   size_t wcap;                  // capacity of wbuf in cells
   int chunk_cap;                // capacity of partial in chunks
   float *pf;                    // per-particle single-precision parameters (mixed form)
+  double *pd = nullptr;         // per-particle parameters of the indicator (double-precision form)
+  double2 *tanh_tab = nullptr;  // tanh and sech^2 at multiples of 1/16 (double-precision form)
   int4 *tdesc;                  // task table: particle, row, columns and image of every chunk
   // weights of the last indicator evaluation in a sub-iteration loop (mixed form), with
   // the particles' geometry words, boxes and first tasks (WeightMemo in ibm_device.cuh)

@@ -54,8 +54,8 @@ __global__ void __launch_bounds__(TT_WARPS * 32) k_task_table_scan(const int *__
 // one function, compiled alike in both translation units, gives both kernels the same
 // bits.
 __global__ void __launch_bounds__(256) k_ibm_work(WorkArgs a) {
-  // per warp: body-frame offsets of its near cells, overwritten by their weights
-  __shared__ double2 slot_buf[8][CHUNK];
+  // per warp: the columns of its near cells, overwritten by their weights
+  __shared__ double slot_buf[8][CHUNK];
   const int wmode = a.iter ? (*a.iter == 0u ? 2 : 0) : a.wmode;
   ibm_work_tasks<false>(a, wmode, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
                         slot_buf[threadIdx.x >> 5]);
@@ -370,7 +370,17 @@ int ibm_reserve(eif_ctx *c, size_t chunks) {
   EIF_CK(c, cudaMalloc((void **)&c->partial, sizeof(double) * 3 * chunks));
   EIF_CK(c, cudaMalloc((void **)&c->wbuf, sizeof(double2) * c->wcap));
   EIF_CK(c, cudaMalloc((void **)&c->wcache, sizeof(double) * c->wcap));
-  EIF_CK(c, cudaMalloc((void **)&c->pf, sizeof(float) * PF_WORDS * c->np));
+  if (c->cfg.precision == EIF_PREC_MIXED) EIF_CK(c, cudaMalloc((void **)&c->pf, sizeof(float) * PF_WORDS * c->np));
+  else EIF_CK(c, cudaMalloc((void **)&c->pd, sizeof(double) * PD_WORDS * c->np));
+  if (c->cfg.precision != EIF_PREC_MIXED && !c->tanh_tab) {
+    std::vector<double2> tab(TANH_N);
+    for (int k = 0; k < TANH_N; k++) {
+      const long double z = (long double)k / TANH_STEPS, ch = coshl(z);
+      tab[k] = make_double2((double)tanhl(z), (double)(1.L / (ch * ch)));
+    }
+    EIF_CK(c, cudaMalloc((void **)&c->tanh_tab, sizeof(double2) * TANH_N));
+    EIF_CK(c, cudaMemcpy(c->tanh_tab, tab.data(), sizeof(double2) * TANH_N, cudaMemcpyHostToDevice));
+  }
   EIF_CK(c, cudaMalloc((void **)&c->tdesc, sizeof(int4) * (size_t)chunks));
   const int nbands = (c->jtot + GTY - 1) / GTY;
   c->band_cap = 3 * c->np;
@@ -397,6 +407,8 @@ void ibm_free(eif_ctx *c) {
   if (c->wbuf) cudaFree(c->wbuf);
   if (c->wcache) cudaFree(c->wcache);
   if (c->pf) cudaFree(c->pf);
+  if (c->pd) cudaFree(c->pd);
+  if (c->tanh_tab) cudaFree(c->tanh_tab);
   if (c->tdesc) cudaFree(c->tdesc);
   if (c->band_lists) cudaFree(c->band_lists);
   if (c->band_counts) cudaFree(c->band_counts);
@@ -410,7 +422,7 @@ void ibm_free(eif_ctx *c) {
   c->band_lists = nullptr; c->band_counts = nullptr; c->band_marks = nullptr; c->edesc = nullptr;
   c->box = nullptr; c->chunk_off = nullptr; c->partial = nullptr; c->wbuf = nullptr; c->wcache = nullptr;
   c->weights_x_valid = false;
-  c->pf = nullptr; c->tdesc = nullptr;
+  c->pf = nullptr; c->pd = nullptr; c->tanh_tab = nullptr; c->tdesc = nullptr;
   c->chunk_cap = 0; c->wcap = 0;
 }
 
@@ -427,7 +439,7 @@ static int launch_boxes(eif_ctx *c, bool use_increment) {
   int *cnt = b.nchunk;
   EIF_PROF(c, "ibm_boxes", c->np <= TT_MAX_NP ? 2 : 3);
   EIF_CK(c, cudaMemsetAsync(cnt, 0, sizeof(int) * c->np, c->stream));
-  k_boxes<<<dim3((c->np + 31) / 32, b.pf ? BOX_PARTS : 3), 32, 0, c->stream>>>(b);
+  k_boxes<<<dim3((c->np + 31) / 32, BOX_PARTS), 32, 0, c->stream>>>(b);
   EIF_LAUNCH_CK(c);
   if (c->np <= TT_MAX_NP) {
     k_task_table_scan<<<(c->np + TT_WARPS - 1) / TT_WARPS, TT_WARPS * 32, 0, c->stream>>>(
@@ -625,6 +637,8 @@ namespace {
 
 struct AdjWorkArgs {
   const double *P;
+  const double *pd;         // per-particle parameters at the boxes' positions (PD_WORDS each)
+  const double2 *tanh_tab;
   const double *ux, *uy, *xc, *yc, *dt;
   const int *off;
   const int4 *tdesc;
@@ -645,7 +659,6 @@ __global__ void __launch_bounds__(256) k_ibm_adj(AdjWorkArgs a) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int total = EIF_CHK(a.bd.rec, a.np, a.bd.off, 70) ? __ldg(a.off + a.np) : 0;
-  const double rh = 1. / a.h;
   const double dxdy = a.dx * a.dy;
   const double kdt = a.mode == 1 ? dxdy / __ldg(a.dt) : 0.;
   const int pc = a.pcap, ld = a.ld;
@@ -657,22 +670,25 @@ __global__ void __launch_bounds__(256) k_ibm_adj(AdjWorkArgs a) {
     RowTask t;
     const bool task = task_of(dsc, a.np, t) && EIF_CHK(a.bd.rec, t.j, a.bd.yc - 1, 73);
     const double *P = a.P;
-    const double pden = __ldg(P + EIF_P_DEN * pc + n), pa = __ldg(P + EIF_P_A * pc + n), pb = __ldg(P + EIF_P_B * pc + n);
-    double px = __ldg(P + EIF_P_X * pc + n), py = __ldg(P + EIF_P_Y * pc + n), paz = __ldg(P + EIF_P_AZ * pc + n);
-    if (a.use_increment) {
-      px = px + __ldg(P + EIF_P_DX * pc + n);
-      py = py + __ldg(P + EIF_P_DY * pc + n);
-      paz = paz + __ldg(P + EIF_P_DAZ * pc + n);
-    }
-    const double pm = pmass(pden, pa, pb), pim = pmoi(pden, pa, pb);
+    const double *pd = a.pd + (size_t)PD_WORDS * n;
+    const float *pdf = reinterpret_cast<const float *>(pd + PD_F);
+    const double px = __ldg(pd + PD_X), py_ = __ldg(pd + PD_Y) + a.ly * (task ? t.img : 0);
+    const double rpm = __ldg(pd + PD_RPM), rpim = __ldg(pd + PD_RPIM);
     const double pux = __ldg(P + EIF_P_UX * pc + n), puy = __ldg(P + EIF_P_UY * pc + n), pvz = __ldg(P + EIF_P_VZ * pc + n);
-    const double b0 = __ldg(a.bar + n), b1 = __ldg(a.bar + a.np + n), b2 = __ldg(a.bar + 2 * a.np + n);
-    const Ell e = make_ell(pa, pb, px, py, paz);
-    const double py_ = py + a.ly * (task ? t.img : 0);
+    // cotangents per unit mass and moment of inertia
+    const double kf = a.mode == 1 ? kdt : 1.;
+    const double b0 = __ldg(a.bar + n) * (kf * rpm), b1 = __ldg(a.bar + a.np + n) * (kf * rpm),
+                 b2 = __ldg(a.bar + 2 * a.np + n) * (kf * rpim);
+    const double cz = __ldg(pd + PD_CZ), sz = __ldg(pd + PD_SZ), pa = __ldg(pd + PD_A), pb = __ldg(pd + PD_B);
+    EllF ef;
+    ef.a = __ldg(pdf + PDF_A); ef.b = __ldg(pdf + PDF_B); ef.kex = __ldg(pdf + PDF_KEX); ef.key = __ldg(pdf + PDF_KEY);
+    ef.cz = 0.f; ef.sz = 0.f;
     const int j = task ? t.j : 1;
     const double y = __ldg(a.yc + j);
     const double ry = y - py_;
-    const double mn = fmin(pa, pb);
+    float olo, ohi, ilo, ihi;
+    row_chords(__ldg(pdf + PDF_AL), __ldg(pdf + PDF_KA), __ldg(pdf + PDF_DE), __ldg(pdf + PDF_SO2), __ldg(pdf + PDF_SI2),
+               __ldg(pdf + PDF_RO2), eifd::d2f(ry), olo, ohi, ilo, ihi);
     double sX = 0., sY = 0., sA = 0., sU = 0., sV = 0., sW = 0.;
 #pragma unroll 1
     for (int half = 0; half < CHUNK / 32; half++) {
@@ -686,10 +702,6 @@ __global__ void __launch_bounds__(256) k_ibm_adj(AdjWorkArgs a) {
       if (in) {
         const double x = __ldg(a.xc + i);
         const double rx = x - px;
-        const double qx = e.cz * rx - e.sz * ry, qy = e.sz * rx + e.cz * ry;
-        // distance bound from the gauge of the ellipse: beyond FAR_CELLS_D cells tanh(2D)
-        // is +-1 in double precision and both weights' derivatives vanish
-        const double rho = sqrt((qx / pa) * (qx / pa) + (qy / pb) * (qy / pb));
         double th, gwx = 0., gwy = 0.;
         const long long slot = (long long)c * CHUNK + half * 32 + lane;
         const bool cached = a.geo == 2 && EIF_CHK(a.bd.rec, slot, a.nslot, 81);
@@ -697,25 +709,21 @@ __global__ void __launch_bounds__(256) k_ibm_adj(AdjWorkArgs a) {
           th = a.geom[slot];
           gwx = a.geom[a.nslot + slot];
           gwy = a.geom[2 * a.nslot + slot];
-        } else if (mn * fabs(rho - 1.) * rh >= FAR_CELLS_D) {
-          th = rho < 1. ? 1. : -1.;
         } else {
-          const double f0 = 1. - (qx / pa) * (qx / pa) - (qy / pb) * (qy / pb);
-          const double sign = f0 > 0. ? 1. : -1.;
-          const double tt = normal_t(e, qx, qy);
-          double st, ct;
-          sincos(tt, &st, &ct);
-          const double fx = pa * ct - qx, fy = pb * st - qy;
-          th = tanh(BETA * (sign * sqrt(fx * fx + fy * fy) * rh));
-          // outward normal at the foot (cos t / a, sin t / b); dD/dq = -n / h
-          double nx = ct / pa, ny = st / pb;
-          const double nn = 1. / sqrt(nx * nx + ny * ny);
-          nx *= nn;
-          ny *= nn;
-          const double gbx = -nx * rh, gby = -ny * rh;
-          // g = R(az) dD/dq with cz = cos(-az), sz = sin(-az)
-          gwx = e.cz * gbx + e.sz * gby;
-          gwy = -e.sz * gbx + e.cz * gby;
+          // far cells (row_chords): tanh(2D) is +-1 in double precision and both weights'
+          // derivatives vanish
+          const float Xf = eifd::d2f(rx);
+          const int side = !(Xf > olo && Xf < ohi) ? -1 : ((Xf >= ilo && Xf <= ihi) ? 1 : 0);
+          if (side != 0) {
+            th = side > 0 ? 1. : -1.;
+          } else {
+            // g = R(az) dD/dq, dD/dq = -n / h with the outward normal n at the foot; cz and
+            // sz carry the factor BETA / h
+            double nx, ny;
+            th = indicator_d<true>(pa, pb, ef, fma(cz, rx, -(sz * ry)), fma(sz, rx, cz * ry), a.tanh_tab, nx, ny);
+            gwx = (-1. / BETA) * fma(cz, nx, sz * ny);
+            gwy = (-1. / BETA) * fma(cz, ny, -(sz * nx));
+          }
         }
         if (a.geo == 1 && EIF_CHK(a.bd.rec, slot, a.nslot, 82)) {
           a.geom[slot] = th;
@@ -728,27 +736,27 @@ __global__ void __launch_bounds__(256) k_ibm_adj(AdjWorkArgs a) {
         const double dDdaz = gwx * ry - gwy * rx;
         if (a.mode == 0) {
           const double wv = 0.5 * (1. + th);
-          const double cx = b0 / pm, cy = b1 / pm, cz = b2 / pim;
-          contrib = make_double2(wv * dxdy * (cx - cz * ry), wv * dxdy * (cy + cz * rx));
-          const double sv = dxdy * (cx * uxf + cy * uyf + cz * (-ry * uxf + rx * uyf));
+          const double cx = b0, cy = b1, cw = b2;
+          contrib = make_double2(wv * dxdy * (cx - cw * ry), wv * dxdy * (cy + cw * rx));
+          const double sv = dxdy * (cx * uxf + cy * uyf + cw * (-ry * uxf + rx * uyf));
           const double dw = ws * sv;
-          sX += -dw * gwx - wv * dxdy * cz * uyf;
-          sY += -dw * gwy + wv * dxdy * cz * uxf;
+          sX += -dw * gwx - wv * dxdy * cw * uyf;
+          sY += -dw * gwy + wv * dxdy * cw * uxf;
           sA += dw * dDdaz;
         } else {
           const int cc = j * ld + i;
           const double urx = pux - pvz * ry, ury = puy + pvz * rx;
           const double ex = urx - uxf, ey = ury - uyf;
-          const double Cx = __ldg(a.gx + cc) - b0 * kdt / pm + b2 * ry * kdt / pim;
-          const double Cy = __ldg(a.gy + cc) - b1 * kdt / pm - b2 * rx * kdt / pim;
+          const double Cx = __ldg(a.gx + cc) - b0 + b2 * ry;
+          const double Cy = __ldg(a.gy + cc) - b1 - b2 * rx;
           const double Ex = ws * Cx, Ey = ws * Cy;
           contrib = make_double2(-Ex, -Ey);
           sU += Ex;
           sV += Ey;
           sW += -ry * Ex + rx * Ey;
           const double dw = (ex * Cx + ey * Cy) * (-2. * BETA * th * ws);
-          sX += -dw * gwx - pvz * Ey + b2 * ws * ey * kdt / pim;
-          sY += -dw * gwy + pvz * Ex - b2 * ws * ex * kdt / pim;
+          sX += -dw * gwx - pvz * Ey + b2 * ws * ey;
+          sY += -dw * gwy + pvz * Ex - b2 * ws * ex;
           sA += dw * dDdaz;
         }
       }
@@ -799,7 +807,7 @@ int launch_adj_pass(eif_ctx *c, const AdjPass &p) {
   int rc = launch_boxes(c, p.use_increment);
   if (rc) return rc;
   AdjWorkArgs w;
-  w.P = c->P; w.ux = p.ux; w.uy = p.uy; w.xc = c->xc; w.yc = c->yc; w.dt = c->d_scal;
+  w.P = c->P; w.pd = c->pd; w.tanh_tab = c->tanh_tab; w.ux = p.ux; w.uy = p.uy; w.xc = c->xc; w.yc = c->yc; w.dt = c->d_scal;
   w.off = c->chunk_off; w.tdesc = c->tdesc;
   w.bar = p.bar; w.gx = p.gx; w.gy = p.gy;
   w.part = p.part;

@@ -40,22 +40,6 @@ constexpr int GTX = 128, GTY = 8, GTHREADS = 256;  // gather tile and block
 constexpr int GCOLS = 64;   // columns covered by the threads of one pass (GTX / GCOLS passes)
 constexpr int LMAX = 256;       // gather entries staged in shared memory at a time (GTHREADS)
 
-// per-particle geometry needed by a box cell evaluation
-struct Ell {
-  double a, b, px, py, cz, sz;   // semi-axes, centre, cos(-az), sin(-az)
-  double kex, key, ab2;          // a(1-(b/a)^2), b(1-(a/b)^2), a*a+b*b
-};
-
-__device__ __forceinline__ Ell make_ell(double a, double b, double px, double py, double az) {
-  Ell e;
-  e.a = a; e.b = b; e.px = px; e.py = py;
-  sincos(-az, &e.sz, &e.cz);
-  e.kex = a * (1. - (b / a) * (b / a));
-  e.key = b * (1. - (a / b) * (a / b));
-  e.ab2 = a * a + b * b;
-  return e;
-}
-
 // ---------------------------------------------------------------------------
 // The normal-foot iteration of ellipse.c:30-65 in single precision (the mixed form's
 // indicator, and the start of the double-precision iteration below). The distance at
@@ -106,52 +90,180 @@ __device__ __forceinline__ float normal_t_f(const EllF &e, float x_, float y_) {
 }
 
 
-// ellipse.c:30-65 (x_, y_ in the body frame). The iteration, its stopping rule and its
-// cap are the reference's; it starts from the foot that the same iteration finds in
-// single precision (on the FP32 pipe, about 1e-4 or closer) instead of from pi/4. The
-// fixed point is the same, and the double-precision iterations (the expensive part on
-// this GPU's FP64 pipe) drop from about four to two: the first moves t by the start's
-// error, the second by its square, below the 1e-8 stop. Not inlined, like
-// ibm_work_tasks: compiled on its own it gives the same bits in every kernel.
-__device__ __noinline__ double normal_t(const Ell &e, double x_, double y_) {
-  const double px = fabs(x_), py = fabs(y_);
-  EllF ef;
-  ef.a = eifd::d2f(e.a); ef.b = eifd::d2f(e.b); ef.kex = eifd::d2f(e.kex); ef.key = eifd::d2f(e.key);
-  ef.cz = 0.f; ef.sz = 0.f;
-  double t = eifd::f2d(normal_t_f_q1(ef, eifd::d2f(px), eifd::d2f(py)));
+// Per-particle parameters of the double-precision form, PD_WORDS doubles per particle,
+// written with the boxes (box_part): what every row task of a particle needs, formed once
+// per particle instead of once per task by all lanes (about 150 FP64 operations a task:
+// the stored-weight sums took 0.95 ms at 2048 x 4096 with 2048 ellipses that way, nearly
+// all of it this set-up). Lengths with a bar are in units of h / BETA, so that the distance
+// the cells compute is the argument of tanh.
+constexpr int PD_WORDS = 14;
+enum { PD_X, PD_Y,            // centre (with the increments where the boxes have them)
+       PD_CZ, PD_SZ,          // cos(-az), sin(-az) times BETA / h
+       PD_A, PD_B,            // semi-axes, barred
+       PD_RPM, PD_RPIM,       // 1 / mass, 1 / moment of inertia
+       PD_F };                // single-precision words from here:
+enum { PDF_AL, PDF_KA, PDF_DE, PDF_SO2, PDF_SI2, PDF_RO2,   // row_chords
+       PDF_A, PDF_B, PDF_KEX, PDF_KEY, PDF_WORDS };         // the foot iteration, barred
+static_assert(2 * (PD_WORDS - PD_F) >= PDF_WORDS && PD_WORDS % 2 == 0, "per-particle parameter block");
+
+// The iteration of ellipse.c:30-65 in double precision with its stopping rule and cap, from
+// the foot t that normal_t_f_q1 finds, for offsets (px, py) in the first quadrant: the foot's
+// parameter. Only for the few cells next to the evolute, where foot_d does not settle.
+__device__ __noinline__ double normal_t_q1(double a, double b, double px, double py, double t) {
+  const double kex = a * (1. - (b / a) * (b / a)), key = b * (1. - (a / b) * (a / b)), ab2 = a * a + b * b;
   for (int n = 0;; n++) {
     double st, ct;
     sincos(t, &st, &ct);
-    const double x = e.a * ct, y = e.b * st;
-    const double ex = e.kex * (ct * ct * ct);
-    const double ey = e.key * (st * st * st);
+    const double x = a * ct, y = b * st;
+    const double ex = kex * (ct * ct * ct);
+    const double ey = key * (st * st * st);
     const double rx = x - ex, ry = y - ey;
     const double qx = px - ex, qy = py - ey;
     const double r = sqrt(ry * ry + rx * rx);
     const double q = sqrt(qy * qy + qx * qx);
     const double dc = r * asin((rx * qy - ry * qx) / (r * q));
-    const double dt = dc / sqrt(e.ab2 - x * x - y * y);
+    const double dt = dc / sqrt(ab2 - x * x - y * y);
     t += dt;
     t = fmin(0.5 * M_PI, t);
     t = fmax(0., t);
     if (fabs(dt) < 1.e-8) break;
     if (n > EIF_NORMAL_MAX_ITER - 1) break;
   }
-  if (x_ < 0.) t = M_PI - t;
-  if (y_ < 0.) t = -t;
   return t;
 }
 
-// auxiliary.c:19-47, in units of the grid size h (rh = 1/h), from the body-frame
-// offset (x_, y_) = R(-az) (x - px, y - py)
-__device__ __forceinline__ double signed_dist_body(const Ell &e, double x_, double y_, double rh) {
-  const double f0 = 1. - (x_ / e.a) * (x_ / e.a) - (y_ / e.b) * (y_ / e.b);
-  const double sign = f0 > 0. ? 1. : -1.;
-  const double t = normal_t(e, x_, y_);
-  double st, ct;
-  sincos(t, &st, &ct);
-  const double dxx = e.a * ct - x_, dyy = e.b * st - y_;
-  return sign * sqrt(dxx * dxx + dyy * dyy) * rh;
+// The normal foot of (px, py), first quadrant, on the ellipse (a, b), and the distance to
+// it, positive outside. Bound by the FP64 pipe (one warp instruction in 16 cycles), so the
+// double-precision work is kept to what carries the precision:
+//  * the foot (c, s) = (cos t, sin t) comes from the single-precision iteration and one
+//    Newton step there, to about 2e-7, and is put on the unit circle in double precision;
+//  * with v = (px, py) - (a c, b s), T the derivative of the ellipse in t (w = |T|) and N
+//    its outward normal, the remaining angle to the foot is d = v.T / K,
+//    K = w^2 + v.(a c, b s) = w^2 (1 + nu / R) with nu = v.N / w the distance to the
+//    tangent and R = w^3 / (a b) the radius of curvature; the distance to the foot is
+//    nu + (v.T / w)^2 / (2 (R + nu)) up to terms of third order in d. v.T, N and w^2 need
+//    double precision, the correction and d only single;
+//  * for |d| <= FOOT_TOL the terms left out are below 1e-16 a; a larger d is taken as a
+//    Newton step (rare: the start is closer than that nearly everywhere).
+// 28 FP64 instructions against about 460 for two passes of ellipse.c's iteration with their
+// sincos, asin, square roots and divisions. NORMAL: the outward normal (nx, ny) as well, for
+// which the foot itself is iterated to 1e-12 (one more step). Returns false next to the evolute (K small, or
+// no convergence): the caller takes the general iteration.
+constexpr float FOOT_TOL = 4.e-6f;
+constexpr float FOOT_TOL_N = 1.e-12f;  // with the normal, which is not stationary in t
+constexpr int FOOT_MAX = 6;
+template <bool NORMAL>
+__device__ __forceinline__ bool foot_d(double a, double b, const EllF &ef, double px, double py, float &t0,
+                                       double &dist, double &nx, double &ny) {
+  const float pxf = eifd::d2f(px), pyf = eifd::d2f(py), abf = ef.a * ef.b;
+  t0 = normal_t_f_q1(ef, pxf, pyf);
+  float s0, c0;
+  sincosf(t0, &s0, &c0);
+  {
+    const float ac = ef.a * c0, bs = ef.b * s0, as = ef.a * s0, bc = ef.b * c0;
+    const float vx = pxf - ac, vy = pyf - bs;
+    const float K = as * as + bc * bc + vx * ac + vy * bs;
+    const float g = vy * bc - vx * as;
+    const float d = K > 0.f ? fminf(fmaxf(__fdividef(g, K), -0.01f), 0.01f) : 0.f;
+    const float c1 = c0 - d * s0;
+    s0 = s0 + d * c0;
+    c0 = c1;
+  }
+  double c = eifd::f2d(c0), s = eifd::f2d(s0);
+  // c, s only a few 1e-5 off the unit circle: three terms of (1 + dn)^(-1/2)
+  for (int n = 0; n < FOOT_MAX; n++) {
+    const double dn = fma(c, c, fma(s, s, -1.));
+    const double r = fma(dn, fma(dn, fma(dn, -0.3125, 0.375), -0.5), 1.);
+    c *= r;
+    s *= r;
+    const double vx = fma(-a, c, px), vy = fma(-b, s, py);
+    const double as = a * s, bc = b * c;
+    const double g = fma(vy, bc, -(vx * as));
+    const double w2 = fma(as, as, bc * bc);
+    const double nw = fma(vx, bc, vy * as);
+    const float w2f = eifd::d2f(w2), gf = eifd::d2f(g), nwf = eifd::d2f(nw);
+    const float rw = rsqrtf(w2f);
+    const float K = fmaf(nwf * abf, rw * rw, w2f);
+    if (!(K > 0.02f * w2f)) return false;
+    const float d = __fdividef(gf, K);
+    const bool done = fabsf(d) <= (NORMAL ? FOOT_TOL_N : FOOT_TOL);
+    if (done) {
+      const float corr = 0.5f * gf * d * abf * (rw * rw * rw);
+      // 1 / w from its single-precision value by one third-order step
+      const double y0 = eifd::f2d(rw);
+      const double e = fma(-(w2 * y0), y0, 1.);
+      const double p = e * fma(e, 0.375, 0.5);
+      const double u = nw * y0;
+      dist = fma(u, p, u) + eifd::f2d(corr);
+      if (NORMAL) {
+        const double y = fma(y0, p, y0);
+        nx = bc * y;
+        ny = as * y;
+      }
+      return true;
+    }
+    if (!(fabsf(d) < 0.1f)) return false;
+    const double dd = eifd::f2d(d), h = fma(dd, -0.5 * dd, 1.);
+    const double c1 = fma(-dd, s, c * h);
+    s = fma(dd, c, s * h);
+    c = c1;
+  }
+  return false;
+}
+
+// tanh(z) for z >= 0 from the values at multiples of 1/16 (tab: tanh and sech^2 there, up to
+// TANH_TOP) by the addition theorem, tanh(z_k + d) = T + S t / (1 + T t), t = tanh(d) from
+// its Taylor series (|d| <= 1/32: the first term left out is 3e-19); the quotient from a
+// single-precision reciprocal and one third-order step. 15 FP64 instructions; absolute
+// error about 1e-16.
+constexpr int TANH_STEPS = 16, TANH_TOP = 20, TANH_N = TANH_STEPS * TANH_TOP + 1;
+__device__ __forceinline__ double tanh_tab(double z, const double2 *__restrict__ tab) {
+  const float zf = eifd::d2f(z);
+  if (!(zf < (float)TANH_TOP)) return z > 0. ? 1. : z;   // a NaN stays one
+  const float kf = rintf(zf * (float)TANH_STEPS);
+  const double2 ts = __ldg(tab + (int)kf);
+  const double d = z - eifd::f2d(kf * (1.f / TANH_STEPS));
+  const double u = d * d;
+  const double p = fma(u, fma(u, fma(u, 62. / 2835., -17. / 315.), 2. / 15.), -1. / 3.);
+  const double t = fma(d * u, p, d);
+  const double den = fma(ts.x, t, 1.);
+  const double r = eifd::f2d(__fdividef(1.f, eifd::d2f(den)));
+  const double e = fma(-den, r, 1.);
+  const double q = ts.y * t * r;
+  return ts.x + fma(q, fma(e, e, e), q);
+}
+
+// tanh(BETA D) of the signed distance D in units of h (auxiliary.c:19-59), positive
+// inside, from the barred body-frame offset (x_, y_); NORMAL: the outward unit normal at the
+// foot in the body frame
+template <bool NORMAL>
+__device__ __forceinline__ double indicator_d(double a, double b, const EllF &ef, double x_, double y_,
+                                              const double2 *__restrict__ tab, double &nx, double &ny) {
+  const double px = fabs(x_), py = fabs(y_);
+  float t0;
+  double dist;
+  if (!foot_d<NORMAL>(a, b, ef, px, py, t0, dist, nx, ny)) {
+    const double t = normal_t_q1(a, b, px, py, eifd::f2d(t0));
+    double st, ct;
+    sincos(t, &st, &ct);
+    const double fx = px - a * ct, fy = py - b * st;
+    const bool in = 1. - (px / a) * (px / a) - (py / b) * (py / b) > 0.;
+    dist = sqrt(fx * fx + fy * fy);
+    if (in) dist = -dist;
+    if (NORMAL) {
+      nx = ct / a;
+      ny = st / b;
+      const double nn = 1. / sqrt(nx * nx + ny * ny);
+      nx *= nn;
+      ny *= nn;
+    }
+  }
+  if (NORMAL) {
+    if (x_ < 0.) nx = -nx;
+    if (y_ < 0.) ny = -ny;
+  }
+  const double th = tanh_tab(fabs(dist), tab);
+  return dist > 0. ? -th : th;
 }
 
 // Cells far from the interface. With rho = sqrt((x/a)^2 + (y/b)^2) (the gauge of
@@ -198,6 +310,8 @@ struct BoxArgs {
   int pcap, np, itot, jtot, use_increment;
   double dx, dy, ly, yf1;
   float *pf;                // PF_WORDS per particle, or null (double-precision form)
+  double *pd;               // PD_WORDS per particle (double-precision form), or null
+  double kb;                // BETA / h: scale of the barred lengths
   int *box, *nchunk;
   const int *bd_off_base;   // start of the buffer nchunk points into
   // inside the sub-iteration loop of a step graph: the loop's counter. In the first
@@ -212,8 +326,7 @@ struct BoxArgs {
 // chain (divisions, sincos) and the FP64 pipe takes a warp instruction at a time, so
 // the work is split into eight parts run by different warps, each over 32
 // particles: parts 0-2 the boxes of images -1, 0, +1 (their task counts are added to
-// nchunk, zeroed before), parts 3-7 groups of parameters (mixed form only). One
-// thread: particle n, part sub.
+// nchunk, zeroed before), parts 3-7 groups of parameters. One thread: particle n, part sub.
 constexpr int BOX_PARTS = 8;
 __device__ __forceinline__ void box_part(const BoxArgs &a, int n, int sub) {
   const double *P = a.P;
@@ -230,6 +343,8 @@ __device__ __forceinline__ void box_part(const BoxArgs &a, int n, int sub) {
     }
     const double r = fmax(pa, pb);
     float *q = a.pf ? a.pf + (size_t)PF_WORDS * n : nullptr;
+    double *d = a.pd ? a.pd + (size_t)PD_WORDS * n : nullptr;
+    float *df = reinterpret_cast<float *>(d + PD_F);
     if (sub < 3) {
       const int per = sub - 1;
       int imin, imax, jmin, jmax;
@@ -285,6 +400,41 @@ __device__ __forceinline__ void box_part(const BoxArgs &a, int n, int sub) {
       q[PF_SO2] = (float)(so * so);
       q[PF_SI2] = si > 0. ? (float)(si * si) : -1.f;
       q[PF_RO2] = (float)((mx + md) * (mx + md));
+    } else if (d && sub == 3) {
+      double az = P[EIF_P_AZ * pc + n];
+      if (a.use_increment) az = az + P[EIF_P_DAZ * pc + n];
+      double sz, cz;
+      sincos(-az, &sz, &cz);
+      d[PD_CZ] = cz * a.kb;
+      d[PD_SZ] = sz * a.kb;
+      // the far cells' row bounds in single precision: the far distance (10.5 cells) exceeds
+      // the saturation distance of tanh (9.53 cells) by far more than their rounding
+      const float fa = eifd::d2f(pa), fb = eifd::d2f(pb), cf = eifd::d2f(cz), sf = eifd::d2f(sz);
+      df[PDF_AL] = cf * cf / (fa * fa) + sf * sf / (fb * fb);
+      df[PDF_KA] = cf * sf * (1.f / (fb * fb) - 1.f / (fa * fa));
+      df[PDF_DE] = sf * sf / (fa * fa) + cf * cf / (fb * fb);
+    } else if (d && sub == 4) {
+      const double ba = pa * a.kb, bb = pb * a.kb;
+      d[PD_A] = ba;
+      d[PD_B] = bb;
+      const float fa = eifd::d2f(ba), fb = eifd::d2f(bb);
+      df[PDF_A] = fa;
+      df[PDF_B] = fb;
+      df[PDF_KEX] = (fa - fb) * (fa + fb) / fa;
+      df[PDF_KEY] = (fb - fa) * (fb + fa) / fb;
+    } else if (d && sub == 5) {
+      d[PD_RPM] = 1. / pmass(P[EIF_P_DEN * pc + n], pa, pb);
+    } else if (d && sub == 6) {
+      d[PD_RPIM] = 1. / pmoi(P[EIF_P_DEN * pc + n], pa, pb);
+    } else if (d && sub == 7) {
+      d[PD_X] = px;
+      d[PD_Y] = py;
+      const float fa = eifd::d2f(pa), fb = eifd::d2f(pb), md = eifd::d2f(FAR_CELLS_D * fmin(a.dx, a.dy));
+      const float mn = fminf(fa, fb), mx = fmaxf(fa, fb);
+      const float so = 1.f + md / mn, si = 1.f - md / mn;
+      df[PDF_SO2] = so * so;
+      df[PDF_SI2] = si > 0.f ? si * si : -1.f;
+      df[PDF_RO2] = (mx + md) * (mx + md);
     }
   }
   if (on && tasks && EIF_CHK(a.bd.rec, (a.nchunk - a.bd_off_base) + n, a.bd.off, 3)) atomicAdd(a.nchunk + n, tasks);
@@ -424,6 +574,8 @@ struct WorkArgs {
   int pcap, np, ld, mode, cn;   // mode 0: inertia (cn), 1: exchange
   double dx, dy, ly, h;
   const float *pf;       // per-particle single-precision parameters (mixed form)
+  const double *pd;      // per-particle parameters (double-precision form)
+  const double2 *tanh_tab;   // tanh_tab's values (double-precision form)
   const int4 *tdesc;     // task table (k_task_table)
   const float *coef;     // single-precision dt products; [9] = 1/dt
   float rh_f, dx_f, dy_f, dxdy_f;
@@ -454,6 +606,22 @@ struct WorkArgs {
   Bounds bd;
 };
 
+// Sums of three values over the warp, in 6 additions instead of 15: in each of the first
+// two steps the two halves of a group of lanes keep different values. The additions pair the
+// same lanes as warp_sum's. The sums are in lane 0 (v0), 16 (v1) and 8 (v2).
+__device__ __forceinline__ double warp_sum3(double v0, double v1, double v2, int lane) {
+  const bool h16 = lane & 16, h8 = lane & 8;
+  const double o = __shfl_xor_sync(0xffffffffu, h16 ? v0 : v1, 16);
+  double v = (h16 ? v1 : v0) + o;
+  v2 += __shfl_xor_sync(0xffffffffu, v2, 16);
+  // lanes 0-7, 16-23 go on with v, lanes 8-15, 24-31 with v2
+  const double q = __shfl_xor_sync(0xffffffffu, h8 ? v : v2, 8);
+  v = (h8 ? v2 : v) + q;
+#pragma unroll
+  for (int d = 4; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+  return v;
+}
+
 // One warp per row task: indicator weights, partial sums, and (for the exchange)
 // per-cell field contributions. The warp runs the tasks first, first + stride, ...
 // with the weight mode wmode; slots: CHUNK entries of shared memory of its own.
@@ -461,14 +629,13 @@ struct WorkArgs {
 // into fused multiply-adds) is the same in every kernel that calls it, so the batch's
 // stage kernel gives the bits of the stand-alone kernel.
 template <bool NC>
-__device__ __noinline__ void ibm_work_tasks(const WorkArgs &a, int wmode, int first, int stride, double2 *slots) {
+__device__ __noinline__ void ibm_work_tasks(const WorkArgs &a, int wmode, int first, int stride, double *slots) {
   const int lane = threadIdx.x & 31;
   const int total = EIF_CHK(a.bd.rec, a.np, a.bd.off, 10) ? ldro<NC>(a.off + a.np) : 0;
-  const double rh = 1. / a.h;
   const double dxdy = a.dx * a.dy;
-  const double dtv = a.mode == 1 ? __ldg(a.dt) : 0.;
-  const double rdtv = a.mode == 1 ? 1. / dtv : 0.;
-  const double md = FAR_CELLS_D * a.h;
+  // factors of the sums: inertia.c:51-59 with 1/2 (1 + th) and the two face averages,
+  // exchange.c:61-76
+  const double scale = a.mode == 0 ? 0.25 * dxdy : dxdy / __ldg(a.dt);
   const int pc = a.pcap, ld = a.ld;
   double *wcache = static_cast<double *>(a.wcache);
   for (int c = first; c < total; c += stride) {
@@ -479,161 +646,130 @@ __device__ __noinline__ void ibm_work_tasks(const WorkArgs &a, int wmode, int fi
     if (!EIF_CHK(a.bd.rec, EIF_P_VZ * pc + n, a.bd.P, 13)) continue;
     RowTask t;
     const bool task = task_of(dsc, a.np, t) && EIF_CHK(a.bd.rec, t.j, a.bd.yc - 1, 15);
-    const double *P = a.P;
-    const double pden = ldro<NC>(P + EIF_P_DEN * pc + n), pa = ldro<NC>(P + EIF_P_A * pc + n),
-                 pb = ldro<NC>(P + EIF_P_B * pc + n);
-    double px = ldro<NC>(P + EIF_P_X * pc + n), py = ldro<NC>(P + EIF_P_Y * pc + n), paz = ldro<NC>(P + EIF_P_AZ * pc + n);
-    if (a.mode == 0) {
-      // inertia.c:29-31: positions at k + increment
-      px = px + ldro<NC>(P + EIF_P_DX * pc + n);
-      py = py + ldro<NC>(P + EIF_P_DY * pc + n);
-      paz = paz + ldro<NC>(P + EIF_P_DAZ * pc + n);
-    }
-    // reciprocals of the mass and the moment of inertia, once per task: the per-cell
-    // divisions of inertia.c and exchange.c become multiplications (a division costs
-    // about ten FP64 operations; the results change by an ulp per term)
-    const double rpm = 1. / pmass(pden, pa, pb);
-    const double rpim = 1. / pmoi(pden, pa, pb);
-    const double pux = ldro<NC>(P + EIF_P_UX * pc + n), puy = ldro<NC>(P + EIF_P_UY * pc + n),
-                 pvz = ldro<NC>(P + EIF_P_VZ * pc + n);
-    const Ell e = make_ell(pa, pb, px, py, paz);
-    const double py_ = py + a.ly * (task ? t.img : 0);
+    const double *pd = a.pd + (size_t)PD_WORDS * n;
+    const float *pdf = reinterpret_cast<const float *>(pd + PD_F);
+    const double px = ldro<NC>(pd + PD_X), py_ = ldro<NC>(pd + PD_Y) + a.ly * (task ? t.img : 0);
     const int j = task ? t.j : 1;
-    const double y = __ldg(a.yc + j);
-    const double Y = y - py_;
-    int rank[2];
-    bool cin[2];
+    const double Y = __ldg(a.yc + j) - py_;
+    const int ib = task ? t.ib : 1;
     double th2[2];
-    unsigned near_mask[2];
-    if (wmode == 2) {
-      // weights of the same geometry from an earlier evaluation
-#pragma unroll
-      for (int half = 0; half < CHUNK / 32; half++) {
-        const int i = (task ? t.ib : 1) + half * 32 + lane;
-        bool in = task && i <= t.ie;
-        if (in) {
-          in = EIF_CHK(a.bd.rec, i, a.bd.xc - 1, 14) && EIF_CHK(a.bd.rec, j * ld + i, a.bd.field, 16) &&
-               EIF_CHK(a.bd.rec, (j + 1) * ld + i, a.bd.field, 17) &&
-               EIF_CHK(a.bd.rec, j * ld + (i - 1), a.bd.field, 18) &&
-               EIF_CHK(a.bd.rec, (long long)c * CHUNK + half * 32 + lane, a.bd.wbuf, 22);
-        }
-        cin[half] = in;
-        th2[half] = in ? wcache[(size_t)c * CHUNK + half * 32 + lane] : 0.;
-      }
-    } else {
-    // far cells of this row (row_chords), in single precision: the far distance
-    // (10.5 cells) exceeds the saturation distance of tanh (9.53 cells) by far more
-    // than the rounding of the column bounds
-    float olo, ohi, ilo, ihi;
-    {
-      const float fa = eifd::d2f(pa), fb = eifd::d2f(pb), cz = eifd::d2f(e.cz), sz = eifd::d2f(e.sz);
-      const float mn = fminf(fa, fb), mx = fmaxf(fa, fb), fmd = eifd::d2f(md);
-      const float so = 1.f + fmd / mn, si = 1.f - fmd / mn;
-      const float al = cz * cz / (fa * fa) + sz * sz / (fb * fb);
-      const float ka = cz * sz * (1.f / (fb * fb) - 1.f / (fa * fa));
-      const float de = sz * sz / (fa * fa) + cz * cz / (fb * fb);
-      row_chords(al, ka, de, so * so, si > 0.f ? si * si : -1.f, (mx + fmd) * (mx + fmd), eifd::d2f(Y), olo, ohi,
-                 ilo, ihi);
-    }
-    // pass 1: cells of the row, far cells settled, body-frame offsets of the near ones
+    bool cin[2];
 #pragma unroll
     for (int half = 0; half < CHUNK / 32; half++) {
-      const int i = (task ? t.ib : 1) + half * 32 + lane;
+      const int i = ib + half * 32 + lane;
       bool in = task && i <= t.ie;
       if (in) {
         in = EIF_CHK(a.bd.rec, i, a.bd.xc - 1, 14) && EIF_CHK(a.bd.rec, j * ld + i, a.bd.field, 16) &&
              EIF_CHK(a.bd.rec, (j + 1) * ld + i, a.bd.field, 17) && EIF_CHK(a.bd.rec, j * ld + (i - 1), a.bd.field, 18);
       }
       cin[half] = in;
-      bool near = false;
-      double x_ = 0., y_ = 0.;
-      th2[half] = 0.;
-      if (in) {
-        const double X = __ldg(a.xc + i) - e.px;
-        const float Xf = eifd::d2f(X);
-        // reference sign convention: +1 inside (auxiliary.c:36-38); tanh saturated
-        const int side = !(Xf > olo && Xf < ohi) ? -1 : ((Xf >= ilo && Xf <= ihi) ? 1 : 0);
-        th2[half] = (double)side;
-        near = side == 0;
-        x_ = e.cz * X - e.sz * Y;
-        y_ = e.sz * X + e.cz * Y;
-      }
-      near_mask[half] = __ballot_sync(0xffffffffu, near);
-      rank[half] = (half ? __popc(near_mask[0]) : 0) + __popc(near_mask[half] & ((1u << lane) - 1u));
-      if (near) slots[rank[half]] = make_double2(x_, y_);
     }
-    // pass 2: the near cells, packed onto consecutive lanes
-    const int nnear = __popc(near_mask[0]) + __popc(near_mask[1]);
-    if (a.count) {
-      const unsigned in0 = __ballot_sync(0xffffffffu, cin[0]), in1 = __ballot_sync(0xffffffffu, cin[1]);
-      if (lane == 0) {
-        atomicAdd(a.count, (unsigned long long)(__popc(in0) + __popc(in1)));
-        atomicAdd(a.count + 1, (unsigned long long)nnear);
-      }
-    }
-    __syncwarp();
-    for (int k = lane; k < nnear; k += 32) {
-      const double2 o = slots[k];
-      slots[k].x = tanh(BETA * signed_dist_body(e, o.x, o.y, rh));
-    }
-    __syncwarp();
+    if (wmode == 2) {
+      // weights of the same geometry from an earlier evaluation
 #pragma unroll
-    for (int half = 0; half < CHUNK / 32; half++)
-      if ((near_mask[half] >> lane) & 1u) th2[half] = slots[rank[half]].x;
-    __syncwarp();
-    if (wmode == 1) {
+      for (int half = 0; half < CHUNK / 32; half++) {
+        if (cin[half]) cin[half] = EIF_CHK(a.bd.rec, (long long)c * CHUNK + half * 32 + lane, a.bd.wbuf, 22);
+        th2[half] = cin[half] ? wcache[(size_t)c * CHUNK + half * 32 + lane] : 0.;
+      }
+    } else {
+      // pass 1: cells of the row, far cells settled, the near ones listed
+      int rank[2];
+      unsigned near_mask[2];
+      float olo, ohi, ilo, ihi;
+      row_chords(ldro<NC>(pdf + PDF_AL), ldro<NC>(pdf + PDF_KA), ldro<NC>(pdf + PDF_DE), ldro<NC>(pdf + PDF_SO2),
+                 ldro<NC>(pdf + PDF_SI2), ldro<NC>(pdf + PDF_RO2), eifd::d2f(Y), olo, ohi, ilo, ihi);
+#pragma unroll
+      for (int half = 0; half < CHUNK / 32; half++) {
+        const int i = ib + half * 32 + lane;
+        bool near = false;
+        th2[half] = 0.;
+        if (cin[half]) {
+          const float Xf = eifd::d2f(__ldg(a.xc + i) - px);
+          // reference sign convention: +1 inside (auxiliary.c:36-38); tanh saturated
+          const int side = !(Xf > olo && Xf < ohi) ? -1 : ((Xf >= ilo && Xf <= ihi) ? 1 : 0);
+          th2[half] = side > 0 ? 1. : (side < 0 ? -1. : 0.);
+          near = side == 0;
+        }
+        near_mask[half] = __ballot_sync(0xffffffffu, near);
+        rank[half] = (half ? __popc(near_mask[0]) : 0) + __popc(near_mask[half] & ((1u << lane) - 1u));
+        if (near) slots[rank[half]] = __hiloint2double(0, half * 32 + lane);
+      }
+      // pass 2: the near cells, packed onto consecutive lanes
+      const int nnear = __popc(near_mask[0]) + __popc(near_mask[1]);
+      if (a.count) {
+        const unsigned in0 = __ballot_sync(0xffffffffu, cin[0]), in1 = __ballot_sync(0xffffffffu, cin[1]);
+        if (lane == 0) {
+          atomicAdd(a.count, (unsigned long long)(__popc(in0) + __popc(in1)));
+          atomicAdd(a.count + 1, (unsigned long long)nnear);
+        }
+      }
+      __syncwarp();
+      if (nnear) {
+        const double cz = ldro<NC>(pd + PD_CZ), sz = ldro<NC>(pd + PD_SZ), pa = ldro<NC>(pd + PD_A),
+                     pb = ldro<NC>(pd + PD_B);
+        EllF ef;
+        ef.a = ldro<NC>(pdf + PDF_A); ef.b = ldro<NC>(pdf + PDF_B);
+        ef.kex = ldro<NC>(pdf + PDF_KEX); ef.key = ldro<NC>(pdf + PDF_KEY);
+        ef.cz = 0.f; ef.sz = 0.f;
+        const double szY = sz * Y, czY = cz * Y;
+        for (int k = lane; k < nnear; k += 32) {
+          const int i = ib + __double2loint(slots[k]);
+          const double X = __ldg(a.xc + i) - px;
+          double nx, ny;
+          slots[k] = indicator_d<false>(pa, pb, ef, fma(cz, X, -szY), fma(sz, X, czY), a.tanh_tab, nx, ny);
+        }
+      }
+      __syncwarp();
 #pragma unroll
       for (int half = 0; half < CHUNK / 32; half++)
-        if (EIF_CHK(a.bd.rec, (long long)c * CHUNK + half * 32 + lane, a.bd.wbuf, 23))
-          wcache[(size_t)c * CHUNK + half * 32 + lane] = th2[half];
+        if ((near_mask[half] >> lane) & 1u) th2[half] = slots[rank[half]];
+      __syncwarp();
+      if (wmode == 1) {
+#pragma unroll
+        for (int half = 0; half < CHUNK / 32; half++)
+          if (EIF_CHK(a.bd.rec, (long long)c * CHUNK + half * 32 + lane, a.bd.wbuf, 23))
+            wcache[(size_t)c * CHUNK + half * 32 + lane] = th2[half];
+      }
     }
-    }
+    const double pux = ldro<NC>(a.P + EIF_P_UX * pc + n), puy = ldro<NC>(a.P + EIF_P_UY * pc + n),
+                 pvz = ldro<NC>(a.P + EIF_P_VZ * pc + n);
     double s0 = 0., s1 = 0., s2 = 0.;
 #pragma unroll
     for (int half = 0; half < CHUNK / 32; half++) {
-      const int i = (task ? t.ib : 1) + half * 32 + lane;
+      const int i = ib + half * 32 + lane;
       double2 contrib = make_double2(0., 0.);
       // cells of weight exactly zero (inertia: far outside; exchange: any far cell) are skipped
-      const double th_ = th2[half];
-      const bool live = a.mode == 0 ? th_ != -1. : fabs(th_) != 1.;
+      const double th = th2[half];
+      const bool live = a.mode == 0 ? th != -1. : fabs(th) != 1.;
       if (cin[half] && live) {
-        const double x = __ldg(a.xc + i);
-        const double th = th_;
-        const double uxf = 0.5 * (__ldg(a.ux + j * ld + (i - 1)) + __ldg(a.ux + j * ld + i));
-        const double uyf = 0.5 * (__ldg(a.uy + j * ld + i) + __ldg(a.uy + (j + 1) * ld + i));
+        const double X = __ldg(a.xc + i) - px;
+        const double us = __ldg(a.ux + j * ld + (i - 1)) + __ldg(a.ux + j * ld + i);
+        const double vs = __ldg(a.uy + j * ld + i) + __ldg(a.uy + (j + 1) * ld + i);
         if (a.mode == 0) {
-          // inertia.c:51-59
-          const double w = 0.5 * (1. + th);
-          const double valx = w * 0.5 * (2. * uxf) * dxdy;
-          const double valy = w * 0.5 * (2. * uyf) * dxdy;
-          s0 += valx * rpm;
-          s1 += valy * rpm;
-          s2 += (-(y - py_) * valx * rpim) + ((x - px) * valy * rpim);
+          // inertia.c:51-59, the constant factors after the sum
+          const double w = 1. + th;
+          const double wu = w * us, wv = w * vs;
+          s0 += wu;
+          s1 += wv;
+          s2 = fma(X, wv, fma(-Y, wu, s2));
         } else {
-          // exchange.c:61-76
-          const double w = 0.5 * BETA * (1. - th * th);
-          const double uxp = pux - pvz * (y - py_);
-          const double uyp = puy + pvz * (x - px);
-          const double fx = w * (uxp - uxf) * rdtv;
-          const double fy = w * (uyp - uyf) * rdtv;
-          contrib = a.weights_only ? make_double2(w, w) : make_double2(fx * dtv, fy * dtv);
-          const double Fx = fx * a.dx * a.dy, Fy = fy * a.dx * a.dy;
-          s0 += -(Fx * rpm);
-          s1 += -(Fy * rpm);
-          s2 += ((y - py_) * Fx * rpim) - ((x - px) * Fy * rpim);
+          // exchange.c:61-76 (BETA / 2 = 1)
+          const double w = fma(-th, th, 1.);
+          const double gx = w * fma(-0.5, us, fma(-pvz, Y, pux));
+          const double gy = w * fma(-0.5, vs, fma(pvz, X, puy));
+          contrib = a.weights_only ? make_double2(w, w) : make_double2(gx, gy);
+          s0 -= gx;
+          s1 -= gy;
+          s2 = fma(Y, gx, fma(-X, gy, s2));
         }
       }
       if (a.mode == 1 && EIF_CHK(a.bd.rec, (long long)c * CHUNK + half * 32 + lane, a.bd.wbuf, 19))
         a.wbuf[(size_t)c * CHUNK + half * 32 + lane] = contrib;
     }
-    s0 = eifd::warp_sum(s0);
-    s1 = eifd::warp_sum(s1);
-    s2 = eifd::warp_sum(s2);
-    if (lane == 0 && EIF_CHK(a.bd.rec, 3LL * c + 2, a.bd.partial, 20)) {
-      a.partial[3 * (size_t)c + 0] = s0;
-      a.partial[3 * (size_t)c + 1] = s1;
-      a.partial[3 * (size_t)c + 2] = s2;
-    }
+    const double v = warp_sum3(s0, s1, s2, lane);
+    const int slot = lane == 0 ? 0 : (lane == 16 ? 1 : (lane == 8 ? 2 : -1));
+    if (slot >= 0 && EIF_CHK(a.bd.rec, 3LL * c + 2, a.bd.partial, 20))
+      a.partial[3 * (size_t)c + slot] = v * (scale * ldro<NC>(pd + (slot == 2 ? PD_RPIM : PD_RPM)));
   }
 }
 
@@ -1184,6 +1320,8 @@ inline BoxArgs box_args(const eif_ctx *c, bool use_increment) {
   b.dx = c->dx; b.dy = c->dy; b.ly = c->ly; b.yf1 = c->h_yf[0];
   b.box = c->box;
   b.pf = c->cfg.precision == EIF_PREC_MIXED ? c->pf : nullptr;
+  b.pd = c->cfg.precision == EIF_PREC_MIXED ? nullptr : c->pd;
+  b.kb = BETA / (c->dx < c->dy ? c->dx : c->dy);
   b.iter = nullptr;
   b.nchunk = c->chunk_off + (c->np + 1);
   return b;
@@ -1200,6 +1338,8 @@ inline WorkArgs work_args(const eif_ctx *c, int mode, int cn) {
   w.dx = c->dx; w.dy = c->dy; w.ly = c->ly; w.h = c->dx < c->dy ? c->dx : c->dy;
   w.bd = bounds_of(c);
   w.pf = c->pf;
+  w.pd = c->pd;
+  w.tanh_tab = c->tanh_tab;
   w.tdesc = c->tdesc;
   w.coef = c->d_coef;
   w.rh_f = (float)(1. / w.h);

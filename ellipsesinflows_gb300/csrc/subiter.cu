@@ -128,7 +128,7 @@ enum { ST_NP, ST_UBOX, ST_UCOLL, ST_UTAB, ST_UPART, ST_MIXED, ST_TASKS, ST_WORDS
 __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
   __shared__ unsigned act[SUB_MAX / 32];   // suspensions still iterating
   __shared__ float2 slot_f[SUB_WARPS][CHUNK];
-  __shared__ double2 slot_d[SUB_WARPS][CHUNK];
+  __shared__ double slot_d[SUB_WARPS][CHUNK];
   extern __shared__ int stab[];            // ST_WORDS per suspension
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int G = gridDim.x, W = G * SUB_WARPS, T = G * SUB_THREADS;
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
         if (!active(j)) continue;
         const int *e = stab + ST_WORDS * j;
         const int groups = (e[ST_NP] + 31) / 32;
-        const int units = groups * (e[ST_MIXED] ? BOX_PARTS : 3);
+        const int units = groups * BOX_PARTS;
         int u = first_unit(wid, e[ST_UBOX], W);
         if (u >= units) continue;
         const SubDesc &d = s.d[j];
@@ -431,7 +431,7 @@ int subiter_upload(SubiterPlan *p, std::string *err) {
       d.u_coll = u_coll;
       d.u_tab = u_tab;
       d.u_part = u_part;
-      u_box += ((d.np + 31) / 32) * (d.mixed ? BOX_PARTS : 3);
+      u_box += ((d.np + 31) / 32) * BOX_PARTS;
       u_coll += (d.np + PAIR_WARPS - 1) / PAIR_WARPS;
       u_tab += (d.np + TT_WARPS - 1) / TT_WARPS;
       u_part += d.np;
