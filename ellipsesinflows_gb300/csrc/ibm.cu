@@ -53,9 +53,9 @@ __global__ void __launch_bounds__(TT_WARPS * 32) k_task_table_scan(const int *__
 // The double-precision body is the batch stage kernel's instantiation (ordinary loads):
 // one function, compiled alike in both translation units, gives both kernels the same
 // bits.
-__global__ void __launch_bounds__(256) k_ibm_work(WorkArgs a) {
-  // per warp: the columns of its near cells, overwritten by their weights
-  __shared__ double slot_buf[8][CHUNK];
+__global__ void __launch_bounds__(256, 3) k_ibm_work(WorkArgs a) {
+  // per warp: its near cells, their feet and their weights
+  __shared__ double2 slot_buf[8][WORK_SLOTS];
   const int wmode = a.iter ? (*a.iter == 0u ? 2 : 0) : a.wmode;
   ibm_work_tasks<false>(a, wmode, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
                         slot_buf[threadIdx.x >> 5]);
@@ -682,7 +682,7 @@ __global__ void __launch_bounds__(256) k_ibm_adj(AdjWorkArgs a) {
     const double cz = __ldg(pd + PD_CZ), sz = __ldg(pd + PD_SZ), pa = __ldg(pd + PD_A), pb = __ldg(pd + PD_B);
     EllF ef;
     ef.a = __ldg(pdf + PDF_A); ef.b = __ldg(pdf + PDF_B); ef.kex = __ldg(pdf + PDF_KEX); ef.key = __ldg(pdf + PDF_KEY);
-    ef.cz = 0.f; ef.sz = 0.f;
+    ef.cz = eifd::d2f(cz); ef.sz = eifd::d2f(sz);
     const int j = task ? t.j : 1;
     const double y = __ldg(a.yc + j);
     const double ry = y - py_;
@@ -720,7 +720,10 @@ __global__ void __launch_bounds__(256) k_ibm_adj(AdjWorkArgs a) {
             // g = R(az) dD/dq, dD/dq = -n / h with the outward normal n at the foot; cz and
             // sz carry the factor BETA / h
             double nx, ny;
-            th = indicator_d<true>(pa, pb, ef, fma(cz, rx, -(sz * ry)), fma(sz, rx, cz * ry), a.tanh_tab, nx, ny);
+            float c0, s0, d0;
+            const double qx = fma(cz, rx, -(sz * ry)), qy = fma(sz, rx, cz * ry);
+            foot_f(ef, eifd::d2f(fabs(qx)), eifd::d2f(fabs(qy)), c0, s0, d0);
+            th = indicator_d<true>(pa, pb, ef.a * ef.b, c0, s0, qx, qy, a.tanh_tab, nx, ny);
             gwx = (-1. / BETA) * fma(cz, nx, sz * ny);
             gwy = (-1. / BETA) * fma(cz, ny, -(sz * nx));
           }

@@ -132,11 +132,29 @@ __device__ __noinline__ double normal_t_q1(double a, double b, double px, double
   return t;
 }
 
-// The normal foot of (px, py), first quadrant, on the ellipse (a, b), and the distance to
-// it, positive outside. Bound by the FP64 pipe (one warp instruction in 16 cycles), so the
-// double-precision work is kept to what carries the precision:
-//  * the foot (c, s) = (cos t, sin t) comes from the single-precision iteration and one
-//    Newton step there, to about 2e-7, and is put on the unit circle in double precision;
+// The normal foot of (px, py), first quadrant, in single precision: (c, s) = (cos t, sin t)
+// to about 2e-7 (the iteration above, whose hardware sines shift its fixed point a little,
+// and one Newton step, d); returns the distance to the foot, positive outside.
+__device__ __forceinline__ float foot_f(const EllF &e, float px, float py, float &c, float &s, float &d) {
+  const float t = normal_t_f_q1(e, px, py);
+  sincosf(t, &s, &c);
+  float ac = e.a * c, bs = e.b * s, as = e.a * s, bc = e.b * c;
+  float vx = px - ac, vy = py - bs;
+  const float K = as * as + bc * bc + vx * ac + vy * bs;
+  const float g = vy * bc - vx * as;
+  d = K > 0.f ? fminf(fmaxf(__fdividef(g, K), -0.01f), 0.01f) : 0.01f;
+  const float c1 = c - d * s;
+  s = s + d * c;
+  c = c1;
+  bc = e.b * c; as = e.a * s;
+  vx = px - e.a * c; vy = py - e.b * s;
+  return (vx * bc + vy * as) * rsqrtf(bc * bc + as * as);
+}
+
+// The same foot and distance in double precision, from foot_f's (c0, s0). Bound by the FP64
+// pipe (one warp instruction in 16 cycles), so the double-precision work is kept to what
+// carries the precision:
+//  * (c, s) is put on the unit circle in double precision;
 //  * with v = (px, py) - (a c, b s), T the derivative of the ellipse in t (w = |T|) and N
 //    its outward normal, the remaining angle to the foot is d = v.T / K,
 //    K = w^2 + v.(a c, b s) = w^2 (1 + nu / R) with nu = v.N / w the distance to the
@@ -147,28 +165,14 @@ __device__ __noinline__ double normal_t_q1(double a, double b, double px, double
 //    Newton step (rare: the start is closer than that nearly everywhere).
 // 28 FP64 instructions against about 460 for two passes of ellipse.c's iteration with their
 // sincos, asin, square roots and divisions. NORMAL: the outward normal (nx, ny) as well, for
-// which the foot itself is iterated to 1e-12 (one more step). Returns false next to the evolute (K small, or
-// no convergence): the caller takes the general iteration.
+// which the foot itself is iterated to 1e-12 (one more step). Returns false next to the
+// evolute (K small, or no convergence): the caller takes the general iteration.
 constexpr float FOOT_TOL = 4.e-6f;
 constexpr float FOOT_TOL_N = 1.e-12f;  // with the normal, which is not stationary in t
 constexpr int FOOT_MAX = 6;
 template <bool NORMAL>
-__device__ __forceinline__ bool foot_d(double a, double b, const EllF &ef, double px, double py, float &t0,
+__device__ __forceinline__ bool foot_d(double a, double b, float abf, float c0, float s0, double px, double py,
                                        double &dist, double &nx, double &ny) {
-  const float pxf = eifd::d2f(px), pyf = eifd::d2f(py), abf = ef.a * ef.b;
-  t0 = normal_t_f_q1(ef, pxf, pyf);
-  float s0, c0;
-  sincosf(t0, &s0, &c0);
-  {
-    const float ac = ef.a * c0, bs = ef.b * s0, as = ef.a * s0, bc = ef.b * c0;
-    const float vx = pxf - ac, vy = pyf - bs;
-    const float K = as * as + bc * bc + vx * ac + vy * bs;
-    const float g = vy * bc - vx * as;
-    const float d = K > 0.f ? fminf(fmaxf(__fdividef(g, K), -0.01f), 0.01f) : 0.f;
-    const float c1 = c0 - d * s0;
-    s0 = s0 + d * c0;
-    c0 = c1;
-  }
   double c = eifd::f2d(c0), s = eifd::f2d(s0);
   // c, s only a few 1e-5 off the unit circle: three terms of (1 + dn)^(-1/2)
   for (int n = 0; n < FOOT_MAX; n++) {
@@ -234,16 +238,15 @@ __device__ __forceinline__ double tanh_tab(double z, const double2 *__restrict__
 }
 
 // tanh(BETA D) of the signed distance D in units of h (auxiliary.c:19-59), positive
-// inside, from the barred body-frame offset (x_, y_); NORMAL: the outward unit normal at the
-// foot in the body frame
+// inside, from the barred body-frame offset (x_, y_) and foot_f's (c0, s0); NORMAL: the
+// outward unit normal at the foot in the body frame
 template <bool NORMAL>
-__device__ __forceinline__ double indicator_d(double a, double b, const EllF &ef, double x_, double y_,
+__device__ __forceinline__ double indicator_d(double a, double b, float abf, float c0, float s0, double x_, double y_,
                                               const double2 *__restrict__ tab, double &nx, double &ny) {
   const double px = fabs(x_), py = fabs(y_);
-  float t0;
   double dist;
-  if (!foot_d<NORMAL>(a, b, ef, px, py, t0, dist, nx, ny)) {
-    const double t = normal_t_q1(a, b, px, py, eifd::f2d(t0));
+  if (!foot_d<NORMAL>(a, b, abf, c0, s0, px, py, dist, nx, ny)) {
+    const double t = normal_t_q1(a, b, px, py, eifd::f2d(fminf(fmaxf(atan2f(s0, c0), 0.f), 1.5707963f)));
     double st, ct;
     sincos(t, &st, &ct);
     const double fx = px - a * ct, fy = py - b * st;
@@ -263,7 +266,20 @@ __device__ __forceinline__ double indicator_d(double a, double b, const EllF &ef
     if (y_ < 0.) ny = -ny;
   }
   const double th = tanh_tab(fabs(dist), tab);
-  return dist > 0. ? -th : th;
+  return __double2hiint(dist) < 0 ? th : -th;
+}
+
+// Cells of which single precision gives tanh(BETA D) to the last bit of the double: with z
+// = |BETA D|, tanh z = 1 - x, x = 2 / (exp(2 z) + 1), and an error dz of the distance changes
+// it by 4 exp(-2 z) dz. foot_f's distance is good to about 1e-6 of the major semi-axis A (in
+// the same barred units) once its Newton step is below 1e-3; at z >= 14 + A / 200 the change is below 3e-17, for every A. Such
+// cells (7 cells from the interface and farther) leave the FP64 pipe nothing but the
+// subtraction.
+__device__ __forceinline__ float z_single(float A) { return fmaf(0.005f, A, 14.f); }
+__device__ __forceinline__ double tanh_far(float dist) {
+  const float x = 2.f * __expf(-2.f * fabsf(dist));   // exp(-2 z) < 1e-12: the 1 + exp is 1
+  const double th = 1. - eifd::f2d(x);
+  return dist < 0.f ? th : -th;
 }
 
 // Cells far from the interface. With rho = sqrt((x/a)^2 + (y/b)^2) (the gauge of
@@ -624,20 +640,23 @@ __device__ __forceinline__ double warp_sum3(double v0, double v1, double v2, int
 
 // One warp per row task: indicator weights, partial sums, and (for the exchange)
 // per-cell field contributions. The warp runs the tasks first, first + stride, ...
-// with the weight mode wmode; slots: CHUNK entries of shared memory of its own.
-// Not inlined: compiled on its own, the double-precision arithmetic (its contractions
-// into fused multiply-adds) is the same in every kernel that calls it, so the batch's
-// stage kernel gives the bits of the stand-alone kernel.
+// with the weight mode wmode; slots: WORK_SLOTS entries of shared memory of its own.
+// Bound by the FP64 pipe in both uses: about 30 FP64 instructions per task for the sums and
+// 45 for each pass of 32 cells next to the interface. Not inlined, and every product that
+// could be fused is written as fma: the batch's stage kernel gives the bits of the
+// stand-alone kernel.
+constexpr int WORK_SLOTS = CHUNK + CHUNK / (int)sizeof(double2);   // double2 entries per warp
 template <bool NC>
-__device__ __noinline__ void ibm_work_tasks(const WorkArgs &a, int wmode, int first, int stride, double *slots) {
+__device__ __noinline__ void ibm_work_tasks(const WorkArgs &a, int wmode, int first, int stride, double2 *slots) {
   const int lane = threadIdx.x & 31;
   const int total = EIF_CHK(a.bd.rec, a.np, a.bd.off, 10) ? ldro<NC>(a.off + a.np) : 0;
   const double dxdy = a.dx * a.dy;
   // factors of the sums: inertia.c:51-59 with 1/2 (1 + th) and the two face averages,
   // exchange.c:61-76
-  const double scale = a.mode == 0 ? 0.25 * dxdy : dxdy / __ldg(a.dt);
+  const double scale = a.mode == 0 ? 0.25 * dxdy : -dxdy / __ldg(a.dt);
   const int pc = a.pcap, ld = a.ld;
   double *wcache = static_cast<double *>(a.wcache);
+  unsigned char *list = reinterpret_cast<unsigned char *>(slots + CHUNK);   // the cells of pass 3
   for (int c = first; c < total; c += stride) {
     if (!EIF_CHK(a.bd.rec, c, a.bd.partial / 3, 21)) continue;
     const int4 dsc = ldro<NC>(a.tdesc + c);
@@ -648,7 +667,8 @@ __device__ __noinline__ void ibm_work_tasks(const WorkArgs &a, int wmode, int fi
     const bool task = task_of(dsc, a.np, t) && EIF_CHK(a.bd.rec, t.j, a.bd.yc - 1, 15);
     const double *pd = a.pd + (size_t)PD_WORDS * n;
     const float *pdf = reinterpret_cast<const float *>(pd + PD_F);
-    const double px = ldro<NC>(pd + PD_X), py_ = ldro<NC>(pd + PD_Y) + a.ly * (task ? t.img : 0);
+    const int img = task ? t.img : 0;
+    const double px = ldro<NC>(pd + PD_X), py_ = ldro<NC>(pd + PD_Y) + (img == 0 ? 0. : (img > 0 ? a.ly : -a.ly));
     const int j = task ? t.j : 1;
     const double Y = __ldg(a.yc + j) - py_;
     const int ib = task ? t.ib : 1;
@@ -692,9 +712,10 @@ __device__ __noinline__ void ibm_work_tasks(const WorkArgs &a, int wmode, int fi
         }
         near_mask[half] = __ballot_sync(0xffffffffu, near);
         rank[half] = (half ? __popc(near_mask[0]) : 0) + __popc(near_mask[half] & ((1u << lane) - 1u));
-        if (near) slots[rank[half]] = __hiloint2double(0, half * 32 + lane);
+        if (near) slots[rank[half]].x = __hiloint2double(0, half * 32 + lane);
       }
-      // pass 2: the near cells, packed onto consecutive lanes
+      // pass 2: the near cells packed onto consecutive lanes, single precision; the cells it
+      // settles get their weights, the others are packed once more
       const int nnear = __popc(near_mask[0]) + __popc(near_mask[1]);
       if (a.count) {
         const unsigned in0 = __ballot_sync(0xffffffffu, cin[0]), in1 = __ballot_sync(0xffffffffu, cin[1]);
@@ -710,19 +731,48 @@ __device__ __noinline__ void ibm_work_tasks(const WorkArgs &a, int wmode, int fi
         EllF ef;
         ef.a = ldro<NC>(pdf + PDF_A); ef.b = ldro<NC>(pdf + PDF_B);
         ef.kex = ldro<NC>(pdf + PDF_KEX); ef.key = ldro<NC>(pdf + PDF_KEY);
-        ef.cz = 0.f; ef.sz = 0.f;
+        ef.cz = eifd::d2f(cz); ef.sz = eifd::d2f(sz);
+        const float zs = z_single(fmaxf(ef.a, ef.b)), Yf = eifd::d2f(Y);
+        int ndbl = 0;
+        for (int base = 0; base < nnear; base += 32) {
+          const int k = base + lane;
+          bool dbl = false;
+          int at = 0;
+          float c0 = 0.f, s0 = 0.f;
+          if (k < nnear) {
+            at = __double2loint(slots[k].x);
+            const float Xf = eifd::d2f(__ldg(a.xc + ib + at) - px);
+            float d;
+            const float dist = foot_f(ef, fabsf(ef.cz * Xf - ef.sz * Yf), fabsf(ef.sz * Xf + ef.cz * Yf), c0, s0, d);
+            dbl = !(fabsf(dist) >= zs && fabsf(d) < 1.e-3f);
+            if (!dbl) slots[at].y = tanh_far(dist);
+          }
+          const unsigned mask = __ballot_sync(0xffffffffu, dbl);
+          if (dbl) {
+            // list positions at or before the ones already read; .y is indexed by cell
+            const int q = ndbl + __popc(mask & ((1u << lane) - 1u));
+            slots[q].x = __hiloint2double(__float_as_int(c0), __float_as_int(s0));
+            list[q] = (unsigned char)at;
+          }
+          ndbl += __popc(mask);
+          __syncwarp();
+        }
+        // pass 3: double precision
         const double szY = sz * Y, czY = cz * Y;
-        for (int k = lane; k < nnear; k += 32) {
-          const int i = ib + __double2loint(slots[k]);
-          const double X = __ldg(a.xc + i) - px;
+        for (int k = lane; k < ndbl; k += 32) {
+          const int at = list[k];
+          const double cs = slots[k].x;
+          const double X = __ldg(a.xc + ib + at) - px;
           double nx, ny;
-          slots[k] = indicator_d<false>(pa, pb, ef, fma(cz, X, -szY), fma(sz, X, czY), a.tanh_tab, nx, ny);
+          slots[at].y = indicator_d<false>(pa, pb, ef.a * ef.b, __int_as_float(__double2hiint(cs)),
+                                           __int_as_float(__double2loint(cs)), fma(cz, X, -szY), fma(sz, X, czY),
+                                           a.tanh_tab, nx, ny);
         }
       }
       __syncwarp();
 #pragma unroll
       for (int half = 0; half < CHUNK / 32; half++)
-        if ((near_mask[half] >> lane) & 1u) th2[half] = slots[rank[half]];
+        if ((near_mask[half] >> lane) & 1u) th2[half] = slots[half * 32 + lane].y;
       __syncwarp();
       if (wmode == 1) {
 #pragma unroll
@@ -738,38 +788,43 @@ __device__ __noinline__ void ibm_work_tasks(const WorkArgs &a, int wmode, int fi
     for (int half = 0; half < CHUNK / 32; half++) {
       const int i = ib + half * 32 + lane;
       double2 contrib = make_double2(0., 0.);
-      // cells of weight exactly zero (inertia: far outside; exchange: any far cell) are skipped
+      // cells of weight exactly zero (inertia: far outside; exchange: any far cell) are
+      // skipped; compared as integers, the FP64 pipe does comparisons too
       const double th = th2[half];
-      const bool live = a.mode == 0 ? th != -1. : fabs(th) != 1.;
-      if (cin[half] && live) {
+      const int hi = __double2hiint(th), lo = __double2loint(th);
+      const bool one = (a.mode == 0 ? hi : hi | (int)0x80000000) == (int)0xbff00000 && lo == 0;
+      if (cin[half] && !one) {
         const double X = __ldg(a.xc + i) - px;
         const double us = __ldg(a.ux + j * ld + (i - 1)) + __ldg(a.ux + j * ld + i);
         const double vs = __ldg(a.uy + j * ld + i) + __ldg(a.uy + (j + 1) * ld + i);
         if (a.mode == 0) {
-          // inertia.c:51-59, the constant factors after the sum
-          const double w = 1. + th;
-          const double wu = w * us, wv = w * vs;
-          s0 += wu;
+          // inertia.c:51-59: the constant factors, and the row's Y in the moment, after the sum
+          const double w = 1. + th, wv = w * vs;
+          s0 = fma(w, us, s0);
           s1 += wv;
-          s2 = fma(X, wv, fma(-Y, wu, s2));
+          s2 = fma(X, wv, s2);
         } else {
           // exchange.c:61-76 (BETA / 2 = 1)
           const double w = fma(-th, th, 1.);
           const double gx = w * fma(-0.5, us, fma(-pvz, Y, pux));
           const double gy = w * fma(-0.5, vs, fma(pvz, X, puy));
           contrib = a.weights_only ? make_double2(w, w) : make_double2(gx, gy);
-          s0 -= gx;
-          s1 -= gy;
-          s2 = fma(Y, gx, fma(-X, gy, s2));
+          s0 += gx;
+          s1 += gy;
+          s2 = fma(X, gy, s2);
         }
       }
       if (a.mode == 1 && EIF_CHK(a.bd.rec, (long long)c * CHUNK + half * 32 + lane, a.bd.wbuf, 19))
         a.wbuf[(size_t)c * CHUNK + half * 32 + lane] = contrib;
     }
-    const double v = warp_sum3(s0, s1, s2, lane);
+    // sum_x, sum_y in lanes 0 and 16, the moment sum X f_y in lane 8, which takes Y sum_x off it
+    double v = warp_sum3(s0, s1, s2, lane);
+    const double sx = __shfl_sync(0xffffffffu, v, 0);
     const int slot = lane == 0 ? 0 : (lane == 16 ? 1 : (lane == 8 ? 2 : -1));
-    if (slot >= 0 && EIF_CHK(a.bd.rec, 3LL * c + 2, a.bd.partial, 20))
+    if (slot >= 0 && EIF_CHK(a.bd.rec, 3LL * c + 2, a.bd.partial, 20)) {
+      if (slot == 2) v = fma(-Y, sx, v);
       a.partial[3 * (size_t)c + slot] = v * (scale * ldro<NC>(pd + (slot == 2 ? PD_RPIM : PD_RPM)));
+    }
   }
 }
 

@@ -128,7 +128,7 @@ enum { ST_NP, ST_UBOX, ST_UCOLL, ST_UTAB, ST_UPART, ST_MIXED, ST_TASKS, ST_WORDS
 __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
   __shared__ unsigned act[SUB_MAX / 32];   // suspensions still iterating
   __shared__ float2 slot_f[SUB_WARPS][CHUNK];
-  __shared__ double slot_d[SUB_WARPS][CHUNK];
+  __shared__ double2 slot_d[SUB_WARPS][WORK_SLOTS];
   extern __shared__ int stab[];            // ST_WORDS per suspension
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int G = gridDim.x, W = G * SUB_WARPS, T = G * SUB_THREADS;
