@@ -13,17 +13,16 @@
 // kernel writes them between its phases.
 #pragma once
 #include "eif_internal.cuh"
+#include "foot_device.cuh"
 #include <cfloat>
 
 namespace {
 
-struct EllD { double a, b, x, y, angle; };
-
 using eifd::pmass;
 using eifd::pmoi;
 
-// ellipse.c:30-65 with per-call evaluation of the evolute coefficients
-__device__ double normal_t_d(double a, double b, double x_, double y_) {
+// ellipse.c:30-65, for the few feet that foot_newton leaves
+__device__ __noinline__ double normal_t_d(double a, double b, double x_, double y_) {
   const double px = fabs(x_), py = fabs(y_);
   const double kex = a * (1. - (b / a) * (b / a));
   const double key = b * (1. - (a / b) * (a / b));
@@ -50,68 +49,93 @@ __device__ double normal_t_d(double a, double b, double x_, double y_) {
   return t;
 }
 
-// ellipse.c:17-28
-__device__ __forceinline__ double curvature(double a, double b, double t) {
-  double st, ct;
-  sincos(t, &st, &ct);
-  const double ct2 = ct * ct, st2 = st * st;
-  return a * b * (ct2 + st2) / pow(a * a * st2 + b * b * ct2, 1.5);
+// One ellipse of an equivalent-circle fit: what its evolute points need, formed once per fit
+struct FitEllipse {
+  double a, b, x, y, cp, sp;     // semi-axes, centre, cos and sin of the angle
+  double kex, key, rab;          // a(1-(b/a)^2), b(1-(a/b)^2), 1 / (a b)
+  EllF f;
+};
+
+__device__ __forceinline__ FitEllipse fit_ellipse(double a, double b, double x, double y, double angle) {
+  FitEllipse e;
+  e.a = a; e.b = b; e.x = x; e.y = y;
+  sincos(angle, &e.sp, &e.cp);
+  e.kex = a * fma(-(b / a), b / a, 1.);
+  e.key = b * fma(-(a / b), a / b, 1.);
+  e.rab = 1. / (a * b);
+  e.f.a = eifd::d2f(a); e.f.b = eifd::d2f(b); e.f.cz = 1.f; e.f.sz = 0.f;
+  e.f.kex = eifd::d2f(e.kex); e.f.key = eifd::d2f(e.key);
+  return e;
 }
 
-// collision.c:75-109
-__device__ void evolute(const EllD &e, double x, double y, double &ex, double &ey, double &ix, double &iy, double &r) {
-  double sn, cs;
-  sincos(-e.angle, &sn, &cs);
-  const double x__ = x - e.x, y__ = y - e.y;
-  double x_ = cs * x__ - sn * y__;
-  double y_ = sn * x__ + cs * y__;
-  const double t = normal_t_d(e.a, e.b, x_, y_);
-  r = 1. / fmax(curvature(e.a, e.b, t), DBL_EPSILON);
-  double st, ct;
-  sincos(t, &st, &ct);
-  x_ = e.a * (1. - (e.b / e.a) * (e.b / e.a)) * (ct * ct * ct);
-  y_ = e.b * (1. - (e.a / e.b) * (e.a / e.b)) * (st * st * st);
-  double sp, cp;
-  sincos(e.angle, &sp, &cp);
-  ex = cp * x_ - sp * y_;
-  ey = sp * x_ + cp * y_;
-  ex = ex + e.x;
-  ey = ey + e.y;
-  x_ = e.a * ct;
-  y_ = e.b * st;
-  ix = cp * x_ - sp * y_;
-  iy = sp * x_ + cp * y_;
-}
-
-// collision.c:111-135; returns false when the iteration cap is reached
-__device__ bool fit_pair(const EllD &e0, const EllD &e1, double c0[3], double c1[3], double &ix0, double &iy0,
-                         double &ix1, double &iy1) {
-  c0[0] = e0.x; c0[1] = e0.y;
-  c1[0] = e1.x; c1[1] = e1.y;
-  for (int n = 0; n < EIF_FIT_MAX_ITER; n++) {
-    double c0x, c0y, c1x, c1y;
-    evolute(e0, c1[0], c1[1], c0x, c0y, ix0, iy0, c0[2]);
-    evolute(e1, c0[0], c0[1], c1x, c1y, ix1, iy1, c1[2]);
-    const double d0x = c0x - c0[0], d0y = c0y - c0[1];
-    const double d1x = c1x - c1[0], d1y = c1y - c1[1];
-    c0[0] += d0x; c0[1] += d0y;
-    c1[0] += d1x; c1[1] += d1y;
-    if (fmax(fmax(fabs(d0x), fabs(d0y)), fmax(fabs(d1x), fabs(d1y))) < 1.e-8) return true;
+// The foot of the normal from (px, py), first quadrant, as (c, s) = (cos t, sin t), by
+// Newton steps from the (c, s) given: with v = (px, py) - (a c, b s) and T the derivative of
+// the ellipse in t, the angle to the foot is v.T / K, K = T^2 + v.(a c, b s). Returns false
+// where K is small (next to the evolute) or the start is too far off.
+__device__ __forceinline__ bool foot_newton(const FitEllipse &e, double px, double py, double &c, double &s) {
+  for (int n = 0; n < 8; n++) {
+    // back onto the unit circle
+    double dn = fma(c, c, fma(s, s, -1.));
+    double h = fma(dn, fma(dn, 0.375, -0.5), 1.);
+    c *= h;
+    s *= h;
+    const double ac = e.a * c, bs = e.b * s, as = e.a * s, bc = e.b * c;
+    const double vx = px - ac, vy = py - bs;
+    const double g = fma(vy, bc, -(vx * as));
+    const double w2 = fma(as, as, bc * bc);
+    const double K = fma(vx, ac, fma(vy, bs, w2));
+    const float Kf = eifd::d2f(K);
+    if (!(Kf > 0.02f * eifd::d2f(w2))) return false;
+    // g / K from a single-precision reciprocal and one Newton step
+    const double r = eifd::f2d(__fdividef(1.f, Kf)), gr = g * r;
+    const double d = fma(gr, fma(-K, r, 1.), gr);
+    if (!(fabs(d) < 0.1)) return false;
+    h = fma(d, -0.5 * d, 1.);
+    const double c1 = fmax(fma(-d, s, c * h), 0.);
+    s = fmax(fma(d, c, s * h), 0.);
+    c = c1;
+    if (fabs(d) < 2.e-8) {   // the next step would be below 1e-15
+      dn = fma(c, c, fma(s, s, -1.));
+      h = fma(dn, -0.5, 1.);
+      c *= h;
+      s *= h;
+      return true;
+    }
   }
   return false;
 }
 
-// collision.c:137-154
-__device__ bool fit_wall(const EllD &e, double wallx, double cc[3], double &ix, double &iy) {
-  cc[0] = e.x; cc[1] = e.y;
-  for (int n = 0; n < EIF_FIT_MAX_ITER; n++) {
-    double cx, cy;
-    evolute(e, 2. * wallx - cc[0], cc[1], cx, cy, ix, iy, cc[2]);
-    const double dcx = cx - cc[0], dcy = cy - cc[1];
-    cc[0] += dcx; cc[1] += dcy;
-    if (fmax(fabs(dcx), fabs(dcy)) < 1.e-8) return true;
+// compute_evolute, collision.c:75-109: the centre (ex, ey) and the radius r of the circle of
+// curvature at the foot of (x, y), and the foot's offset (ix, iy) from the ellipse's centre;
+// (c, s): the foot of the fit's last iteration on entry (first: none yet), this one's on
+// return. A serial chain of FP64 operations, of about 25 ns each here: the foot is iterated
+// on (cos t, sin t), from the last foot or the one that single precision finds, so that
+// nothing but a square root is left of ellipse.c's sincos, asin, divisions and the curvature's
+// pow, and evaluated to the same accuracy (the foot to 1e-15 and better, where ellipse.c
+// stops once the step is below 1e-8). Every product-sum is an explicit fma: the same bits in
+// whatever kernel this is compiled.
+__device__ __forceinline__ void evolute(const FitEllipse &e, bool first, double x, double y, double &c, double &s,
+                                        double &ex, double &ey, double &ix, double &iy, double &r) {
+  const double X = x - e.x, Y = y - e.y;
+  const double x_ = fma(e.cp, X, e.sp * Y), y_ = fma(e.cp, Y, -(e.sp * X));
+  const double px = fabs(x_), py = fabs(y_);
+  if (first || !foot_newton(e, px, py, c, s)) {
+    float sf, cf;
+    sincosf(normal_t_f_q1(e.f, eifd::d2f(px), eifd::d2f(py)), &sf, &cf);
+    c = eifd::f2d(cf);
+    s = eifd::f2d(sf);
+    if (!foot_newton(e, px, py, c, s)) sincos(normal_t_d(e.a, e.b, px, py), &s, &c);
   }
-  return false;
+  const double cs = x_ < 0. ? -c : c, ss = y_ < 0. ? -s : s;
+  const double as = e.a * s, bc = e.b * c;
+  const double w2 = fma(as, as, bc * bc);
+  r = fmin(w2 * sqrt(w2) * e.rab, 1. / DBL_EPSILON);   // ellipse.c:17-28
+  const double vx = e.kex * (cs * cs * cs), vy = e.key * (ss * ss * ss);
+  ex = fma(e.cp, vx, -(e.sp * vy)) + e.x;
+  ey = fma(e.sp, vx, e.cp * vy) + e.y;
+  const double fx = e.a * cs, fy = e.b * ss;
+  ix = fma(e.cp, fx, -(e.sp * fy));
+  iy = fma(e.sp, fx, e.cp * fy);
 }
 
 __device__ __forceinline__ double harmonic(double v0, double v1) { return 1. / (0.5 * (1. / v0 + 1. / v1)); }
@@ -159,85 +183,150 @@ __device__ __forceinline__ bool bounding_overlap(const PV &p0, const PV &p1, dou
 // Candidate normals: the centre line, the four semi-axis directions and 16 fixed
 // directions; along a unit normal n the ellipses' extents are their support values
 // sqrt(a^2 (n.u)^2 + b^2 (n.v)^2) about the centres.
-__device__ bool apart(const PV &p0, const PV &p1, double ly) {
-  const double yoff = image_offset(p0.y, p1.y, ly);
-  const double dx = p1.x - p0.x, dy = (p1.y + yoff) - p0.y;
-  double s0, c0, s1, c1;
-  sincos(p0.az, &s0, &c0);
-  sincos(p1.az, &s1, &c1);
-  const double margin = 0.01 * fmin(fmin(p0.a, p0.b), fmin(p1.a, p1.b));
-  auto gap = [&](double nx, double ny) {
-    const double u0 = nx * c0 + ny * s0, v0 = ny * c0 - nx * s0;
-    const double u1 = nx * c1 + ny * s1, v1 = ny * c1 - nx * s1;
-    const double h0 = sqrt(p0.a * p0.a * u0 * u0 + p0.b * p0.b * v0 * v0);
-    const double h1 = sqrt(p1.a * p1.a * u1 * u1 + p1.b * p1.b * v1 * v1);
-    return fabs(nx * dx + ny * dy) - h0 - h1;
-  };
-  const double d = hypot(dx, dy);
-  if (d > 0. && gap(dx / d, dy / d) > margin) return true;
-  if (gap(c0, s0) > margin || gap(-s0, c0) > margin || gap(c1, s1) > margin || gap(-s1, c1) > margin) return true;
-  for (int q = 0; q < 16; q++) {
-    double s, c;
-    sincospi(q / 16., &s, &c);
-    if (gap(c, s) > margin) return true;
-  }
-  return false;
+struct PairFrame {
+  double dx, dy, s0, c0, s1, c1, margin;
+};
+__device__ __forceinline__ PairFrame pair_frame(const PV &p0, const PV &p1, double ly) {
+  PairFrame f;
+  f.dx = p1.x - p0.x;
+  f.dy = (p1.y + image_offset(p0.y, p1.y, ly)) - p0.y;
+  sincos(p0.az, &f.s0, &f.c0);
+  sincos(p1.az, &f.s1, &f.c1);
+  f.margin = 0.01 * fmin(fmin(p0.a, p0.b), fmin(p1.a, p1.b));
+  return f;
+}
+__device__ __forceinline__ bool separated(const PairFrame &f, const PV &p0, const PV &p1, double nx, double ny) {
+  const double u0 = nx * f.c0 + ny * f.s0, v0 = ny * f.c0 - nx * f.s0;
+  const double u1 = nx * f.c1 + ny * f.s1, v1 = ny * f.c1 - nx * f.s1;
+  const double h0 = sqrt(p0.a * p0.a * u0 * u0 + p0.b * p0.b * v0 * v0);
+  const double h1 = sqrt(p1.a * p1.a * u1 * u1 + p1.b * p1.b * v1 * v1);
+  return fabs(nx * f.dx + ny * f.dy) - h0 - h1 > f.margin;
+}
+// the centre line alone, which settles most pairs: one pair per lane
+__device__ __forceinline__ bool apart_centres(const PV &p0, const PV &p1, double ly) {
+  const PairFrame f = pair_frame(p0, p1, ly);
+  const double d = hypot(f.dx, f.dy);
+  return d > 0. && separated(f, p0, p1, f.dx / d, f.dy / d);
+}
+// the other directions of one pair, one per lane
+__device__ __forceinline__ bool apart_warp(const PV &p0, const PV &p1, double ly, int lane) {
+  const PairFrame f = pair_frame(p0, p1, ly);
+  double ny, nx;
+  sincospi((lane - 4) / 16., &ny, &nx);
+  if (lane == 0) { nx = f.c0; ny = f.s0; }
+  if (lane == 1) { nx = -f.s0; ny = f.c0; }
+  if (lane == 2) { nx = f.c1; ny = f.s1; }
+  if (lane == 3) { nx = -f.s1; ny = f.c1; }
+  return __any_sync(0xffffffffu, lane < 20 && separated(f, p0, p1, nx, ny));
 }
 
-// force/torque contribution of pair (n0 < n1) on particle `self` (collision.c:190-246)
-__device__ void pair_contribution(const PV &p0, const PV &p1, bool self_is_0, double ly, double out[3], bool &ok) {
-  out[0] = out[1] = out[2] = 0.;
-  const double yoff = image_offset(p0.y, p1.y, ly);
-  EllD e0{p0.a, p0.b, p0.x, p0.y, p0.az};
-  EllD e1{p1.a, p1.b, p1.x, p1.y + yoff, p1.az};
-  double c0[3], c1[3], ix0, iy0, ix1, iy1;
-  ok = fit_pair(e0, e1, c0, c1, ix0, iy0, ix1, iy1);
-  const double m0 = pmass(p0.den, p0.a, p0.b), m1 = pmass(p1.den, p1.a, p1.b);
-  const double i0 = pmoi(p0.den, p0.a, p0.b), i1 = pmoi(p1.den, p1.a, p1.b);
-  const double mass = harmonic(m0, m1);
-  const double reft = pow(harmonic(sqrt(p0.a * p0.b), sqrt(p1.a * p1.b)), 1.5);
-  const double k = mass * (M_PI * M_PI) / (reft * reft);
-  double nx = c1[0] - c0[0], ny = c1[1] - c0[1];
-  const double norm = fmax(hypot(nx, ny), DBL_EPSILON);
-  nx /= norm;
-  ny /= norm;
-  const double overlap = c0[2] + c1[2] - norm;
-  if (overlap > 0.) {
-    const double cfx = k * overlap * nx, cfy = k * overlap * ny;
-    if (self_is_0) {
-      out[0] = 1. / m0 * (-cfx);
-      out[1] = 1. / m0 * (-cfy);
-      out[2] = 1. / i0 * (ix0 * (-cfy) - iy0 * (-cfx));
-    } else {
-      out[0] = 1. / m1 * (+cfx);
-      out[1] = 1. / m1 * (+cfy);
-      out[2] = 1. / i1 * (ix1 * (+cfy) - iy1 * (+cfx));
+constexpr int FIT_SLOTS = 16;   // pairs a warp fits at a time, two lanes each
+// The contacts of particle k, its pairs with the listed particles (in partner order) and the
+// walls at x = 0 and x = lx: equivalent-circle fits (collision.c:111-154), forces and torques
+// (collision.c:190-304), summed in partner order and then the walls (lane 0 has the sums).
+// The two ellipses of a pair are iterated by two neighbouring lanes, since each iteration
+// needs of the other ellipse only its last centre; the walls take one more pair of lanes, with
+// the mirrored centre in the place of the other's. A fit is a serial chain of a hundred and more
+// evolute points in double precision and sets the time of the launch.
+__device__ __forceinline__ void contact_forces(const double *P, int pcap, int k, const PV &pk, const int *list, int ncon,
+                                               double ly, double lx, double (*cval)[3], double acc[3], bool &ok_all) {
+  const int lane = threadIdx.x & 31, role = lane & 1;
+  const double wallx = role ? lx : 0.;
+  const bool near_wall = !(fmax(pk.a, pk.b) - fabs(wallx - pk.x) < 0.);
+  const bool walls = __any_sync(0xffffffffu, near_wall);
+  const int items = ncon + (walls ? 1 : 0);
+  acc[0] = acc[1] = acc[2] = 0.;
+  ok_all = true;
+  for (int base = 0; base < items; base += FIT_SLOTS) {
+    const int q = base + (lane >> 1);
+    const bool wall = q == ncon;
+    bool act = q < ncon || (wall && near_wall);
+    PV p0 = pk, p1 = pk;
+    bool self0 = true;
+    if (q < ncon) {
+      const int m = list[q];
+      self0 = k < m;
+      const PV o = load_pv(P, pcap, m);
+      p0 = self0 ? pk : o;
+      p1 = self0 ? o : pk;
     }
+    const double yoff = wall ? 0. : image_offset(p0.y, p1.y, ly);
+    const PV &pe = role ? p1 : p0;
+    const FitEllipse e = fit_ellipse(pe.a, pe.b, pe.x, pe.y + (role ? yoff : 0.), pe.az);
+    double cx = e.x, cy = e.y, r = 0., ix = 0., iy = 0., c = 0., s = 0.;
+    bool ok = !act;
+    for (int n = 0; n < EIF_FIT_MAX_ITER && __any_sync(0xffffffffu, act); n++) {
+      double ox = __shfl_xor_sync(0xffffffffu, cx, 1), oy = __shfl_xor_sync(0xffffffffu, cy, 1);
+      if (wall) {
+        ox = fma(2., wallx, -cx);
+        oy = cy;
+      }
+      double change = 0.;
+      if (act) {
+        double nx, ny;
+        evolute(e, n == 0, ox, oy, c, s, nx, ny, ix, iy, r);
+        const double dx = nx - cx, dy = ny - cy;
+        cx += dx;
+        cy += dy;
+        change = fmax(fabs(dx), fabs(dy));
+      }
+      const double other = __shfl_xor_sync(0xffffffffu, change, 1);
+      if (act && (wall ? change : fmax(change, other)) < 1.e-8) {
+        act = false;
+        ok = true;
+      }
+    }
+    ok_all &= ok;
+    const double ocx = __shfl_xor_sync(0xffffffffu, cx, 1), ocy = __shfl_xor_sync(0xffffffffu, cy, 1),
+                 orr = __shfl_xor_sync(0xffffffffu, r, 1);
+    double out[3] = {0., 0., 0.};
+    if (q < ncon && (role == 0) == self0) {
+      const double m0 = pmass(p0.den, p0.a, p0.b), m1 = pmass(p1.den, p1.a, p1.b);
+      const double mass = harmonic(m0, m1);
+      const double h = harmonic(sqrt(p0.a * p0.b), sqrt(p1.a * p1.b));
+      const double kc = mass * (M_PI * M_PI) / (h * h * h);   // the square of h^(3/2)
+      // from this particle's circle to the other's
+      double nx = ocx - cx, ny = ocy - cy;
+      const double norm = fmax(hypot(nx, ny), DBL_EPSILON);
+      nx /= norm;
+      ny /= norm;
+      const double overlap = r + orr - norm;
+      if (overlap > 0.) {
+        const double cfx = -(kc * overlap * nx), cfy = -(kc * overlap * ny);
+        out[0] = 1. / (self0 ? m0 : m1) * cfx;
+        out[1] = 1. / (self0 ? m0 : m1) * cfy;
+        out[2] = 1. / pmoi(pe.den, pe.a, pe.b) * fma(ix, cfy, -(iy * cfx));
+      }
+    }
+    if (wall && near_wall) {
+      const double pm = pmass(pk.den, pk.a, pk.b), h = sqrt(pk.a * pk.b);
+      const double kc = pm * (M_PI * M_PI) / (h * h * h);
+      double nx = wallx - cx;
+      const double norm = fabs(nx);
+      nx /= norm;
+      const double overlap = r - norm;
+      if (overlap > 0.) {
+        const double cfx = kc * overlap * nx;
+        out[0] = 1. / pm * (-cfx);
+        out[2] = 1. / pmoi(pk.den, pk.a, pk.b) * (iy * cfx);
+      }
+    }
+    if (q < ncon && (role == 0) == self0)
+      for (int f = 0; f < 3; f++) cval[lane >> 1][f] = out[f];
+    if (wall)
+      for (int f = 0; f < 3; f++) cval[FIT_SLOTS + role][f] = out[f];
+    __syncwarp();
+    if (lane == 0) {
+      const int pairs = min(FIT_SLOTS, ncon - base);
+      for (int t = 0; t < pairs; t++)
+        for (int f = 0; f < 3; f++) acc[f] += cval[t][f];
+      if (base + FIT_SLOTS >= items && walls)
+        for (int t = 0; t < 2; t++)
+          for (int f = 0; f < 3; f++) acc[f] += cval[FIT_SLOTS + t][f];
+    }
+    __syncwarp();
   }
-}
-
-// collision.c:249-304
-__device__ void wall_contribution(const PV &p, double wallx, double out[3], bool &ok) {
-  out[0] = out[1] = out[2] = 0.;
-  ok = true;
-  const double r = fmax(p.a, p.b);
-  if (r - fabs(wallx - p.x) < 0.) return;
-  EllD e{p.a, p.b, p.x, p.y, p.az};
-  double cc[3], ix, iy;
-  ok = fit_wall(e, wallx, cc, ix, iy);
-  const double pm = pmass(p.den, p.a, p.b), pim = pmoi(p.den, p.a, p.b);
-  const double reft = pow(sqrt(p.a * p.b), 1.5);
-  const double k = pm * (M_PI * M_PI) / (reft * reft);
-  double nx = wallx - cc[0];
-  const double norm = fabs(nx);
-  nx /= norm;
-  const double overlap = cc[2] - norm;
-  if (overlap > 0.) {
-    const double cfx = k * overlap * nx, cfy = 0.;
-    out[0] = 1. / pm * (-cfx);
-    out[1] = 1. / pm * (-cfy);
-    out[2] = 1. / pim * (ix * (-cfy) - iy * (-cfx));
-  }
+  ok_all = __all_sync(0xffffffffu, ok_all);
 }
 
 // Collision forces (collision.c:306-367) in one launch, one warp per particle k:
@@ -248,8 +337,8 @@ __device__ void wall_contribution(const PV &p, double wallx, double out[3], bool
 //     prefix count);
 //  2. the lanes give the listed pairs the exact double-precision bounding-circle test of
 //     collision.c:173-189 (canonical orientation) and compact the hits in order;
-//  3. the hits are evaluated one per lane (circle fit, force and torque) and summed in
-//     partner order by lane 0, then the walls at x = 0 and x = lx are added.
+//  3. hits whose ellipses a line separates are dropped, the others and the walls are
+//     evaluated (contact_forces).
 constexpr int CAND_CAP = EIF_CAND_CAP;   // candidates per particle
 constexpr int PAIR_WARPS = 8;
 constexpr int PAIR_TILE = 1024;
@@ -266,7 +355,7 @@ __device__ __forceinline__ void collision_block(double *P, int pcap, int np, int
                                                 unsigned *flags, int block) {
   __shared__ float4 tile[PAIR_TILE];
   __shared__ int list[PAIR_WARPS][CAND_CAP];
-  __shared__ double cval[PAIR_WARPS][32][3];
+  __shared__ double cval[PAIR_WARPS][FIT_SLOTS + 2][3];
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int k = block * PAIR_WARPS + wl;
   const bool on = k < np;   // uniform over the warp
@@ -315,7 +404,8 @@ __device__ __forceinline__ void collision_block(double *P, int pcap, int np, int
   if (nmaybe > CAND_CAP && lane == 0) atomicOr(flags, EIF_FLAG_NOCONV);
   nmaybe = min(nmaybe, CAND_CAP);
   const PV pk = load_pv(P, pcap, k);
-  // exact test, hits compacted in place (a write never passes the entries still to read)
+  // exact test and the centre line, hits compacted in place (a write never passes the
+  // entries still to read)
   int cnt = 0;
   for (int base = 0; base < nmaybe; base += 32) {
     const int q = base + lane;
@@ -323,57 +413,35 @@ __device__ __forceinline__ void collision_block(double *P, int pcap, int np, int
     int m = 0;
     if (q < nmaybe) {
       m = list[wl][q];
-      const PV pm_ = load_pv(P, pcap, m);
-      hit = m < k ? bounding_overlap(pm_, pk, ly) : bounding_overlap(pk, pm_, ly);
+      const PV o = load_pv(P, pcap, m);
+      const PV p0 = m < k ? o : pk, p1 = m < k ? pk : o;
+      hit = bounding_overlap(p0, p1, ly) && !apart_centres(p0, p1, ly);
     }
     const unsigned mask = __ballot_sync(0xffffffffu, hit);
     if (hit) list[wl][cnt + __popc(mask & ((1u << lane) - 1u))] = m;
     cnt += __popc(mask);
     __syncwarp();
   }
-  // forces of the hits, summed in partner order
-  double acc0 = 0., acc1 = 0., acc2 = 0.;
-  bool ok_all = true;
-  for (int base = 0; base < cnt; base += 32) {
-    const int q = base + lane;
-    const int ncand = min(32, cnt - base);
-    if (q < cnt) {
-      const int mm = list[wl][q];
-      const PV pmm = load_pv(P, pcap, mm);
-      double out[3] = {0., 0., 0.};
-      bool ok = true;
-      if (mm < k) {
-        if (!apart(pmm, pk, ly)) pair_contribution(pmm, pk, false, ly, out, ok);
-      } else {
-        if (!apart(pk, pmm, ly)) pair_contribution(pk, pmm, true, ly, out, ok);
-      }
-      ok_all &= ok;
-      cval[wl][lane][0] = out[0];
-      cval[wl][lane][1] = out[1];
-      cval[wl][lane][2] = out[2];
-    }
+  // the other directions, in order again
+  int ncon = 0;
+  for (int q = 0; q < cnt; q++) {
+    const int m = list[wl][q];
+    const PV o = load_pv(P, pcap, m);
+    const PV p0 = m < k ? o : pk, p1 = m < k ? pk : o;
+    if (apart_warp(p0, p1, ly, lane)) continue;
     __syncwarp();
-    if (lane == 0) {
-      for (int t = 0; t < ncand; t++) {
-        acc0 += cval[wl][t][0];
-        acc1 += cval[wl][t][1];
-        acc2 += cval[wl][t][2];
-      }
-    }
-    __syncwarp();
+    if (lane == 0) list[wl][ncon] = m;
+    ncon++;
   }
-  const bool ok_warp = __all_sync(0xffffffffu, ok_all);
+  __syncwarp();
+  double acc[3];
+  bool ok;
+  contact_forces(P, pcap, k, pk, list[wl], ncon, ly, lx, cval[wl], acc, ok);
   if (lane == 0) {
-    double out[3];
-    bool ok0, ok1;
-    wall_contribution(pk, 0., out, ok0);
-    acc0 += out[0]; acc1 += out[1]; acc2 += out[2];
-    wall_contribution(pk, lx, out, ok1);
-    acc0 += out[0]; acc1 += out[1]; acc2 += out[2];
-    P[(EIF_P_CFX0 + cn) * pcap + k] = acc0;
-    P[(EIF_P_CFY0 + cn) * pcap + k] = acc1;
-    P[(EIF_P_CTZ0 + cn) * pcap + k] = acc2;
-    if (!(ok_warp && ok0 && ok1)) atomicOr(flags, EIF_FLAG_NOCONV);
+    P[(EIF_P_CFX0 + cn) * pcap + k] = acc[0];
+    P[(EIF_P_CFY0 + cn) * pcap + k] = acc[1];
+    P[(EIF_P_CTZ0 + cn) * pcap + k] = acc[2];
+    if (!ok) atomicOr(flags, EIF_FLAG_NOCONV);
   }
 }
 
