@@ -73,8 +73,11 @@ struct PoissonPlan {
   float *tdm_inv_f = nullptr, *tdm_up_f = nullptr, *tdm_g_f = nullptr;
   float2 *qdf = nullptr;   // right-hand side of the first pass as (hi, lo) pairs, jtot rows of pitch ld
   // tridiagonal solver along y (jtot rows, one system per wavenumber)
-  int blk;          // interior rows per block + 1 (EIF_TDM_M), or 0: serial path
-  int nblk;         // blocks per column (jtot / blk)
+  int blk;          // interior rows per block + 1 (EIF_TDM_M), or 0: odd_blk or the serial path
+  int nblk;         // blocks per column
+  // lengths that no block size divides: blocks of odd_blk rows, the last one of odd_len
+  int odd_blk = 0, odd_len = 0;
+  double *tdm_gl = nullptr;  // [i][k]  tdm_g of the last block, i < odd_len-1
   double *tdm_inv;  // [k][i]  1/pivot of the interior Thomas sweep, i < blk-1
   double *tdm_up;   // [k][i]  modified upper diagonal, i < blk-1
   double *tdm_g;    // [k][i]  response of the interior block to its left neighbour
@@ -83,14 +86,19 @@ struct PoissonPlan {
   double *red_inv;  // [k][b]  reduced cyclic system: Thomas pivots (b < nblk-1)
   double *red_up;   // [k][b]
   double *red_q1;   // [k][b]  correction vector of the reduced cyclic system
-  double *red_coef; // [k][4]  A, B, den, pin flag
+  double *red_coef; // [k][4]  A, A of the last block, den, pin flag
   // second-level partition of the reduced system (g2 values per group, q2 groups; 0: not used)
   int g2 = 0, q2 = 0;
   double *r2_inv = nullptr, *r2_up = nullptr, *r2_phi = nullptr;   // [i][k], i < g2-1
   double *r2_qinv = nullptr, *r2_qup = nullptr, *r2_q1 = nullptr;  // [q][k], q < q2-1
-  double *r2_coef = nullptr;                                        // [k][4] A2, B2, den2, pin flag
+  double *r2_coef = nullptr;                                        // [k][4] A2, A2 of the last group, den2, pin flag
+  // the last group where it differs (r2_gl values): factors and responses to both sides, i < r2_gl-1
+  bool r2_odd = false;
+  int r2_gl = 0;
+  double *r2l_inv = nullptr, *r2l_up = nullptr, *r2l_phl = nullptr, *r2l_phr = nullptr;
   double *lam;      // [k]     eigenvalue of the DCT direction
-  double *ywork;    // nblk*itot: reduced right-hand sides / interface values
+  double *ywork;    // 2*nblk*itot: reduced right-hand sides / interface values; the sequential solve's pivots
+  double *ser_up = nullptr, *ser_q1 = nullptr, *ser_den = nullptr, *ser_last = nullptr;  // its other tables (in ywork)
   float *iface_f = nullptr;  // nblk*itot: the solved interface values rounded to float (refined solve)
 };
 

@@ -17,7 +17,8 @@
 //   2. k_tdm_local: the column of each wavenumber is cut into blocks of
 //      EIF_TDM_M rows: EIF_TDM_M-1 interior rows and one interface row. Each
 //      thread solves the interior rows of one block in registers with
-//      pre-factored Thomas coefficients (the matrix is constant along y).
+//      pre-factored Thomas coefficients (the matrix is constant along y). Column
+//      lengths that are no multiple of a block size end in a shorter block.
 //   3. k_tdm_reduced: one thread per wavenumber solves the cyclic system of
 //      the interface values, which again has constant coefficients and is
 //      solved with the reference's cyclic algorithm (tdm.c:64-108), on
@@ -178,29 +179,66 @@ __global__ void __launch_bounds__(256) k_dct2(Dct2Args a) {
   }
 }
 
-// interior Thomas solve of one block in registers
-template <int M>
+// interior Thomas solve of one block in registers; ODD: the last block of a column has
+// `last` rows (1..M; without an interior its one row is the interface row)
+template <int M, bool ODD>
 __global__ void __launch_bounds__(256) k_tdm_local(double *__restrict__ qhat, const double *__restrict__ inv,
                                                   const double *__restrict__ up, double *__restrict__ iface_a,
-                                                  double *__restrict__ first, double l, int itot, int nblk, int ld) {
+                                                  double *__restrict__ first, double l, int itot, int nblk, int ld,
+                                                  int last) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
   if (k >= itot) return;
+  const int m = ODD && b == nblk - 1 ? last - 1 : M - 1;   // interior rows
   double v[M - 1];
   const size_t base = (size_t)b * M * ld + k;
 #pragma unroll
-  for (int r = 0; r < M - 1; r++) v[r] = qhat[base + (size_t)r * ld];
-  const double rif = qhat[base + (size_t)(M - 1) * ld];
+  for (int r = 0; r < M - 1; r++) v[r] = !ODD || r < m ? qhat[base + (size_t)r * ld] : 0.;
+  const double rif = qhat[base + (size_t)m * ld];
   v[0] = v[0] * __ldg(inv + k);
 #pragma unroll
-  for (int r = 1; r < M - 1; r++) v[r] = (v[r] - l * v[r - 1]) * __ldg(inv + r * itot + k);
+  for (int r = 1; r < M - 1; r++)
+    if (!ODD || r < m) v[r] = (v[r] - l * v[r - 1]) * __ldg(inv + r * itot + k);
+  double vl = v[M - 2];
+  if (ODD) {
+    vl = 0.;
 #pragma unroll
-  for (int r = M - 3; r >= 0; r--) v[r] = v[r] - __ldg(up + r * itot + k) * v[r + 1];
+    for (int r = 0; r < M - 1; r++)
+      if (r == m - 1) vl = v[r];
+  }
 #pragma unroll
-  for (int r = 0; r < M - 1; r++) qhat[base + (size_t)r * ld] = v[r];
+  for (int r = M - 3; r >= 0; r--)
+    if (!ODD || r < m - 1) v[r] = v[r] - __ldg(up + r * itot + k) * v[r + 1];
+#pragma unroll
+  for (int r = 0; r < M - 1; r++)
+    if (!ODD || r < m) qhat[base + (size_t)r * ld] = v[r];
   // interface equation: r_iface - l y[M-2] (this block) - l y[0] (next block)
-  iface_a[(size_t)b * itot + k] = rif - l * v[M - 2];
+  iface_a[(size_t)b * itot + k] = rif - l * vl;
   first[(size_t)b * itot + k] = v[0];
+}
+
+// The solution of the columns with a shorter last block, written whole (the transforms
+// that follow reconstruct equal blocks only): y + s_{b-1} g[r] + s_b g[m-1-r], with the
+// response gl of the last block's interior
+template <int M>
+__global__ void __launch_bounds__(256) k_tdm_finish(double *__restrict__ qhat, const double *__restrict__ iface,
+                                                    const double *__restrict__ g, const double *__restrict__ gl,
+                                                    int itot, int nblk, int ld, int last) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int b = blockIdx.y;
+  if (k >= itot) return;
+  const bool end = b == nblk - 1;
+  const int m = end ? last - 1 : M - 1;
+  const double *gb = (end ? gl : g) + k;
+  const double sl = __ldg(iface + (size_t)(b == 0 ? nblk - 1 : b - 1) * itot + k), sr = __ldg(iface + (size_t)b * itot + k);
+  const size_t base = (size_t)b * M * ld + k;
+#pragma unroll
+  for (int r = 0; r < M - 1; r++)
+    if (r < m) {
+      double &q = qhat[base + (size_t)r * ld];
+      q = q + sl * __ldg(gb + (size_t)r * itot) + sr * __ldg(gb + (size_t)(m - 1 - r) * itot);
+    }
+  qhat[base + (size_t)m * ld] = sr;
 }
 
 // cyclic system of the interface values of one wavenumber. One thread per
@@ -233,7 +271,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_tdm_reduced(double *__restrict_
   const int t = threadIdx.x;
   if (t < cols) {
     const int kk = min(k0 + t, itot - 1);
-    const double A = rcoef[4 * kk + 0];
+    const double A = rcoef[4 * kk + 0], Al = rcoef[4 * kk + 1];   // Al: through the last block
     const double den = rcoef[4 * kk + 2];
     const bool pin = rcoef[4 * kk + 3] != 0.;
     const double rP = zs[(P - 1) * cols + t];
@@ -251,7 +289,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_tdm_reduced(double *__restrict_
       zs[b * cols + t] = zprev;
     }
     const double z0 = zs[t], zl = zs[(P - 2) * cols + t];
-    const double num = rP - A * z0 - A * zl;
+    const double num = rP - A * z0 - Al * zl;
     lastv[t] = pin ? 0. : num / den;
   }
   __syncthreads();
@@ -279,15 +317,23 @@ __global__ void __launch_bounds__(RED_THREADS) k_tdm_reduced(double *__restrict_
 // the factors of the Q-value solve are staged in shared memory by the whole block
 // before its serial sweep. iface_f (optional): the solved values rounded to float, as in
 // k_tdm_reduced.
+// ODD: the last block of the columns (and so the last row's neighbour, P-2, and the coupling
+// Al between the two) or the last group differs from the others; the last group has Gl
+// values (1..G) and tables of its own, with the responses to both sides. One-level sweeps of
+// such lengths were serial over P values, and before them over all rows of the column.
 constexpr int RED2_K = 8;
+struct Red2Last {
+  const double *inv, *up, *phi_l, *phi_r;   // [i][k], i < Gl - 1
+  int Gl;
+};
 constexpr size_t red2_smem_bytes(int Q) { return sizeof(double) * 6 * RED2_K * (size_t)Q; }
-template <int G>
-__global__ void __launch_bounds__(1024) k_tdm_reduced2(double *__restrict__ iface, const double *__restrict__ first,
-                                                       const double *__restrict__ rcoef, const double *__restrict__ inv2,
-                                                       const double *__restrict__ up2, const double *__restrict__ phi2,
-                                                       const double *__restrict__ ri2, const double *__restrict__ ru2,
-                                                       const double *__restrict__ rq2, const double *__restrict__ rc2,
-                                                       double l, int itot, int P, int Q, float *__restrict__ iface_f) {
+template <int G, bool ODD>
+__global__ void __launch_bounds__(ODD ? 256 : 1024)
+    k_tdm_reduced2(double *__restrict__ iface, const double *__restrict__ first, const double *__restrict__ rcoef,
+                   const double *__restrict__ inv2, const double *__restrict__ up2, const double *__restrict__ phi2,
+                   const double *__restrict__ ri2, const double *__restrict__ ru2, const double *__restrict__ rq2,
+                   const double *__restrict__ rc2, double l, int itot, int P, int Q, float *__restrict__ iface_f,
+                   Red2Last last) {
   // [Q][RED2_K] first interior values, right-hand sides, interface values, and the
   // second-level factors ri2, ru2, rq2
   extern __shared__ double sm2[];
@@ -299,6 +345,11 @@ __global__ void __launch_bounds__(1024) k_tdm_reduced2(double *__restrict__ ifac
   const bool on = k < itot;
   const int kc = on ? k : itot - 1;
   const double A = rcoef[4 * kc + 0];
+  // the last group: interior values m, coupling to its interface value, factors
+  const bool end = ODD && g == Q - 1;
+  const int m = end ? last.Gl - 1 : G - 1;
+  const double Ag = end ? rcoef[4 * kc + 1] : A;
+  const double *inv_g = end ? last.inv : inv2, *up_g = end ? last.up : up2;
   // the factors of the second-level sweep (q < Q - 1; the tables hold max(G, Q) rows)
   if (g < Q - 1) {
     s_ri[g * K + kk] = ri2[(size_t)g * itot + kc];
@@ -310,20 +361,38 @@ __global__ void __launch_bounds__(1024) k_tdm_reduced2(double *__restrict__ ifac
 #pragma unroll
   for (int i = 0; i < G; i++) {
     const int b = g * G + i;
-    y[i] = iface[(size_t)b * itot + kc] - l * first[(size_t)((b + 1) % P) * itot + kc];
+    y[i] = 0.;
+    if (!ODD || i <= m) y[i] = iface[(size_t)b * itot + kc] - l * first[(size_t)((b + 1) % P) * itot + kc];
   }
-  const double rlast = y[G - 1];
-  y[0] = y[0] * inv2[kc];
+  double rlast = y[G - 1];
+  if (ODD) {
 #pragma unroll
-  for (int i = 1; i < G - 1; i++) y[i] = (y[i] - A * y[i - 1]) * inv2[(size_t)i * itot + kc];
+    for (int i = 0; i < G - 1; i++)
+      if (i == m) {
+        rlast = y[i];
+        y[i] = 0.;
+      }
+  }
+  if (!ODD || m > 0) y[0] = y[0] * inv_g[kc];
 #pragma unroll
-  for (int i = G - 3; i >= 0; i--) y[i] = y[i] - up2[(size_t)i * itot + kc] * y[i + 1];
+  for (int i = 1; i < G - 1; i++)
+    if (!ODD || i < m) y[i] = (y[i] - A * y[i - 1]) * inv_g[(size_t)i * itot + kc];
+  double yl = y[G - 2];
+  if (ODD) {
+    yl = 0.;
+#pragma unroll
+    for (int i = 0; i < G - 1; i++)
+      if (i == m - 1) yl = y[i];
+  }
+#pragma unroll
+  for (int i = G - 3; i >= 0; i--)
+    if (!ODD || i < m - 1) y[i] = y[i] - up_g[(size_t)i * itot + kc] * y[i + 1];
   y0s[g * K + kk] = y[0];
   __syncthreads();
-  rhs[g * K + kk] = rlast - A * y[G - 2] - A * y0s[((g + 1) % Q) * K + kk];
+  rhs[g * K + kk] = rlast - Ag * yl - A * y0s[((g + 1) % Q) * K + kk];
   __syncthreads();
   if (g == 0) {
-    const double A2 = rc2[4 * kc + 0], den2 = rc2[4 * kc + 2];
+    const double A2 = rc2[4 * kc + 0], A2l = rc2[4 * kc + 1], den2 = rc2[4 * kc + 2];
     const bool pin = rc2[4 * kc + 3] != 0.;
     double zprev = rhs[kk] * s_ri[kk];
     ts[kk] = zprev;
@@ -335,22 +404,25 @@ __global__ void __launch_bounds__(1024) k_tdm_reduced2(double *__restrict__ ifac
       zprev = ts[q * K + kk] - s_ru[q * K + kk] * zprev;
       ts[q * K + kk] = zprev;
     }
-    const double num = rhs[(Q - 1) * K + kk] - A2 * ts[kk] - A2 * ts[(Q - 2) * K + kk];
-    const double last = pin ? 0. : num / den2;
-    for (int q = 0; q < Q - 1; q++) ts[q * K + kk] = ts[q * K + kk] + last * s_rq[q * K + kk];
-    ts[(Q - 1) * K + kk] = last;
+    const double num = rhs[(Q - 1) * K + kk] - A2 * ts[kk] - A2l * ts[(Q - 2) * K + kk];
+    const double last_t = pin ? 0. : num / den2;
+    for (int q = 0; q < Q - 1; q++) ts[q * K + kk] = ts[q * K + kk] + last_t * s_rq[q * K + kk];
+    ts[(Q - 1) * K + kk] = last_t;
   }
   __syncthreads();
   if (!on) return;
   const double tl = ts[((g + Q - 1) % Q) * K + kk], tr = ts[g * K + kk];
 #pragma unroll
   for (int i = 0; i < G - 1; i++) {
-    const double v = y[i] + tl * phi2[(size_t)i * itot + k] + tr * phi2[(size_t)(G - 2 - i) * itot + k];
+    if (ODD && i >= m) continue;
+    const double pl = end ? last.phi_l[(size_t)i * itot + k] : phi2[(size_t)i * itot + k];
+    const double pr = end ? last.phi_r[(size_t)i * itot + k] : phi2[(size_t)(G - 2 - i) * itot + k];
+    const double v = y[i] + tl * pl + tr * pr;
     iface[(size_t)(g * G + i) * itot + k] = v;
     if (iface_f) iface_f[(size_t)(g * G + i) * itot + k] = eifd::d2f(v);
   }
-  iface[(size_t)(g * G + G - 1) * itot + k] = tr;
-  if (iface_f) iface_f[(size_t)(g * G + G - 1) * itot + k] = eifd::d2f(tr);
+  iface[(size_t)(g * G + m) * itot + k] = tr;
+  if (iface_f) iface_f[(size_t)(g * G + m) * itot + k] = eifd::d2f(tr);
 }
 
 // columns per block of k_tdm_reduced that fit its shared memory
@@ -362,44 +434,117 @@ static int red_cols(int nblk) {
 }
 static size_t red_smem_bytes(int nblk, int cols) { return sizeof(double) * ((size_t)3 * nblk * cols + cols); }
 
-// fallback for column lengths without a suitable block size: the reference's
-// sequential cyclic algorithm per wavenumber on global memory
-__global__ void k_tdm_serial(double *__restrict__ qhat, double *__restrict__ scratch, const double *__restrict__ lam,
-                             double l, int itot, int jtot, int ld) {
+// The reference's sequential cyclic algorithm (tdm.c:64-108), one thread per wavenumber: the
+// mixed form's columns that no block size divides (a partition rounds differently, and single
+// precision evaluations downstream are not continuous in their rounding: whether a stage takes
+// 4 or 102 sub-iterations depends on it), and columns of fewer than 9 rows. The matrix is the
+// same at every solve, so its factors, the correction vector and the last pivot are tables,
+// formed once per context by the sweep that the solve itself used to run: [i][k], i < n - 1.
+__global__ void k_tdm_serial_tables(double *__restrict__ val, double *__restrict__ up, double *__restrict__ q1,
+                                    double *__restrict__ den, const double *__restrict__ lam, double l, int itot,
+                                    int jtot) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= itot) return;
   const int n = jtot;
   const double c = -l - l + lam[k];
-  double *u0 = scratch + k;                     // [i*itot + k]
-  double *q1 = scratch + (size_t)n * itot + k;  // [i*itot + k]
-  auto Q = [&](int i) -> double & { return qhat[(size_t)i * ld + k]; };
-  auto U0 = [&](int i) -> double & { return u0[(size_t)i * itot]; };
-  auto Q1 = [&](int i) -> double & { return q1[(size_t)i * itot]; };
-  for (int i = 0; i < n - 1; i++) Q1(i) = i == 0 ? -l : (i == n - 2 ? -l : 0.);
-  // Thomas on rows 0..n-2 for q and q1 together (same factors)
-  U0(0) = l / c;
-  Q(0) = Q(0) / c;
-  Q1(0) = Q1(0) / c;
+  double u = l / c, w = -l / c;
+  up[k] = u;
+  val[k] = 0.;   // row 0 is divided by c
+  q1[k] = w;
   for (int i = 1; i <= n - 2; i++) {
-    double val = c - l * U0(i - 1);
-    if (fabs(val) < 2.220446049250313e-16) {
-      U0(i) = 0.; Q(i) = 0.; Q1(i) = 0.;
+    double v = fma(-l, u, c);
+    const double r = i == n - 2 ? -l : 0.;
+    if (fabs(v) < 2.220446049250313e-16) {
+      v = u = w = 0.;
     } else {
-      val = 1. / val;
-      U0(i) = val * l;
-      Q(i) = val * (Q(i) - l * Q(i - 1));
-      Q1(i) = val * (Q1(i) - l * Q1(i - 1));
+      v = 1. / v;
+      u = v * l;
+      w = v * fma(-l, w, r);
     }
+    val[(size_t)i * itot + k] = v;
+    up[(size_t)i * itot + k] = u;
+    q1[(size_t)i * itot + k] = w;
   }
+  const double wl = w;
   for (int i = n - 3; i >= 0; i--) {
-    Q(i) -= U0(i) * Q(i + 1);
-    Q1(i) -= U0(i) * Q1(i + 1);
+    w = fma(-up[(size_t)i * itot + k], w, q1[(size_t)i * itot + k]);
+    q1[(size_t)i * itot + k] = w;
   }
-  const double num = Q(n - 1) - l * Q(0) - l * Q(n - 2);
-  const double den = c + l * Q1(0) + l * Q1(n - 2);
-  const double last = (k == 0 || fabs(den) < 2.220446049250313e-16) ? 0. : num / den;
-  Q(n - 1) = last;
-  for (int i = 0; i <= n - 2; i++) Q(i) = Q(i) + last * Q1(i);
+  den[k] = fma(l, wl, fma(l, w, c));
+}
+
+// Both sweeps of the right-hand side and the last unknown. A chain of two dependent FP64
+// operations a row down and one up, which sets the time; the rows of SER_B steps ahead are in
+// registers before the chain reaches them. With the division and the correction vector's
+// sweeps in the solve, and every row loaded when its turn came, 216 x 430 took 578 us.
+constexpr int SER_B = 16;
+__global__ void __launch_bounds__(32) k_tdm_serial(double *__restrict__ qhat, const double *__restrict__ val,
+                                                   const double *__restrict__ up, const double *__restrict__ q1,
+                                                   const double *__restrict__ den, double *__restrict__ last_,
+                                                   const double *__restrict__ lam, double l, int itot, int jtot, int ld) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= itot) return;
+  const int n = jtot;
+  double *Q = qhat + k;
+  double a[SER_B], f[SER_B], an[SER_B], fn[SER_B];
+  auto load = [&](int i0, int dir, const double *t) {
+#pragma unroll
+    for (int r = 0; r < SER_B; r++) {
+      const int i = i0 + dir * r;
+      const bool in = i >= 0 && i <= n - 2;
+      an[r] = in ? Q[(size_t)i * ld] : 0.;
+      fn[r] = in ? __ldg(t + (size_t)i * itot + k) : 0.;
+    }
+  };
+  auto take = [&]() {
+#pragma unroll
+    for (int r = 0; r < SER_B; r++) {
+      a[r] = an[r];
+      f[r] = fn[r];
+    }
+  };
+  double q = Q[0] / (-l - l + lam[k]);
+  Q[0] = q;
+  load(1, 1, val);
+  for (int i0 = 1; i0 <= n - 2; i0 += SER_B) {
+    take();
+    load(i0 + SER_B, 1, val);
+#pragma unroll
+    for (int r = 0; r < SER_B; r++)
+      if (i0 + r <= n - 2) {
+        q = f[r] * fma(-l, q, a[r]);
+        Q[(size_t)(i0 + r) * ld] = q;
+      }
+  }
+  const double ql = q;
+  load(n - 3, -1, up);
+  for (int i0 = n - 3; i0 >= 0; i0 -= SER_B) {
+    take();
+    load(i0 - SER_B, -1, up);
+#pragma unroll
+    for (int r = 0; r < SER_B; r++)
+      if (i0 - r >= 0) {
+        q = fma(-f[r], q, a[r]);
+        Q[(size_t)(i0 - r) * ld] = q;
+      }
+  }
+  const double num = fma(-l, ql, fma(-l, q, Q[(size_t)(n - 1) * ld]));
+  const double d = den[k];
+  const double last = (k == 0 || fabs(d) < 2.220446049250313e-16) ? 0. : num / d;
+  Q[(size_t)(n - 1) * ld] = last;
+  last_[k] = last;
+}
+
+// the last unknown's correction of the other rows
+__global__ void __launch_bounds__(128) k_tdm_serial_last(double *__restrict__ qhat, const double *__restrict__ q1,
+                                                         const double *__restrict__ last, int itot, int jtot, int ld) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= itot) return;
+  const double s = last[k];
+  for (int i = blockIdx.y; i < jtot - 1; i += gridDim.y) {
+    double &q = qhat[(size_t)i * ld + k];
+    q = fma(s, __ldg(q1 + (size_t)i * itot + k), q);
+  }
 }
 
 struct Dct3Args {
@@ -1597,6 +1742,17 @@ int poisson_init(eif_ctx *c) {
   for (int ci = 0; ci < 3; ci++) {
     if (jt % cand[ci] == 0 && jt / cand[ci] >= 3) { pp.blk = cand[ci]; pp.nblk = jt / cand[ci]; break; }
   }
+  // other lengths (double-precision form; the mixed form: see k_tdm_serial_tables): the largest
+  // block size with three blocks, the last one shorter
+  const bool fp64 = c->cfg.precision == EIF_PREC_FP64;
+  for (int ci = 0; ci < 3 && fp64 && pp.blk == 0 && pp.odd_blk == 0; ci++) {
+    const int P = (jt + cand[ci] - 1) / cand[ci];
+    if (P >= 3 && red_cols(P) > 0) {
+      pp.odd_blk = cand[ci];
+      pp.nblk = P;
+      pp.odd_len = jt - (P - 1) * cand[ci];
+    }
+  }
   auto up_load = [&](void **dst, const void *src, size_t bytes) -> cudaError_t {
     cudaError_t e = cudaMalloc(dst, bytes);
     if (e != cudaSuccess) return e;
@@ -1643,8 +1799,9 @@ int poisson_init(eif_ctx *c) {
   EIF_CK(c, up_load((void **)&pp.rot, rot.data(), sizeof(double2) * n));
   EIF_CK(c, up_load((void **)&pp.wn, wn.data(), sizeof(double2) * n));
   EIF_CK(c, up_load((void **)&pp.lam, lam.data(), sizeof(double) * n));
-  if (pp.blk > 0) {
-    const int M = pp.blk, P = pp.nblk;
+  if (pp.blk > 0 || pp.odd_blk > 0) {
+    const int M = pp.blk > 0 ? pp.blk : pp.odd_blk, P = pp.nblk;
+    const int ml = pp.blk > 0 ? M - 1 : pp.odd_len - 1;   // interior rows of the last block
     std::vector<double> inv((size_t)(M - 1) * n), up((size_t)(M - 1) * n), g((size_t)(M - 1) * n);
     std::vector<double> rinv((size_t)P * n), rup((size_t)P * n), rq1((size_t)P * n), rcoef((size_t)4 * n);
     std::vector<double> ti(M), tu(M), tg(M), ri(P), ru(P), rq(P);
@@ -1656,8 +1813,26 @@ int poisson_init(eif_ctx *c) {
       if (q < 3 || q > 32) continue;
       if (G2 == 0 || gsz + q < G2 + Q2) { G2 = gsz; Q2 = q; }
     }
+    // a last block of its own, or no such G (double-precision form): groups of 4 to 32, the
+    // last one with GL <= G2 values
+    int GL = G2;
+    pp.r2_odd = fp64 && (ml != M - 1 || G2 == 0);
+    if (pp.r2_odd) {
+      G2 = 0;
+      for (int gsz : {32, 16, 8, 4}) {
+        const int q = (P + gsz - 1) / gsz;
+        if (q < 3 || q > 32) continue;
+        if (G2 == 0 || gsz + q < G2 + Q2) { G2 = gsz; Q2 = q; GL = P - (q - 1) * gsz; }
+      }
+    }
+    const int mi = GL - 1;   // interior values of the last group
     pp.g2 = G2;
     pp.q2 = Q2;
+    pp.r2_gl = GL;
+    const bool odd2 = G2 > 0 && pp.r2_odd;
+    const size_t ll = odd2 ? (size_t)std::max(mi, 1) * n : 1;
+    std::vector<double> l_inv(ll), l_up(ll), l_phl(ll), l_phr(ll), gl((size_t)std::max(ml, 1) * n);
+    std::vector<double> tl(M), l2i(std::max(G2, 1)), l2u(std::max(G2, 1)), l2l(std::max(G2, 1)), l2r(std::max(G2, 1));
     const size_t l2 = G2 > 0 ? (size_t)std::max(G2, Q2) * n : 1;
     std::vector<double> inv2(l2), up2(l2), phi2(l2), ri2(l2), ru2(l2), rq2(l2), rc2(G2 > 0 ? (size_t)4 * n : 1);
     std::vector<double> t2i(std::max(G2, 1)), t2u(std::max(G2, 1)), t2g(std::max(G2, 1));
@@ -1676,10 +1851,20 @@ int poisson_init(eif_ctx *c) {
       // reduced cyclic system A s_{b-1} + B s_b + A s_{b+1} = R_b
       const double A = l * tg[M - 2];
       const double B = cc + 2. * l * tg[0];
+      // the last block: coupling Al of rows P-2 and P-1, their diagonal Bl
+      double Al = A, Bl = B;
+      if (ml != M - 1) {
+        for (int i = 0; i < ml; i++) tl[i] = i == 0 ? -l : 0.;
+        if (ml > 0) thomas_apply(ml, l, ti.data(), tu.data(), tl.data());
+        for (int i = 0; i < ml; i++) gl[(size_t)i * n + k] = tl[i];
+        Al = ml > 0 ? l * tl[ml - 1] : l;
+        Bl = cc + l * tg[0] + (ml > 0 ? l * tl[0] : 0.);
+      }
       thomas_factors(P - 1, A, B, ri.data(), ru.data());
+      ri[P - 2] = 1. / (Bl - A * ru[P - 3]);
       for (int b = 0; b < P - 1; b++) rq[b] = 0.;
       rq[0] = -A;
-      rq[P - 2] += -A;
+      rq[P - 2] += -Al;
       thomas_apply(P - 1, A, ri.data(), ru.data(), rq.data());
       for (int b = 0; b < P - 1; b++) {
         rinv[(size_t)b * n + k] = ri[b];
@@ -1687,8 +1872,8 @@ int poisson_init(eif_ctx *c) {
         rq1[(size_t)b * n + k] = rq[b];
       }
       rcoef[4 * k + 0] = A;
-      rcoef[4 * k + 1] = B;
-      rcoef[4 * k + 2] = B + A * rq[0] + A * rq[P - 2];
+      rcoef[4 * k + 1] = Al;
+      rcoef[4 * k + 2] = Bl + A * rq[0] + Al * rq[P - 2];
       rcoef[4 * k + 3] = k == 0 ? 1. : 0.;
       if (G2 > 0) {
         // second level: interior factors and left response of a group, then the
@@ -1704,10 +1889,35 @@ int poisson_init(eif_ctx *c) {
         }
         const double A2 = A * t2g[G2 - 2];
         const double B2 = B + 2. * A * t2g[0];
+        // the last group: coupling A2l of its interface value to the one before, whose
+        // diagonal is B2p, and its own diagonal B2l
+        double A2l = A2, B2p = B2, B2l = B2;
+        if (odd2) {
+          for (int i = 0; i < mi; i++) {
+            l2i[i] = i < mi - 1 ? t2i[i] : 1. / (Bl - (i > 0 ? A * t2u[i - 1] : 0.));
+            l2u[i] = A * l2i[i];
+            l2l[i] = i == 0 ? -A : 0.;
+            l2r[i] = i == mi - 1 ? -Al : 0.;
+          }
+          if (mi > 0) {
+            thomas_apply(mi, A, l2i.data(), l2u.data(), l2l.data());
+            thomas_apply(mi, A, l2i.data(), l2u.data(), l2r.data());
+          }
+          for (int i = 0; i < mi; i++) {
+            l_inv[(size_t)i * n + k] = l2i[i];
+            l_up[(size_t)i * n + k] = l2u[i];
+            l_phl[(size_t)i * n + k] = l2l[i];
+            l_phr[(size_t)i * n + k] = l2r[i];
+          }
+          A2l = mi > 0 ? Al * l2l[mi - 1] : Al;
+          B2p = mi > 0 ? B + A * t2g[0] + A * l2l[0] : Bl + A * t2g[0];
+          B2l = Bl + A * t2g[0] + (mi > 0 ? Al * l2r[mi - 1] : 0.);
+        }
         thomas_factors(Q2 - 1, A2, B2, q2i.data(), q2u.data());
+        q2i[Q2 - 2] = 1. / (B2p - A2 * q2u[Q2 - 3]);
         for (int q = 0; q < Q2 - 1; q++) q2q[q] = 0.;
         q2q[0] = -A2;
-        q2q[Q2 - 2] += -A2;
+        q2q[Q2 - 2] += -A2l;
         thomas_apply(Q2 - 1, A2, q2i.data(), q2u.data(), q2q.data());
         for (int q = 0; q < Q2 - 1; q++) {
           ri2[(size_t)q * n + k] = q2i[q];
@@ -1715,8 +1925,8 @@ int poisson_init(eif_ctx *c) {
           rq2[(size_t)q * n + k] = q2q[q];
         }
         rc2[4 * k + 0] = A2;
-        rc2[4 * k + 1] = B2;
-        rc2[4 * k + 2] = B2 + A2 * q2q[0] + A2 * q2q[Q2 - 2];
+        rc2[4 * k + 1] = A2l;
+        rc2[4 * k + 2] = B2l + A2 * q2q[0] + A2l * q2q[Q2 - 2];
         rc2[4 * k + 3] = k == 0 ? 1. : 0.;
       }
     }
@@ -1759,13 +1969,29 @@ int poisson_init(eif_ctx *c) {
       EIF_CK(c, up_load((void **)&pp.r2_q1, rq2.data(), sizeof(double) * l2));
       EIF_CK(c, up_load((void **)&pp.r2_coef, rc2.data(), sizeof(double) * rc2.size()));
     }
+    if (odd2) {
+      EIF_CK(c, up_load((void **)&pp.r2l_inv, l_inv.data(), sizeof(double) * ll));
+      EIF_CK(c, up_load((void **)&pp.r2l_up, l_up.data(), sizeof(double) * ll));
+      EIF_CK(c, up_load((void **)&pp.r2l_phl, l_phl.data(), sizeof(double) * ll));
+      EIF_CK(c, up_load((void **)&pp.r2l_phr, l_phr.data(), sizeof(double) * ll));
+    }
+    if (pp.odd_blk > 0) EIF_CK(c, up_load((void **)&pp.tdm_gl, gl.data(), sizeof(double) * gl.size()));
     EIF_CK(c, cudaMalloc((void **)&pp.ywork, sizeof(double) * 2 * (size_t)P * n));
   } else {
-    EIF_CK(c, cudaMalloc((void **)&pp.ywork, sizeof(double) * 2 * (size_t)jt * n));
+    // the tables of the sequential solve and the last unknowns
+    const size_t tab = (size_t)(jt - 1) * n;
+    EIF_CK(c, cudaMalloc((void **)&pp.ywork, sizeof(double) * (3 * tab + 2 * (size_t)n)));
+    pp.ser_up = pp.ywork + tab;
+    pp.ser_q1 = pp.ser_up + tab;
+    pp.ser_den = pp.ser_q1 + tab;
+    pp.ser_last = pp.ser_den + n;
+    EIF_CK(c, cudaStreamSynchronize(nullptr));   // lam's upload
+    k_tdm_serial_tables<<<(n + 31) / 32, 32, 0, c->stream>>>(pp.ywork, pp.ser_up, pp.ser_q1, pp.ser_den, pp.lam, l, n, jt);
+    EIF_LAUNCH_CK(c);
   }
-  const int rcols = red_cols(pp.blk > 0 ? pp.nblk : 1);
+  const int rcols = red_cols(pp.nblk);
   if (rcols == 0) return fail(c, EIF_ERR_ARG, "jtot %d needs too many tridiagonal blocks", jt);
-  const size_t red_smem = red_smem_bytes(pp.blk > 0 ? pp.nblk : 1, rcols);
+  const size_t red_smem = red_smem_bytes(pp.nblk, rcols);
   if (red_smem > 48 * 1024) {
     EIF_CK(c, cudaFuncSetAttribute(k_tdm_reduced, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)red_smem));
   }
@@ -1798,7 +2024,7 @@ void poisson_free(eif_ctx *c) {
   void *ptrs[] = {pp.r2_inv, pp.r2_up, pp.r2_phi, pp.r2_qinv, pp.r2_qup, pp.r2_q1, pp.r2_coef,
                   pp.tw, pp.rot, pp.wn, pp.tw_f, pp.rot_f, pp.wn_f, pp.lam, pp.tdm_inv, pp.tdm_up, pp.tdm_g, pp.tdm_g_df, pp.tdm_inv_df, pp.tdm_up_df,
                   pp.red_inv, pp.red_up, pp.red_q1, pp.red_coef, pp.ywork, pp.tw2, pp.rot2, pp.wn2, pp.tdm_inv_f,
-                  pp.tdm_up_f, pp.tdm_g_f, pp.qdf, pp.iface_f};
+                  pp.tdm_up_f, pp.tdm_g_f, pp.qdf, pp.iface_f, pp.r2l_inv, pp.r2l_up, pp.r2l_phl, pp.r2l_phr, pp.tdm_gl};
   for (void *p : ptrs) if (p) cudaFree(p);
   pp = PoissonPlan{};
 }
@@ -1814,19 +2040,24 @@ static int reduced_solve(eif_ctx *c, double *iface, double *first, float *iface_
     const int Q = pp.q2;
     const size_t sm = red2_smem_bytes(Q);
     const dim3 grid((n + RED2_K - 1) / RED2_K);
-    if (pp.g2 == 16) {
-      k_tdm_reduced2<16><<<grid, RED2_K * Q, sm, c->stream>>>(iface, first, pp.red_coef, pp.r2_inv, pp.r2_up, pp.r2_phi,
-                                                          pp.r2_qinv, pp.r2_qup, pp.r2_q1, pp.r2_coef, l, n, pp.nblk, Q,
-                                                         iface_f);
+    const Red2Last last{pp.r2l_inv, pp.r2l_up, pp.r2l_phl, pp.r2l_phr, pp.r2_gl};
+#define EIF_RED2(G, ODD)                                                                                              \
+  k_tdm_reduced2<G, ODD><<<grid, RED2_K * Q, sm, c->stream>>>(iface, first, pp.red_coef, pp.r2_inv, pp.r2_up,         \
+                                                              pp.r2_phi, pp.r2_qinv, pp.r2_qup, pp.r2_q1, pp.r2_coef, \
+                                                              l, n, pp.nblk, Q, iface_f, last)
+    if (pp.r2_odd) {
+      if (pp.g2 == 32) EIF_RED2(32, true);
+      else if (pp.g2 == 16) EIF_RED2(16, true);
+      else if (pp.g2 == 8) EIF_RED2(8, true);
+      else EIF_RED2(4, true);
+    } else if (pp.g2 == 16) {
+      EIF_RED2(16, false);
     } else if (pp.g2 == 8) {
-      k_tdm_reduced2<8><<<grid, RED2_K * Q, sm, c->stream>>>(iface, first, pp.red_coef, pp.r2_inv, pp.r2_up, pp.r2_phi,
-                                                         pp.r2_qinv, pp.r2_qup, pp.r2_q1, pp.r2_coef, l, n, pp.nblk, Q,
-                                                         iface_f);
+      EIF_RED2(8, false);
     } else {
-      k_tdm_reduced2<4><<<grid, RED2_K * Q, sm, c->stream>>>(iface, first, pp.red_coef, pp.r2_inv, pp.r2_up, pp.r2_phi,
-                                                         pp.r2_qinv, pp.r2_qup, pp.r2_q1, pp.r2_coef, l, n, pp.nblk, Q,
-                                                         iface_f);
+      EIF_RED2(4, false);
     }
+#undef EIF_RED2
   } else {
     const int rcols = red_cols(pp.nblk);
     k_tdm_reduced<<<(n + rcols - 1) / rcols, RED_THREADS, red_smem_bytes(pp.nblk, rcols), c->stream>>>(
@@ -1995,39 +2226,41 @@ int launch_potential(eif_ctx *c, int rk, bool with_ibm) {
         k_tdm_local_df<4><<<g, tt, 0, c->stream>>>(qf, pp.tdm_inv_df, pp.tdm_up_df, iface, first, ldf, n, pp.nblk, c->ld);
       }
     } else if (pp.blk == 16) {
-      k_tdm_local<16><<<g, tt, 0, c->stream>>>(c->qhat, pp.tdm_inv, pp.tdm_up, iface, first, l, n, pp.nblk, c->ld);
+      k_tdm_local<16, false><<<g, tt, 0, c->stream>>>(c->qhat, pp.tdm_inv, pp.tdm_up, iface, first, l, n, pp.nblk, c->ld, 16);
     } else if (pp.blk == 8) {
-      k_tdm_local<8><<<g, tt, 0, c->stream>>>(c->qhat, pp.tdm_inv, pp.tdm_up, iface, first, l, n, pp.nblk, c->ld);
+      k_tdm_local<8, false><<<g, tt, 0, c->stream>>>(c->qhat, pp.tdm_inv, pp.tdm_up, iface, first, l, n, pp.nblk, c->ld, 8);
     } else {
-      k_tdm_local<4><<<g, tt, 0, c->stream>>>(c->qhat, pp.tdm_inv, pp.tdm_up, iface, first, l, n, pp.nblk, c->ld);
+      k_tdm_local<4, false><<<g, tt, 0, c->stream>>>(c->qhat, pp.tdm_inv, pp.tdm_up, iface, first, l, n, pp.nblk, c->ld, 4);
     }
     EIF_LAUNCH_CK(c);
-    if (pp.g2 > 0) {
-      const int Q = pp.q2;
-      const size_t sm = red2_smem_bytes(Q);
-      const dim3 grid((n + RED2_K - 1) / RED2_K);
-      if (pp.g2 == 16) {
-        k_tdm_reduced2<16><<<grid, RED2_K * Q, sm, c->stream>>>(iface, first, pp.red_coef, pp.r2_inv, pp.r2_up, pp.r2_phi,
-                                                            pp.r2_qinv, pp.r2_qup, pp.r2_q1, pp.r2_coef, l, n,
-                                                            pp.nblk, Q, nullptr);
-      } else if (pp.g2 == 8) {
-        k_tdm_reduced2<8><<<grid, RED2_K * Q, sm, c->stream>>>(iface, first, pp.red_coef, pp.r2_inv, pp.r2_up, pp.r2_phi,
-                                                           pp.r2_qinv, pp.r2_qup, pp.r2_q1, pp.r2_coef, l, n,
-                                                           pp.nblk, Q, nullptr);
-      } else {
-        k_tdm_reduced2<4><<<grid, RED2_K * Q, sm, c->stream>>>(iface, first, pp.red_coef, pp.r2_inv, pp.r2_up, pp.r2_phi,
-                                                           pp.r2_qinv, pp.r2_qup, pp.r2_q1, pp.r2_coef, l, n,
-                                                           pp.nblk, Q, nullptr);
-      }
+    int rc = reduced_solve(c, iface, first, nullptr);
+    if (rc) return rc;
+  } else if (pp.odd_blk > 0) {
+    EIF_PROF(c, "poisson_tdm", 3);
+    const int tt = 64;
+    dim3 g((n + tt - 1) / tt, pp.nblk);
+#define EIF_ODD_TDM(M)                                                                                                \
+  k_tdm_local<M, true><<<g, tt, 0, c->stream>>>(c->qhat, pp.tdm_inv, pp.tdm_up, iface, first, l, n, pp.nblk, c->ld,   \
+                                                pp.odd_len);                                                          \
+  EIF_LAUNCH_CK(c);                                                                                                   \
+  if (int rc = reduced_solve(c, iface, first, nullptr)) return rc;                                                    \
+  k_tdm_finish<M><<<g, tt, 0, c->stream>>>(c->qhat, iface, pp.tdm_g, pp.tdm_gl, n, pp.nblk, c->ld, pp.odd_len)
+    if (pp.odd_blk == 16) {
+      EIF_ODD_TDM(16);
+    } else if (pp.odd_blk == 8) {
+      EIF_ODD_TDM(8);
     } else {
-      const int rcols = red_cols(pp.nblk);
-      k_tdm_reduced<<<(n + rcols - 1) / rcols, RED_THREADS, red_smem_bytes(pp.nblk, rcols), c->stream>>>(
-          iface, first, pp.red_inv, pp.red_up, pp.red_q1, pp.red_coef, l, n, pp.nblk, rcols, nullptr);
+      EIF_ODD_TDM(4);
     }
+#undef EIF_ODD_TDM
     EIF_LAUNCH_CK(c);
   } else {
-    EIF_PROF(c, "poisson_tdm", 1);
-    k_tdm_serial<<<(n + 63) / 64, 64, 0, c->stream>>>(c->qhat, pp.ywork, pp.lam, l, n, jt, c->ld);
+    EIF_PROF(c, "poisson_tdm", 2);
+    k_tdm_serial<<<(n + 31) / 32, 32, 0, c->stream>>>(c->qhat, pp.ywork, pp.ser_up, pp.ser_q1, pp.ser_den, pp.ser_last,
+                                                      pp.lam, l, n, jt, c->ld);
+    EIF_LAUNCH_CK(c);
+    k_tdm_serial_last<<<dim3((n + 127) / 128, std::min(jt - 1, 512)), 128, 0, c->stream>>>(c->qhat, pp.ser_q1,
+                                                                                          pp.ser_last, n, jt, c->ld);
     EIF_LAUNCH_CK(c);
   }
   if (mixed) {
