@@ -7,6 +7,7 @@
 #include <cstdlib>
 #include <cmath>
 #include <new>
+#include <algorithm>
 #include <vector>
 
 namespace eif {
@@ -593,7 +594,8 @@ int eif_push_particles(eif_ctx *c, int n, const double *rec) {
   // The IBM buffers, and the step graphs that hold them, are kept when the particle
   // count is unchanged and the buffers already cover the pushed radii (a driver that
   // re-pushes the state every step); otherwise they are rebuilt.
-  const size_t chunks = ibm_tasks_needed(c, rec, n);
+  size_t most = 0;
+  const size_t chunks = ibm_tasks_needed(c, rec, n, &most);
   const bool reuse = c->P && n == c->np && n <= c->pcap && (n == 0 || (c->box && chunks <= (size_t)c->chunk_cap));
   if (!reuse) {
     graphs_free(c);
@@ -616,7 +618,12 @@ int eif_push_particles(eif_ctx *c, int n, const double *rec) {
     EIF_CK(c, cudaMemcpy(c->P, soa.data(), sizeof(double) * soa.size(), cudaMemcpyHostToDevice));
   }
   c->np = n;
-  return reuse ? EIF_OK : ibm_reserve(c, chunks);
+  c->max_tasks = (int)std::min<size_t>(most, 1u << 30);
+  if (!reuse) {
+    int rc = ibm_reserve(c, chunks);
+    if (rc) return rc;
+  }
+  return ibm_task_bases(c);
 }
 
 int eif_pull_particles(eif_ctx *c, int n, double *rec) {

@@ -105,6 +105,7 @@ struct PoissonPlan {
 struct Adjoint;  // adjoint.cu
 struct Snapshot;  // snapshot.cu
 struct Stats;     // stats.cu
+struct SubiterPlan;  // subiter.cu
 }  // namespace eif
 
 struct eif_ctx {
@@ -176,6 +177,7 @@ struct eif_ctx {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int cur0 = -1, scur0 = -1, cur1 = 0, scur1 = 0;
+    eif::SubiterPlan *plan = nullptr;   // stage kernels of the sub-iteration loops
   } graphs[2];
   bool use_graphs = true;
   // tile shapes of the stencil and block-Thomas kernels, chosen once per grid size by the
@@ -212,6 +214,10 @@ struct eif_ctx {
   // immersed-boundary work
   int *box;                     // per particle: 3 images x {imin,imax,jmin,jmax}
   int *chunk_off;               // per particle: first chunk (exclusive scan), [np] = total
+  // first task slots that hold for any position of the particles (sums of the bounds from the
+  // radii), and the largest bound of one particle
+  int *task_base = nullptr;
+  int max_tasks = 0;
   double *partial;              // per chunk: 3 partial sums
   double *wbuf;                 // per box cell: dux, duy contribution
   size_t wcap;                  // capacity of wbuf in cells
@@ -276,18 +282,21 @@ int check_records(eif_ctx *c);
 // ---- step graphs (graph.cu) ----
 int step_graph_launch(eif_ctx *c);
 void graphs_free(eif_ctx *c);
-int capture_step(eif_ctx *c, cudaGraph_t g, int *cur1, int *scur1);
+struct SubiterPlan;
+// plan: where set and the context is subiter_alone, the sub-iteration loops are stage kernels
+// of the plan it receives, conditional nodes otherwise
+int capture_step(eif_ctx *c, cudaGraph_t g, int *cur1, int *scur1, SubiterPlan **plan);
 int step_capture_begin(eif_ctx *c);
 void step_capture_end(eif_ctx *c, int cur0, int scur0);
 int capture_step_part(eif_ctx *c, cudaGraph_t g, const std::vector<cudaGraphNode_t> &deps, int part,
-                      std::vector<cudaGraphNode_t> *sinks, bool particles_in_stage_kernel = false);
+                      std::vector<cudaGraphNode_t> *sinks, bool particles_in_stage_kernel, bool fields_event);
 int capture_subiteration_loop(eif_ctx *c, cudaGraph_t g, const std::vector<cudaGraphNode_t> &deps, int rk,
                               std::vector<cudaGraphNode_t> *sinks);
 
-// ---- sub-iterations of many suspensions in one persistent kernel per stage (subiter.cu) ----
-struct SubiterPlan;
+// ---- sub-iterations in one persistent kernel per stage (subiter.cu) ----
 constexpr size_t SUBITER_MAX = 1024;   // suspensions per stage kernel
 bool subiter_joinable(const eif_ctx *c);
+bool subiter_alone(const eif_ctx *c);
 int subiter_plan_create(eif_ctx *const *ctx, int n, SubiterPlan **out, std::string *err);
 void subiter_plan_destroy(SubiterPlan *p);
 // the descriptor of suspension j (context c) in RK stage rk, from the state of c after
@@ -337,7 +346,8 @@ int launch_potential(eif_ctx *c, int rk, bool with_ibm);
 int launch_psi_to_double(eif_ctx *c, double *dst);
 
 // ---- immersed boundary (ibm.cu) ----
-size_t ibm_tasks_needed(const eif_ctx *c, const double *rec, int n);
+size_t ibm_tasks_needed(const eif_ctx *c, const double *rec, int n, size_t *most);
+int ibm_task_bases(eif_ctx *c);
 int ibm_reserve(eif_ctx *c, size_t chunks);
 void ibm_free(eif_ctx *c);
 int launch_inertia(eif_ctx *c, int cn);

@@ -1,21 +1,21 @@
 // Step graphs: one time step of eif_advance as a single CUDA graph.
 //
 // The graph holds, in launch order, the dt decision and for each RK stage the
-// stage kernels, a conditional WHILE node whose body is one particle
-// sub-iteration (inertia at the increment, collisions, increments), and the
-// particle update (src/main.c:13-53). Work that the stage driver puts on the side
-// stream is captured as a parallel branch of the same graph. The last block of
-// k_increment sets the loop condition on the device from the residual and the
-// sub-iteration count, so a step needs
+// stage kernels and one persistent kernel for its particle sub-iterations and the
+// particle update (subiter.cu; src/main.c:13-53). Work that the stage driver puts on the side
+// stream is captured as a parallel branch of the same graph. A step needs
 // no host round trip; the host synchronises once per step to read dt and the
-// error flags. The kernels and their order are those of the host-driven path
-// (rk_stage), so both paths give bit-identical results.
+// error flags. The kernels' bodies and their order are those of the host-driven path
+// (rk_stage), so both paths give bit-identical results. Contexts of many particles
+// (subiter_alone) have a conditional WHILE node per stage whose body is one
+// sub-iteration; the last block of k_increment sets its condition.
 //
 // The stage kernels swap the double-buffered velocity and source arrays, so the
 // buffers a step touches depend on the buffer indices at its start; one graph
 // is kept per starting pair of indices (at most two occur). Graphs are rebuilt
 // after the particle buffers are reallocated.
 #include "eif_internal.cuh"
+#include <string>
 #include <vector>
 
 namespace eif {
@@ -83,12 +83,12 @@ void step_capture_end(eif_ctx *c, int cur0, int scur0) {
 // and the front of RK stage 0 (src/main.c:14-35), parts 1 and 2 the particle update
 // of the stage before (main.c:51-53) and the front of the next stage, part 3 the
 // particle update of stage 2. The sub-iteration loops (main.c:36-50) go between the
-// parts: a conditional node per context (capture_subiteration_loop), or one kernel for
-// all the suspensions of a batch, which then also updates the particles at the end of the
+// parts: a conditional node per context (capture_subiteration_loop), or one kernel (for
+// all the suspensions of a batch), which then also updates the particles at the end of the
 // stage and resets the increments for the next (particles_in_stage_kernel: those launches
-// are left out of parts 1-3).
+// are left out of parts 1-3). fields_event: ev_fields is recorded once the fields are final.
 int capture_step_part(eif_ctx *c, cudaGraph_t g, const std::vector<cudaGraphNode_t> &deps, int part,
-                      std::vector<cudaGraphNode_t> *sinks, bool particles_in_stage_kernel) {
+                      std::vector<cudaGraphNode_t> *sinks, bool particles_in_stage_kernel, bool fields_event) {
   cudaError_t e = cudaStreamBeginCaptureToGraph(c->stream, g, deps.data(), nullptr, deps.size(),
                                                 cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return check_cuda(c, e, "cudaStreamBeginCaptureToGraph");
@@ -110,7 +110,7 @@ int capture_step_part(eif_ctx *c, cudaGraph_t g, const std::vector<cudaGraphNode
     c->reset_in_stage_kernel = false;
     if (rc) return rc;
   }
-  if (part == 2 && !particles_in_stage_kernel && c->ev_fields) {
+  if (part == 2 && fields_event && c->ev_fields) {
     // the last stage's projection is done: the fields are final for this step
     // (eif_advance_pull copies them to the host beside the particle work that follows)
     const cudaError_t e = cudaEventRecordWithFlags(c->ev_fields, c->stream, cudaEventRecordExternal);
@@ -121,7 +121,8 @@ int capture_step_part(eif_ctx *c, cudaGraph_t g, const std::vector<cudaGraphNode
 
 // The sub-iteration loop of RK stage rk of c as a conditional WHILE node after the
 // nodes deps (its counter reset before it); sinks = {the loop node}. The last block
-// of k_increment sets the loop condition on the device.
+// of k_increment sets the loop condition on the device. Without particles one
+// sub-iteration is all there is: no loop.
 int capture_subiteration_loop(eif_ctx *c, cudaGraph_t g, const std::vector<cudaGraphNode_t> &deps, int rk,
                               std::vector<cudaGraphNode_t> *sinks) {
   std::vector<cudaGraphNode_t> tail;
@@ -131,8 +132,12 @@ int capture_subiteration_loop(eif_ctx *c, cudaGraph_t g, const std::vector<cudaG
   // the sub-iteration counter starts at zero for every stage
   e = cudaMemsetAsync(reinterpret_cast<unsigned *>(c->d_inc + 1), 0, sizeof(unsigned), c->stream);
   if (e != cudaSuccess) return check_cuda(c, e, "cudaMemsetAsync");
-  int rc = end_capture(c, &tail);
-  if (rc) return rc;
+  int rc = c->np == 0 ? sub_iteration(c, rk) : EIF_OK;
+  if (rc || (rc = end_capture(c, &tail))) return rc;
+  if (c->np == 0) {
+    *sinks = tail;
+    return EIF_OK;
+  }
   cudaGraphConditionalHandle h;
   e = cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault);
   if (e != cudaSuccess) return check_cuda(c, e, "cudaGraphConditionalHandleCreate");
@@ -163,21 +168,42 @@ int capture_subiteration_loop(eif_ctx *c, cudaGraph_t g, const std::vector<cudaG
 // nodes have no dependences) and returns the buffer indices the step ends with. The
 // host state of c is left as before the capture; on failure g may hold a partial
 // branch and should be discarded.
-int capture_step(eif_ctx *c, cudaGraph_t g, int *cur1, int *scur1) {
+int capture_step(eif_ctx *c, cudaGraph_t g, int *cur1, int *scur1, SubiterPlan **plan) {
   int rc = step_capture_begin(c);
   if (rc) return rc;
   const int cur0 = c->cur, scur0 = c->scur;
+  const bool stage_kernels = plan && subiter_alone(c);
+  SubiterPlan *p = nullptr;
+  std::string err;
   std::vector<cudaGraphNode_t> tail;
+  cudaGraphNode_t reset = nullptr;
+  auto failed = [&](int code, bool stage) {
+    subiter_plan_destroy(p);
+    step_capture_end(c, cur0, scur0);
+    return stage ? fail(c, code, "stage kernel: %s", err.c_str()) : code;
+  };
+  if (stage_kernels) {
+    if ((rc = subiter_plan_create(&c, 1, &p, &err)) || (rc = subiter_add_reset(p, g, &reset, &err)))
+      return failed(rc, true);
+  }
   for (int part = 0; part < 4; part++) {
-    if ((rc = capture_step_part(c, g, tail, part, &tail)) ||
-        (part < 3 && (rc = capture_subiteration_loop(c, g, tail, part, &tail)))) {
-      step_capture_end(c, cur0, scur0);
-      return rc;
+    if ((rc = capture_step_part(c, g, tail, part, &tail, stage_kernels, true))) return failed(rc, false);
+    if (part == 3) break;
+    if (stage_kernels) {
+      subiter_describe(p, part, 0, c);
+      if (part == 0) tail.push_back(reset);
+      cudaGraphNode_t node = nullptr;
+      if ((rc = subiter_add_stage(p, part, g, tail, &node, &err))) return failed(rc, true);
+      tail.assign(1, node);
+    } else if ((rc = capture_subiteration_loop(c, g, tail, part, &tail))) {
+      return failed(rc, false);
     }
   }
+  if (stage_kernels && (rc = subiter_upload(p, &err))) return failed(rc, true);
   *cur1 = c->cur;
   *scur1 = c->scur;
   step_capture_end(c, cur0, scur0);
+  if (plan) *plan = p;
   return EIF_OK;
 }
 
@@ -187,7 +213,8 @@ int build(eif_ctx *c, eif_ctx::StepGraph &sg) {
   cudaGraph_t g = nullptr;
   EIF_CK(c, cudaGraphCreate(&g, 0));
   int cur1 = 0, scur1 = 0;
-  int rc = capture_step(c, g, &cur1, &scur1);
+  SubiterPlan *plan = nullptr;
+  int rc = capture_step(c, g, &cur1, &scur1, &plan);
   if (rc) {
     cudaGraphDestroy(g);
     return rc;
@@ -196,10 +223,12 @@ int build(eif_ctx *c, eif_ctx::StepGraph &sg) {
   const cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
   if (e != cudaSuccess) {
     cudaGraphDestroy(g);
+    subiter_plan_destroy(plan);
     return check_cuda(c, e, "cudaGraphInstantiate");
   }
   sg.graph = g;
   sg.exec = exec;
+  sg.plan = plan;
   sg.cur0 = c->cur;
   sg.scur0 = c->scur;
   sg.cur1 = cur1;
@@ -213,6 +242,7 @@ void graphs_free(eif_ctx *c) {
   for (auto &sg : c->graphs) {
     if (sg.exec) cudaGraphExecDestroy(sg.exec);
     if (sg.graph) cudaGraphDestroy(sg.graph);
+    subiter_plan_destroy(sg.plan);
     sg = eif_ctx::StepGraph{};
   }
 }

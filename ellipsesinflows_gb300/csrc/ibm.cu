@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(256, 3) k_ibm_work(WorkArgs a) {
   __shared__ double2 slot_buf[8][WORK_SLOTS];
   const int wmode = a.iter ? (*a.iter == 0u ? 2 : 0) : a.wmode;
   ibm_work_tasks<false>(a, wmode, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
-                        slot_buf[threadIdx.x >> 5]);
+                        slot_buf[threadIdx.x >> 5], nullptr);
 }
 
 __global__ void __launch_bounds__(256, 3) k_ibm_work_f(WorkArgs a) {
@@ -75,12 +75,15 @@ __global__ void __launch_bounds__(256, 4) k_ibm_memo_f(WorkArgs a) {
 
 __global__ void __launch_bounds__(256, 4) k_ibm_sum_f(WorkArgs a) {
   if (a.gate && ((a.gate == 1) != (*a.iter == 0u))) return;
-  ibm_sum_f_tasks<true>(a, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5);
+  ibm_sum_f_tasks<true>(a, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
+                        EIF_CHK(a.bd.rec, a.np, a.bd.off, 70) ? __ldg(a.off + a.np) : 0);
 }
 
 __global__ void k_chunk_reduce(const double *__restrict__ partial, const int *__restrict__ off, double *__restrict__ P,
                                int pcap, int np, int f0, int f1, int f2, Bounds bd) {
-  chunk_reduce_warp(partial, off, P, pcap, np, f0, f1, f2, bd, (blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (n >= np || !EIF_CHK(bd.rec, n + 1, bd.off, 30)) return;
+  chunk_reduce_warp(partial, off[n], off[n + 1], P, pcap, f0, f1, f2, bd, n);
 }
 
 // save: after an indicator evaluation that stored its weights in the memo (with iter:
@@ -89,9 +92,10 @@ __global__ void k_chunk_reduce_f(const float *__restrict__ partial, const int *_
                                  int pcap, int np, int f0, int f1, int f2, Bounds bd, WeightMemo memo, int save,
                                  const unsigned *__restrict__ iter, const float *__restrict__ pf,
                                  const int *__restrict__ box) {
-  const bool s = save && (!iter || *iter != 0u);
-  chunk_reduce_f_warp(partial, off, P, pcap, np, f0, f1, f2, bd, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
-                      s ? &memo : nullptr, pf, box);
+  const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (n >= np || !EIF_CHK(bd.rec, n + 1, bd.off, 33)) return;
+  if (save && (!iter || *iter != 0u)) memo_particle(memo, pf + (size_t)PF_WORDS * n, box + 12 * (size_t)n, off[n], n);
+  chunk_reduce_f_warp(partial, off[n], off[n + 1], P, pcap, f0, f1, f2, bd, n);
 }
 
 // exclusive scan of the chunk counts (one block); off[np] = total
@@ -119,6 +123,45 @@ __global__ void k_scan(const int *__restrict__ cnt, int *__restrict__ off, int n
     __syncthreads();
   }
   if (threadIdx.x == 0 && EIF_CHK(bd.rec, np, bd.off, 6)) off[np] = carry;
+}
+
+// Bound on the box cells of one particle over its three images. A box spans at
+// most 2r/h + 2 + 2*NEXTRA + 1 cells per direction before clipping; the three
+// images are shifted by exactly jtot rows, so their clipped row ranges together
+// never exceed the unclipped height.
+__host__ __device__ inline size_t tasks_bound(double r, double dx, double dy, int itot, int jtot) {
+  const long w = (long)ceil(2. * r / dx) + 2 + 2 * NEXTRA + 2;
+  const long h = (long)ceil(2. * r / dy) + 2 + 2 * NEXTRA + 2;
+  const long wc = w < itot ? w : itot;
+  const long hc = h < 3L * jtot ? h : 3L * jtot;
+  return (size_t)hc * (size_t)box_segs((int)wc);
+}
+
+// exclusive sums of the bounds (one block of 1024): first task slots of the particles
+__global__ void __launch_bounds__(1024) k_task_bases(const double *__restrict__ P, int pcap, int np, double dx, double dy,
+                                                     int itot, int jtot, int *__restrict__ base) {
+  __shared__ int w[32];
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  int run = 0;
+  for (int n0 = 0; n0 < np; n0 += 1024) {
+    const int n = n0 + threadIdx.x;
+    const int v = n < np ? (int)tasks_bound(fmax(P[EIF_P_A * pcap + n], P[EIF_P_B * pcap + n]), dx, dy, itot, jtot) : 0;
+    int sc = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, sc, o);
+      if (lane >= o) sc += u;
+    }
+    if (lane == 31) w[wl] = sc;
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int q = 0; q < 32; q++) {
+      before += q < wl ? w[q] : 0;
+      all += w[q];
+    }
+    if (n < np) base[n] = run + before + sc - v;
+    run += all;
+    __syncthreads();
+  }
 }
 
 // The task table: one int4 per task (chunk) {particle, row, first column, last
@@ -326,16 +369,8 @@ __global__ void k_ibm_halo(T *__restrict__ dux, T *__restrict__ duy, int itot, i
 
 namespace eif {
 
-// Bound on the box cells of one particle over its three images. A box spans at
-// most 2r/h + 2 + 2*NEXTRA + 1 cells per direction before clipping; the three
-// images are shifted by exactly jtot rows, so their clipped row ranges together
-// never exceed the unclipped height.
 static size_t box_tasks_bound(const eif_ctx *c, double r) {
-  const long w = (long)std::ceil(2. * r / c->dx) + 2 + 2 * NEXTRA + 2;
-  const long h = (long)std::ceil(2. * r / c->dy) + 2 + 2 * NEXTRA + 2;
-  const long wc = std::min<long>(w, c->itot);
-  const long hc = std::min<long>(h, 3L * c->jtot);
-  return (size_t)hc * (size_t)box_segs((int)wc);
+  return tasks_bound(r, c->dx, c->dy, c->itot, c->jtot);
 }
 
 // resident CTAs per SM of the IBM work kernels (a host query; done before any graph capture)
@@ -350,13 +385,26 @@ int ibm_prepare(eif_ctx *c) {
   return EIF_OK;
 }
 
-// task bound of a particle set, from the radii in the host records (EIF_NFIELDS per particle)
-size_t ibm_tasks_needed(const eif_ctx *c, const double *rec, int n) {
+// task bound of a particle set, from the radii in the host records (EIF_NFIELDS per particle);
+// most: the largest of one particle
+size_t ibm_tasks_needed(const eif_ctx *c, const double *rec, int n, size_t *most) {
   size_t chunks = 0;
+  *most = 0;
   for (int k = 0; k < n; k++) {
-    chunks += box_tasks_bound(c, std::max(rec[(size_t)k * EIF_NFIELDS + EIF_P_A], rec[(size_t)k * EIF_NFIELDS + EIF_P_B]));
+    const size_t b =
+        box_tasks_bound(c, std::max(rec[(size_t)k * EIF_NFIELDS + EIF_P_A], rec[(size_t)k * EIF_NFIELDS + EIF_P_B]));
+    chunks += b;
+    *most = std::max(*most, b);
   }
   return chunks;
+}
+
+// the first task slots of the pushed particles (box_tasks_bound summed on the device)
+int ibm_task_bases(eif_ctx *c) {
+  if (c->np == 0) return EIF_OK;
+  k_task_bases<<<1, 1024, 0, c->stream>>>(c->P, c->pcap, c->np, c->dx, c->dy, c->itot, c->jtot, c->task_base);
+  EIF_LAUNCH_CK(c);
+  return EIF_OK;
 }
 
 int ibm_reserve(eif_ctx *c, size_t chunks) {
@@ -367,6 +415,7 @@ int ibm_reserve(eif_ctx *c, size_t chunks) {
   c->wcap = chunks * CHUNK;
   EIF_CK(c, cudaMalloc((void **)&c->box, sizeof(int) * 12 * c->np));
   EIF_CK(c, cudaMalloc((void **)&c->chunk_off, sizeof(int) * 2 * (c->np + 1)));
+  EIF_CK(c, cudaMalloc((void **)&c->task_base, sizeof(int) * c->np));
   EIF_CK(c, cudaMalloc((void **)&c->partial, sizeof(double) * 3 * chunks));
   EIF_CK(c, cudaMalloc((void **)&c->wbuf, sizeof(double2) * c->wcap));
   EIF_CK(c, cudaMalloc((void **)&c->wcache, sizeof(double) * c->wcap));
@@ -403,6 +452,8 @@ int ibm_reserve(eif_ctx *c, size_t chunks) {
 void ibm_free(eif_ctx *c) {
   if (c->box) cudaFree(c->box);
   if (c->chunk_off) cudaFree(c->chunk_off);
+  if (c->task_base) cudaFree(c->task_base);
+  c->task_base = nullptr;
   if (c->partial) cudaFree(c->partial);
   if (c->wbuf) cudaFree(c->wbuf);
   if (c->wcache) cudaFree(c->wcache);

@@ -414,6 +414,95 @@ __device__ __forceinline__ void box_part(const BoxArgs &a, int n, int sub) {
   if (on && tasks && EIF_CHK(a.bd.rec, (a.nchunk - a.bd_off_base) + n, a.bd.off, 3)) atomicAdd(a.nchunk + n, tasks);
 }
 
+// The same for one particle by one warp, into shared memory (bx: 12 ints, pf or pd: its
+// parameter block), at X + dX in a sub-iteration: the values of box_part bit for bit. An FP64
+// warp instruction holds the pipe 16 cycles whether one lane or all take part, so the divisions
+// (the boxes' bounds, the grid offsets, the quadratic form) are one division of 22 lanes; the
+// words that do not change within a stage are copied from the blocks at X. With a part of
+// box_part per warp, one lane each, this took ten times as long, most of a sub-iteration.
+__device__ __forceinline__ void box_warp(const BoxArgs &a, int n, int *bx, float *pf, double *pd) {
+  const double *P = a.P;
+  const int pc = a.pcap, lane = threadIdx.x & 31;
+  const double pa = P[EIF_P_A * pc + n], pb = P[EIF_P_B * pc + n];
+  const double px = P[EIF_P_X * pc + n] + P[EIF_P_DX * pc + n], py = P[EIF_P_Y * pc + n] + P[EIF_P_DY * pc + n];
+  const double az = P[EIF_P_AZ * pc + n] + P[EIF_P_DAZ * pc + n];
+  const double r = fmax(pa, pb);
+  double sz, cz;
+  sincos(-az, &sz, &cz);
+  double num = 1., den = 1.;
+  if (lane < 12) {
+    // image lane / 4 - 1: imin, imax, jmin, jmax (loop_size)
+    const bool row = lane & 2;
+    const double gc = row ? py + a.ly * (double)(lane / 4 - 1) - a.yf1 : px;
+    num = lane & 1 ? gc + r : gc - r;
+    den = row ? a.dy : a.dx;
+  } else if (lane < 16) {
+    num = lane == 12 ? px : py + a.ly * (double)(lane - 14);
+    den = lane == 12 ? a.dx : a.dy;
+  } else if (lane < 22) {
+    const int k = lane - 16;
+    num = k == 0 || k == 3 ? cz * cz : (k < 3 ? sz * sz : 1.);
+    den = k == 0 || k == 2 || k == 5 ? pa * pa : pb * pb;
+  }
+  const double v = num / den;
+  if (lane < 12) {
+    const int lb = 1, ub = lane & 2 ? a.jtot : a.itot;
+    int w;
+    if (lane & 1) {
+      w = (int)(ceil(v) + NEXTRA);
+      w = w > ub ? ub : w;
+    } else {
+      w = (int)(floor(v) - NEXTRA);
+      w = w < lb ? lb : w;
+    }
+    bx[lane] = w;
+  }
+  if (pf) {
+    const float *c = a.pf + (size_t)PF_WORDS * n;
+    constexpr unsigned keep = 1u << PF_A | 1u << PF_B | 1u << PF_KEX | 1u << PF_KEY | 1u << PF_RPM | 1u << PF_RPIM |
+                              1u << PF_UX | 1u << PF_UY | 1u << PF_VZ | 1u << PF_SO2 | 1u << PF_SI2 | 1u << PF_RO2;
+    if ((keep >> lane) & 1u) pf[lane] = c[lane];
+    const double v1 = __shfl_down_sync(0xffffffffu, v, 1);
+    if (lane == 0) {
+      pf[PF_CZ] = (float)cz;
+      pf[PF_SZ] = (float)sz;
+    }
+    if (lane >= 12 && lane < 16) {
+      const int i0 = (int)floor(v);
+      pf[lane == 12 ? PF_I0 : PF_J0 + (lane - 13)] = __int_as_float(i0);
+      pf[lane == 12 ? PF_GX : PF_GY + (lane - 13)] = (float)(v - i0 + 0.5);
+    }
+    if (lane == 16) pf[PF_AL] = (float)(v + v1);
+    if (lane == 18) pf[PF_DE] = (float)(v + v1);
+    if (lane == 20) pf[PF_KA] = (float)(cz * sz * (v - v1));
+  } else {
+    const double *c = a.pd + (size_t)PD_WORDS * n;
+    // everything but the first words and those of the quadratic form
+    if (lane >= PD_A && lane < PD_F) pd[lane] = c[lane];
+    float *df = reinterpret_cast<float *>(pd + PD_F);
+    if (lane >= PDF_SO2 && lane < PDF_WORDS) df[lane] = reinterpret_cast<const float *>(c + PD_F)[lane];
+    if (lane == 0) {
+      pd[PD_X] = px;
+      pd[PD_Y] = py;
+      pd[PD_CZ] = cz * a.kb;
+      pd[PD_SZ] = sz * a.kb;
+      const float fa = eifd::d2f(pa), fb = eifd::d2f(pb), cf = eifd::d2f(cz), sf = eifd::d2f(sz);
+      df[PDF_AL] = cf * cf / (fa * fa) + sf * sf / (fb * fb);
+      df[PDF_KA] = cf * sf * (1.f / (fb * fb) - 1.f / (fa * fa));
+      df[PDF_DE] = sf * sf / (fa * fa) + cf * cf / (fb * fb);
+    }
+  }
+}
+__device__ __forceinline__ int box_tasks(const int *bx) {
+  int t = 0;
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    const int w = bx[4 * q + 1] - bx[4 * q] + 1, h = bx[4 * q + 3] - bx[4 * q + 2] + 1;
+    if (w > 0 && h > 0) t += h * box_segs(w);
+  }
+  return t;
+}
+
 // A particle's tasks: image by image, row by row, segment by segment.
 struct RowTask {
   int img, j, ib, ie;   // image -1..1, row, first and last column of the segment
@@ -580,6 +669,22 @@ struct WorkArgs {
   Bounds bd;
 };
 
+// The tasks of one particle for the persistent sub-iteration kernel, which forms the boxes and
+// parameters of the particle at hand in shared memory instead of tables over all particles:
+// tasks r = 0 .. of the boxes, numbered base + r in the scratch buffers. box null: the tasks of
+// the table up to number `total`.
+struct OneParticle {
+  const int4 *box;      // the three images' boxes, or null
+  const float *pf;
+  const double *pd;
+  int n, base, total;
+};
+__device__ __forceinline__ int4 task_desc(const OneParticle &o, int r) {
+  RowTask t;
+  return row_task(o.box[0], o.box[1], o.box[2], r, t) ? make_int4(o.n, t.j, t.ib, t.ie * 4 + t.img + 1)
+                                                      : make_int4(-1, 0, 0, 0);
+}
+
 // Sums of three values over the warp, in 6 additions instead of 15: in each of the first
 // two steps the two halves of a group of lanes keep different values. The additions pair the
 // same lanes as warp_sum's. The sums are in lane 0 (v0), 16 (v1) and 8 (v2).
@@ -605,9 +710,11 @@ __device__ __forceinline__ double warp_sum3(double v0, double v1, double v2, int
 // stand-alone kernel.
 constexpr int WORK_SLOTS = CHUNK + CHUNK / (int)sizeof(double2);   // double2 entries per warp
 template <bool NC>
-__device__ __noinline__ void ibm_work_tasks(const WorkArgs &a, int wmode, int first, int stride, double2 *slots) {
+__device__ __noinline__ void ibm_work_tasks(const WorkArgs &a, int wmode, int first, int stride, double2 *slots,
+                                            const OneParticle *one) {
   const int lane = threadIdx.x & 31;
-  const int total = EIF_CHK(a.bd.rec, a.np, a.bd.off, 10) ? ldro<NC>(a.off + a.np) : 0;
+  const int total = one ? one->total : (EIF_CHK(a.bd.rec, a.np, a.bd.off, 10) ? ldro<NC>(a.off + a.np) : 0);
+  const bool own = one && one->box;
   const double dxdy = a.dx * a.dy;
   // factors of the sums: inertia.c:51-59 with 1/2 (1 + th) and the two face averages,
   // exchange.c:61-76
@@ -615,15 +722,16 @@ __device__ __noinline__ void ibm_work_tasks(const WorkArgs &a, int wmode, int fi
   const int pc = a.pcap, ld = a.ld;
   double *wcache = static_cast<double *>(a.wcache);
   unsigned char *list = reinterpret_cast<unsigned char *>(slots + CHUNK);   // the cells of pass 3
-  for (int c = first; c < total; c += stride) {
+  for (int k = first; k < total; k += stride) {
+    const int c = own ? one->base + k : k;
     if (!EIF_CHK(a.bd.rec, c, a.bd.partial / 3, 21)) continue;
-    const int4 dsc = ldro<NC>(a.tdesc + c);
+    const int4 dsc = own ? task_desc(*one, k) : ldro<NC>(a.tdesc + c);
     const int n = dsc.x;
     if (!EIF_CHK(a.bd.rec, n, a.np, 11)) continue;
     if (!EIF_CHK(a.bd.rec, EIF_P_VZ * pc + n, a.bd.P, 13)) continue;
     RowTask t;
     const bool task = task_of(dsc, a.np, t) && EIF_CHK(a.bd.rec, t.j, a.bd.yc - 1, 15);
-    const double *pd = a.pd + (size_t)PD_WORDS * n;
+    const double *pd = own ? one->pd : a.pd + (size_t)PD_WORDS * n;
     const float *pdf = reinterpret_cast<const float *>(pd + PD_F);
     const int img = task ? t.img : 0;
     const double px = ldro<NC>(pd + PD_X), py_ = ldro<NC>(pd + PD_Y) + (img == 0 ? 0. : (img > 0 ? a.ly : -a.ly));
@@ -822,14 +930,20 @@ __device__ __forceinline__ void inertia_cell_f(float th, float X, float Y, float
   s2 = __fmaf_rn(__fmaf_rn(X, valy, __fmul_rn(-Y, valx)), rpim, s2);
 }
 
-// one warp per row task, single precision (see ibm_work_tasks)
-template <bool NC>
-__device__ __forceinline__ void ibm_work_f_tasks(const WorkArgs &a, int wmode, int first, int stride, float2 *slots) {
+// one warp per row task, single precision (see ibm_work_tasks); ONE: the tasks of one particle
+template <bool NC, bool ONE = false>
+__device__ __forceinline__ void ibm_work_f_tasks(const WorkArgs &a, int wmode, int first, int stride, float2 *slots,
+                                                 const OneParticle *one = nullptr) {
   const int lane = threadIdx.x & 31;
   // all tasks, or (with a.only) the listed ones: task number c of list entry k
-  const int total = a.only ? (int)min((long long)ldro<NC>(a.only), (long long)(a.bd.partial / 3))
-                           : (EIF_CHK(a.bd.rec, a.np, a.bd.off, 50) ? ldro<NC>(a.off + a.np) : 0);
-  auto task_no = [&](int k) { return a.only ? ldro<NC>(a.only + 1 + k) : k; };
+  const int total = ONE ? one->total
+                        : (a.only ? (int)min((long long)ldro<NC>(a.only), (long long)(a.bd.partial / 3))
+                                  : (EIF_CHK(a.bd.rec, a.np, a.bd.off, 50) ? ldro<NC>(a.off + a.np) : 0));
+  auto task_no = [&](int k) { return ONE ? one->base + k : (a.only ? ldro<NC>(a.only + 1 + k) : k); };
+  auto desc = [&](int k, int c) {
+    if constexpr (ONE) return task_desc(*one, k);
+    else return ldro<NC>(a.tdesc + c);
+  };
   const float rh = a.rh_f, dxf = a.dx_f, dyf = a.dy_f, dxdy = a.dxdy_f;
   const float rdtv = a.mode == 1 ? __ldg(a.coef + 9) : 0.f;
   const int ld = a.ld;
@@ -839,20 +953,20 @@ __device__ __forceinline__ void ibm_work_f_tasks(const WorkArgs &a, int wmode, i
   int4 nxt = make_int4(-1, 0, 0, 0);
   if (first < total) {
     const int cf = task_no(first);
-    if (EIF_CHK(a.bd.rec, cf, a.bd.partial / 3, 51)) nxt = ldro<NC>(a.tdesc + cf);
+    if (EIF_CHK(a.bd.rec, cf, a.bd.partial / 3, 51)) nxt = desc(first, cf);
   }
   for (int k = first; k < total; k += stride) {
     const int c = task_no(k);
     const int4 dsc = nxt;
     if (k + stride < total) {
       const int cn = task_no(k + stride);
-      if (EIF_CHK(a.bd.rec, cn, a.bd.partial / 3, 51)) nxt = ldro<NC>(a.tdesc + cn);
+      if (EIF_CHK(a.bd.rec, cn, a.bd.partial / 3, 51)) nxt = desc(k + stride, cn);
     }
     const int n = dsc.x;
     if (!EIF_CHK(a.bd.rec, n, a.np, 52)) continue;
     RowTask t;
     const bool task = task_of(dsc, a.np, t);
-    const float4 *q4 = reinterpret_cast<const float4 *>(a.pf + (size_t)PF_WORDS * n);
+    const float4 *q4 = reinterpret_cast<const float4 *>(ONE ? one->pf : a.pf + (size_t)PF_WORDS * n);
     const float4 qA = ldro<NC>(q4), qB = ldro<NC>(q4 + 1), qC = ldro<NC>(q4 + 2), qD = ldro<NC>(q4 + 3),
                  qE = ldro<NC>(q4 + 4);
     const float4 qF = ldro<NC>(q4 + 5), qG = ldro<NC>(q4 + 6);
@@ -1108,10 +1222,9 @@ __device__ __forceinline__ void ibm_memo_f_tasks(const WorkArgs &a, int first, i
 // few registers and many resident warps, which hide the latency of its loads.
 // The warp runs the tasks first, first + stride, ...
 template <bool NC>
-__device__ __forceinline__ void ibm_sum_f_tasks(const WorkArgs &a, int first, int stride) {
+__device__ __forceinline__ void ibm_sum_f_tasks(const WorkArgs &a, int first, int stride, int total) {
   const int lane = threadIdx.x & 31;
   const int warp = first, nwarps = stride;
-  const int total = EIF_CHK(a.bd.rec, a.np, a.bd.off, 70) ? ldro<NC>(a.off + a.np) : 0;
   const float dxf = a.dx_f, dyf = a.dy_f, dxdy = a.dxdy_f;
   const float rdtv = a.mode == 1 ? __ldg(a.coef + 9) : 0.f;
   const int ld = a.ld;
@@ -1219,13 +1332,10 @@ __device__ __forceinline__ void ibm_sum_f_tasks(const WorkArgs &a, int first, in
   }
 }
 
-// per-particle sums over chunks in a fixed order (one warp: particle n)
-__device__ __forceinline__ void chunk_reduce_warp(const double *partial, const int *off, double *P, int pcap, int np,
-                                                  int f0, int f1, int f2, const Bounds &bd, int n) {
+// sums of particle n over its chunks c0 .. c1 - 1 in a fixed order (one warp)
+__device__ __forceinline__ void chunk_reduce_warp(const double *partial, int c0, int c1, double *P, int pcap, int f0,
+                                                  int f1, int f2, const Bounds &bd, int n) {
   const int lane = threadIdx.x & 31;
-  if (n >= np) return;
-  if (!EIF_CHK(bd.rec, n + 1, bd.off, 30)) return;
-  const int c0 = off[n], c1 = off[n + 1];
   double s0 = 0., s1 = 0., s2 = 0.;
   for (int c = c0 + lane; c < c1; c += 32) {
     if (!EIF_CHK(bd.rec, 3LL * c + 2, bd.partial, 31)) break;
@@ -1247,27 +1357,9 @@ __device__ __forceinline__ void chunk_reduce_warp(const double *partial, const i
 // accumulated in double-float arithmetic (TwoSum) on the FP32 pipe: the sum of at most
 // a few hundred floats is kept to about 48 bits, and the result is rounded once to
 // double.
-// With memo set (after a sub-iteration's indicator evaluation that stored its weights in
-// it), the particle's geometry words, boxes and first task are copied to the memo.
-__device__ __forceinline__ void chunk_reduce_f_warp(const float *partial, const int *off, double *P, int pcap, int np,
-                                                    int f0, int f1, int f2, const Bounds &bd, int n,
-                                                    const WeightMemo *memo = nullptr, const float *pf = nullptr,
-                                                    const int *box = nullptr) {
+__device__ __forceinline__ void chunk_reduce_f_warp(const float *partial, int c0, int c1, double *P, int pcap, int f0,
+                                                    int f1, int f2, const Bounds &bd, int n) {
   const int lane = threadIdx.x & 31;
-  if (n >= np) return;
-  if (memo) {
-    if (lane < 20) {
-      const size_t q = (size_t)PF_WORDS * n + memo_word(lane);
-      memo->pf[q] = pf[q];
-    } else {
-      const size_t q = 12 * (size_t)n + (lane - 20);
-      memo->box[q] = box[q];
-    }
-    if (lane == 0) memo->off[n] = off[n];
-    if (lane == 0 && n == 0) *memo->valid = 1;
-  }
-  if (!EIF_CHK(bd.rec, n + 1, bd.off, 33)) return;
-  const int c0 = off[n], c1 = off[n + 1];
   float h[3] = {0.f, 0.f, 0.f}, l[3] = {0.f, 0.f, 0.f};
   for (int c = c0 + lane; c < c1; c += 32) {
     if (!EIF_CHK(bd.rec, 3LL * c + 2, 2 * bd.partial, 34)) break;
@@ -1294,6 +1386,16 @@ __device__ __forceinline__ void chunk_reduce_f_warp(const float *partial, const 
     P[f1 * pcap + n] = eifd::f2d(h[1]) + eifd::f2d(l[1]);
     P[f2 * pcap + n] = eifd::f2d(h[2]) + eifd::f2d(l[2]);
   }
+}
+
+// The geometry words (pf: PF_WORDS words), boxes (12 ints) and first task c0 of particle n to
+// the memo, after a sub-iteration's indicator evaluation that stored its weights there (one warp).
+__device__ __forceinline__ void memo_particle(const WeightMemo &memo, const float *pf, const int *box, int c0, int n) {
+  const int lane = threadIdx.x & 31;
+  if (lane < 20) memo.pf[(size_t)PF_WORDS * n + memo_word(lane)] = pf[memo_word(lane)];
+  else memo.box[12 * (size_t)n + (lane - 20)] = box[lane - 20];
+  if (lane == 0) memo.off[n] = c0;
+  if (lane == 0 && n == 0) *memo.valid = 1;
 }
 
 // ---- arguments of the box, table and task bodies from a context (host) ----

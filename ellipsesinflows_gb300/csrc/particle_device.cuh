@@ -19,7 +19,6 @@
 namespace {
 
 using eifd::pmass;
-using eifd::pmoi;
 
 // ellipse.c:30-65, for the few feet that foot_newton leaves
 __device__ __noinline__ double normal_t_d(double a, double b, double x_, double y_) {
@@ -60,25 +59,25 @@ __device__ __forceinline__ FitEllipse fit_ellipse(double a, double b, double x, 
   FitEllipse e;
   e.a = a; e.b = b; e.x = x; e.y = y;
   sincos(angle, &e.sp, &e.cp);
-  e.kex = a * fma(-(b / a), b / a, 1.);
-  e.key = b * fma(-(a / b), a / b, 1.);
-  e.rab = 1. / (a * b);
-  e.f.a = eifd::d2f(a); e.f.b = eifd::d2f(b); e.f.cz = 1.f; e.f.sz = 0.f;
+  const double ra = 1. / a, rb = 1. / b, d = (a - b) * (a + b);
+  e.kex = d * ra;      // a (1 - (b/a)^2)
+  e.key = -(d * rb);
+  e.rab = ra * rb;
+  e.f.a = eifd::d2f(a); e.f.b = eifd::d2f(b);
+  e.f.cz = eifd::d2f(d); e.f.sz = 0.f;   // a^2 - b^2 (the angle's words are not used here)
   e.f.kex = eifd::d2f(e.kex); e.f.key = eifd::d2f(e.key);
   return e;
 }
 
-// The foot of the normal from (px, py), first quadrant, as (c, s) = (cos t, sin t), by
-// Newton steps from the (c, s) given: with v = (px, py) - (a c, b s) and T the derivative of
-// the ellipse in t, the angle to the foot is v.T / K, K = T^2 + v.(a c, b s). Returns false
-// where K is small (next to the evolute) or the start is too far off.
+// The foot of the normal from (px, py), first quadrant, as (c, s) = (cos t, sin t), from the
+// (c, s) given: with v = (px, py) - (a c, b s) and T the derivative of the ellipse in t, the
+// angle to the foot solves g - K t + f t^2 / 2 = 0 up to third order, g = v.T, K = T^2 + v.(a c,
+// b s), f = -(g + 3 (a^2 - b^2) c s): t = g / K to double precision and the quadratic term, which
+// needs no more than single precision. Below FIT_STEP what is left out is below 1e-16. Returns
+// false where K is small (next to the evolute) or the start is too far off.
+constexpr double FIT_STEP = 4.e-6;
 __device__ __forceinline__ bool foot_newton(const FitEllipse &e, double px, double py, double &c, double &s) {
   for (int n = 0; n < 8; n++) {
-    // back onto the unit circle
-    double dn = fma(c, c, fma(s, s, -1.));
-    double h = fma(dn, fma(dn, 0.375, -0.5), 1.);
-    c *= h;
-    s *= h;
     const double ac = e.a * c, bs = e.b * s, as = e.a * s, bc = e.b * c;
     const double vx = px - ac, vy = py - bs;
     const double g = fma(vy, bc, -(vx * as));
@@ -87,35 +86,35 @@ __device__ __forceinline__ bool foot_newton(const FitEllipse &e, double px, doub
     const float Kf = eifd::d2f(K);
     if (!(Kf > 0.02f * eifd::d2f(w2))) return false;
     // g / K from a single-precision reciprocal and one Newton step
-    const double r = eifd::f2d(__fdividef(1.f, Kf)), gr = g * r;
+    const float rf = __fdividef(1.f, Kf);
+    const double r = eifd::f2d(rf), gr = g * r;
     const double d = fma(gr, fma(-K, r, 1.), gr);
     if (!(fabs(d) < 0.1)) return false;
-    h = fma(d, -0.5 * d, 1.);
-    const double c1 = fmax(fma(-d, s, c * h), 0.);
-    s = fmax(fma(d, c, s * h), 0.);
-    c = c1;
-    if (fabs(d) < 2.e-8) {   // the next step would be below 1e-15
-      dn = fma(c, c, fma(s, s, -1.));
-      h = fma(dn, -0.5, 1.);
-      c *= h;
-      s *= h;
-      return true;
-    }
+    const float df = eifd::d2f(d), f3 = __fmul_rn(3.f * e.f.cz, __fmul_rn(eifd::d2f(c), eifd::d2f(s)));
+    const float q = __fmul_rn(__fmul_rn(0.5f * rf, __fadd_rn(eifd::d2f(g), f3)), __fmul_rn(df, df));
+    const double t = d - eifd::f2d(q);
+    const double h = fma(t, -0.5 * t, 1.);
+    const double c1 = fmax(fma(-t, s, c * h), 0.), s1 = fmax(fma(t, c, s * h), 0.);
+    // back onto the unit circle: the step leaves t^4 / 4, a start from single precision 1e-7
+    const double dn = fma(c1, c1, fma(s1, s1, -1.));
+    const double u = fma(dn, fma(dn, 0.375, -0.5), 1.);
+    c = c1 * u;
+    s = s1 * u;
+    if (fabs(d) < FIT_STEP) return true;
   }
   return false;
 }
 
-// compute_evolute, collision.c:75-109: the centre (ex, ey) and the radius r of the circle of
-// curvature at the foot of (x, y), and the foot's offset (ix, iy) from the ellipse's centre;
-// (c, s): the foot of the fit's last iteration on entry (first: none yet), this one's on
-// return. A serial chain of FP64 operations, of about 25 ns each here: the foot is iterated
-// on (cos t, sin t), from the last foot or the one that single precision finds, so that
-// nothing but a square root is left of ellipse.c's sincos, asin, divisions and the curvature's
-// pow, and evaluated to the same accuracy (the foot to 1e-15 and better, where ellipse.c
-// stops once the step is below 1e-8). Every product-sum is an explicit fma: the same bits in
-// whatever kernel this is compiled.
+// compute_evolute, collision.c:75-109: the centre (ex, ey) of the circle of curvature at the
+// foot of (x, y). (c, s), both signs positive: the foot of the fit's last iteration on entry
+// (first: none yet), this one's on return; cs, ss: with its signs. A serial chain of FP64
+// operations, of about 25 ns each here: the foot is iterated on (cos t, sin t), from the last
+// foot or the one that single precision finds, so that nothing is left of ellipse.c's sincos,
+// asin, square roots and divisions, and evaluated to the same accuracy (the foot to 1e-15 and
+// better, where ellipse.c stops once the step is below 1e-8). Every product-sum is an explicit
+// fma: the same bits in whatever kernel this is compiled.
 __device__ __forceinline__ void evolute(const FitEllipse &e, bool first, double x, double y, double &c, double &s,
-                                        double &ex, double &ey, double &ix, double &iy, double &r) {
+                                        double &cs, double &ss, double &ex, double &ey) {
   const double X = x - e.x, Y = y - e.y;
   const double x_ = fma(e.cp, X, e.sp * Y), y_ = fma(e.cp, Y, -(e.sp * X));
   const double px = fabs(x_), py = fabs(y_);
@@ -126,31 +125,49 @@ __device__ __forceinline__ void evolute(const FitEllipse &e, bool first, double 
     s = eifd::f2d(sf);
     if (!foot_newton(e, px, py, c, s)) sincos(normal_t_d(e.a, e.b, px, py), &s, &c);
   }
-  const double cs = x_ < 0. ? -c : c, ss = y_ < 0. ? -s : s;
-  const double as = e.a * s, bc = e.b * c;
-  const double w2 = fma(as, as, bc * bc);
-  r = fmin(w2 * sqrt(w2) * e.rab, 1. / DBL_EPSILON);   // ellipse.c:17-28
+  cs = x_ < 0. ? -c : c;
+  ss = y_ < 0. ? -s : s;
   const double vx = e.kex * (cs * cs * cs), vy = e.key * (ss * ss * ss);
-  ex = fma(e.cp, vx, -(e.sp * vy)) + e.x;
-  ey = fma(e.sp, vx, e.cp * vy) + e.y;
+  ex = fma(e.cp, vx, fma(-e.sp, vy, e.x));
+  ey = fma(e.sp, vx, fma(e.cp, vy, e.y));
+}
+// the rest of compute_evolute, wanted of the last iteration only: the circle's radius r
+// (ellipse.c:17-28) and the foot's offset (ix, iy) from the ellipse's centre
+__device__ __forceinline__ void evolute_end(const FitEllipse &e, double cs, double ss, double &ix, double &iy, double &r) {
+  const double as = e.a * ss, bc = e.b * cs;
+  const double w2 = fma(as, as, bc * bc);
+  r = fmin(w2 * sqrt(w2) * e.rab, 1. / DBL_EPSILON);
   const double fx = e.a * cs, fy = e.b * ss;
   ix = fma(e.cp, fx, -(e.sp * fy));
   iy = fma(e.sp, fx, e.cp * fy);
 }
 
-__device__ __forceinline__ double harmonic(double v0, double v1) { return 1. / (0.5 * (1. / v0 + 1. / v1)); }
+// Where the centres X^k + dX are taken from: formed from the records, from X^k alone (zero
+// increments), or from a list (the persistent sub-iteration kernel, which writes the records'
+// increments while other blocks still read the centres)
+struct Places {
+  const double2 *pos = nullptr;
+  const float4 *near = nullptr;   // with pos: pair_prefilter's values
+  bool at_x = false;
+};
+__device__ __forceinline__ double2 place_of(const Places &s, const double *P, int pc, int n) {
+  if (s.pos) return s.pos[n];
+  const double x = P[EIF_P_X * pc + n], y = P[EIF_P_Y * pc + n];
+  return s.at_x ? make_double2(x, y) : make_double2(x + P[EIF_P_DX * pc + n], y + P[EIF_P_DY * pc + n]);
+}
 
 struct PV {  // particle view at the positions X^k + dX
   double den, a, b, x, y, az;
 };
 
-__device__ __forceinline__ PV load_pv(const double *P, int pc, int n) {
+__device__ __forceinline__ PV load_pv(const Places &s, const double *P, int pc, int n) {
   PV v;
   v.den = P[EIF_P_DEN * pc + n];
   v.a = P[EIF_P_A * pc + n];
   v.b = P[EIF_P_B * pc + n];
-  v.x = P[EIF_P_X * pc + n] + P[EIF_P_DX * pc + n];
-  v.y = P[EIF_P_Y * pc + n] + P[EIF_P_DY * pc + n];
+  const double2 c = place_of(s, P, pc, n);
+  v.x = c.x;
+  v.y = c.y;
   v.az = P[EIF_P_AZ * pc + n];
   return v;
 }
@@ -165,12 +182,16 @@ __device__ __forceinline__ double image_offset(double p0y, double p1y, double ly
   return yoff;
 }
 
-// exact early-out of collision.c:173-189: true when the bounding circles overlap
+// exact early-out of collision.c:173-189: true when the bounding circles overlap. The distance
+// itself (hypot: a chain of about 40 FP64 operations) only where the squares leave it open.
 __device__ __forceinline__ bool bounding_overlap(const PV &p0, const PV &p1, double ly) {
   const double yoff = image_offset(p0.y, p1.y, ly);
   const double nx = p1.x - p0.x, ny = (p1.y + yoff) - p0.y;
-  const double norm = fmax(hypot(nx, ny), DBL_EPSILON);
-  return !(fmax(p0.a, p0.b) + fmax(p1.a, p1.b) - norm < 0.);
+  const double sum = fmax(p0.a, p0.b) + fmax(p1.a, p1.b);
+  const double d2 = fma(nx, nx, ny * ny), s2 = sum * sum;
+  if (d2 < s2 * (1. - 1e-12)) return true;
+  if (d2 > s2 * (1. + 1e-12)) return false;
+  return !(sum - fmax(hypot(nx, ny), DBL_EPSILON) < 0.);
 }
 
 // Pairs whose bounding circles overlap (collision.c:173-189) but whose ellipses are
@@ -182,42 +203,46 @@ __device__ __forceinline__ bool bounding_overlap(const PV &p0, const PV &p1, dou
 // the fit's stopping error) proves the same zero contribution without the iteration.
 // Candidate normals: the centre line, the four semi-axis directions and 16 fixed
 // directions; along a unit normal n the ellipses' extents are their support values
-// sqrt(a^2 (n.u)^2 + b^2 (n.v)^2) about the centres.
+// sqrt(a^2 (n.u)^2 + b^2 (n.v)^2) about the centres. Single precision: whatever it finds apart
+// by the margin, which is at least 2e-5 of the radii, forty times its rounding, is apart.
 struct PairFrame {
-  double dx, dy, s0, c0, s1, c1, margin;
+  float dx, dy, s0, c0, s1, c1, a0, b0, a1, b1, margin;
 };
 __device__ __forceinline__ PairFrame pair_frame(const PV &p0, const PV &p1, double ly) {
   PairFrame f;
-  f.dx = p1.x - p0.x;
-  f.dy = (p1.y + image_offset(p0.y, p1.y, ly)) - p0.y;
-  sincos(p0.az, &f.s0, &f.c0);
-  sincos(p1.az, &f.s1, &f.c1);
-  f.margin = 0.01 * fmin(fmin(p0.a, p0.b), fmin(p1.a, p1.b));
+  f.dx = eifd::d2f(p1.x - p0.x);
+  f.dy = eifd::d2f((p1.y + image_offset(p0.y, p1.y, ly)) - p0.y);
+  sincosf(eifd::d2f(p0.az), &f.s0, &f.c0);
+  sincosf(eifd::d2f(p1.az), &f.s1, &f.c1);
+  f.a0 = eifd::d2f(p0.a); f.b0 = eifd::d2f(p0.b);
+  f.a1 = eifd::d2f(p1.a); f.b1 = eifd::d2f(p1.b);
+  f.margin = fmaxf(0.01f * fminf(fminf(f.a0, f.b0), fminf(f.a1, f.b1)),
+                   2.e-5f * (fmaxf(f.a0, f.b0) + fmaxf(f.a1, f.b1)));
   return f;
 }
-__device__ __forceinline__ bool separated(const PairFrame &f, const PV &p0, const PV &p1, double nx, double ny) {
-  const double u0 = nx * f.c0 + ny * f.s0, v0 = ny * f.c0 - nx * f.s0;
-  const double u1 = nx * f.c1 + ny * f.s1, v1 = ny * f.c1 - nx * f.s1;
-  const double h0 = sqrt(p0.a * p0.a * u0 * u0 + p0.b * p0.b * v0 * v0);
-  const double h1 = sqrt(p1.a * p1.a * u1 * u1 + p1.b * p1.b * v1 * v1);
-  return fabs(nx * f.dx + ny * f.dy) - h0 - h1 > f.margin;
+__device__ __forceinline__ bool separated(const PairFrame &f, float nx, float ny) {
+  const float u0 = nx * f.c0 + ny * f.s0, v0 = ny * f.c0 - nx * f.s0;
+  const float u1 = nx * f.c1 + ny * f.s1, v1 = ny * f.c1 - nx * f.s1;
+  const float h0 = sqrtf(f.a0 * f.a0 * u0 * u0 + f.b0 * f.b0 * v0 * v0);
+  const float h1 = sqrtf(f.a1 * f.a1 * u1 * u1 + f.b1 * f.b1 * v1 * v1);
+  return fabsf(nx * f.dx + ny * f.dy) - h0 - h1 > f.margin;
 }
 // the centre line alone, which settles most pairs: one pair per lane
 __device__ __forceinline__ bool apart_centres(const PV &p0, const PV &p1, double ly) {
   const PairFrame f = pair_frame(p0, p1, ly);
-  const double d = hypot(f.dx, f.dy);
-  return d > 0. && separated(f, p0, p1, f.dx / d, f.dy / d);
+  const float d = sqrtf(f.dx * f.dx + f.dy * f.dy);
+  return d > 0.f && separated(f, f.dx / d, f.dy / d);
 }
 // the other directions of one pair, one per lane
 __device__ __forceinline__ bool apart_warp(const PV &p0, const PV &p1, double ly, int lane) {
   const PairFrame f = pair_frame(p0, p1, ly);
-  double ny, nx;
-  sincospi((lane - 4) / 16., &ny, &nx);
+  float ny, nx;
+  sincospif((lane - 4) / 16.f, &ny, &nx);
   if (lane == 0) { nx = f.c0; ny = f.s0; }
   if (lane == 1) { nx = -f.s0; ny = f.c0; }
   if (lane == 2) { nx = f.c1; ny = f.s1; }
   if (lane == 3) { nx = -f.s1; ny = f.c1; }
-  return __any_sync(0xffffffffu, lane < 20 && separated(f, p0, p1, nx, ny));
+  return __any_sync(0xffffffffu, lane < 20 && separated(f, nx, ny));
 }
 
 constexpr int FIT_SLOTS = 16;   // pairs a warp fits at a time, two lanes each
@@ -228,7 +253,7 @@ constexpr int FIT_SLOTS = 16;   // pairs a warp fits at a time, two lanes each
 // needs of the other ellipse only its last centre; the walls take one more pair of lanes, with
 // the mirrored centre in the place of the other's. A fit is a serial chain of a hundred and more
 // evolute points in double precision and sets the time of the launch.
-__device__ __forceinline__ void contact_forces(const double *P, int pcap, int k, const PV &pk, const int *list, int ncon,
+__device__ __forceinline__ void contact_forces(const Places &where, const double *P, int pcap, int k, const PV &pk, const int *list, int ncon,
                                                double ly, double lx, double (*cval)[3], double acc[3], bool &ok_all) {
   const int lane = threadIdx.x & 31, role = lane & 1;
   const double wallx = role ? lx : 0.;
@@ -246,14 +271,14 @@ __device__ __forceinline__ void contact_forces(const double *P, int pcap, int k,
     if (q < ncon) {
       const int m = list[q];
       self0 = k < m;
-      const PV o = load_pv(P, pcap, m);
+      const PV o = load_pv(where, P, pcap, m);
       p0 = self0 ? pk : o;
       p1 = self0 ? o : pk;
     }
     const double yoff = wall ? 0. : image_offset(p0.y, p1.y, ly);
-    const PV &pe = role ? p1 : p0;
+    const PV pe = role ? p1 : p0;
     const FitEllipse e = fit_ellipse(pe.a, pe.b, pe.x, pe.y + (role ? yoff : 0.), pe.az);
-    double cx = e.x, cy = e.y, r = 0., ix = 0., iy = 0., c = 0., s = 0.;
+    double cx = e.x, cy = e.y, r = 0., ix = 0., iy = 0., c = 0., s = 0., cs = 0., ss = 0.;
     bool ok = !act;
     for (int n = 0; n < EIF_FIT_MAX_ITER && __any_sync(0xffffffffu, act); n++) {
       double ox = __shfl_xor_sync(0xffffffffu, cx, 1), oy = __shfl_xor_sync(0xffffffffu, cy, 1);
@@ -264,7 +289,7 @@ __device__ __forceinline__ void contact_forces(const double *P, int pcap, int k,
       double change = 0.;
       if (act) {
         double nx, ny;
-        evolute(e, n == 0, ox, oy, c, s, nx, ny, ix, iy, r);
+        evolute(e, n == 0, ox, oy, c, s, cs, ss, nx, ny);
         const double dx = nx - cx, dy = ny - cy;
         cx += dx;
         cy += dy;
@@ -277,41 +302,37 @@ __device__ __forceinline__ void contact_forces(const double *P, int pcap, int k,
       }
     }
     ok_all &= ok;
+    evolute_end(e, cs, ss, ix, iy, r);
     const double ocx = __shfl_xor_sync(0xffffffffu, cx, 1), ocy = __shfl_xor_sync(0xffffffffu, cy, 1),
                  orr = __shfl_xor_sync(0xffffffffu, r, 1);
+    // the force over this particle's mass and the torque over its moment of inertia
+    // (collision.c:190-304: k = m (pi / h^(3/2))^2 with the harmonic means m of the masses and
+    // h of the radii sqrt(a b)), in few and independent divisions
     double out[3] = {0., 0., 0.};
-    if (q < ncon && (role == 0) == self0) {
-      const double m0 = pmass(p0.den, p0.a, p0.b), m1 = pmass(p1.den, p1.a, p1.b);
-      const double mass = harmonic(m0, m1);
-      const double h = harmonic(sqrt(p0.a * p0.b), sqrt(p1.a * p1.b));
-      const double kc = mass * (M_PI * M_PI) / (h * h * h);   // the square of h^(3/2)
-      // from this particle's circle to the other's
-      double nx = ocx - cx, ny = ocy - cy;
-      const double norm = fmax(hypot(nx, ny), DBL_EPSILON);
-      nx /= norm;
-      ny /= norm;
-      const double overlap = r + orr - norm;
+    const bool mine = q < ncon && (role == 0) == self0;
+    if (mine || (wall && near_wall)) {
+      double nx = wallx - cx, ny = 0., norm = fabs(nx), overlap = r - norm, w = 1., hs = 1., hp = sqrt(pk.a * pk.b);
+      if (mine) {
+        // from this particle's circle to the other's
+        nx = ocx - cx;
+        ny = ocy - cy;
+        norm = fmax(sqrt(fma(nx, nx, ny * ny)), DBL_EPSILON);
+        overlap = r + orr - norm;
+        const PV po = role ? p0 : p1;
+        const double ms = pmass(pe.den, pe.a, pe.b), mo = pmass(po.den, po.a, po.b), ho = sqrt(po.a * po.b);
+        w = 2. * mo / (ms + mo);
+        hs = hp + ho;
+        hp = 2. * hp * ho;
+      }
       if (overlap > 0.) {
-        const double cfx = -(kc * overlap * nx), cfy = -(kc * overlap * ny);
-        out[0] = 1. / (self0 ? m0 : m1) * cfx;
-        out[1] = 1. / (self0 ? m0 : m1) * cfy;
-        out[2] = 1. / pmoi(pe.den, pe.a, pe.b) * fma(ix, cfy, -(iy * cfx));
+        const double rh = hs / hp;
+        const double f = -(M_PI * M_PI * w * overlap * (rh * rh * rh)) / norm;
+        out[0] = f * nx;
+        out[1] = f * ny;
+        out[2] = 4. / fma(pe.a, pe.a, pe.b * pe.b) * fma(ix, out[1], -(iy * out[0]));
       }
     }
-    if (wall && near_wall) {
-      const double pm = pmass(pk.den, pk.a, pk.b), h = sqrt(pk.a * pk.b);
-      const double kc = pm * (M_PI * M_PI) / (h * h * h);
-      double nx = wallx - cx;
-      const double norm = fabs(nx);
-      nx /= norm;
-      const double overlap = r - norm;
-      if (overlap > 0.) {
-        const double cfx = kc * overlap * nx;
-        out[0] = 1. / pm * (-cfx);
-        out[2] = 1. / pmoi(pk.den, pk.a, pk.b) * (iy * cfx);
-      }
-    }
-    if (q < ncon && (role == 0) == self0)
+    if (mine)
       for (int f = 0; f < 3; f++) cval[lane >> 1][f] = out[f];
     if (wall)
       for (int f = 0; f < 3; f++) cval[FIT_SLOTS + role][f] = out[f];
@@ -344,14 +365,14 @@ constexpr int PAIR_WARPS = 8;
 constexpr int PAIR_TILE = 1024;
 constexpr int PAIR_LOADS = PAIR_TILE / (PAIR_WARPS * 32);
 
-__device__ __forceinline__ float4 pair_prefilter(const double *P, int pcap, int n) {
-  const double x = P[EIF_P_X * pcap + n] + P[EIF_P_DX * pcap + n];
-  const double y = P[EIF_P_Y * pcap + n] + P[EIF_P_DY * pcap + n];
-  return make_float4(eifd::d2f(x), eifd::d2f(y), eifd::d2f(fmax(P[EIF_P_A * pcap + n], P[EIF_P_B * pcap + n])), 0.f);
+__device__ __forceinline__ float4 pair_prefilter(const Places &where, const double *P, int pcap, int n) {
+  if (where.near) return where.near[n];
+  const double2 c = place_of(where, P, pcap, n);
+  return make_float4(eifd::d2f(c.x), eifd::d2f(c.y), eifd::d2f(fmax(P[EIF_P_A * pcap + n], P[EIF_P_B * pcap + n])), 0.f);
 }
 
 // One block of PAIR_WARPS warps: particles block * PAIR_WARPS ...
-__device__ __forceinline__ void collision_block(double *P, int pcap, int np, int cn, double ly, double lx,
+__device__ __forceinline__ void collision_block(const Places &where, double *P, int pcap, int np, int cn, double ly, double lx,
                                                 unsigned *flags, int block) {
   __shared__ float4 tile[PAIR_TILE];
   __shared__ int list[PAIR_WARPS][CAND_CAP];
@@ -359,7 +380,7 @@ __device__ __forceinline__ void collision_block(double *P, int pcap, int np, int
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int k = block * PAIR_WARPS + wl;
   const bool on = k < np;   // uniform over the warp
-  const float4 fk = on ? pair_prefilter(P, pcap, k) : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 fk = on ? pair_prefilter(where, P, pcap, k) : make_float4(0.f, 0.f, 0.f, 0.f);
   const float lyf = eifd::d2f(ly);
   int nmaybe = 0;
   for (int t0 = 0; t0 < np; t0 += PAIR_TILE) {
@@ -368,7 +389,7 @@ __device__ __forceinline__ void collision_block(double *P, int pcap, int np, int
 #pragma unroll
     for (int r = 0; r < PAIR_LOADS; r++) {
       const int q = threadIdx.x + r * PAIR_WARPS * 32;
-      st[r] = q < nt ? pair_prefilter(P, pcap, t0 + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+      st[r] = q < nt ? pair_prefilter(where, P, pcap, t0 + q) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
 #pragma unroll
@@ -403,7 +424,7 @@ __device__ __forceinline__ void collision_block(double *P, int pcap, int np, int
   __syncwarp();
   if (nmaybe > CAND_CAP && lane == 0) atomicOr(flags, EIF_FLAG_NOCONV);
   nmaybe = min(nmaybe, CAND_CAP);
-  const PV pk = load_pv(P, pcap, k);
+  const PV pk = load_pv(where, P, pcap, k);
   // exact test and the centre line, hits compacted in place (a write never passes the
   // entries still to read)
   int cnt = 0;
@@ -413,7 +434,7 @@ __device__ __forceinline__ void collision_block(double *P, int pcap, int np, int
     int m = 0;
     if (q < nmaybe) {
       m = list[wl][q];
-      const PV o = load_pv(P, pcap, m);
+      const PV o = load_pv(where, P, pcap, m);
       const PV p0 = m < k ? o : pk, p1 = m < k ? pk : o;
       hit = bounding_overlap(p0, p1, ly) && !apart_centres(p0, p1, ly);
     }
@@ -426,7 +447,7 @@ __device__ __forceinline__ void collision_block(double *P, int pcap, int np, int
   int ncon = 0;
   for (int q = 0; q < cnt; q++) {
     const int m = list[wl][q];
-    const PV o = load_pv(P, pcap, m);
+    const PV o = load_pv(where, P, pcap, m);
     const PV p0 = m < k ? o : pk, p1 = m < k ? pk : o;
     if (apart_warp(p0, p1, ly, lane)) continue;
     __syncwarp();
@@ -436,7 +457,7 @@ __device__ __forceinline__ void collision_block(double *P, int pcap, int np, int
   __syncwarp();
   double acc[3];
   bool ok;
-  contact_forces(P, pcap, k, pk, list[wl], ncon, ly, lx, cval[wl], acc, ok);
+  contact_forces(where, P, pcap, k, pk, list[wl], ncon, ly, lx, cval[wl], acc, ok);
   if (lane == 0) {
     P[(EIF_P_CFX0 + cn) * pcap + k] = acc[0];
     P[(EIF_P_CFY0 + cn) * pcap + k] = acc[1];
@@ -447,9 +468,11 @@ __device__ __forceinline__ void collision_block(double *P, int pcap, int np, int
 
 // increment.c:10-72 for particle n: new increments from the forces, inertia integrals
 // and collision forces of the sub-iteration, the position increments from them; returns
-// res raised to the largest change of the velocity increments
+// res raised to the largest change of the velocity increments; pos (optional): the centre
+// X^k + dX of the new increments, rounded as load_pv forms it from the records, and near the
+// partner search's values of it
 __device__ __forceinline__ double increment_particle(double *p, int pcap, int n, double gamma, double Fr2, double dt,
-                                                     double res) {
+                                                     double res, double2 *pos = nullptr, float4 *near = nullptr) {
   const double den = p[EIF_P_DEN * pcap + n];
   const double px = p[EIF_P_DUX * pcap + n], py = p[EIF_P_DUY * pcap + n], pz = p[EIF_P_DVZ * pcap + n];
   const double hgd = 0.5 * gamma * dt;
@@ -466,8 +489,14 @@ __device__ __forceinline__ double increment_particle(double *p, int pcap, int n,
   res = fmax(res, fabs(duy - py));
   res = fmax(res, fabs(dvz - pz));
   const double ux0 = p[EIF_P_UX * pcap + n], uy0 = p[EIF_P_UY * pcap + n], vz0 = p[EIF_P_VZ * pcap + n];
-  p[EIF_P_DX * pcap + n] = hgd * (ux0 + (ux0 + dux));
-  p[EIF_P_DY * pcap + n] = hgd * (uy0 + (uy0 + duy));
+  const double dx = hgd * (ux0 + (ux0 + dux)), dy = hgd * (uy0 + (uy0 + duy));
+  p[EIF_P_DX * pcap + n] = dx;
+  p[EIF_P_DY * pcap + n] = dy;
+  if (pos) {
+    const double2 c = make_double2(__dadd_rn(p[EIF_P_X * pcap + n], dx), __dadd_rn(p[EIF_P_Y * pcap + n], dy));
+    pos[n] = c;
+    near[n] = make_float4(eifd::d2f(c.x), eifd::d2f(c.y), eifd::d2f(fmax(p[EIF_P_A * pcap + n], p[EIF_P_B * pcap + n])), 0.f);
+  }
   p[EIF_P_DAZ * pcap + n] = hgd * (vz0 + (vz0 + dvz));
   return res;
 }

@@ -23,7 +23,7 @@ namespace {
 
 __global__ void __launch_bounds__(PAIR_WARPS * 32) k_collision(double *__restrict__ P, int pcap, int np, int cn,
                                                                double ly, double lx, unsigned *__restrict__ flags) {
-  collision_block(P, pcap, np, cn, ly, lx, flags, blockIdx.x);
+  collision_block(Places{}, P, pcap, np, cn, ly, lx, flags, blockIdx.x);
 }
 
 __global__ void k_reset(double *__restrict__ P, int pcap, int np) {

@@ -1,44 +1,40 @@
-// Sub-iterations of the particles (src/main.c:36-50) of many suspensions in one
-// persistent kernel per RK stage.
+// Sub-iterations of the particles (src/main.c:36-50) in one persistent kernel per RK stage:
+// of one suspension (eif_advance) or of many (a batch, batch.cu, whose stage fronts join
+// before the kernel and fork after it).
 //
-// A batch (batch.cu) captures each suspension's stage front as a graph branch; the
-// branches join before one cooperative kernel that runs the sub-iteration loops of all
-// joined suspensions, and fork again after it for the particle updates and the next
-// stage. The kernel's CTAs (all resident: a cooperative launch of as many CTAs as fit
-// on the GPU at once) loop over the sub-iterations; a sub-iteration has four phases
-// separated by grid barriers:
-//   1. the collision forces at X + dX (block units of PAIR_WARPS particles) and, after
-//      the first sub-iteration, the boxes at X + dX (warp units: 32 particles, one
-//      part); in the first one the increments are zero and the boxes and weights that
-//      the stage front built at X are still in place;
-//   2. (after the first) the task tables (block units of TT_WARPS particles);
-//   3. the row tasks of the inertia integrals of all suspensions in one index space (a
-//      warp per task; cached weights in the first sub-iteration); the task counts are
-//      zeroed for the next boxes;
-//   4. per particle (a warp) the sum over its tasks, then its increment and the
-//      suspension's residual (an integer max of the IEEE bits, independent of order).
-// After phase 4 every CTA evaluates the stopping rule of each suspension (main.c:40-48:
-// go on while the residual is not below 1e-8 and at most 101 sub-iterations ran) from
-// the same residuals, so all CTAs agree on the set still iterating; a suspension that
-// stops takes no part in later sub-iterations. Every body is the one of the stand-alone
-// kernels (ibm_device.cuh, particle_device.cuh) with the same decomposition per task,
-// particle and block, so each suspension gets the same bits as in its own loop.
-// When no suspension iterates any more, the kernel updates every suspension's particles
-// (update.c) and, before stages 1 and 2, resets their increments (reset.c): the particle
-// launches around the loop, which the suspensions' own branches then leave out.
+// The kernel's CTAs (all resident: a cooperative launch) loop over the sub-iterations. The
+// work of one is a list of units, the collision forces of PAIR_WARPS particles each, and for
+// every particle ns slices of the row tasks of its inertia integrals:
+//  * a slice forms the boxes and parameters of its particle at X + dX in shared memory
+//    (box_warp) and runs its share of the particle's tasks, a warp per task; in the first
+//    sub-iteration, where the increments are zero, it runs the
+//    stage front's tasks with their stored weights;
+//  * every unit counts itself at its particles; the last one of a particle sums the tasks,
+//    forms the increments (increment.c) and raises the suspension's residual.
+// Nothing else orders the units of a sub-iteration: the new increments go to the records, the
+// centres that the collisions of other particles may still be reading are a list of their own
+// (two, alternating). One grid barrier ends the sub-iteration; every CTA then evaluates the
+// stopping rule of each suspension (main.c:40-48: go on while the residual is not below 1e-8
+// and at most 101 sub-iterations ran) from the same residuals, so all agree on the set still
+// iterating. When none is left the kernel updates every suspension's particles (update.c) and,
+// before stages 1 and 2, resets their increments (reset.c).
 //
-// The units of a phase are numbered suspension by suspension (fixed offsets from the
-// particle counts) and worker w (a CTA or a warp) takes units w, w + W, ... of that
-// numbering; the row tasks are numbered on the device from the task counts of phase 2.
+// As a loop of kernels (boxes, task table, indicator, sums, collisions, increments: a
+// conditional node of the step graph) a sub-iteration was eight launches in a row of 2 to 7 us
+// each, about 30 us before any real work.
 //
-// The grid barrier is an arrival counter per stage, zeroed by a memset node at the
-// start of every step and polled with acquire loads. A poll gives up after 2^22 tries:
-// the CTA sets the plan's error word, which makes the others give up at their next
-// poll, and every suspension's EIF_FLAG_TIMEOUT, and the CTAs return. Data that one
-// phase writes and a later one reads is read with ordinary loads, not through the
-// read-only path. For the tests of that bounded wait, EIF_TEST_HOLD_BARRIER=1 in the
-// environment when a batch's graph is built keeps CTA 0 of the first stage's kernel
-// from arriving at its first barrier: the other CTAs give up, and the step reports it.
+// Every body is the one of the stand-alone kernels (ibm_device.cuh, particle_device.cuh) with
+// the same decomposition per task and particle, so each suspension gets the same bits as from
+// those.
+//
+// The grid barrier is an arrival counter per stage, zeroed with the particles' counters by a
+// memset node at the start of every step and polled with acquire loads. A poll gives up after
+// 2^22 tries: the CTA sets the plan's error word, which makes the others give up at their next
+// poll, and every suspension's EIF_FLAG_TIMEOUT, and the CTAs return. Data that one CTA writes
+// and another reads is read with ordinary loads, not through the read-only path. For the tests
+// of that bounded wait, EIF_TEST_HOLD_BARRIER=1 in the environment when a batch's graph is
+// built keeps CTA 0 of the first stage's kernel from arriving at its first barrier: the other
+// CTAs give up, and the step reports it.
 #ifndef EIF_CHECK
 #define EIF_CHECK 1
 #endif
@@ -55,14 +51,16 @@ struct SubDesc {
   BoxArgs box;     // boxes at X + dX
   WorkArgs work;   // inertia integrals at X + dX (mode 0, integrals 1)
   double *P;
-  int pcap, np, tcap, mixed;
-  int *cnt, *off;
-  int4 *tdesc;
+  int pcap, np, ns, mixed;       // ns: slices per particle
+  int *cnt, *off;                // tasks at X + dX, first tasks at X
+  const int *base;               // first task slots at X + dX (fixed, from the radii)
+  double2 *pos[2];               // centres X + dX
+  float4 *near[2];               // the same for the partner search (pair_prefilter)
+  unsigned *arr;                 // units of the particle that are done
   double ly, lx, gamma, Fr2;
   double *scal;                  // [0] dt, [1] residual
   unsigned *flags, *counter;     // error flags, the stage's sub-iteration count
   unsigned long long *total;     // sub-iterations run (eif_counters)
-  int u_box, u_coll, u_tab, u_part;   // first unit of the suspension in phases 1 (boxes, collisions), 2, 4
 };
 
 struct StageArgs {
@@ -70,8 +68,8 @@ struct StageArgs {
   int n;
   int reset_next;               // the particles' increments are reset for a following stage
   int hold;                     // a CTA that does not arrive at the first barrier (tests), or -1
-  unsigned *sync;               // [0] arrivals, [1] error
-  unsigned long long *res;      // two residual words per suspension (alternating sub-iterations)
+  unsigned *sync;               // [0] arrivals, [1] error, [2..4] units taken (by sub-iteration mod 3)
+  unsigned long long *res;      // three residual words per suspension (by sub-iteration mod 3)
 };
 
 constexpr int SUB_THREADS = 256;
@@ -79,12 +77,19 @@ constexpr int SUB_WARPS = SUB_THREADS / 32;
 constexpr int SUB_MAX = (int)eif::SUBITER_MAX;
 constexpr unsigned SUB_CAP = 102;      // the stopping rule ends every loop by the 102nd sub-iteration
 constexpr unsigned SPIN_MAX = 1u << 22;
-constexpr int SYNC_WORDS = 32;         // per stage (arrivals and error word, padded)
-static_assert(PAIR_WARPS == SUB_WARPS && TT_WARPS == SUB_WARPS, "block units of the phases");
+constexpr int SYNC_WORDS = 32;         // per stage (arrivals, error word, unit counters; padded)
+static_assert(PAIR_WARPS == SUB_WARPS, "units of the sub-iterations");
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// adds 1, ordering what this thread has seen and written before with what it does after
+__device__ __forceinline__ unsigned atom_acq_rel(unsigned *p) {
+  unsigned v;
+  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 
@@ -95,182 +100,194 @@ __device__ bool grid_barrier(unsigned *sync, unsigned idx, bool arrive) {
   __syncthreads();
   if (threadIdx.x == 0) {
     const unsigned target = gridDim.x * (idx + 1u);
-    __threadfence();
-    if (arrive) atomicAdd(sync, 1u);
-    int good = 0;
-    for (unsigned k = 0; k < SPIN_MAX; k++) {
-      if (ld_acquire(sync) >= target) {
-        good = 1;
-        break;
+    int good = arrive && atom_acq_rel(sync) + 1u >= target;
+    for (unsigned k = 0; !good && k < SPIN_MAX; k++) {
+      good = ld_acquire(sync) >= target;
+      if (!good && k % 16u == 15u) {
+        if (ld_acquire(sync + 1) != 0u) break;
+        __nanosleep(64);
       }
-      if (ld_acquire(sync + 1) != 0u) break;
-      __nanosleep(64);
     }
     if (!good) atomicOr(sync + 1, 1u);
-    __threadfence();
     ok = good;
   }
   __syncthreads();
   return ok != 0;
 }
 
-// the first of the units u = 0, 1, ... that worker w of W takes when the units are
-// numbered from `base`
-__device__ __forceinline__ int first_unit(int w, int base, int W) {
-  const int r = (w - base) % W;
-  return r < 0 ? r + W : r;
+// per suspension, in shared memory: the loop control, so that the units are found without
+// loading the descriptors; running numbers of the units, collisions first, then slices
+enum { ST_NP, ST_NS, ST_CEND, ST_SEND, ST_WORDS };
+
+// a warp counts a unit of particle n as done; true (for all lanes) when it was the last one
+__device__ __forceinline__ bool unit_done(const SubDesc &d, int n, int lane) {
+  unsigned last = 0u;
+  __syncwarp();
+  if (lane == 0) {
+    last = atom_acq_rel(d.arr + n) == (unsigned)d.ns ? 1u : 0u;   // ns slices and the collisions
+    if (last) d.arr[n] = 0u;
+  }
+  last = __shfl_sync(0xffffffffu, last, 0);
+  __syncwarp();
+  return last != 0u;
 }
 
-// per suspension, in shared memory: the loop control of the phases, so that a worker
-// walks the suspensions without loading their descriptors
-enum { ST_NP, ST_UBOX, ST_UCOLL, ST_UTAB, ST_UPART, ST_MIXED, ST_TASKS, ST_WORDS = 8 };
+// the particle's sums and increments (one warp), after its last unit
+__device__ __forceinline__ void finish_particle(const SubDesc &d, int n, unsigned it, unsigned long long *res) {
+  const bool first = it == 0u;
+  const int c0 = first ? d.off[n] : d.base[n], c1 = first ? d.off[n + 1] : c0 + d.cnt[n];
+  if (d.mixed)
+    chunk_reduce_f_warp(reinterpret_cast<const float *>(d.work.partial), c0, c1, d.P, d.pcap, EIF_P_IUX0 + 1,
+                        EIF_P_IUY0 + 1, EIF_P_IVZ0 + 1, d.box.bd, n);
+  else
+    chunk_reduce_warp(d.work.partial, c0, c1, d.P, d.pcap, EIF_P_IUX0 + 1, EIF_P_IUY0 + 1, EIF_P_IVZ0 + 1, d.box.bd, n);
+  if ((threadIdx.x & 31) == 0) {
+    const double r = increment_particle(d.P, d.pcap, n, d.gamma, d.Fr2, d.scal[0], 0., d.pos[(it + 1u) & 1u], d.near[(it + 1u) & 1u]);
+    if (r > 0.) atomicMax(res, (unsigned long long)__double_as_longlong(r));
+  }
+}
 
 __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
   __shared__ unsigned act[SUB_MAX / 32];   // suspensions still iterating
   __shared__ float2 slot_f[SUB_WARPS][CHUNK];
   __shared__ double2 slot_d[SUB_WARPS][WORK_SLOTS];
+  __shared__ __align__(16) int bx[12];
+  __shared__ __align__(16) float pf[PF_WORDS];
+  __shared__ __align__(16) double pd[PD_WORDS];
+  __shared__ int unit[2];                  // suspension and unit within it
   extern __shared__ int stab[];            // ST_WORDS per suspension
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  const int G = gridDim.x, W = G * SUB_WARPS, T = G * SUB_THREADS;
-  const int wid = blockIdx.x * SUB_WARPS + wl, tid = blockIdx.x * SUB_THREADS + threadIdx.x;
-  const int n = s.n;
+  const int G = gridDim.x, n = s.n;
   for (int q = threadIdx.x; q < SUB_MAX / 32; q += SUB_THREADS) {
     const int lo = 32 * q;
     act[q] = lo >= n ? 0u : (n - lo >= 32 ? 0xffffffffu : ((1u << (n - lo)) - 1u));
   }
   for (int j = threadIdx.x; j < n; j += SUB_THREADS) {
-    const SubDesc &d = s.d[j];
-    int *e = stab + ST_WORDS * j;
-    e[ST_NP] = d.np;
-    e[ST_UBOX] = d.u_box;
-    e[ST_UCOLL] = d.u_coll;
-    e[ST_UTAB] = d.u_tab;
-    e[ST_UPART] = d.u_part;
-    e[ST_MIXED] = d.mixed;
-    e[ST_TASKS] = 0;
+    stab[ST_WORDS * j + ST_NP] = s.d[j].np;
+    stab[ST_WORDS * j + ST_NS] = s.d[j].ns;
   }
-  if (blockIdx.x == 0)
-    for (int j = threadIdx.x; j < 2 * n; j += SUB_THREADS) s.res[j] = 0ull;
   __syncthreads();
-  auto active = [&](int j) { return ((act[j >> 5] >> (j & 31)) & 1u) != 0u; };
   unsigned bar = 0;
-  bool ok = true;
   auto barrier = [&]() {
     const bool arrive = bar != 0u || (int)blockIdx.x != s.hold;
     return grid_barrier(s.sync, bar++, arrive);
   };
+  bool ok = true;
+  auto active = [&](int j) { return ((act[j >> 5] >> (j & 31)) & 1u) != 0u; };
+  int ncoll = 0, units = 0;
+  bool changed = true;
   for (unsigned it = 0; it < SUB_CAP; it++) {
-    // 1. collision forces; boxes after the first sub-iteration
-    for (int j = 0; j < n; j++) {
-      if (!active(j)) continue;
-      const int *e = stab + ST_WORDS * j;
-      const int units = (e[ST_NP] + PAIR_WARPS - 1) / PAIR_WARPS;
-      int b = first_unit(blockIdx.x, e[ST_UCOLL], G);
-      if (b >= units) continue;
-      const SubDesc &d = s.d[j];
-      for (; b < units; b += G) {
-        collision_block(d.P, d.pcap, d.np, 1, d.ly, d.lx, d.flags, b);
-        __syncthreads();
+    if (changed) {
+      // the units of the suspensions still iterating
+      if (threadIdx.x < 32) {
+        int run = 0;
+        for (int pass = 0; pass < 2; pass++) {
+          for (int j0 = 0; j0 < n; j0 += 32) {
+            const int j = j0 + lane;
+            int v = 0;
+            if (j < n && active(j)) {
+              const int np = stab[ST_WORDS * j + ST_NP];
+              v = pass == 0 ? (np + PAIR_WARPS - 1) / PAIR_WARPS : np * stab[ST_WORDS * j + ST_NS];
+            }
+            int sc = v;
+            for (int o = 1; o < 32; o <<= 1) {
+              const int w = __shfl_up_sync(0xffffffffu, sc, o);
+              if (lane >= o) sc += w;
+            }
+            if (j < n) stab[ST_WORDS * j + (pass == 0 ? ST_CEND : ST_SEND)] = run + sc;
+            run += __shfl_sync(0xffffffffu, sc, 31);
+          }
+        }
       }
+      __syncthreads();
+      ncoll = stab[ST_WORDS * (n - 1) + ST_CEND];
+      units = stab[ST_WORDS * (n - 1) + ST_SEND];
     }
-    if (it > 0) {
-      for (int j = 0; j < n; j++) {
-        if (!active(j)) continue;
-        const int *e = stab + ST_WORDS * j;
-        const int groups = (e[ST_NP] + 31) / 32;
-        const int units = groups * BOX_PARTS;
-        int u = first_unit(wid, e[ST_UBOX], W);
-        if (u >= units) continue;
-        const SubDesc &d = s.d[j];
-        for (; u < units; u += W) box_part(d.box, (u % groups) * 32 + lane, u / groups);
+    const unsigned m3 = it % 3u;
+    // words of the next sub-iteration: last used two barriers ago
+    if (blockIdx.x == 0) {
+      for (int j = threadIdx.x; j < n; j += SUB_THREADS) s.res[3 * j + (it + 1u) % 3u] = 0ull;
+      if (threadIdx.x == 0) s.sync[2 + (it + 1u) % 3u] = 0u;
+    }
+    // units in order: the first by the CTA's number, the next ones as CTAs come free
+    int next = blockIdx.x;
+    for (;;) {
+      if (threadIdx.x == 0) {
+        const int u = next;
+        if (units > G) next = G + (int)atomicAdd(s.sync + 2 + m3, 1u);
+        else next = units;
+        // the first suspension whose running number is above u
+        const int col = u < ncoll ? ST_CEND : ST_SEND;
+        int lo = 0, hi = n - 1;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (stab[ST_WORDS * mid + col] > u) hi = mid;
+          else lo = mid + 1;
+        }
+        unit[0] = u < units ? lo : -1;
+        unit[1] = u - (lo > 0 ? stab[ST_WORDS * (lo - 1) + col] : (col == ST_SEND ? ncoll : 0)) +
+                  (col == ST_CEND ? (1 << 30) : 0);
       }
-      if (!(ok = barrier())) break;
-      // 2. task tables
-      for (int j = 0; j < n; j++) {
-        if (!active(j)) continue;
-        const int *e = stab + ST_WORDS * j;
-        const int units = (e[ST_NP] + TT_WARPS - 1) / TT_WARPS;
-        int b = first_unit(blockIdx.x, e[ST_UTAB], G);
-        if (b >= units) continue;
-        const SubDesc &d = s.d[j];
-        for (; b < units; b += G) {
-          task_table_block(d.box.box, d.cnt, d.off, d.tdesc, d.np, d.box.bd, d.tcap, b);
+      __syncthreads();
+      const int j = unit[0];
+      if (j < 0) break;
+      const bool coll = unit[1] >= (1 << 30);
+      const int q = unit[1] & ((1 << 30) - 1);
+      const SubDesc &d = s.d[j];
+      unsigned long long *res = s.res + 3 * j + m3;
+      if (coll) {
+        collision_block(it > 0 ? Places{d.pos[it & 1u], d.near[it & 1u], false} : Places{nullptr, nullptr, true}, d.P, d.pcap, d.np, 1, d.ly, d.lx, d.flags, q);
+        const int k = q * PAIR_WARPS + wl;
+        if (k < d.np && unit_done(d, k, lane)) finish_particle(d, k, it, res);
+      } else {
+        const int p = q / d.ns, sl = q - p * d.ns;
+        if (it == 0) {
+          const int c0 = d.off[p], cnt = d.off[p + 1] - c0;
+          const int r0 = (int)((long long)cnt * sl / d.ns), r1 = (int)((long long)cnt * (sl + 1) / d.ns);
+          if (d.mixed) {
+            ibm_sum_f_tasks<false>(d.work, c0 + r0 + wl, SUB_WARPS, c0 + r1);
+          } else {
+            const OneParticle one{nullptr, nullptr, nullptr, p, 0, c0 + r1};
+            ibm_work_tasks<false>(d.work, 2, c0 + r0 + wl, SUB_WARPS, slot_d[wl], &one);
+          }
+        } else {
+          if (wl == 0) box_warp(d.box, p, bx, d.mixed ? pf : nullptr, pd);
           __syncthreads();
+          const int cnt = box_tasks(bx);
+          const int r0 = (int)((long long)cnt * sl / d.ns), r1 = (int)((long long)cnt * (sl + 1) / d.ns);
+          const OneParticle one{reinterpret_cast<const int4 *>(bx), pf, pd, p, d.base[p], r1};
+          if (d.mixed) {
+            ibm_work_f_tasks<false, true>(d.work, 0, r0 + wl, SUB_WARPS, slot_f[wl], &one);
+            if (sl == 0 && wl == SUB_WARPS - 1 && d.work.memo_mode == 2) memo_particle(d.work.memo, pf, bx, one.base, p);
+          } else {
+            ibm_work_tasks<false>(d.work, 0, r0 + wl, SUB_WARPS, slot_d[wl], &one);
+          }
+          if (threadIdx.x == 0) d.cnt[p] = cnt;
         }
+        __syncthreads();
+        if (wl == 0 && unit_done(d, p, lane)) finish_particle(d, p, it, res);
       }
-    }
-    if (!(ok = barrier())) break;
-    // 3. row tasks of the inertia integrals; task counts zeroed for the next boxes. The
-    // task totals of phase 2 are read into shared memory first, one load per suspension.
-    for (int j = threadIdx.x; j < n; j += SUB_THREADS) {
-      int *e = stab + ST_WORDS * j;
-      e[ST_TASKS] = active(j) && e[ST_NP] > 0 ? s.d[j].off[e[ST_NP]] : 0;
-    }
-    __syncthreads();
-    int base = 0;
-    for (int j = 0; j < n; j++) {
-      if (!active(j)) continue;
-      const int *e = stab + ST_WORDS * j;
-      const int np = e[ST_NP], total = e[ST_TASKS];
-      if (np == 0) continue;
-      const int first = first_unit(wid, base, W);
-      base += total;
-      const bool zero_cnt = blockIdx.x * SUB_THREADS < np;
-      if (first >= total && !zero_cnt) continue;
-      const SubDesc &d = s.d[j];
-      if (first < total) {
-        if (e[ST_MIXED]) {
-          if (it == 0) ibm_sum_f_tasks<false>(d.work, first, W);
-          else ibm_work_f_tasks<false>(d.work, 0, first, W, slot_f[wl]);
-        } else {
-          ibm_work_tasks<false>(d.work, it == 0 ? 2 : 0, first, W, slot_d[wl]);
-        }
-      }
-      for (int q = tid; q < np; q += T) d.cnt[q] = 0;
-    }
-    if (!(ok = barrier())) break;
-    // 4. sums over the tasks, increments, residuals
-    for (int j = 0; j < n; j++) {
-      if (!active(j)) continue;
-      const int *e = stab + ST_WORDS * j;
-      int m = first_unit(wid, e[ST_UPART], W);
-      if (m >= e[ST_NP]) continue;
-      const SubDesc &d = s.d[j];
-      const double dt = d.scal[0];
-      unsigned long long *res = s.res + 2 * j + (it & 1u);
-      for (; m < d.np; m += W) {
-        if (d.mixed) {
-          // after a sub-iteration with the indicator geometry: its weights are in the memo
-          chunk_reduce_f_warp(reinterpret_cast<const float *>(d.work.partial), d.off, d.P, d.pcap, d.np,
-                              EIF_P_IUX0 + 1, EIF_P_IUY0 + 1, EIF_P_IVZ0 + 1, d.box.bd, m,
-                              it > 0 && d.work.memo_mode == 2 ? &d.work.memo : nullptr, d.work.pf, d.box.box);
-        } else {
-          chunk_reduce_warp(d.work.partial, d.off, d.P, d.pcap, d.np, EIF_P_IUX0 + 1, EIF_P_IUY0 + 1,
-                            EIF_P_IVZ0 + 1, d.box.bd, m);
-        }
-        if (lane == 0) {
-          const double r = increment_particle(d.P, d.pcap, m, d.gamma, d.Fr2, dt, 0.);
-          if (r > 0.) atomicMax(res, (unsigned long long)__double_as_longlong(r));
-        }
-      }
+      if (units <= G) break;
     }
     if (!(ok = barrier())) break;
     // the stopping rule of every suspension, evaluated alike by all CTAs
+    bool stop = false;
     for (int j = threadIdx.x; j < n; j += SUB_THREADS) {
       if (!active(j)) continue;
-      const double r = __longlong_as_double(
-          (long long)*reinterpret_cast<volatile unsigned long long *>(s.res + 2 * j + (it & 1u)));
+      const double r = __longlong_as_double((long long)*reinterpret_cast<volatile unsigned long long *>(s.res + 3 * j + m3));
       const unsigned count = it + 1u;
-      if (!(!(r < 1.e-8) && count <= 101u)) atomicAnd(&act[j >> 5], ~(1u << (j & 31)));
+      if (!(!(r < 1.e-8) && count <= 101u)) {
+        atomicAnd(&act[j >> 5], ~(1u << (j & 31)));
+        stop = true;
+      }
       if (blockIdx.x == 0) {
         const SubDesc &d = s.d[j];
         d.scal[1] = r;
         *d.counter = count;
         *d.total += 1ull;
-        s.res[2 * j + ((it + 1u) & 1u)] = 0ull;
       }
     }
-    __syncthreads();
+    changed = __syncthreads_or(stop);
     bool any = false;
     for (int q = 0; q < SUB_MAX / 32; q++) any |= act[q] != 0u;
     if (!any) break;
@@ -283,15 +300,18 @@ __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
   // the particle update of the stage (update.c:8-34) and, before a following stage, the
   // reset of the increments (reset.c:7-18); the last increments were written before the
   // last grid barrier
+  const int T = G * SUB_THREADS;
+  int at = blockIdx.x * SUB_THREADS + threadIdx.x;
   for (int j = 0; j < n; j++) {
-    const int *e = stab + ST_WORDS * j;
-    int m = first_unit(tid, e[ST_UPART], T);
-    if (m >= e[ST_NP]) continue;
-    const SubDesc &d = s.d[j];
-    for (; m < d.np; m += T) {
-      update_particle(d.P, d.pcap, m, d.ly);
-      if (s.reset_next) reset_particle(d.P, d.pcap, m);
+    const int np = stab[ST_WORDS * j + ST_NP];
+    if (at < np) {
+      const SubDesc &d = s.d[j];
+      for (int m = at; m < np; m += T) {
+        update_particle(d.P, d.pcap, m, d.ly);
+        if (s.reset_next) reset_particle(d.P, d.pcap, m);
+      }
     }
+    at = (at + T - np % T) % T;   // the suspensions' particles spread over all CTAs
   }
 }
 
@@ -303,18 +323,36 @@ struct SubiterPlan {
   int n = 0, grid = 0;
   std::vector<SubDesc> h;               // 3 stages x n
   SubDesc *d_desc = nullptr;
-  unsigned *d_sync = nullptr;           // 3 stages x SYNC_WORDS
-  unsigned long long *d_res = nullptr;  // 3 stages x 2n
+  // zeroed at the start of every step: residuals (3 stages x 3n), then barriers and counters
+  // (3 stages x SYNC_WORDS), then the particles' unit counters
+  unsigned long long *d_res = nullptr;
+  unsigned *d_sync = nullptr;
+  size_t zero_words = 0;
+  double2 *d_pos = nullptr;             // two lists of centres of all particles
+  float4 *d_near = nullptr;             // the same for the partner search
+  std::vector<int> first;               // first particle of every suspension in these arrays
+  std::vector<int> ns;                  // slices per particle
+  int np = 0;
   int hold = -1;                        // EIF_TEST_HOLD_BARRIER: CTA 0 of stage 0 held back
 };
 
 bool subiter_joinable(const eif_ctx *c) { return c->np <= TT_MAX_NP; }
 
+// One suspension's loops in stage kernels: while every unit has a CTA of its own. With more, a
+// loop of kernels is faster: the stand-alone indicator has 24 warps on an SM and no
+// CTA-wide steps, the stage kernel 16 (registers of the fits). 768 x 1536 with 512 ellipses, 177
+// sub-iterations: 15.2 ms against 18.5; 2048 x 4096 with 2048: 54 against 83 (mixed form); with
+// 128 at 512 x 1024 11.3 against 10.8, with 24 at 216 x 430 8.4 against 7.2.
+bool subiter_alone(const eif_ctx *c) {
+  return c->np > 0 && c->np + (c->np + PAIR_WARPS - 1) / PAIR_WARPS <= 2 * c->sms;
+}
+
 void subiter_plan_destroy(SubiterPlan *p) {
   if (!p) return;
   if (p->d_desc) cudaFree(p->d_desc);
-  if (p->d_sync) cudaFree(p->d_sync);
   if (p->d_res) cudaFree(p->d_res);
+  if (p->d_pos) cudaFree(p->d_pos);
+  if (p->d_near) cudaFree(p->d_near);
   delete p;
 }
 
@@ -349,16 +387,33 @@ int subiter_plan_create(eif_ctx *const *ctx, int n, SubiterPlan **out, std::stri
   SubiterPlan *p = new (std::nothrow) SubiterPlan;
   if (!p) return EIF_ERR_NOMEM;
   p->n = n;
-  p->grid = occ * ctx[0]->sms;
+  // slices: as many as give every warp of the GPU a task when the particles are few, none
+  // without a task for each of its warps
+  const int most = occ * ctx[0]->sms;
+  long long units = 0;
+  for (int j = 0; j < n; j++) {
+    p->first.push_back(p->np);
+    p->np += ctx[j]->np;
+  }
+  for (int j = 0; j < n; j++) {
+    const int by_gpu = std::max(1, most / std::max(1, p->np));
+    const int by_tasks = std::max(1, (ctx[j]->max_tasks + SUB_WARPS - 1) / SUB_WARPS);
+    p->ns.push_back(std::min(by_gpu, by_tasks));
+    units += (long long)ctx[j]->np * p->ns[j] + (ctx[j]->np + PAIR_WARPS - 1) / PAIR_WARPS;
+  }
+  p->zero_words = (size_t)18 * n + 3 * SYNC_WORDS + p->np;
+  p->grid = (int)std::max<long long>(1, std::min<long long>(most, units));
   const char *hold = std::getenv("EIF_TEST_HOLD_BARRIER");
   p->hold = hold && hold[0] == '1' ? 0 : -1;
   p->h.assign((size_t)3 * n, SubDesc{});
   if ((e = cudaMalloc((void **)&p->d_desc, sizeof(SubDesc) * 3 * n)) != cudaSuccess ||
-      (e = cudaMalloc((void **)&p->d_sync, sizeof(unsigned) * 3 * SYNC_WORDS)) != cudaSuccess ||
-      (e = cudaMalloc((void **)&p->d_res, sizeof(unsigned long long) * 3 * 2 * n)) != cudaSuccess) {
+      (e = cudaMalloc((void **)&p->d_pos, sizeof(double2) * std::max(1, 2 * p->np))) != cudaSuccess ||
+      (e = cudaMalloc((void **)&p->d_near, sizeof(float4) * std::max(1, 2 * p->np))) != cudaSuccess ||
+      (e = cudaMalloc((void **)&p->d_res, sizeof(unsigned) * p->zero_words)) != cudaSuccess) {
     subiter_plan_destroy(p);
     return plan_fail(err, "cudaMalloc", e);
   }
+  p->d_sync = reinterpret_cast<unsigned *>(p->d_res + (size_t)9 * n);
   *out = p;
   return EIF_OK;
 }
@@ -372,11 +427,16 @@ void subiter_describe(SubiterPlan *p, int rk, int j, const eif_ctx *c) {
   d.P = c->P;
   d.pcap = c->pcap;
   d.np = c->np;
-  d.tcap = c->chunk_cap;
+  d.ns = p->ns[j];
+  d.base = c->task_base;
+  for (int k = 0; k < 2; k++) {
+    d.pos[k] = p->d_pos + (size_t)k * p->np + p->first[j];
+    d.near[k] = p->d_near + (size_t)k * p->np + p->first[j];
+  }
+  d.arr = p->d_sync + 3 * SYNC_WORDS + p->first[j];
   d.mixed = c->cfg.precision == EIF_PREC_MIXED ? 1 : 0;
   d.cnt = c->np > 0 ? c->chunk_off + (c->np + 1) : nullptr;
   d.off = c->chunk_off;
-  d.tdesc = c->tdesc;
   d.ly = c->ly;
   d.lx = c->lx;
   d.gamma = rk_coef(rk).gamma;
@@ -389,10 +449,10 @@ void subiter_describe(SubiterPlan *p, int rk, int j, const eif_ctx *c) {
 
 int subiter_add_reset(SubiterPlan *p, cudaGraph_t g, cudaGraphNode_t *node, std::string *err) {
   cudaMemsetParams m = {};
-  m.dst = p->d_sync;
+  m.dst = p->d_res;
   m.value = 0;
   m.elementSize = sizeof(unsigned);
-  m.width = 3 * SYNC_WORDS;
+  m.width = p->zero_words;
   m.height = 1;
   const cudaError_t e = cudaGraphAddMemsetNode(node, g, nullptr, 0, &m);
   return e == cudaSuccess ? EIF_OK : plan_fail(err, "cudaGraphAddMemsetNode", e);
@@ -404,7 +464,7 @@ int subiter_add_stage(SubiterPlan *p, int rk, cudaGraph_t g, const std::vector<c
   a.d = p->d_desc + (size_t)rk * p->n;
   a.n = p->n;
   a.sync = p->d_sync + SYNC_WORDS * rk;
-  a.res = p->d_res + (size_t)2 * p->n * rk;
+  a.res = p->d_res + (size_t)3 * p->n * rk;
   a.reset_next = rk < 2 ? 1 : 0;
   a.hold = rk == 0 ? p->hold : -1;
   void *args[] = {&a};
@@ -423,20 +483,6 @@ int subiter_add_stage(SubiterPlan *p, int rk, cudaGraph_t g, const std::vector<c
 }
 
 int subiter_upload(SubiterPlan *p, std::string *err) {
-  for (int rk = 0; rk < 3; rk++) {
-    int u_box = 0, u_coll = 0, u_tab = 0, u_part = 0;
-    for (int j = 0; j < p->n; j++) {
-      SubDesc &d = p->h[(size_t)rk * p->n + j];
-      d.u_box = u_box;
-      d.u_coll = u_coll;
-      d.u_tab = u_tab;
-      d.u_part = u_part;
-      u_box += ((d.np + 31) / 32) * BOX_PARTS;
-      u_coll += (d.np + PAIR_WARPS - 1) / PAIR_WARPS;
-      u_tab += (d.np + TT_WARPS - 1) / TT_WARPS;
-      u_part += d.np;
-    }
-  }
   const cudaError_t e = cudaMemcpy(p->d_desc, p->h.data(), sizeof(SubDesc) * p->h.size(), cudaMemcpyHostToDevice);
   return e == cudaSuccess ? EIF_OK : plan_fail(err, "cudaMemcpy (stage descriptors)", e);
 }
