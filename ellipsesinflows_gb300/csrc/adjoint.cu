@@ -38,7 +38,8 @@ namespace eif {
 
 struct Adjoint {
   int mode = EIF_ADJOINT_COUPLED;
-  int max_steps = 0, nrec = 0, np = 0;
+  int max_steps = 0, nrec = 0, np = 0, pcap = 0;
+  bool ready = false;   // every buffer is allocated
   // per step: dt, contact seen; per stage (3 per step): inputs u_k, v_k, predictor
   // outputs u*, v* (coupled), particle state (6 x np), sub-iteration count and
   // increments dX_m (m = 1..K, 3 x np each); per step the final velocity (coupled)
@@ -452,6 +453,8 @@ int frozen_stage(eif_ctx *c, int rk) {
   return launch_correct(c, rk, ibm, true);
 }
 
+bool stage_kernels(const eif_ctx *c) { return c->use_graphs && !c->sync_debug && !c->prof.enabled && subiter_alone(c); }
+
 // one RK stage of the full step (src/main.c:14-52), recording for the adjoint when
 // slot >= 0: u_k, u*, the particle state and every sub-iteration's increments
 int coupled_stage(eif_ctx *c, int rk, int slot) {
@@ -483,6 +486,10 @@ int coupled_stage(eif_ctx *c, int rk, int slot) {
     return EIF_OK;
   }
   if ((rc = launch_collision(c, 0))) return rc;
+  if (stage_kernels(c)) {
+    // the sub-iterations and their tape without the host; eif_adjoint_forward reads their number
+    return launch_stage_kernel(c, rk, slot >= 0 ? a->tape_dx[slot] : nullptr, a->d_contact);
+  }
   int m = 0;
   for (;; m++) {
     if ((rc = launch_inertia(c, 1))) return rc;
@@ -506,21 +513,34 @@ int coupled_stage(eif_ctx *c, int rk, int slot) {
 
 }  // namespace
 
+namespace { int adj_clear(eif_ctx *c); }
+
 extern "C" {
 
 int eif_adjoint_begin(eif_ctx *c, int max_steps, int mode) {
   if (!c || max_steps <= 0 || (mode != EIF_ADJOINT_COUPLED && mode != EIF_ADJOINT_FROZEN)) return EIF_ERR_ARG;
   if (c->cfg.precision != EIF_PREC_FP64) return fail(c, EIF_ERR_ARG, "the adjoint is built on the double-precision form");
   if (!c->fluid_pushed) return fail(c, EIF_ERR_STATE, "push the fluid state before eif_adjoint_begin");
+  const bool coupled = mode == EIF_ADJOINT_COUPLED;
+  const size_t bytes = sizeof(double) * c->nfield;
+  const int np = c->np;
+  int rc;
+  // the buffers of an earlier begin of the same shape are taken over (a gradient in a loop: about
+  // seventy allocations, each waiting for the device when it is given back); eif_adjoint_end
+  // and eif_destroy free them
+  if (Adjoint *a = c->adj) {
+    if (a->ready && a->mode == mode && a->max_steps == max_steps && a->np == np && a->pcap == c->pcap) {
+      a->nrec = 0;
+      return adj_clear(c);
+    }
+  }
   adj_free(c);
   Adjoint *a = new Adjoint;
   c->adj = a;
   a->mode = mode;
   a->max_steps = max_steps;
-  a->np = c->np;
-  const bool coupled = mode == EIF_ADJOINT_COUPLED;
-  const size_t bytes = sizeof(double) * c->nfield;
-  const int np = c->np;
+  a->np = np;
+  a->pcap = c->pcap;
   auto field = [&](std::vector<double *> &v, int n) -> int {
     for (int k = 0; k < n; k++) {
       double *p = nullptr;
@@ -529,7 +549,6 @@ int eif_adjoint_begin(eif_ctx *c, int max_steps, int mode) {
     }
     return EIF_OK;
   };
-  int rc;
   if ((rc = field(a->tape_u, 3 * max_steps)) || (rc = field(a->tape_v, 3 * max_steps))) return rc;
   if (coupled) {
     if ((rc = field(a->tape_us, 3 * max_steps)) || (rc = field(a->tape_vs, 3 * max_steps))) return rc;
@@ -550,25 +569,42 @@ int eif_adjoint_begin(eif_ctx *c, int max_steps, int mode) {
   for (double **p : {&a->ub, &a->vb, &a->pb, &a->abx, &a->aby, &a->tu, &a->tv, &a->rhs, &a->w, &a->fcx, &a->fcy,
                      &a->gcx, &a->gcy}) {
     EIF_CK(c, cudaMalloc((void **)p, bytes));
-    EIF_CK(c, cudaMemsetAsync(*p, 0, bytes, c->stream));
   }
   const int n3 = std::max(1, 3 * np);
-  for (double **p : {&a->xb, &a->vpb, &a->dub, &a->fb, &a->i0b, &a->i1b}) {
+  for (double **p : {&a->xb, &a->vpb, &a->dub, &a->fb, &a->i0b, &a->i1b})
     EIF_CK(c, cudaMalloc((void **)p, sizeof(double) * n3));
-    EIF_CK(c, cudaMemsetAsync(*p, 0, sizeof(double) * n3, c->stream));
-  }
   EIF_CK(c, cudaMalloc((void **)&a->pout, sizeof(double) * 2 * n3));
   EIF_CK(c, cudaMalloc((void **)&a->wall_rows, sizeof(double) * 2 * c->jtot));
-  EIF_CK(c, cudaMemsetAsync(a->wall_rows, 0, sizeof(double) * 2 * c->jtot, c->stream));
   EIF_CK(c, cudaMalloc((void **)&a->wall, sizeof(double) * 2));
-  EIF_CK(c, cudaMemsetAsync(a->wall, 0, sizeof(double) * 2, c->stream));
   EIF_CK(c, cudaMalloc((void **)&a->pbackup, sizeof(double) * EIF_NFIELDS * std::max(1, c->pcap)));
   EIF_CK(c, cudaMalloc((void **)&a->d_contact, sizeof(int)));
-  EIF_CK(c, cudaMemsetAsync(a->d_contact, 0, sizeof(int), c->stream));
   if (np > 0) {
     a->part_cap = adj_chunk_cap(c);
     EIF_CK(c, cudaMalloc((void **)&a->part, sizeof(double) * 6 * std::max(1, a->part_cap)));
   }
+  a->ready = true;
+  return adj_clear(c);
+}
+
+}  // extern "C"
+
+namespace {
+
+// the cotangents and scratch of a new recording
+int adj_clear(eif_ctx *c) {
+  Adjoint *a = c->adj;
+  const size_t bytes = sizeof(double) * c->nfield;
+  const int n3 = std::max(1, 3 * a->np);
+  int rc;
+  for (double *p : {a->ub, a->vb, a->pb, a->abx, a->aby, a->tu, a->tv, a->rhs, a->w, a->fcx, a->fcy, a->gcx, a->gcy})
+    EIF_CK(c, cudaMemsetAsync(p, 0, bytes, c->stream));
+  for (double *p : {a->xb, a->vpb, a->dub, a->fb, a->i0b, a->i1b})
+    EIF_CK(c, cudaMemsetAsync(p, 0, sizeof(double) * n3, c->stream));
+  EIF_CK(c, cudaMemsetAsync(a->wall_rows, 0, sizeof(double) * 2 * c->jtot, c->stream));
+  EIF_CK(c, cudaMemsetAsync(a->wall, 0, sizeof(double) * 2, c->stream));
+  EIF_CK(c, cudaMemsetAsync(a->d_contact, 0, sizeof(int), c->stream));
+  const bool coupled = a->mode == EIF_ADJOINT_COUPLED;
+  const int np = a->np;
   // frozen mode: summed indicator weights of the particles, from the exchange with the
   // weights as the cell contributions (double-precision kernels) gathered into dux
   if (!coupled && np > 0) {
@@ -584,6 +620,10 @@ int eif_adjoint_begin(eif_ctx *c, int max_steps, int mode) {
   EIF_CK(c, cudaStreamSynchronize(c->stream));
   return check_records(c);
 }
+
+}  // namespace
+
+extern "C" {
 
 int eif_adjoint_end(eif_ctx *c) {
   if (!c) return EIF_ERR_ARG;
@@ -615,8 +655,19 @@ int eif_adjoint_forward(eif_ctx *c, int record) {
     }
   } else {
     if (record) EIF_CK(c, cudaMemsetAsync(a->d_contact, 0, sizeof(int), c->stream));
-    for (int rk = 0; rk < 3; rk++)
+    const bool graph = !record && c->use_graphs && !c->sync_debug && !c->prof.enabled;
+    if (graph) {
+      // a step that is not recorded: the graph of eif_integrate
+      if ((rc = tune_tiles(c)) || (rc = step_graph_launch(c, false))) return rc;
+      c->incr_zero = false;
+    }
+    for (int rk = 0; !graph && rk < 3; rk++)
       if ((rc = coupled_stage(c, rk, record ? 3 * s + rk : -1))) return rc;
+    if (record && c->np > 0 && stage_kernels(c))
+      EIF_CK(c, cudaMemcpyAsync(c->h_flags + 1, c->d_sub, sizeof(unsigned) * 3, cudaMemcpyDeviceToHost, c->stream));
+    if ((rc = read_scalars(c))) return rc;
+    if (record && c->np > 0 && stage_kernels(c))
+      for (int rk = 0; rk < 3; rk++) a->tape_k[3 * s + rk] = (int)c->h_flags[1 + rk];
     if (record) {
       EIF_CK(c, cudaMemcpyAsync(a->tape_out_u[s], c->ux[c->cur], bytes, cudaMemcpyDeviceToDevice, c->stream));
       EIF_CK(c, cudaMemcpyAsync(a->tape_out_v[s], c->uy[c->cur], bytes, cudaMemcpyDeviceToDevice, c->stream));

@@ -96,6 +96,7 @@ int build_joined(eif_batch *b, eif_batch::Graph &g, const std::vector<size_t> &i
   int rc = eif::subiter_plan_create(cs.data(), m, &plan, &err);
   if (rc) return batch_fail(b, rc, "stage kernel: " + err);
   g.plans.push_back(plan);
+  eif::subiter_test_hold(plan);
   cudaGraphNode_t reset = nullptr;
   if ((rc = eif::subiter_add_reset(plan, g.graph, &reset, &err))) return batch_fail(b, rc, "stage kernel: " + err);
   for (int k = 0; k < m; k++) {
@@ -157,7 +158,7 @@ int build(eif_batch *b, eif_batch::Graph &out) {
       continue;
     }
     int cur1 = 0, scur1 = 0;
-    const int rc = eif::capture_step(c, g.graph, &cur1, &scur1, nullptr);
+    const int rc = eif::capture_step(c, g.graph, &cur1, &scur1, nullptr, true);
     if (rc) {
       free_graph(g);
       return batch_fail(b, rc, "suspension " + std::to_string(i) + ": " + eif_last_error(c));

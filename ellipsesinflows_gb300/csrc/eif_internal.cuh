@@ -178,7 +178,11 @@ struct eif_ctx {
     cudaGraphExec_t exec = nullptr;
     int cur0 = -1, scur0 = -1, cur1 = 0, scur1 = 0;
     eif::SubiterPlan *plan = nullptr;   // stage kernels of the sub-iteration loops
-  } graphs[2];
+  } graphs[2], igraphs[2];              // of eif_advance; of eif_integrate (without the dt decision)
+  // stage kernels launched one by one (adjoint.cu), for the buffers of generation stage_gen
+  eif::SubiterPlan *stage_plan = nullptr;
+  unsigned stage_gen = 0;
+  unsigned *d_sub = nullptr;            // sub-iterations of the stages of a step
   bool use_graphs = true;
   // tile shapes of the stencil and block-Thomas kernels, chosen once per grid size by the
   // tuner (tune.cu) among shapes that give the same results: predictor and projection
@@ -280,16 +284,18 @@ struct ProfScope {
 int profile_flush(eif_ctx *c);
 int check_records(eif_ctx *c);
 // ---- step graphs (graph.cu) ----
-int step_graph_launch(eif_ctx *c);
+// one step as a graph: all of it, or without the dt decision
+int step_graph_launch(eif_ctx *c, bool with_dt);
 void graphs_free(eif_ctx *c);
 struct SubiterPlan;
 // plan: where set and the context is subiter_alone, the sub-iteration loops are stage kernels
 // of the plan it receives, conditional nodes otherwise
-int capture_step(eif_ctx *c, cudaGraph_t g, int *cur1, int *scur1, SubiterPlan **plan);
+int capture_step(eif_ctx *c, cudaGraph_t g, int *cur1, int *scur1, SubiterPlan **plan, bool with_dt);
 int step_capture_begin(eif_ctx *c);
 void step_capture_end(eif_ctx *c, int cur0, int scur0);
 int capture_step_part(eif_ctx *c, cudaGraph_t g, const std::vector<cudaGraphNode_t> &deps, int part,
-                      std::vector<cudaGraphNode_t> *sinks, bool particles_in_stage_kernel, bool fields_event);
+                      std::vector<cudaGraphNode_t> *sinks, bool particles_in_stage_kernel, bool fields_event,
+                      bool with_dt = true);
 int capture_subiteration_loop(eif_ctx *c, cudaGraph_t g, const std::vector<cudaGraphNode_t> &deps, int rk,
                               std::vector<cudaGraphNode_t> *sinks);
 
@@ -297,8 +303,10 @@ int capture_subiteration_loop(eif_ctx *c, cudaGraph_t g, const std::vector<cudaG
 constexpr size_t SUBITER_MAX = 1024;   // suspensions per stage kernel
 bool subiter_joinable(const eif_ctx *c);
 bool subiter_alone(const eif_ctx *c);
-int subiter_plan_create(eif_ctx *const *ctx, int n, SubiterPlan **out, std::string *err);
+// sets: descriptors of the three stages this many times
+int subiter_plan_create(eif_ctx *const *ctx, int n, SubiterPlan **out, std::string *err, int sets = 1);
 void subiter_plan_destroy(SubiterPlan *p);
+void subiter_test_hold(SubiterPlan *p);   // EIF_TEST_HOLD_BARRIER (batches)
 // the descriptor of suspension j (context c) in RK stage rk, from the state of c after
 // the capture of that stage's front
 void subiter_describe(SubiterPlan *p, int rk, int j, const eif_ctx *c);
@@ -307,6 +315,10 @@ int subiter_add_reset(SubiterPlan *p, cudaGraph_t g, cudaGraphNode_t *node, std:
 int subiter_add_stage(SubiterPlan *p, int rk, cudaGraph_t g, const std::vector<cudaGraphNode_t> &deps,
                       cudaGraphNode_t *node, std::string *err);
 int subiter_upload(SubiterPlan *p, std::string *err);
+// the stage kernel of RK stage rk on c's stream (np > 0, subiter_alone): the sub-iterations after
+// a stage front and the particle update; tape (optional): dX after sub-iteration m to
+// tape + 3 np m, and *contact = 1 where a collision force is not zero
+int launch_stage_kernel(eif_ctx *c, int rk, double *tape, int *contact);
 int rk_stage_front(eif_ctx *c, int rk);
 int ibm_prepare(eif_ctx *c);
 void profile_free(eif_ctx *c);

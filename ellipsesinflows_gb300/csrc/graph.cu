@@ -87,14 +87,15 @@ void step_capture_end(eif_ctx *c, int cur0, int scur0) {
 // all the suspensions of a batch), which then also updates the particles at the end of the
 // stage and resets the increments for the next (particles_in_stage_kernel: those launches
 // are left out of parts 1-3). fields_event: ev_fields is recorded once the fields are final.
+// with_dt: false leaves the dt decision out (eif_integrate).
 int capture_step_part(eif_ctx *c, cudaGraph_t g, const std::vector<cudaGraphNode_t> &deps, int part,
-                      std::vector<cudaGraphNode_t> *sinks, bool particles_in_stage_kernel, bool fields_event) {
+                      std::vector<cudaGraphNode_t> *sinks, bool particles_in_stage_kernel, bool fields_event, bool with_dt) {
   cudaError_t e = cudaStreamBeginCaptureToGraph(c->stream, g, deps.data(), nullptr, deps.size(),
                                                 cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return check_cuda(c, e, "cudaStreamBeginCaptureToGraph");
   int rc;
   if (part == 0) {
-    if ((rc = launch_decide_dt(c))) return rc;
+    if (with_dt && (rc = launch_decide_dt(c))) return rc;
   } else {
     // after a sub-iteration loop: the increments are not zero and the boxes of the
     // loop's last positions are not those at X
@@ -164,11 +165,21 @@ int capture_subiteration_loop(eif_ctx *c, cudaGraph_t g, const std::vector<cudaG
   return EIF_OK;
 }
 
+// the loop's count to the stage's place in d_sub
+int capture_loop_count(eif_ctx *c, cudaGraph_t g, int rk, std::vector<cudaGraphNode_t> *tail) {
+  cudaGraphNode_t n = nullptr;
+  const cudaError_t e = cudaGraphAddMemcpyNode1D(&n, g, tail->data(), tail->size(), c->d_sub + rk, c->d_inc + 1,
+                                                 sizeof(unsigned), cudaMemcpyDeviceToDevice);
+  if (e != cudaSuccess) return check_cuda(c, e, "cudaGraphAddMemcpyNode1D");
+  tail->assign(1, n);
+  return EIF_OK;
+}
+
 // Captures one time step of c into g (appended as an independent branch: its first
 // nodes have no dependences) and returns the buffer indices the step ends with. The
 // host state of c is left as before the capture; on failure g may hold a partial
 // branch and should be discarded.
-int capture_step(eif_ctx *c, cudaGraph_t g, int *cur1, int *scur1, SubiterPlan **plan) {
+int capture_step(eif_ctx *c, cudaGraph_t g, int *cur1, int *scur1, SubiterPlan **plan, bool with_dt) {
   int rc = step_capture_begin(c);
   if (rc) return rc;
   const int cur0 = c->cur, scur0 = c->scur;
@@ -187,7 +198,7 @@ int capture_step(eif_ctx *c, cudaGraph_t g, int *cur1, int *scur1, SubiterPlan *
       return failed(rc, true);
   }
   for (int part = 0; part < 4; part++) {
-    if ((rc = capture_step_part(c, g, tail, part, &tail, stage_kernels, true))) return failed(rc, false);
+    if ((rc = capture_step_part(c, g, tail, part, &tail, stage_kernels, true, with_dt))) return failed(rc, false);
     if (part == 3) break;
     if (stage_kernels) {
       subiter_describe(p, part, 0, c);
@@ -195,7 +206,8 @@ int capture_step(eif_ctx *c, cudaGraph_t g, int *cur1, int *scur1, SubiterPlan *
       cudaGraphNode_t node = nullptr;
       if ((rc = subiter_add_stage(p, part, g, tail, &node, &err))) return failed(rc, true);
       tail.assign(1, node);
-    } else if ((rc = capture_subiteration_loop(c, g, tail, part, &tail))) {
+    } else if ((rc = capture_subiteration_loop(c, g, tail, part, &tail)) ||
+               (!with_dt && c->np > 0 && (rc = capture_loop_count(c, g, part, &tail)))) {
       return failed(rc, false);
     }
   }
@@ -209,12 +221,12 @@ int capture_step(eif_ctx *c, cudaGraph_t g, int *cur1, int *scur1, SubiterPlan *
 
 namespace {
 
-int build(eif_ctx *c, eif_ctx::StepGraph &sg) {
+int build(eif_ctx *c, eif_ctx::StepGraph &sg, bool with_dt) {
   cudaGraph_t g = nullptr;
   EIF_CK(c, cudaGraphCreate(&g, 0));
   int cur1 = 0, scur1 = 0;
   SubiterPlan *plan = nullptr;
-  int rc = capture_step(c, g, &cur1, &scur1, &plan);
+  int rc = capture_step(c, g, &cur1, &scur1, &plan, with_dt);
   if (rc) {
     cudaGraphDestroy(g);
     return rc;
@@ -238,8 +250,8 @@ int build(eif_ctx *c, eif_ctx::StepGraph &sg) {
 
 }  // namespace
 
-void graphs_free(eif_ctx *c) {
-  for (auto &sg : c->graphs) {
+static void free_graphs(eif_ctx::StepGraph (&graphs)[2]) {
+  for (auto &sg : graphs) {
     if (sg.exec) cudaGraphExecDestroy(sg.exec);
     if (sg.graph) cudaGraphDestroy(sg.graph);
     subiter_plan_destroy(sg.plan);
@@ -247,20 +259,28 @@ void graphs_free(eif_ctx *c) {
   }
 }
 
-int step_graph_launch(eif_ctx *c) {
+void graphs_free(eif_ctx *c) {
+  free_graphs(c->graphs);
+  free_graphs(c->igraphs);
+  subiter_plan_destroy(c->stage_plan);
+  c->stage_plan = nullptr;
+}
+
+int step_graph_launch(eif_ctx *c, bool with_dt) {
+  auto &graphs = with_dt ? c->graphs : c->igraphs;
   eif_ctx::StepGraph *sg = nullptr;
-  for (auto &g : c->graphs) {
+  for (auto &g : graphs) {
     if (g.exec && g.cur0 == c->cur && g.scur0 == c->scur) sg = &g;
   }
   if (!sg) {
-    for (auto &g : c->graphs) {
+    for (auto &g : graphs) {
       if (!g.exec) { sg = &g; break; }
     }
     if (!sg) {
-      graphs_free(c);
-      sg = &c->graphs[0];
+      free_graphs(graphs);
+      sg = &graphs[0];
     }
-    int rc = build(c, *sg);
+    int rc = build(c, *sg, with_dt);
     if (rc) return rc;
   }
   EIF_CK(c, cudaGraphLaunch(sg->exec, c->stream));

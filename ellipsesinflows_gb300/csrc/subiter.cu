@@ -70,6 +70,8 @@ struct StageArgs {
   int hold;                     // a CTA that does not arrive at the first barrier (tests), or -1
   unsigned *sync;               // [0] arrivals, [1] error, [2..4] units taken (by sub-iteration mod 3)
   unsigned long long *res;      // three residual words per suspension (by sub-iteration mod 3)
+  double *tape;                 // dX after sub-iteration m to tape + 3 np m (one suspension), or null
+  int *contact;                 // with tape: set where a collision force is not zero
 };
 
 constexpr int SUB_THREADS = 256;
@@ -133,7 +135,8 @@ __device__ __forceinline__ bool unit_done(const SubDesc &d, int n, int lane) {
 }
 
 // the particle's sums and increments (one warp), after its last unit
-__device__ __forceinline__ void finish_particle(const SubDesc &d, int n, unsigned it, unsigned long long *res) {
+__device__ __forceinline__ void finish_particle(const SubDesc &d, int n, unsigned it, unsigned long long *res,
+                                                double *tape, int *contact) {
   const bool first = it == 0u;
   const int c0 = first ? d.off[n] : d.base[n], c1 = first ? d.off[n + 1] : c0 + d.cnt[n];
   if (d.mixed)
@@ -144,6 +147,15 @@ __device__ __forceinline__ void finish_particle(const SubDesc &d, int n, unsigne
   if ((threadIdx.x & 31) == 0) {
     const double r = increment_particle(d.P, d.pcap, n, d.gamma, d.Fr2, d.scal[0], 0., d.pos[(it + 1u) & 1u], d.near[(it + 1u) & 1u]);
     if (r > 0.) atomicMax(res, (unsigned long long)__double_as_longlong(r));
+    if (tape) {
+      double *t = tape + (size_t)3 * d.np * (it + 1u) + n;
+      t[0] = d.P[EIF_P_DX * d.pcap + n];
+      t[d.np] = d.P[EIF_P_DY * d.pcap + n];
+      t[2 * (size_t)d.np] = d.P[EIF_P_DAZ * d.pcap + n];
+      bool any = false;
+      for (int f = EIF_P_CFX0; f <= EIF_P_CTZ1; f++) any |= d.P[f * d.pcap + n] != 0.;
+      if (any) *contact = 1;
+    }
   }
 }
 
@@ -238,7 +250,7 @@ __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
       if (coll) {
         collision_block(it > 0 ? Places{d.pos[it & 1u], d.near[it & 1u], false} : Places{nullptr, nullptr, true}, d.P, d.pcap, d.np, 1, d.ly, d.lx, d.flags, q);
         const int k = q * PAIR_WARPS + wl;
-        if (k < d.np && unit_done(d, k, lane)) finish_particle(d, k, it, res);
+        if (k < d.np && unit_done(d, k, lane)) finish_particle(d, k, it, res, s.tape, s.contact);
       } else {
         const int p = q / d.ns, sl = q - p * d.ns;
         if (it == 0) {
@@ -265,7 +277,7 @@ __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
           if (threadIdx.x == 0) d.cnt[p] = cnt;
         }
         __syncthreads();
-        if (wl == 0 && unit_done(d, p, lane)) finish_particle(d, p, it, res);
+        if (wl == 0 && unit_done(d, p, lane)) finish_particle(d, p, it, res, s.tape, s.contact);
       }
       if (units <= G) break;
     }
@@ -321,7 +333,7 @@ namespace eif {
 
 struct SubiterPlan {
   int n = 0, grid = 0;
-  std::vector<SubDesc> h;               // 3 stages x n
+  std::vector<SubDesc> h;               // 3 stages x n (x 2 buffer indices, launch_stage_kernel)
   SubDesc *d_desc = nullptr;
   // zeroed at the start of every step: residuals (3 stages x 3n), then barriers and counters
   // (3 stages x SYNC_WORDS), then the particles' unit counters
@@ -361,7 +373,7 @@ static int plan_fail(std::string *err, const char *what, cudaError_t e) {
   return EIF_ERR_CUDA;
 }
 
-int subiter_plan_create(eif_ctx *const *ctx, int n, SubiterPlan **out, std::string *err) {
+int subiter_plan_create(eif_ctx *const *ctx, int n, SubiterPlan **out, std::string *err, int sets) {
   *out = nullptr;
   if (n <= 0 || n > SUB_MAX) {
     *err = "a stage kernel takes 1 to " + std::to_string(SUB_MAX) + " suspensions";
@@ -403,10 +415,8 @@ int subiter_plan_create(eif_ctx *const *ctx, int n, SubiterPlan **out, std::stri
   }
   p->zero_words = (size_t)18 * n + 3 * SYNC_WORDS + p->np;
   p->grid = (int)std::max<long long>(1, std::min<long long>(most, units));
-  const char *hold = std::getenv("EIF_TEST_HOLD_BARRIER");
-  p->hold = hold && hold[0] == '1' ? 0 : -1;
-  p->h.assign((size_t)3 * n, SubDesc{});
-  if ((e = cudaMalloc((void **)&p->d_desc, sizeof(SubDesc) * 3 * n)) != cudaSuccess ||
+  p->h.assign((size_t)3 * sets * n, SubDesc{});
+  if ((e = cudaMalloc((void **)&p->d_desc, sizeof(SubDesc) * p->h.size())) != cudaSuccess ||
       (e = cudaMalloc((void **)&p->d_pos, sizeof(double2) * std::max(1, 2 * p->np))) != cudaSuccess ||
       (e = cudaMalloc((void **)&p->d_near, sizeof(float4) * std::max(1, 2 * p->np))) != cudaSuccess ||
       (e = cudaMalloc((void **)&p->d_res, sizeof(unsigned) * p->zero_words)) != cudaSuccess) {
@@ -418,8 +428,7 @@ int subiter_plan_create(eif_ctx *const *ctx, int n, SubiterPlan **out, std::stri
   return EIF_OK;
 }
 
-void subiter_describe(SubiterPlan *p, int rk, int j, const eif_ctx *c) {
-  SubDesc &d = p->h[(size_t)rk * p->n + j];
+static void describe(SubiterPlan *p, SubDesc &d, int rk, int j, const eif_ctx *c) {
   d.box = box_args(c, true);
   d.work = work_args(c, 0, 1);
   // the evaluations with geometry (sub-iterations after the first) store their weights
@@ -443,8 +452,17 @@ void subiter_describe(SubiterPlan *p, int rk, int j, const eif_ctx *c) {
   d.Fr2 = c->cfg.Fr * c->cfg.Fr;
   d.scal = c->d_scal;
   d.flags = c->d_flags;
-  d.counter = reinterpret_cast<unsigned *>(c->d_inc + 1);
+  d.counter = c->d_sub + rk;
   d.total = c->d_inc + 2;
+}
+
+void subiter_describe(SubiterPlan *p, int rk, int j, const eif_ctx *c) {
+  describe(p, p->h[(size_t)rk * p->n + j], rk, j, c);
+}
+
+void subiter_test_hold(SubiterPlan *p) {
+  const char *hold = std::getenv("EIF_TEST_HOLD_BARRIER");
+  p->hold = hold && hold[0] == '1' ? 0 : -1;
 }
 
 int subiter_add_reset(SubiterPlan *p, cudaGraph_t g, cudaGraphNode_t *node, std::string *err) {
@@ -458,15 +476,23 @@ int subiter_add_reset(SubiterPlan *p, cudaGraph_t g, cudaGraphNode_t *node, std:
   return e == cudaSuccess ? EIF_OK : plan_fail(err, "cudaGraphAddMemsetNode", e);
 }
 
-int subiter_add_stage(SubiterPlan *p, int rk, cudaGraph_t g, const std::vector<cudaGraphNode_t> &deps,
-                      cudaGraphNode_t *node, std::string *err) {
+// arguments of stage rk's kernel with the descriptors d
+static StageArgs stage_args(SubiterPlan *p, int rk, const SubDesc *d) {
   StageArgs a;
-  a.d = p->d_desc + (size_t)rk * p->n;
+  a.d = d;
   a.n = p->n;
   a.sync = p->d_sync + SYNC_WORDS * rk;
   a.res = p->d_res + (size_t)3 * p->n * rk;
   a.reset_next = rk < 2 ? 1 : 0;
   a.hold = rk == 0 ? p->hold : -1;
+  a.tape = nullptr;
+  a.contact = nullptr;
+  return a;
+}
+
+int subiter_add_stage(SubiterPlan *p, int rk, cudaGraph_t g, const std::vector<cudaGraphNode_t> &deps,
+                      cudaGraphNode_t *node, std::string *err) {
+  StageArgs a = stage_args(p, rk, p->d_desc + (size_t)rk * p->n);
   void *args[] = {&a};
   cudaKernelNodeParams k = {};
   k.func = reinterpret_cast<void *>(k_subiterations);
@@ -485,6 +511,45 @@ int subiter_add_stage(SubiterPlan *p, int rk, cudaGraph_t g, const std::vector<c
 int subiter_upload(SubiterPlan *p, std::string *err) {
   const cudaError_t e = cudaMemcpy(p->d_desc, p->h.data(), sizeof(SubDesc) * p->h.size(), cudaMemcpyHostToDevice);
   return e == cudaSuccess ? EIF_OK : plan_fail(err, "cudaMemcpy (stage descriptors)", e);
+}
+
+int launch_stage_kernel(eif_ctx *c, int rk, double *tape, int *contact) {
+  std::string err;
+  int rc;
+  if (c->stage_plan && c->stage_gen != c->buf_gen) {
+    subiter_plan_destroy(c->stage_plan);
+    c->stage_plan = nullptr;
+  }
+  if (!c->stage_plan) {
+    SubiterPlan *p = nullptr;
+    if ((rc = subiter_plan_create(&c, 1, &p, &err, 2))) return fail(c, rc, "stage kernel: %s", err.c_str());
+    const int cur = c->cur;
+    for (int k = 0; k < 6; k++) {
+      c->cur = k / 3;
+      describe(p, p->h[k], k % 3, 0, c);
+    }
+    c->cur = cur;
+    if ((rc = subiter_upload(p, &err))) {
+      subiter_plan_destroy(p);
+      return fail(c, rc, "stage kernel: %s", err.c_str());
+    }
+    c->stage_plan = p;
+    c->stage_gen = c->buf_gen;
+  }
+  SubiterPlan *p = c->stage_plan;
+  EIF_CK(c, cudaMemsetAsync(p->d_res, 0, sizeof(unsigned) * p->zero_words, c->stream));
+  StageArgs a = stage_args(p, rk, p->d_desc + 3 * c->cur + rk);
+  a.reset_next = 0;
+  a.tape = tape;
+  a.contact = contact;
+  void *args[] = {&a};
+  EIF_CK(c, cudaLaunchCooperativeKernel(reinterpret_cast<void *>(k_subiterations), dim3(p->grid), dim3(SUB_THREADS), args,
+                                        sizeof(int) * ST_WORDS, c->stream));
+  EIF_LAUNCH_CK(c);
+  c->incr_zero = false;
+  c->boxes_x_valid = false;
+  c->weights_x_valid = false;
+  return EIF_OK;
 }
 
 }  // namespace eif
