@@ -83,7 +83,9 @@ __global__ void k_chunk_reduce(const double *__restrict__ partial, const int *__
                                int pcap, int np, int f0, int f1, int f2, Bounds bd) {
   const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (n >= np || !EIF_CHK(bd.rec, n + 1, bd.off, 30)) return;
-  chunk_reduce_warp(partial, off[n], off[n + 1], P, pcap, f0, f1, f2, bd, n);
+  const double v = chunk_sum_warp(partial, off[n], off[n + 1], bd);
+  const int lane = threadIdx.x & 31;
+  if (lane < 3 && EIF_CHK(bd.rec, f2 * pcap + n, bd.P, 32)) P[(lane == 0 ? f0 : (lane == 1 ? f1 : f2)) * pcap + n] = v;
 }
 
 // save: after an indicator evaluation that stored its weights in the memo (with iter:
@@ -95,7 +97,9 @@ __global__ void k_chunk_reduce_f(const float *__restrict__ partial, const int *_
   const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (n >= np || !EIF_CHK(bd.rec, n + 1, bd.off, 33)) return;
   if (save && (!iter || *iter != 0u)) memo_particle(memo, pf + (size_t)PF_WORDS * n, box + 12 * (size_t)n, off[n], n);
-  chunk_reduce_f_warp(partial, off[n], off[n + 1], P, pcap, f0, f1, f2, bd, n);
+  const double v = chunk_sum_f_warp(partial, off[n], off[n + 1], bd);
+  const int lane = threadIdx.x & 31;
+  if (lane < 3 && EIF_CHK(bd.rec, f2 * pcap + n, bd.P, 35)) P[(lane == 0 ? f0 : (lane == 1 ? f1 : f2)) * pcap + n] = v;
 }
 
 // exclusive scan of the chunk counts (one block); off[np] = total

@@ -414,83 +414,84 @@ __device__ __forceinline__ void box_part(const BoxArgs &a, int n, int sub) {
   if (on && tasks && EIF_CHK(a.bd.rec, (a.nchunk - a.bd_off_base) + n, a.bd.off, 3)) atomicAdd(a.nchunk + n, tasks);
 }
 
-// The same for one particle by one warp, into shared memory (bx: 12 ints, pf or pd: its
-// parameter block), at X + dX in a sub-iteration: the values of box_part bit for bit. An FP64
-// warp instruction holds the pipe 16 cycles whether one lane or all take part, so the divisions
-// (the boxes' bounds, the grid offsets, the quadratic form) are one division of 22 lanes; the
-// words that do not change within a stage are copied from the blocks at X. With a part of
-// box_part per warp, one lane each, this took ten times as long, most of a sub-iteration.
-__device__ __forceinline__ void box_warp(const BoxArgs &a, int n, int *bx, float *pf, double *pd) {
+// The same for one particle by the first four warps of a CTA, into shared memory (bx: 12 ints,
+// pf or pd: its parameter block), at X + dX in a sub-iteration: the values of box_part bit for
+// bit. An FP64 instruction holds its scheduler 64 cycles whether one lane or all take part and
+// whatever else the warp has ready, so the work is one instruction stream per scheduler: the
+// angle and the quadratic form (six divisions in six lanes), the boxes' bounds (twelve lanes),
+// the grid offsets (four); the words that do not change within a stage are copied from the
+// blocks at X. About 45 FP64 instructions in the longest; all in one warp took 7400 cycles, and
+// with a part of box_part per warp, one lane each, 30 000.
+__device__ __forceinline__ void box_warps(const BoxArgs &a, int n, int part, int *bx, float *pf, double *pd) {
   const double *P = a.P;
   const int pc = a.pcap, lane = threadIdx.x & 31;
-  const double pa = P[EIF_P_A * pc + n], pb = P[EIF_P_B * pc + n];
-  const double px = P[EIF_P_X * pc + n] + P[EIF_P_DX * pc + n], py = P[EIF_P_Y * pc + n] + P[EIF_P_DY * pc + n];
-  const double az = P[EIF_P_AZ * pc + n] + P[EIF_P_DAZ * pc + n];
-  const double r = fmax(pa, pb);
-  double sz, cz;
-  sincos(-az, &sz, &cz);
-  double num = 1., den = 1.;
-  if (lane < 12) {
-    // image lane / 4 - 1: imin, imax, jmin, jmax (loop_size)
-    const bool row = lane & 2;
-    const double gc = row ? py + a.ly * (double)(lane / 4 - 1) - a.yf1 : px;
-    num = lane & 1 ? gc + r : gc - r;
-    den = row ? a.dy : a.dx;
-  } else if (lane < 16) {
-    num = lane == 12 ? px : py + a.ly * (double)(lane - 14);
-    den = lane == 12 ? a.dx : a.dy;
-  } else if (lane < 22) {
-    const int k = lane - 16;
-    num = k == 0 || k == 3 ? cz * cz : (k < 3 ? sz * sz : 1.);
-    den = k == 0 || k == 2 || k == 5 ? pa * pa : pb * pb;
-  }
-  const double v = num / den;
-  if (lane < 12) {
-    const int lb = 1, ub = lane & 2 ? a.jtot : a.itot;
-    int w;
-    if (lane & 1) {
-      w = (int)(ceil(v) + NEXTRA);
-      w = w > ub ? ub : w;
-    } else {
-      w = (int)(floor(v) - NEXTRA);
-      w = w < lb ? lb : w;
-    }
-    bx[lane] = w;
-  }
-  if (pf) {
-    const float *c = a.pf + (size_t)PF_WORDS * n;
-    constexpr unsigned keep = 1u << PF_A | 1u << PF_B | 1u << PF_KEX | 1u << PF_KEY | 1u << PF_RPM | 1u << PF_RPIM |
-                              1u << PF_UX | 1u << PF_UY | 1u << PF_VZ | 1u << PF_SO2 | 1u << PF_SI2 | 1u << PF_RO2;
-    if ((keep >> lane) & 1u) pf[lane] = c[lane];
-    const double v1 = __shfl_down_sync(0xffffffffu, v, 1);
-    if (lane == 0) {
-      pf[PF_CZ] = (float)cz;
-      pf[PF_SZ] = (float)sz;
-    }
-    if (lane >= 12 && lane < 16) {
-      const int i0 = (int)floor(v);
-      pf[lane == 12 ? PF_I0 : PF_J0 + (lane - 13)] = __int_as_float(i0);
-      pf[lane == 12 ? PF_GX : PF_GY + (lane - 13)] = (float)(v - i0 + 0.5);
-    }
-    if (lane == 16) pf[PF_AL] = (float)(v + v1);
-    if (lane == 18) pf[PF_DE] = (float)(v + v1);
-    if (lane == 20) pf[PF_KA] = (float)(cz * sz * (v - v1));
-  } else {
-    const double *c = a.pd + (size_t)PD_WORDS * n;
-    // everything but the first words and those of the quadratic form
-    if (lane >= PD_A && lane < PD_F) pd[lane] = c[lane];
-    float *df = reinterpret_cast<float *>(pd + PD_F);
-    if (lane >= PDF_SO2 && lane < PDF_WORDS) df[lane] = reinterpret_cast<const float *>(c + PD_F)[lane];
-    if (lane == 0) {
-      pd[PD_X] = px;
-      pd[PD_Y] = py;
+  if (part == 0) {
+    const double pa = P[EIF_P_A * pc + n], pb = P[EIF_P_B * pc + n];
+    double sz, cz;
+    sincos(-(P[EIF_P_AZ * pc + n] + P[EIF_P_DAZ * pc + n]), &sz, &cz);
+    if (pf) {
+      // cz^2/pa^2, sz^2/pb^2, sz^2/pa^2, cz^2/pb^2, 1/pb^2, 1/pa^2
+      const double x = lane == 0 || lane == 3 ? cz : (lane < 3 ? sz : 1.);
+      const double y = lane == 0 || lane == 2 || lane == 5 ? pa : pb;
+      const double v = x * x / (y * y), v1 = __shfl_down_sync(0xffffffffu, v, 1);
+      // AL, -, DE, -, KA; CZ and SZ in the lanes between
+      const double w = lane == 4 ? cz * sz * (v - v1) : (lane == 1 ? cz : (lane == 3 ? sz : v + v1));
+      if (lane < 5) pf[lane == 0 ? PF_AL : (lane == 1 ? PF_CZ : (lane == 2 ? PF_DE : (lane == 3 ? PF_SZ : PF_KA)))] = (float)w;
+    } else if (lane == 0) {
       pd[PD_CZ] = cz * a.kb;
       pd[PD_SZ] = sz * a.kb;
+      float *df = reinterpret_cast<float *>(pd + PD_F);
       const float fa = eifd::d2f(pa), fb = eifd::d2f(pb), cf = eifd::d2f(cz), sf = eifd::d2f(sz);
       df[PDF_AL] = cf * cf / (fa * fa) + sf * sf / (fb * fb);
       df[PDF_KA] = cf * sf * (1.f / (fb * fb) - 1.f / (fa * fa));
       df[PDF_DE] = sf * sf / (fa * fa) + cf * cf / (fb * fb);
     }
+  } else if (part == 1) {
+    // lane: image lane / 4 - 1; imin, imax, jmin, jmax (loop_size)
+    const double px = P[EIF_P_X * pc + n] + P[EIF_P_DX * pc + n], py = P[EIF_P_Y * pc + n] + P[EIF_P_DY * pc + n];
+    const double r = fmax(P[EIF_P_A * pc + n], P[EIF_P_B * pc + n]);
+    const bool row = lane & 2;
+    const double gc = row ? py + a.ly * (double)(lane / 4 - 1) - a.yf1 : px;
+    const double v = (gc + (lane & 1 ? r : -r)) / (row ? a.dy : a.dx);
+    if (lane < 12) {
+      const int lb = 1, ub = row ? a.jtot : a.itot;
+      // floor, or ceil as -floor(-v)
+      const double e = floor(lane & 1 ? -v : v);
+      int w;
+      if (lane & 1) {
+        w = (int)(-e + NEXTRA);
+        w = w > ub ? ub : w;
+      } else {
+        w = (int)(e - NEXTRA);
+        w = w < lb ? lb : w;
+      }
+      bx[lane] = w;
+    }
+  } else if (part == 2) {
+    const double px = P[EIF_P_X * pc + n] + P[EIF_P_DX * pc + n], py = P[EIF_P_Y * pc + n] + P[EIF_P_DY * pc + n];
+    if (pf) {
+      const double v = (lane == 0 ? px : py + a.ly * (double)(lane - 2)) / (lane == 0 ? a.dx : a.dy);
+      const int i0 = (int)floor(v);
+      const float g = (float)(v - i0 + 0.5);
+      if (lane < 4) {
+        pf[lane == 0 ? PF_I0 : PF_J0 + (lane - 1)] = __int_as_float(i0);
+        pf[lane == 0 ? PF_GX : PF_GY + (lane - 1)] = g;
+      }
+    } else if (lane == 0) {
+      pd[PD_X] = px;
+      pd[PD_Y] = py;
+    }
+  } else if (pf) {
+    const float *c = a.pf + (size_t)PF_WORDS * n;
+    constexpr unsigned keep = 1u << PF_A | 1u << PF_B | 1u << PF_KEX | 1u << PF_KEY | 1u << PF_RPM | 1u << PF_RPIM |
+                              1u << PF_UX | 1u << PF_UY | 1u << PF_VZ | 1u << PF_SO2 | 1u << PF_SI2 | 1u << PF_RO2;
+    if ((keep >> lane) & 1u) pf[lane] = c[lane];
+  } else {
+    // everything but the first words and those of the quadratic form
+    const double *c = a.pd + (size_t)PD_WORDS * n;
+    if (lane >= PD_A && lane < PD_F) pd[lane] = c[lane];
+    float *df = reinterpret_cast<float *>(pd + PD_F);
+    if (lane >= PDF_SO2 && lane < PDF_WORDS) df[lane] = reinterpret_cast<const float *>(c + PD_F)[lane];
   }
 }
 __device__ __forceinline__ int box_tasks(const int *bx) {
@@ -1332,9 +1333,8 @@ __device__ __forceinline__ void ibm_sum_f_tasks(const WorkArgs &a, int first, in
   }
 }
 
-// sums of particle n over its chunks c0 .. c1 - 1 in a fixed order (one warp)
-__device__ __forceinline__ void chunk_reduce_warp(const double *partial, int c0, int c1, double *P, int pcap, int f0,
-                                                  int f1, int f2, const Bounds &bd, int n) {
+// sums over the chunks c0 .. c1 - 1 in a fixed order (one warp): lane k < 3 has sum k
+__device__ __forceinline__ double chunk_sum_warp(const double *partial, int c0, int c1, const Bounds &bd) {
   const int lane = threadIdx.x & 31;
   double s0 = 0., s1 = 0., s2 = 0.;
   for (int c = c0 + lane; c < c1; c += 32) {
@@ -1346,19 +1346,14 @@ __device__ __forceinline__ void chunk_reduce_warp(const double *partial, int c0,
   s0 = eifd::warp_sum(s0);
   s1 = eifd::warp_sum(s1);
   s2 = eifd::warp_sum(s2);
-  if (lane == 0 && EIF_CHK(bd.rec, f2 * pcap + n, bd.P, 32)) {
-    P[f0 * pcap + n] = s0;
-    P[f1 * pcap + n] = s1;
-    P[f2 * pcap + n] = s2;
-  }
+  return lane == 0 ? s0 : (lane == 1 ? s1 : s2);
 }
 
 // The same per-particle sums from the single-precision partials of the mixed form,
 // accumulated in double-float arithmetic (TwoSum) on the FP32 pipe: the sum of at most
 // a few hundred floats is kept to about 48 bits, and the result is rounded once to
 // double.
-__device__ __forceinline__ void chunk_reduce_f_warp(const float *partial, int c0, int c1, double *P, int pcap, int f0,
-                                                    int f1, int f2, const Bounds &bd, int n) {
+__device__ __forceinline__ double chunk_sum_f_warp(const float *partial, int c0, int c1, const Bounds &bd) {
   const int lane = threadIdx.x & 31;
   float h[3] = {0.f, 0.f, 0.f}, l[3] = {0.f, 0.f, 0.f};
   for (int c = c0 + lane; c < c1; c += 32) {
@@ -1381,11 +1376,14 @@ __device__ __forceinline__ void chunk_reduce_f_warp(const float *partial, int c0
       h[k] = s;
     }
   }
-  if (lane == 0 && EIF_CHK(bd.rec, f2 * pcap + n, bd.P, 35)) {
-    P[f0 * pcap + n] = eifd::f2d(h[0]) + eifd::f2d(l[0]);
-    P[f1 * pcap + n] = eifd::f2d(h[1]) + eifd::f2d(l[1]);
-    P[f2 * pcap + n] = eifd::f2d(h[2]) + eifd::f2d(l[2]);
+  // lane 0's (the lanes' trailing parts differ in their last bits)
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    h[k] = __shfl_sync(0xffffffffu, h[k], 0);
+    l[k] = __shfl_sync(0xffffffffu, l[k], 0);
   }
+  const float hk = lane == 0 ? h[0] : (lane == 1 ? h[1] : h[2]), lk = lane == 0 ? l[0] : (lane == 1 ? l[1] : l[2]);
+  return eifd::f2d(hk) + eifd::f2d(lk);
 }
 
 // The geometry words (pf: PF_WORDS words), boxes (12 ints) and first task c0 of particle n to

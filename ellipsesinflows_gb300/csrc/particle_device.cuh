@@ -466,38 +466,44 @@ __device__ __forceinline__ void collision_block(const Places &where, double *P, 
   }
 }
 
-// increment.c:10-72 for particle n: new increments from the forces, inertia integrals
-// and collision forces of the sub-iteration, the position increments from them; returns
-// res raised to the largest change of the velocity increments; pos (optional): the centre
-// X^k + dX of the new increments, rounded as load_pv forms it from the records, and near the
-// partner search's values of it
+// increment.c:10-72, one component (x, y or the rotation) of a particle: the new velocity
+// increment from the collision forces c0, c1, the fluid force f, the inertia integrals i0, i1 and
+// the constant part g (gravity_increment in x), and the position increment from it. Every
+// rounding is explicit: the kernels that form increments give the same bits.
+__device__ __forceinline__ double velocity_increment(double hgd, double dt, double c0, double c1, double f, double i0,
+                                                     double i1) {
+  return __dadd_rn(fma(hgd, __dadd_rn(c0, c1), __dmul_rn(dt, f)), __dadd_rn(i1, -i0));
+}
+__device__ __forceinline__ double gravity_increment(double gamma, double dt, double den, double Fr2) {
+  return __ddiv_rn(__dmul_rn(__dmul_rn(gamma, dt), __dadd_rn(1., -den)), Fr2);
+}
+__device__ __forceinline__ double position_increment(double hgd, double u, double du) {
+  return __dmul_rn(hgd, __dadd_rn(u, __dadd_rn(u, du)));
+}
+
+// the three components of particle n (one thread); returns res raised to the largest change of
+// the velocity increments
 __device__ __forceinline__ double increment_particle(double *p, int pcap, int n, double gamma, double Fr2, double dt,
-                                                     double res, double2 *pos = nullptr, float4 *near = nullptr) {
-  const double den = p[EIF_P_DEN * pcap + n];
+                                                     double res) {
   const double px = p[EIF_P_DUX * pcap + n], py = p[EIF_P_DUY * pcap + n], pz = p[EIF_P_DVZ * pcap + n];
-  const double hgd = 0.5 * gamma * dt;
-  const double dux = hgd * (p[EIF_P_CFX0 * pcap + n] + p[EIF_P_CFX1 * pcap + n]) + dt * p[EIF_P_FUX * pcap + n] +
-                     (p[EIF_P_IUX1 * pcap + n] - p[EIF_P_IUX0 * pcap + n]) + 1.0 * gamma * dt * (1. - den) / Fr2;
-  const double duy = hgd * (p[EIF_P_CFY0 * pcap + n] + p[EIF_P_CFY1 * pcap + n]) + dt * p[EIF_P_FUY * pcap + n] +
-                     (p[EIF_P_IUY1 * pcap + n] - p[EIF_P_IUY0 * pcap + n]);
-  const double dvz = hgd * (p[EIF_P_CTZ0 * pcap + n] + p[EIF_P_CTZ1 * pcap + n]) + dt * p[EIF_P_TVZ * pcap + n] +
-                     (p[EIF_P_IVZ1 * pcap + n] - p[EIF_P_IVZ0 * pcap + n]);
+  const double hgd = __dmul_rn(0.5 * gamma, dt);
+  const double dux =
+      __dadd_rn(velocity_increment(hgd, dt, p[EIF_P_CFX0 * pcap + n], p[EIF_P_CFX1 * pcap + n], p[EIF_P_FUX * pcap + n],
+                                   p[EIF_P_IUX0 * pcap + n], p[EIF_P_IUX1 * pcap + n]),
+                gravity_increment(gamma, dt, p[EIF_P_DEN * pcap + n], Fr2));
+  const double duy = velocity_increment(hgd, dt, p[EIF_P_CFY0 * pcap + n], p[EIF_P_CFY1 * pcap + n],
+                                        p[EIF_P_FUY * pcap + n], p[EIF_P_IUY0 * pcap + n], p[EIF_P_IUY1 * pcap + n]);
+  const double dvz = velocity_increment(hgd, dt, p[EIF_P_CTZ0 * pcap + n], p[EIF_P_CTZ1 * pcap + n],
+                                        p[EIF_P_TVZ * pcap + n], p[EIF_P_IVZ0 * pcap + n], p[EIF_P_IVZ1 * pcap + n]);
   p[EIF_P_DUX * pcap + n] = dux;
   p[EIF_P_DUY * pcap + n] = duy;
   p[EIF_P_DVZ * pcap + n] = dvz;
   res = fmax(res, fabs(dux - px));
   res = fmax(res, fabs(duy - py));
   res = fmax(res, fabs(dvz - pz));
-  const double ux0 = p[EIF_P_UX * pcap + n], uy0 = p[EIF_P_UY * pcap + n], vz0 = p[EIF_P_VZ * pcap + n];
-  const double dx = hgd * (ux0 + (ux0 + dux)), dy = hgd * (uy0 + (uy0 + duy));
-  p[EIF_P_DX * pcap + n] = dx;
-  p[EIF_P_DY * pcap + n] = dy;
-  if (pos) {
-    const double2 c = make_double2(__dadd_rn(p[EIF_P_X * pcap + n], dx), __dadd_rn(p[EIF_P_Y * pcap + n], dy));
-    pos[n] = c;
-    near[n] = make_float4(eifd::d2f(c.x), eifd::d2f(c.y), eifd::d2f(fmax(p[EIF_P_A * pcap + n], p[EIF_P_B * pcap + n])), 0.f);
-  }
-  p[EIF_P_DAZ * pcap + n] = hgd * (vz0 + (vz0 + dvz));
+  p[EIF_P_DX * pcap + n] = position_increment(hgd, p[EIF_P_UX * pcap + n], dux);
+  p[EIF_P_DY * pcap + n] = position_increment(hgd, p[EIF_P_UY * pcap + n], duy);
+  p[EIF_P_DAZ * pcap + n] = position_increment(hgd, p[EIF_P_VZ * pcap + n], dvz);
   return res;
 }
 

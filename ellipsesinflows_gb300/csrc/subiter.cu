@@ -6,7 +6,7 @@
 // work of one is a list of units, the collision forces of PAIR_WARPS particles each, and for
 // every particle ns slices of the row tasks of its inertia integrals:
 //  * a slice forms the boxes and parameters of its particle at X + dX in shared memory
-//    (box_warp) and runs its share of the particle's tasks, a warp per task; in the first
+//    (box_warps) and runs its share of the particle's tasks, a warp per task; in the first
 //    sub-iteration, where the increments are zero, it runs the
 //    stage front's tasks with their stored weights;
 //  * every unit counts itself at its particles; the last one of a particle sums the tasks,
@@ -134,29 +134,63 @@ __device__ __forceinline__ bool unit_done(const SubDesc &d, int n, int lane) {
   return last != 0u;
 }
 
-// the particle's sums and increments (one warp), after its last unit
-__device__ __forceinline__ void finish_particle(const SubDesc &d, int n, unsigned it, unsigned long long *res,
-                                                double *tape, int *contact) {
-  const bool first = it == 0u;
-  const int c0 = first ? d.off[n] : d.base[n], c1 = first ? d.off[n + 1] : c0 + d.cnt[n];
-  if (d.mixed)
-    chunk_reduce_f_warp(reinterpret_cast<const float *>(d.work.partial), c0, c1, d.P, d.pcap, EIF_P_IUX0 + 1,
-                        EIF_P_IUY0 + 1, EIF_P_IVZ0 + 1, d.box.bd, n);
-  else
-    chunk_reduce_warp(d.work.partial, c0, c1, d.P, d.pcap, EIF_P_IUX0 + 1, EIF_P_IUY0 + 1, EIF_P_IVZ0 + 1, d.box.bd, n);
-  if ((threadIdx.x & 31) == 0) {
-    const double r = increment_particle(d.P, d.pcap, n, d.gamma, d.Fr2, d.scal[0], 0., d.pos[(it + 1u) & 1u], d.near[(it + 1u) & 1u]);
-    if (r > 0.) atomicMax(res, (unsigned long long)__double_as_longlong(r));
+// What a particle's increments need and no unit of the sub-iteration writes, component k in
+// lane k < 3 (x, y, rotation): loaded before the units are counted, so that the loads and the
+// gravity's division are in flight with the counter's round trip.
+struct FinishIn {
+  double c0, f, i0, u, du, x, g, dt;
+};
+__device__ __forceinline__ FinishIn finish_load(const SubDesc &d, int n) {
+  const int k = min(threadIdx.x & 31u, 2u);
+  const double *p = d.P + n;
+  const int pc = d.pcap;
+  FinishIn v;
+  v.c0 = p[(k == 0 ? EIF_P_CFX0 : (k == 1 ? EIF_P_CFY0 : EIF_P_CTZ0)) * pc];
+  v.f = p[(k == 0 ? EIF_P_FUX : (k == 1 ? EIF_P_FUY : EIF_P_TVZ)) * pc];
+  v.i0 = p[(k == 0 ? EIF_P_IUX0 : (k == 1 ? EIF_P_IUY0 : EIF_P_IVZ0)) * pc];
+  v.u = p[(k == 0 ? EIF_P_UX : (k == 1 ? EIF_P_UY : EIF_P_VZ)) * pc];
+  v.du = p[(k == 0 ? EIF_P_DUX : (k == 1 ? EIF_P_DUY : EIF_P_DVZ)) * pc];
+  v.x = p[(k == 1 ? EIF_P_Y : EIF_P_X) * pc];
+  v.dt = d.scal[0];
+  v.g = k == 0 ? gravity_increment(d.gamma, v.dt, p[EIF_P_DEN * pc], d.Fr2) : 0.;
+  return v;
+}
+
+// the particle's sums over its tasks q0 .. q1 - 1 and its increments (one warp), after its last unit
+__device__ __forceinline__ void finish_particle(const SubDesc &d, int n, unsigned it, int q0, int q1,
+                                                unsigned long long *res, const FinishIn &v, double *tape, int *contact) {
+  const int lane = threadIdx.x & 31, k = min(lane, 2), pc = d.pcap;
+  double *p = d.P + n;
+  const double c1 = p[(k == 0 ? EIF_P_CFX1 : (k == 1 ? EIF_P_CFY1 : EIF_P_CTZ1)) * pc];
+  const double i1 = d.mixed ? chunk_sum_f_warp(reinterpret_cast<const float *>(d.work.partial), q0, q1, d.box.bd)
+                            : chunk_sum_warp(d.work.partial, q0, q1, d.box.bd);
+  const double hgd = __dmul_rn(0.5 * d.gamma, v.dt);
+  double du = velocity_increment(hgd, v.dt, v.c0, c1, v.f, v.i0, i1);
+  if (k == 0) du = __dadd_rn(du, v.g);
+  const double dx = position_increment(hgd, v.u, du);
+  const double at = __dadd_rn(v.x, dx);
+  // the largest change of the three as bits (non-negative; a NaN does not count, as in fmax)
+  const double change = fabs(du - v.du);
+  long long r = change > 0. ? __double_as_longlong(change) : 0ll;
+  if (lane < 3) {
+    p[(k == 0 ? EIF_P_IUX1 : (k == 1 ? EIF_P_IUY1 : EIF_P_IVZ1)) * pc] = i1;
+    p[(k == 0 ? EIF_P_DUX : (k == 1 ? EIF_P_DUY : EIF_P_DVZ)) * pc] = du;
+    p[(k == 0 ? EIF_P_DX : (k == 1 ? EIF_P_DY : EIF_P_DAZ)) * pc] = dx;
+    const unsigned o = (it + 1u) & 1u;
+    // the centre, rounded as load_pv forms it from the records, and pair_prefilter's values of it
+    if (k < 2) {
+      reinterpret_cast<double *>(d.pos[o] + n)[k] = at;
+      reinterpret_cast<float *>(d.near[o] + n)[k] = eifd::d2f(at);
+    } else {
+      reinterpret_cast<float *>(d.near[o] + n)[2] = eifd::d2f(fmax(p[EIF_P_A * pc], p[EIF_P_B * pc]));
+    }
     if (tape) {
-      double *t = tape + (size_t)3 * d.np * (it + 1u) + n;
-      t[0] = d.P[EIF_P_DX * d.pcap + n];
-      t[d.np] = d.P[EIF_P_DY * d.pcap + n];
-      t[2 * (size_t)d.np] = d.P[EIF_P_DAZ * d.pcap + n];
-      bool any = false;
-      for (int f = EIF_P_CFX0; f <= EIF_P_CTZ1; f++) any |= d.P[f * d.pcap + n] != 0.;
-      if (any) *contact = 1;
+      tape[(size_t)3 * d.np * (it + 1u) + (size_t)k * d.np + n] = dx;
+      if (v.c0 != 0. || c1 != 0.) *contact = 1;
     }
   }
+  r = max(r, max(__shfl_sync(0xffffffffu, r, 1), __shfl_sync(0xffffffffu, r, 2)));
+  if (lane == 0 && r > 0ll) atomicMax(res, (unsigned long long)r);
 }
 
 __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
@@ -167,6 +201,11 @@ __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
   __shared__ __align__(16) float pf[PF_WORDS];
   __shared__ __align__(16) double pd[PD_WORDS];
   __shared__ int unit[2];                  // suspension and unit within it
+  // the descriptor of the suspension at hand: read in nearly every instruction of the units,
+  // and from global memory again after every acquire (which empties L1)
+  __shared__ __align__(16) unsigned sd_words[(sizeof(SubDesc) + 15) / 16 * 4];
+  const SubDesc &d = *reinterpret_cast<const SubDesc *>(sd_words);
+  int have = -1;
   extern __shared__ int stab[];            // ST_WORDS per suspension
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int G = gridDim.x, n = s.n;
@@ -245,16 +284,30 @@ __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
       if (j < 0) break;
       const bool coll = unit[1] >= (1 << 30);
       const int q = unit[1] & ((1 << 30) - 1);
-      const SubDesc &d = s.d[j];
+      if (j != have) {
+        const unsigned *src = reinterpret_cast<const unsigned *>(s.d + j);
+        for (int w = threadIdx.x; w < (int)(sizeof(SubDesc) / sizeof(unsigned)); w += SUB_THREADS) sd_words[w] = src[w];
+        have = j;
+        __syncthreads();
+      }
       unsigned long long *res = s.res + 3 * j + m3;
       if (coll) {
         collision_block(it > 0 ? Places{d.pos[it & 1u], d.near[it & 1u], false} : Places{nullptr, nullptr, true}, d.P, d.pcap, d.np, 1, d.ly, d.lx, d.flags, q);
         const int k = q * PAIR_WARPS + wl;
-        if (k < d.np && unit_done(d, k, lane)) finish_particle(d, k, it, res, s.tape, s.contact);
+        if (k < d.np) {
+          const FinishIn in = finish_load(d, k);
+          const int c0 = it == 0 ? d.off[k] : d.base[k];
+          if (unit_done(d, k, lane))
+            finish_particle(d, k, it, c0, it == 0 ? d.off[k + 1] : c0 + d.cnt[k], res, in, s.tape, s.contact);
+        }
       } else {
         const int p = q / d.ns, sl = q - p * d.ns;
+        FinishIn in;
+        if (wl == SUB_WARPS - 1) in = finish_load(d, p);
+        int c0, cnt;
         if (it == 0) {
-          const int c0 = d.off[p], cnt = d.off[p + 1] - c0;
+          c0 = d.off[p];
+          cnt = d.off[p + 1] - c0;
           const int r0 = (int)((long long)cnt * sl / d.ns), r1 = (int)((long long)cnt * (sl + 1) / d.ns);
           if (d.mixed) {
             ibm_sum_f_tasks<false>(d.work, c0 + r0 + wl, SUB_WARPS, c0 + r1);
@@ -263,21 +316,22 @@ __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
             ibm_work_tasks<false>(d.work, 2, c0 + r0 + wl, SUB_WARPS, slot_d[wl], &one);
           }
         } else {
-          if (wl == 0) box_warp(d.box, p, bx, d.mixed ? pf : nullptr, pd);
+          if (wl < 4) box_warps(d.box, p, wl, bx, d.mixed ? pf : nullptr, pd);
           __syncthreads();
-          const int cnt = box_tasks(bx);
+          c0 = d.base[p];
+          cnt = box_tasks(bx);
           const int r0 = (int)((long long)cnt * sl / d.ns), r1 = (int)((long long)cnt * (sl + 1) / d.ns);
-          const OneParticle one{reinterpret_cast<const int4 *>(bx), pf, pd, p, d.base[p], r1};
+          const OneParticle one{reinterpret_cast<const int4 *>(bx), pf, pd, p, c0, r1};
           if (d.mixed) {
             ibm_work_f_tasks<false, true>(d.work, 0, r0 + wl, SUB_WARPS, slot_f[wl], &one);
-            if (sl == 0 && wl == SUB_WARPS - 1 && d.work.memo_mode == 2) memo_particle(d.work.memo, pf, bx, one.base, p);
+            if (sl == 0 && wl == SUB_WARPS - 2 && d.work.memo_mode == 2) memo_particle(d.work.memo, pf, bx, one.base, p);
           } else {
             ibm_work_tasks<false>(d.work, 0, r0 + wl, SUB_WARPS, slot_d[wl], &one);
           }
           if (threadIdx.x == 0) d.cnt[p] = cnt;
         }
         __syncthreads();
-        if (wl == 0 && unit_done(d, p, lane)) finish_particle(d, p, it, res, s.tape, s.contact);
+        if (wl == SUB_WARPS - 1 && unit_done(d, p, lane)) finish_particle(d, p, it, c0, c0 + cnt, res, in, s.tape, s.contact);
       }
       if (units <= G) break;
     }
@@ -293,10 +347,10 @@ __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
         stop = true;
       }
       if (blockIdx.x == 0) {
-        const SubDesc &d = s.d[j];
-        d.scal[1] = r;
-        *d.counter = count;
-        *d.total += 1ull;
+        const SubDesc &e = s.d[j];
+        e.scal[1] = r;
+        *e.counter = count;
+        *e.total += 1ull;
       }
     }
     changed = __syncthreads_or(stop);
@@ -317,10 +371,10 @@ __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
   for (int j = 0; j < n; j++) {
     const int np = stab[ST_WORDS * j + ST_NP];
     if (at < np) {
-      const SubDesc &d = s.d[j];
+      const SubDesc &e = s.d[j];
       for (int m = at; m < np; m += T) {
-        update_particle(d.P, d.pcap, m, d.ly);
-        if (s.reset_next) reset_particle(d.P, d.pcap, m);
+        update_particle(e.P, e.pcap, m, e.ly);
+        if (s.reset_next) reset_particle(e.P, e.pcap, m);
       }
     }
     at = (at + T - np % T) % T;   // the suspensions' particles spread over all CTAs
@@ -399,8 +453,8 @@ int subiter_plan_create(eif_ctx *const *ctx, int n, SubiterPlan **out, std::stri
   SubiterPlan *p = new (std::nothrow) SubiterPlan;
   if (!p) return EIF_ERR_NOMEM;
   p->n = n;
-  // slices: as many as give every warp of the GPU a task when the particles are few, none
-  // without a task for each of its warps
+  // slices: as many as give every CTA of the GPU a unit when the particles are few, none
+  // without four tasks, one for each scheduler of an SM
   const int most = occ * ctx[0]->sms;
   long long units = 0;
   for (int j = 0; j < n; j++) {
@@ -409,7 +463,7 @@ int subiter_plan_create(eif_ctx *const *ctx, int n, SubiterPlan **out, std::stri
   }
   for (int j = 0; j < n; j++) {
     const int by_gpu = std::max(1, most / std::max(1, p->np));
-    const int by_tasks = std::max(1, (ctx[j]->max_tasks + SUB_WARPS - 1) / SUB_WARPS);
+    const int by_tasks = std::max(1, (ctx[j]->max_tasks + 3) / 4);
     p->ns.push_back(std::min(by_gpu, by_tasks));
     units += (long long)ctx[j]->np * p->ns[j] + (ctx[j]->np + PAIR_WARPS - 1) / PAIR_WARPS;
   }
