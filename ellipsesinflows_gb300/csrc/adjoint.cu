@@ -931,6 +931,9 @@ int eif_adjoint_pull(eif_ctx *c, double *ux_bar, double *uy_bar, double *p_bar) 
   const size_t dp = sizeof(double) * c->ld;
   const int rows = c->jtot + 2;
   const size_t wx = sizeof(double) * (c->itot + 1), wy = sizeof(double) * (c->itot + 2);
+  if (ux_bar) touch_pages(ux_bar, wx * rows);
+  if (uy_bar) touch_pages(uy_bar, wy * rows);
+  if (p_bar) touch_pages(p_bar, wy * rows);
   if (ux_bar) EIF_CK(c, cudaMemcpy2DAsync(ux_bar, wx, a->ub, dp, wx, rows, cudaMemcpyDeviceToHost, c->stream));
   if (uy_bar) EIF_CK(c, cudaMemcpy2DAsync(uy_bar, wy, a->vb, dp, wy, rows, cudaMemcpyDeviceToHost, c->stream));
   if (p_bar) EIF_CK(c, cudaMemcpy2DAsync(p_bar, wy, a->pb, dp, wy, rows, cudaMemcpyDeviceToHost, c->stream));

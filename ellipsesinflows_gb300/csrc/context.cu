@@ -48,6 +48,18 @@ int check_records(eif_ctx *c) {
   return fail(c, EIF_ERR_CUDA, "bounds guard %llu: index %llu outside [0, %llu)", tag, idx, bound);
 }
 
+void touch_pages(void *p, size_t bytes) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if (at.type != cudaMemoryTypeUnregistered) return;
+  volatile char *q = static_cast<volatile char *>(p);
+  for (size_t k = 0; k < bytes; k += 4096) q[k] = 0;
+  if (bytes) q[bytes - 1] = 0;
+}
+
 // Particle-only work beside the fluid kernels. The kernels of a stage and their
 // data dependences are unchanged; work that shares no buffer with the fluid kernels
 // launched in between is moved to the side stream, which forks from the main stream
@@ -226,6 +238,7 @@ int rows_out(eif_ctx *c, double *host, const double *src, int w, int rows, cudaS
     EIF_LAUNCH_CK(c);
     return EIF_OK;
   }
+  if (!engine) touch_pages(host, sizeof(double) * w * rows);
   EIF_CK(c, cudaMemcpy2DAsync(host, sizeof(double) * w, src, sizeof(double) * c->ld, sizeof(double) * w, rows,
                               cudaMemcpyDeviceToHost, stream));
   return EIF_OK;

@@ -162,7 +162,9 @@ int eif_stats_pull(eif_ctx *c, double *ux1, double *ux2, double *uy1, double *uy
   const int rows = c->jtot + 2;
   const size_t wx = sizeof(double) * (c->itot + 1), wy = sizeof(double) * (c->itot + 2);
   auto pull = [&](double *dst, const double *src, size_t w) -> int {
-    if (dst) EIF_CK(c, cudaMemcpy2DAsync(dst, w, src, dp, w, rows, cudaMemcpyDeviceToHost, c->stream));
+    if (!dst) return EIF_OK;
+    touch_pages(dst, w * rows);
+    EIF_CK(c, cudaMemcpy2DAsync(dst, w, src, dp, w, rows, cudaMemcpyDeviceToHost, c->stream));
     return EIF_OK;
   };
   int rc;
