@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(TT_WARPS * 32) k_task_table_scan(const int *__
 // bits.
 __global__ void __launch_bounds__(256, 3) k_ibm_work(WorkArgs a) {
   // per warp: its near cells, their feet and their weights
-  __shared__ double2 slot_buf[8][WORK_SLOTS];
+  __shared__ WorkSlots slot_buf[8];
   const int wmode = a.iter ? (*a.iter == 0u ? 2 : 0) : a.wmode;
   ibm_work_tasks<false>(a, wmode, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
                         slot_buf[threadIdx.x >> 5], nullptr);
@@ -426,13 +426,20 @@ int ibm_reserve(eif_ctx *c, size_t chunks) {
   if (c->cfg.precision == EIF_PREC_MIXED) EIF_CK(c, cudaMalloc((void **)&c->pf, sizeof(float) * PF_WORDS * c->np));
   else EIF_CK(c, cudaMalloc((void **)&c->pd, sizeof(double) * PD_WORDS * c->np));
   if (c->cfg.precision != EIF_PREC_MIXED && !c->tanh_tab) {
-    std::vector<double2> tab(TANH_N);
+    // tanh_tab's values, then tanh_mid's (float pairs)
+    std::vector<double2> tab(TANH_N + (MID_N + 1) / 2);
     for (int k = 0; k < TANH_N; k++) {
       const long double z = (long double)k / TANH_STEPS, ch = coshl(z);
       tab[k] = make_double2((double)tanhl(z), (double)(1.L / (ch * ch)));
     }
-    EIF_CK(c, cudaMalloc((void **)&c->tanh_tab, sizeof(double2) * TANH_N));
-    EIF_CK(c, cudaMemcpy(c->tanh_tab, tab.data(), sizeof(double2) * TANH_N, cudaMemcpyHostToDevice));
+    float2 *mid = reinterpret_cast<float2 *>(tab.data() + TANH_N);
+    for (int k = 0; k < MID_N; k++) {
+      const long double x = 2.L * expl(-2.L * (MID_Z0 + (long double)k / MID_STEPS));
+      const float hi = (float)x;
+      mid[k] = make_float2(hi, (float)(x - (long double)hi));
+    }
+    EIF_CK(c, cudaMalloc((void **)&c->tanh_tab, sizeof(double2) * tab.size()));
+    EIF_CK(c, cudaMemcpy(c->tanh_tab, tab.data(), sizeof(double2) * tab.size(), cudaMemcpyHostToDevice));
   }
   EIF_CK(c, cudaMalloc((void **)&c->tdesc, sizeof(int4) * (size_t)chunks));
   const int nbands = (c->jtot + GTY - 1) / GTY;

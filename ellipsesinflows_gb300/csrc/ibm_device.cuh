@@ -21,6 +21,7 @@
 // one instantiation of it.
 #pragma once
 #include "eif_internal.cuh"
+#include "eif_df.cuh"
 #include "foot_device.cuh"
 #include <cfloat>
 
@@ -54,14 +55,17 @@ __device__ __forceinline__ float normal_t_f(const EllF &e, float x_, float y_) {
 // the stored-weight sums took 0.95 ms at 2048 x 4096 with 2048 ellipses that way, nearly
 // all of it this set-up). Lengths with a bar are in units of h / BETA, so that the distance
 // the cells compute is the argument of tanh.
-constexpr int PD_WORDS = 14;
+constexpr int PD_WORDS = 20;
 enum { PD_X, PD_Y,            // centre (with the increments where the boxes have them)
        PD_CZ, PD_SZ,          // cos(-az), sin(-az) times BETA / h
        PD_A, PD_B,            // semi-axes, barred
        PD_RPM, PD_RPIM,       // 1 / mass, 1 / moment of inertia
+       PD_QM, PD_QIM,         // dx dy / 4 over them, the factors of the inertia sums
        PD_F };                // single-precision words from here:
 enum { PDF_AL, PDF_KA, PDF_DE, PDF_SO2, PDF_SI2, PDF_RO2,   // row_chords
-       PDF_A, PDF_B, PDF_KEX, PDF_KEY, PDF_WORDS };         // the foot iteration, barred
+       PDF_A, PDF_B, PDF_KEX, PDF_KEY,                      // the foot iteration, barred
+       PDF_PAIRS,                   // PD_A, PD_B, PD_CZ, PD_SZ as float pairs (dist_mid)
+       PDF_WORDS = PDF_PAIRS + 8 };
 static_assert(2 * (PD_WORDS - PD_F) >= PDF_WORDS && PD_WORDS % 2 == 0, "per-particle parameter block");
 
 // The iteration of ellipse.c:30-65 in double precision with its stopping rule and cap, from
@@ -92,10 +96,11 @@ __device__ __noinline__ double normal_t_q1(double a, double b, double px, double
 
 // The normal foot of (px, py), first quadrant, in single precision: (c, s) = (cos t, sin t)
 // to about 2e-7 (the iteration above, whose hardware sines shift its fixed point a little,
-// and one Newton step, d); returns the distance to the foot, positive outside.
-__device__ __forceinline__ float foot_f(const EllF &e, float px, float py, float &c, float &s, float &d) {
+// and one Newton step, d); returns the distance to the foot, positive outside. Out of line:
+// inlined into the loops around it, the compiler makes 45 KB of copies of it.
+__device__ __noinline__ float foot_f(const EllF &e, float px, float py, float &c, float &s, float &d) {
   const float t = normal_t_f_q1(e, px, py);
-  sincosf(t, &s, &c);
+  sincospif(t * 0.318309886f, &s, &c);
   float ac = e.a * c, bs = e.b * s, as = e.a * s, bc = e.b * c;
   float vx = px - ac, vy = py - bs;
   const float K = as * as + bc * bc + vx * ac + vy * bs;
@@ -112,7 +117,8 @@ __device__ __forceinline__ float foot_f(const EllF &e, float px, float py, float
 // The same foot and distance in double precision, from foot_f's (c0, s0). Bound by the FP64
 // pipe (one warp instruction in 16 cycles), so the double-precision work is kept to what
 // carries the precision:
-//  * (c, s) is put on the unit circle in double precision;
+//  * (c, s) is put on the unit circle in double precision; what is left of c^2 + s^2 - 1
+//    (its rounding, the largest of the distance's errors) is taken off the distance;
 //  * with v = (px, py) - (a c, b s), T the derivative of the ellipse in t (w = |T|) and N
 //    its outward normal, the remaining angle to the foot is d = v.T / K,
 //    K = w^2 + v.(a c, b s) = w^2 (1 + nu / R) with nu = v.N / w the distance to the
@@ -121,7 +127,7 @@ __device__ __forceinline__ float foot_f(const EllF &e, float px, float py, float
 //    double precision, the correction and d only single;
 //  * for |d| <= FOOT_TOL the terms left out are below 1e-16 a; a larger d is taken as a
 //    Newton step (rare: the start is closer than that nearly everywhere).
-// 28 FP64 instructions against about 460 for two passes of ellipse.c's iteration with their
+// 31 FP64 instructions against about 460 for two passes of ellipse.c's iteration with their
 // sincos, asin, square roots and divisions. NORMAL: the outward normal (nx, ny) as well, for
 // which the foot itself is iterated to 1e-12 (one more step). Returns false next to the
 // evolute (K small, or no convergence): the caller takes the general iteration.
@@ -155,7 +161,7 @@ __device__ __forceinline__ bool foot_d(double a, double b, float abf, float c0, 
       const double y0 = eifd::f2d(rw);
       const double e = fma(-(w2 * y0), y0, 1.);
       const double p = e * fma(e, 0.375, 0.5);
-      const double u = nw * y0;
+      const double u = fma(eifd::f2d(0.5f * abf), fma(c, c, fma(s, s, -1.)), nw) * y0;
       dist = fma(u, p, u) + eifd::f2d(corr);
       if (NORMAL) {
         const double y = fma(y0, p, y0);
@@ -195,6 +201,23 @@ __device__ __forceinline__ double tanh_tab(double z, const double2 *__restrict__
   return ts.x + fma(q, fma(e, e, e), q);
 }
 
+// the distance and the normal next to the evolute, by ellipse.c's iteration
+__device__ __noinline__ double foot_general(double a, double b, double px, double py, float c0, float s0, double &nx,
+                                            double &ny) {
+  const double t = normal_t_q1(a, b, px, py, eifd::f2d(fminf(fmaxf(atan2f(s0, c0), 0.f), 1.5707963f)));
+  double st, ct;
+  sincos(t, &st, &ct);
+  const double fx = px - a * ct, fy = py - b * st;
+  const bool in = 1. - (px / a) * (px / a) - (py / b) * (py / b) > 0.;
+  const double d = sqrt(fx * fx + fy * fy);
+  nx = ct / a;
+  ny = st / b;
+  const double nn = 1. / sqrt(nx * nx + ny * ny);
+  nx *= nn;
+  ny *= nn;
+  return in ? -d : d;
+}
+
 // tanh(BETA D) of the signed distance D in units of h (auxiliary.c:19-59), positive
 // inside, from the barred body-frame offset (x_, y_) and foot_f's (c0, s0); NORMAL: the
 // outward unit normal at the foot in the body frame
@@ -203,22 +226,7 @@ __device__ __forceinline__ double indicator_d(double a, double b, float abf, flo
                                               const double2 *__restrict__ tab, double &nx, double &ny) {
   const double px = fabs(x_), py = fabs(y_);
   double dist;
-  if (!foot_d<NORMAL>(a, b, abf, c0, s0, px, py, dist, nx, ny)) {
-    const double t = normal_t_q1(a, b, px, py, eifd::f2d(fminf(fmaxf(atan2f(s0, c0), 0.f), 1.5707963f)));
-    double st, ct;
-    sincos(t, &st, &ct);
-    const double fx = px - a * ct, fy = py - b * st;
-    const bool in = 1. - (px / a) * (px / a) - (py / b) * (py / b) > 0.;
-    dist = sqrt(fx * fx + fy * fy);
-    if (in) dist = -dist;
-    if (NORMAL) {
-      nx = ct / a;
-      ny = st / b;
-      const double nn = 1. / sqrt(nx * nx + ny * ny);
-      nx *= nn;
-      ny *= nn;
-    }
-  }
+  if (!foot_d<NORMAL>(a, b, abf, c0, s0, px, py, dist, nx, ny)) dist = foot_general(a, b, px, py, c0, s0, nx, ny);
   if (NORMAL) {
     if (x_ < 0.) nx = -nx;
     if (y_ < 0.) ny = -ny;
@@ -227,17 +235,65 @@ __device__ __forceinline__ double indicator_d(double a, double b, float abf, flo
   return __double2hiint(dist) < 0 ? th : -th;
 }
 
-// Cells of which single precision gives tanh(BETA D) to the last bit of the double: with z
-// = |BETA D|, tanh z = 1 - x, x = 2 / (exp(2 z) + 1), and an error dz of the distance changes
-// it by 4 exp(-2 z) dz. foot_f's distance is good to about 1e-6 of the major semi-axis A (in
-// the same barred units) once its Newton step is below 1e-3; at z >= 14 + A / 200 the change is below 3e-17, for every A. Such
-// cells (7 cells from the interface and farther) leave the FP64 pipe nothing but the
-// subtraction.
-__device__ __forceinline__ float z_single(float A) { return fmaf(0.005f, A, 14.f); }
-__device__ __forceinline__ double tanh_far(float dist) {
-  const float x = 2.f * __expf(-2.f * fabsf(dist));   // exp(-2 z) < 1e-12: the 1 + exp is 1
-  const double th = 1. - eifd::f2d(x);
-  return dist < 0.f ? th : -th;
+// Cells whose tanh(BETA D) the FP32 pipe gives to the last bit of the double: with z = |BETA D|,
+// tanh z = 1 - x, x = 2 / (exp(2 z) + 1), and an error dz of the distance changes it by
+// 4 exp(-2 z) dz.
+// foot_f's foot (once its Newton step is below 1e-3) and the distance and x in double-float
+// arithmetic (dist_mid, good to 1e-13 rms and 2e-12 at A = 48, in proportion to A; tanh_mid) leave
+// less than 1e-17 rms at z >= 6 + A / 400 for every major semi-axis A (in the same barred units).
+// Only the cells within three of the interface are left to the FP64 pipe, a pass of 32 of them
+// being as long as 3000 instructions of the FP32 pipe.
+__device__ __forceinline__ float z_mid(float A) { return fmaf(0.0025f, A, 6.f); }
+// (1 - m 2^-53) with the sign of -dist; the doubles below 1 are 2^-53 apart
+__device__ __forceinline__ double tanh_of(long long m, float dist) {
+  const long long b = 0x3ff0000000000000ll - m;
+  return __longlong_as_double(dist < 0.f ? b : b | (long long)0x8000000000000000ull);
+}
+
+using eifdf::DF;
+// product with a single
+__device__ __forceinline__ DF df_mulf(DF x, float y) {
+  const float p = x.hi * y;
+  return eifdf::fast_sum(p, fmaf(x.lo, y, fmaf(x.hi, y, -p)));
+}
+// The distance of foot_d (positive outside) for offsets (x, y) in the first quadrant, from
+// foot_f's (c, s), put back onto the unit circle as far as single precision goes; what is left
+// of c^2 + s^2 - 1 is taken off the distance.
+__device__ __forceinline__ DF dist_mid(DF a, DF b, float abf, float c, float s, DF x, DF y) {
+  const float n = fmaf(-0.5f, fmaf(c, c, fmaf(s, s, -1.f)), 1.f);
+  c *= n;
+  s *= n;
+  const DF vx = eifdf::df_add_nw(x, eifdf::df_neg(df_mulf(a, c))), vy = eifdf::df_add_nw(y, eifdf::df_neg(df_mulf(b, s)));
+  const DF as = df_mulf(a, s), bc = df_mulf(b, c);
+  const DF nw = eifdf::df_add_nw(eifdf::df_mul(vx, bc), eifdf::df_mul(vy, as));
+  const DF w2 = eifdf::df_add_nw(eifdf::df_mul(as, as), eifdf::df_mul(bc, bc));
+  const float p = c * c, q = s * s;
+  const float rho = ((fmaxf(p, q) - 1.f) + fminf(p, q)) + (fmaf(c, c, -p) + fmaf(s, s, -q));
+  // 1 / w = y (1 + e / 2), e = 1 - w^2 y^2
+  const float y0 = rsqrtf(w2.hi);
+  const DF t = df_mulf(df_mulf(w2, y0), y0);
+  const float e = (1.f - t.hi) - t.lo;
+  const float g = eifdf::df_add_nw(eifdf::df_mul(vy, bc), eifdf::df_neg(eifdf::df_mul(vx, as))).hi, iw2 = y0 * y0;
+  const float K = fmaf(nw.hi * abf, iw2, w2.hi);
+  const float corr = 0.5f * g * __fdividef(g, K) * abf * (y0 * iw2) + abf * y0 * (0.5f * rho);
+  const DF d = df_mulf(nw, y0);
+  return eifdf::fast_sum(d.hi, d.lo + fmaf(d.hi, 0.5f * e, corr));
+}
+// tanh z of z = |d| from 2 exp(-2 z) at multiples of 1 / MID_STEPS (tab, from MID_Z0 up)
+constexpr int MID_STEPS = 128, MID_Z0 = 6, MID_Z1 = 20, MID_N = (MID_Z1 - MID_Z0) * MID_STEPS + 1;
+__device__ __forceinline__ double tanh_mid(DF d, const float2 *__restrict__ tab) {
+  const float zh = fmaxf(fminf(fabsf(d.hi), (float)MID_Z1), (float)MID_Z0), zl = d.hi < 0.f ? -d.lo : d.lo;
+  const float kf = rintf((zh - (float)MID_Z0) * (float)MID_STEPS);
+  const float2 E = __ldg(tab + (int)kf);
+  // exp(-2 (z - z_k)) = (1 + y + q)(1 + yl); x = E (1 - E / 2 + E^2 / 4)
+  const float y = -2.f * (zh - fmaf(kf, 1.f / MID_STEPS, (float)MID_Z0)), yl = -2.f * zl;
+  const float q = y * y * fmaf(y, fmaf(y, 1.f / 24.f, 1.f / 6.f), 0.5f);
+  const float p = E.x * y;
+  const DF m = eifdf::fast_sum(E.x, p);
+  const float l0 = m.lo + (fmaf(E.x, y, -p) + fmaf(E.x, q + fmaf(yl, y, yl), fmaf(E.y, y, E.y))), x = m.hi + l0;
+  const float lo = l0 - 0.5f * x * x * fmaf(-0.5f, x, 1.f);
+  constexpr float U = 9007199254740992.f;   // 2^53
+  return tanh_of(__float2ll_rn(m.hi * U) + __float2ll_rn(lo * U), d.hi);
 }
 
 // Cells far from the interface. With rho = sqrt((x/a)^2 + (y/b)^2) (the gauge of
@@ -302,6 +358,11 @@ struct BoxArgs {
 // particles: parts 0-2 the boxes of images -1, 0, +1 (their task counts are added to
 // nchunk, zeroed before), parts 3-7 groups of parameters. One thread: particle n, part sub.
 constexpr int BOX_PARTS = 8;
+__device__ __forceinline__ void put_pair(float *p, double v) {
+  const eifdf::DF t = eifdf::df_of(v);
+  p[0] = t.hi;
+  p[1] = t.lo;
+}
 __device__ __forceinline__ void box_part(const BoxArgs &a, int n, int sub) {
   const double *P = a.P;
   const int pc = a.pcap;
@@ -381,6 +442,8 @@ __device__ __forceinline__ void box_part(const BoxArgs &a, int n, int sub) {
       sincos(-az, &sz, &cz);
       d[PD_CZ] = cz * a.kb;
       d[PD_SZ] = sz * a.kb;
+      put_pair(df + PDF_PAIRS + 4, d[PD_CZ]);
+      put_pair(df + PDF_PAIRS + 6, d[PD_SZ]);
       // the far cells' row bounds in single precision: the far distance (10.5 cells) exceeds
       // the saturation distance of tanh (9.53 cells) by far more than their rounding
       const float fa = eifd::d2f(pa), fb = eifd::d2f(pb), cf = eifd::d2f(cz), sf = eifd::d2f(sz);
@@ -391,15 +454,21 @@ __device__ __forceinline__ void box_part(const BoxArgs &a, int n, int sub) {
       const double ba = pa * a.kb, bb = pb * a.kb;
       d[PD_A] = ba;
       d[PD_B] = bb;
+      put_pair(df + PDF_PAIRS, ba);
+      put_pair(df + PDF_PAIRS + 2, bb);
       const float fa = eifd::d2f(ba), fb = eifd::d2f(bb);
       df[PDF_A] = fa;
       df[PDF_B] = fb;
       df[PDF_KEX] = (fa - fb) * (fa + fb) / fa;
       df[PDF_KEY] = (fb - fa) * (fb + fa) / fb;
     } else if (d && sub == 5) {
-      d[PD_RPM] = 1. / pmass(P[EIF_P_DEN * pc + n], pa, pb);
+      const double m = pmass(P[EIF_P_DEN * pc + n], pa, pb);
+      d[PD_RPM] = 1. / m;
+      d[PD_QM] = 0.25 * a.dx * a.dy / m;
     } else if (d && sub == 6) {
-      d[PD_RPIM] = 1. / pmoi(P[EIF_P_DEN * pc + n], pa, pb);
+      const double m = pmoi(P[EIF_P_DEN * pc + n], pa, pb);
+      d[PD_RPIM] = 1. / m;
+      d[PD_QIM] = 0.25 * a.dx * a.dy / m;
     } else if (d && sub == 7) {
       d[PD_X] = px;
       d[PD_Y] = py;
@@ -413,6 +482,8 @@ __device__ __forceinline__ void box_part(const BoxArgs &a, int n, int sub) {
   }
   if (on && tasks && EIF_CHK(a.bd.rec, (a.nchunk - a.bd_off_base) + n, a.bd.off, 3)) atomicAdd(a.nchunk + n, tasks);
 }
+
+__device__ __forceinline__ eifdf::DF get_pair(const float *p) { return eifdf::DF{p[0], p[1]}; }
 
 // The same for one particle by the first four warps of a CTA, into shared memory (bx: 12 ints,
 // pf or pd: its parameter block), at X + dX in a sub-iteration: the values of box_part bit for
@@ -438,9 +509,12 @@ __device__ __forceinline__ void box_warps(const BoxArgs &a, int n, int part, int
       const double w = lane == 4 ? cz * sz * (v - v1) : (lane == 1 ? cz : (lane == 3 ? sz : v + v1));
       if (lane < 5) pf[lane == 0 ? PF_AL : (lane == 1 ? PF_CZ : (lane == 2 ? PF_DE : (lane == 3 ? PF_SZ : PF_KA)))] = (float)w;
     } else if (lane == 0) {
-      pd[PD_CZ] = cz * a.kb;
-      pd[PD_SZ] = sz * a.kb;
+      const double bc = cz * a.kb, bs = sz * a.kb;
+      pd[PD_CZ] = bc;
+      pd[PD_SZ] = bs;
       float *df = reinterpret_cast<float *>(pd + PD_F);
+      put_pair(df + PDF_PAIRS + 4, bc);
+      put_pair(df + PDF_PAIRS + 6, bs);
       const float fa = eifd::d2f(pa), fb = eifd::d2f(pb), cf = eifd::d2f(cz), sf = eifd::d2f(sz);
       df[PDF_AL] = cf * cf / (fa * fa) + sf * sf / (fb * fb);
       df[PDF_KA] = cf * sf * (1.f / (fb * fb) - 1.f / (fa * fa));
@@ -491,7 +565,7 @@ __device__ __forceinline__ void box_warps(const BoxArgs &a, int n, int part, int
     const double *c = a.pd + (size_t)PD_WORDS * n;
     if (lane >= PD_A && lane < PD_F) pd[lane] = c[lane];
     float *df = reinterpret_cast<float *>(pd + PD_F);
-    if (lane >= PDF_SO2 && lane < PDF_WORDS) df[lane] = reinterpret_cast<const float *>(c + PD_F)[lane];
+    if (lane >= PDF_SO2 && lane < PDF_PAIRS + 4) df[lane] = reinterpret_cast<const float *>(c + PD_F)[lane];
   }
 }
 __device__ __forceinline__ int box_tasks(const int *bx) {
@@ -640,6 +714,7 @@ struct WorkArgs {
   const float *pf;       // per-particle single-precision parameters (mixed form)
   const double *pd;      // per-particle parameters (double-precision form)
   const double2 *tanh_tab;   // tanh_tab's values (double-precision form)
+  const float2 *mid_tab;     // tanh_mid's
   const int4 *tdesc;     // task table (k_task_table)
   const float *coef;     // single-precision dt products; [9] = 1/dt
   float rh_f, dx_f, dy_f, dxdy_f;
@@ -704,194 +779,227 @@ __device__ __forceinline__ double warp_sum3(double v0, double v1, double v2, int
 
 // One warp per row task: indicator weights, partial sums, and (for the exchange)
 // per-cell field contributions. The warp runs the tasks first, first + stride, ...
-// with the weight mode wmode; slots: WORK_SLOTS entries of shared memory of its own.
-// Bound by the FP64 pipe in both uses: about 30 FP64 instructions per task for the sums and
-// 45 for each pass of 32 cells next to the interface. Not inlined, and every product that
-// could be fused is written as fma: the batch's stage kernel gives the bits of the
-// stand-alone kernel.
-constexpr int WORK_SLOTS = CHUNK + CHUNK / (int)sizeof(double2);   // double2 entries per warp
+// with the weight mode wmode, WORK_ROWS at a time: the cells of theirs that need double
+// precision are evaluated together, packed onto the lanes.
+// Bound by the FP64 pipe: an instruction of a warp holds its scheduler 64 cycles. About 27 FP64
+// instructions per task for the sums and 48 for each pass of 32 cells next to the interface,
+// of which a task has 15 or so. Not inlined, and every product that could be fused is written
+// as fma: the stage kernel gives the bits of the stand-alone kernel. Kept short (loops not
+// unrolled, the guards' records out of line): with 30 KB of straight code the warps waited for
+// instructions more than half of the time.
+__device__ __noinline__ bool work_chk_fail(unsigned long long *rec, long long idx, long long bound, int tag) {
+  return EIF_CHK(rec, idx, bound, tag);
+}
+#define WORK_CHK(rec, idx, bound, tag) \
+  ((unsigned long long)(idx) < (unsigned long long)(bound) || work_chk_fail((rec), (long long)(idx), (long long)(bound), (tag)))
+constexpr int WORK_ROWS = 4;
+struct WorkSlots {     // shared memory of a warp
+  double th[WORK_ROWS][CHUNK];        // weights; before pass 3 the feet (c, s) of its cells
+  double px[WORK_ROWS], Y[WORK_ROWS];
+  const double *pd[WORK_ROWS];
+  int ib[WORK_ROWS];
+  unsigned char near[CHUNK];          // cells of a row for pass 2
+  unsigned char list[WORK_ROWS * CHUNK];   // row * CHUNK + cell for pass 3
+};
 template <bool NC>
-__device__ __noinline__ void ibm_work_tasks(const WorkArgs &a, int wmode, int first, int stride, double2 *slots,
+__device__ __noinline__ void ibm_work_tasks(const WorkArgs &a, int wmode, int first, int stride, WorkSlots &ws,
                                             const OneParticle *one) {
   const int lane = threadIdx.x & 31;
-  const int total = one ? one->total : (EIF_CHK(a.bd.rec, a.np, a.bd.off, 10) ? ldro<NC>(a.off + a.np) : 0);
+  const int total = one ? one->total : (WORK_CHK(a.bd.rec, a.np, a.bd.off, 10) ? ldro<NC>(a.off + a.np) : 0);
   const bool own = one && one->box;
-  const double dxdy = a.dx * a.dy;
-  // factors of the sums: inertia.c:51-59 with 1/2 (1 + th) and the two face averages,
-  // exchange.c:61-76
-  const double scale = a.mode == 0 ? 0.25 * dxdy : -dxdy / __ldg(a.dt);
+  // factor of the exchange's sums (exchange.c:61-76) over the particle's PD_QM, PD_QIM
+  const double xscale = a.mode == 0 ? 1. : -4. / __ldg(a.dt);
   const int pc = a.pcap, ld = a.ld;
   double *wcache = static_cast<double *>(a.wcache);
-  unsigned char *list = reinterpret_cast<unsigned char *>(slots + CHUNK);   // the cells of pass 3
-  for (int k = first; k < total; k += stride) {
-    const int c = own ? one->base + k : k;
-    if (!EIF_CHK(a.bd.rec, c, a.bd.partial / 3, 21)) continue;
+  // task k: its number c, descriptor and row; false when it is to be skipped
+  auto task_at = [&](int k, int &c, int &n, RowTask &t, bool &task) {
+    c = own ? one->base + k : k;
+    if (!WORK_CHK(a.bd.rec, c, a.bd.partial / 3, 21)) return false;
     const int4 dsc = own ? task_desc(*one, k) : ldro<NC>(a.tdesc + c);
-    const int n = dsc.x;
-    if (!EIF_CHK(a.bd.rec, n, a.np, 11)) continue;
-    if (!EIF_CHK(a.bd.rec, EIF_P_VZ * pc + n, a.bd.P, 13)) continue;
-    RowTask t;
-    const bool task = task_of(dsc, a.np, t) && EIF_CHK(a.bd.rec, t.j, a.bd.yc - 1, 15);
-    const double *pd = own ? one->pd : a.pd + (size_t)PD_WORDS * n;
-    const float *pdf = reinterpret_cast<const float *>(pd + PD_F);
-    const int img = task ? t.img : 0;
-    const double px = ldro<NC>(pd + PD_X), py_ = ldro<NC>(pd + PD_Y) + (img == 0 ? 0. : (img > 0 ? a.ly : -a.ly));
-    const int j = task ? t.j : 1;
-    const double Y = __ldg(a.yc + j) - py_;
-    const int ib = task ? t.ib : 1;
-    double th2[2];
-    bool cin[2];
-#pragma unroll
-    for (int half = 0; half < CHUNK / 32; half++) {
-      const int i = ib + half * 32 + lane;
-      bool in = task && i <= t.ie;
-      if (in) {
-        in = EIF_CHK(a.bd.rec, i, a.bd.xc - 1, 14) && EIF_CHK(a.bd.rec, j * ld + i, a.bd.field, 16) &&
-             EIF_CHK(a.bd.rec, (j + 1) * ld + i, a.bd.field, 17) && EIF_CHK(a.bd.rec, j * ld + (i - 1), a.bd.field, 18);
-      }
-      cin[half] = in;
+    n = dsc.x;
+    if (!WORK_CHK(a.bd.rec, n, a.np, 11)) return false;
+    if (!WORK_CHK(a.bd.rec, EIF_P_VZ * pc + n, a.bd.P, 13)) return false;
+    task = task_of(dsc, a.np, t) && WORK_CHK(a.bd.rec, t.j, a.bd.yc - 1, 15);
+    if (!task) {
+      t.img = 0;
+      t.j = t.ib = 1;
+      t.ie = 0;
     }
-    if (wmode == 2) {
-      // weights of the same geometry from an earlier evaluation
-#pragma unroll
-      for (int half = 0; half < CHUNK / 32; half++) {
-        if (cin[half]) cin[half] = EIF_CHK(a.bd.rec, (long long)c * CHUNK + half * 32 + lane, a.bd.wbuf, 22);
-        th2[half] = cin[half] ? wcache[(size_t)c * CHUNK + half * 32 + lane] : 0.;
-      }
-    } else {
-      // pass 1: cells of the row, far cells settled, the near ones listed
-      int rank[2];
-      unsigned near_mask[2];
-      float olo, ohi, ilo, ihi;
-      row_chords(ldro<NC>(pdf + PDF_AL), ldro<NC>(pdf + PDF_KA), ldro<NC>(pdf + PDF_DE), ldro<NC>(pdf + PDF_SO2),
-                 ldro<NC>(pdf + PDF_SI2), ldro<NC>(pdf + PDF_RO2), eifd::d2f(Y), olo, ohi, ilo, ihi);
-#pragma unroll
-      for (int half = 0; half < CHUNK / 32; half++) {
-        const int i = ib + half * 32 + lane;
-        bool near = false;
-        th2[half] = 0.;
-        if (cin[half]) {
-          const float Xf = eifd::d2f(__ldg(a.xc + i) - px);
-          // reference sign convention: +1 inside (auxiliary.c:36-38); tanh saturated
-          const int side = !(Xf > olo && Xf < ohi) ? -1 : ((Xf >= ilo && Xf <= ihi) ? 1 : 0);
-          th2[half] = side > 0 ? 1. : (side < 0 ? -1. : 0.);
-          near = side == 0;
-        }
-        near_mask[half] = __ballot_sync(0xffffffffu, near);
-        rank[half] = (half ? __popc(near_mask[0]) : 0) + __popc(near_mask[half] & ((1u << lane) - 1u));
-        if (near) slots[rank[half]].x = __hiloint2double(0, half * 32 + lane);
-      }
-      // pass 2: the near cells packed onto consecutive lanes, single precision; the cells it
-      // settles get their weights, the others are packed once more
-      const int nnear = __popc(near_mask[0]) + __popc(near_mask[1]);
-      if (a.count) {
-        const unsigned in0 = __ballot_sync(0xffffffffu, cin[0]), in1 = __ballot_sync(0xffffffffu, cin[1]);
+    return true;
+  };
+  auto centre_y = [&](const double *pd, int img) {
+    return ldro<NC>(pd + PD_Y) + (img == 0 ? 0. : (img > 0 ? a.ly : -a.ly));
+  };
+  for (int k0 = first; k0 < total; k0 += WORK_ROWS * stride) {
+    const int nq = min(WORK_ROWS, (total - k0 + stride - 1) / stride);
+    if (wmode != 2) {
+      int ndbl = 0;
+      for (int q = 0; q < nq; q++) {
+        int c, n;
+        RowTask t;
+        bool task;
+        if (!task_at(k0 + q * stride, c, n, t, task)) continue;
+        const double *pd = own ? one->pd : a.pd + (size_t)PD_WORDS * n;
+        const float *pdf = reinterpret_cast<const float *>(pd + PD_F);
+        const double px = ldro<NC>(pd + PD_X);
+        const double Y = __ldg(a.yc + t.j) - centre_y(pd, t.img);
+        // the columns are dx apart
+        const DF X0 = eifdf::df_of(__ldg(a.xc + t.ib) - px), dxp = eifdf::df_of(a.dx), Yp = eifdf::df_of(Y);
         if (lane == 0) {
-          atomicAdd(a.count, (unsigned long long)(__popc(in0) + __popc(in1)));
+          ws.px[q] = px;
+          ws.Y[q] = Y;
+          ws.pd[q] = pd;
+          ws.ib[q] = t.ib;
+        }
+        // pass 1: cells of the row, far cells settled (tanh +-1), the near ones listed
+        int nnear = 0;
+        float olo, ohi, ilo, ihi;
+        row_chords(ldro<NC>(pdf + PDF_AL), ldro<NC>(pdf + PDF_KA), ldro<NC>(pdf + PDF_DE), ldro<NC>(pdf + PDF_SO2),
+                   ldro<NC>(pdf + PDF_SI2), ldro<NC>(pdf + PDF_RO2), Yp.hi, olo, ohi, ilo, ihi);
+#pragma unroll 1
+        for (int half = 0; half < CHUNK / 32; half++) {
+          const int at = half * 32 + lane;
+          const bool in = t.ib + at <= t.ie;
+          const float Xf = fmaf((float)at, dxp.hi, X0.hi);
+          // reference sign convention: +1 inside (auxiliary.c:36-38)
+          const int side = !(Xf > olo && Xf < ohi) ? -1 : ((Xf >= ilo && Xf <= ihi) ? 1 : 0);
+          const bool near = in && side == 0;
+          ws.th[q][at] = in ? (side > 0 ? 1. : (side < 0 ? -1. : 0.)) : 0.;
+          const unsigned mask = __ballot_sync(0xffffffffu, near);
+          if (near) ws.near[nnear + __popc(mask & ((1u << lane) - 1u))] = (unsigned char)at;
+          nnear += __popc(mask);
+        }
+        if (a.count && lane == 0) {
+          atomicAdd(a.count, (unsigned long long)max(0, min(CHUNK, t.ie - t.ib + 1)));
           atomicAdd(a.count + 1, (unsigned long long)nnear);
         }
-      }
-      __syncwarp();
-      if (nnear) {
-        const double cz = ldro<NC>(pd + PD_CZ), sz = ldro<NC>(pd + PD_SZ), pa = ldro<NC>(pd + PD_A),
-                     pb = ldro<NC>(pd + PD_B);
+        __syncwarp();
+        if (nnear == 0) continue;
+        // pass 2: the near cells packed onto consecutive lanes, on the FP32 pipe; the cells it
+        // settles get their weights, the others are listed for pass 3 with their feet
         EllF ef;
         ef.a = ldro<NC>(pdf + PDF_A); ef.b = ldro<NC>(pdf + PDF_B);
         ef.kex = ldro<NC>(pdf + PDF_KEX); ef.key = ldro<NC>(pdf + PDF_KEY);
-        ef.cz = eifd::d2f(cz); ef.sz = eifd::d2f(sz);
-        const float zs = z_single(fmaxf(ef.a, ef.b)), Yf = eifd::d2f(Y);
-        int ndbl = 0;
+        ef.cz = ef.sz = 0.f;
+        const DF ap = get_pair(pdf + PDF_PAIRS), bp = get_pair(pdf + PDF_PAIRS + 2), czp = get_pair(pdf + PDF_PAIRS + 4),
+                 szp = get_pair(pdf + PDF_PAIRS + 6);
+        const DF szY = eifdf::df_mul(szp, Yp), czY = eifdf::df_mul(czp, Yp);
+        const float zm = z_mid(fmaxf(ef.a, ef.b));
         for (int base = 0; base < nnear; base += 32) {
           const int k = base + lane;
           bool dbl = false;
           int at = 0;
           float c0 = 0.f, s0 = 0.f;
           if (k < nnear) {
-            at = __double2loint(slots[k].x);
-            const float Xf = eifd::d2f(__ldg(a.xc + ib + at) - px);
+            at = ws.near[k];
+            // offset X0 + at dx, then the body frame
+            const float f = (float)at, p = f * dxp.hi;
+            const DF sm = eifdf::two_sum(X0.hi, p);
+            const DF X = eifdf::fast_sum(sm.hi, sm.lo + (fmaf(f, dxp.hi, -p) + fmaf(f, dxp.lo, X0.lo)));
+            DF x = eifdf::df_add_nw(eifdf::df_mul(czp, X), eifdf::df_neg(szY));
+            DF y = eifdf::df_add_nw(eifdf::df_mul(szp, X), czY);
+            if (x.hi < 0.f) x = eifdf::df_neg(x);
+            if (y.hi < 0.f) y = eifdf::df_neg(y);
             float d;
-            const float dist = foot_f(ef, fabsf(ef.cz * Xf - ef.sz * Yf), fabsf(ef.sz * Xf + ef.cz * Yf), c0, s0, d);
-            dbl = !(fabsf(dist) >= zs && fabsf(d) < 1.e-3f);
-            if (!dbl) slots[at].y = tanh_far(dist);
+            const float dist = foot_f(ef, x.hi, y.hi, c0, s0, d);
+            dbl = !(fabsf(dist) >= zm && fabsf(d) < 1.e-3f);
+            if (!dbl) ws.th[q][at] = tanh_mid(dist_mid(ap, bp, ef.a * ef.b, c0, s0, x, y), a.mid_tab);
           }
           const unsigned mask = __ballot_sync(0xffffffffu, dbl);
           if (dbl) {
-            // list positions at or before the ones already read; .y is indexed by cell
-            const int q = ndbl + __popc(mask & ((1u << lane) - 1u));
-            slots[q].x = __hiloint2double(__float_as_int(c0), __float_as_int(s0));
-            list[q] = (unsigned char)at;
+            ws.th[q][at] = __hiloint2double(__float_as_int(c0), __float_as_int(s0));
+            ws.list[ndbl + __popc(mask & ((1u << lane) - 1u))] = (unsigned char)(q * CHUNK + at);
           }
           ndbl += __popc(mask);
-          __syncwarp();
         }
-        // pass 3: double precision
-        const double szY = sz * Y, czY = cz * Y;
-        for (int k = lane; k < ndbl; k += 32) {
-          const int at = list[k];
-          const double cs = slots[k].x;
-          const double X = __ldg(a.xc + ib + at) - px;
-          double nx, ny;
-          slots[at].y = indicator_d<false>(pa, pb, ef.a * ef.b, __int_as_float(__double2hiint(cs)),
-                                           __int_as_float(__double2loint(cs)), fma(cz, X, -szY), fma(sz, X, czY),
-                                           a.tanh_tab, nx, ny);
-        }
+        __syncwarp();
       }
       __syncwarp();
-#pragma unroll
-      for (int half = 0; half < CHUNK / 32; half++)
-        if ((near_mask[half] >> lane) & 1u) th2[half] = slots[half * 32 + lane].y;
-      __syncwarp();
-      if (wmode == 1) {
-#pragma unroll
-        for (int half = 0; half < CHUNK / 32; half++)
-          if (EIF_CHK(a.bd.rec, (long long)c * CHUNK + half * 32 + lane, a.bd.wbuf, 23))
-            wcache[(size_t)c * CHUNK + half * 32 + lane] = th2[half];
+      // pass 3: double precision
+      for (int k = lane; k < ndbl; k += 32) {
+        const int e = ws.list[k], q = e / CHUNK, at = e % CHUNK;
+        const double *pd = ws.pd[q];
+        const double cs = ws.th[q][at];
+        const double cz = ldro<NC>(pd + PD_CZ), sz = ldro<NC>(pd + PD_SZ);
+        const double X = __ldg(a.xc + ws.ib[q] + at) - ws.px[q], Y = ws.Y[q];
+        const float *pdf = reinterpret_cast<const float *>(pd + PD_F);
+        double nx, ny;
+        ws.th[q][at] = indicator_d<false>(ldro<NC>(pd + PD_A), ldro<NC>(pd + PD_B), ldro<NC>(pdf + PDF_A) * ldro<NC>(pdf + PDF_B),
+                                          __int_as_float(__double2hiint(cs)), __int_as_float(__double2loint(cs)),
+                                          fma(cz, X, -(sz * Y)), fma(sz, X, cz * Y), a.tanh_tab, nx, ny);
       }
+      __syncwarp();
     }
-    const double pux = ldro<NC>(a.P + EIF_P_UX * pc + n), puy = ldro<NC>(a.P + EIF_P_UY * pc + n),
-                 pvz = ldro<NC>(a.P + EIF_P_VZ * pc + n);
-    double s0 = 0., s1 = 0., s2 = 0.;
-#pragma unroll
-    for (int half = 0; half < CHUNK / 32; half++) {
-      const int i = ib + half * 32 + lane;
-      double2 contrib = make_double2(0., 0.);
-      // cells of weight exactly zero (inertia: far outside; exchange: any far cell) are
-      // skipped; compared as integers, the FP64 pipe does comparisons too
-      const double th = th2[half];
-      const int hi = __double2hiint(th), lo = __double2loint(th);
-      const bool one = (a.mode == 0 ? hi : hi | (int)0x80000000) == (int)0xbff00000 && lo == 0;
-      if (cin[half] && !one) {
-        const double X = __ldg(a.xc + i) - px;
-        const double us = __ldg(a.ux + j * ld + (i - 1)) + __ldg(a.ux + j * ld + i);
-        const double vs = __ldg(a.uy + j * ld + i) + __ldg(a.uy + (j + 1) * ld + i);
-        if (a.mode == 0) {
-          // inertia.c:51-59: the constant factors, and the row's Y in the moment, after the sum
-          const double w = 1. + th, wv = w * vs;
-          s0 = fma(w, us, s0);
-          s1 += wv;
-          s2 = fma(X, wv, s2);
+    // the sums
+    for (int q = 0; q < nq; q++) {
+      int c, n;
+      RowTask t;
+      bool task;
+      if (!task_at(k0 + q * stride, c, n, t, task)) continue;
+      const double *pd = own ? one->pd : a.pd + (size_t)PD_WORDS * n;
+      const double px = ldro<NC>(pd + PD_X);
+      const int j = t.j;
+      const double Y = __ldg(a.yc + j) - centre_y(pd, t.img);
+      const double pux = ldro<NC>(a.P + EIF_P_UX * pc + n), puy = ldro<NC>(a.P + EIF_P_UY * pc + n),
+                   pvz = ldro<NC>(a.P + EIF_P_VZ * pc + n);
+      double s0 = 0., s1 = 0., s2 = 0.;
+#pragma unroll 1
+      for (int half = 0; half < CHUNK / 32; half++) {
+        const int at = half * 32 + lane, i = t.ib + at;
+        const long long slot = (long long)c * CHUNK + at;
+        bool in = i <= t.ie;
+        if (in) {
+          in = WORK_CHK(a.bd.rec, i, a.bd.xc - 1, 14) && WORK_CHK(a.bd.rec, j * ld + i, a.bd.field, 16) &&
+               WORK_CHK(a.bd.rec, (j + 1) * ld + i, a.bd.field, 17) && WORK_CHK(a.bd.rec, j * ld + (i - 1), a.bd.field, 18);
+        }
+        double th = 0.;
+        if (wmode == 2) {
+          // weights of the same geometry from an earlier evaluation
+          if (in) in = WORK_CHK(a.bd.rec, slot, a.bd.wbuf, 22);
+          if (in) th = wcache[slot];
         } else {
-          // exchange.c:61-76 (BETA / 2 = 1)
-          const double w = fma(-th, th, 1.);
-          const double gx = w * fma(-0.5, us, fma(-pvz, Y, pux));
-          const double gy = w * fma(-0.5, vs, fma(pvz, X, puy));
-          contrib = a.weights_only ? make_double2(w, w) : make_double2(gx, gy);
-          s0 += gx;
-          s1 += gy;
-          s2 = fma(X, gy, s2);
+          if (in) th = ws.th[q][at];
+          if (wmode == 1 && WORK_CHK(a.bd.rec, slot, a.bd.wbuf, 23)) wcache[slot] = th;
         }
+        double2 contrib = make_double2(0., 0.);
+        // cells of weight exactly zero (inertia: far outside; exchange: any far cell) are
+        // skipped; compared as integers, the FP64 pipe does comparisons too
+        const int hi = __double2hiint(th), lo = __double2loint(th);
+        const bool zero = (a.mode == 0 ? hi : hi | (int)0x80000000) == (int)0xbff00000 && lo == 0;
+        if (in && !zero) {
+          const double X = __ldg(a.xc + i) - px;
+          const double us = __ldg(a.ux + j * ld + (i - 1)) + __ldg(a.ux + j * ld + i);
+          const double vs = __ldg(a.uy + j * ld + i) + __ldg(a.uy + (j + 1) * ld + i);
+          if (a.mode == 0) {
+            // inertia.c:51-59: the constant factors, and the row's Y in the moment, after the sum
+            const double w = 1. + th, wv = w * vs;
+            s0 = fma(w, us, s0);
+            s1 += wv;
+            s2 = fma(X, wv, s2);
+          } else {
+            // exchange.c:61-76 (BETA / 2 = 1)
+            const double w = fma(-th, th, 1.);
+            const double gx = w * fma(-0.5, us, fma(-pvz, Y, pux));
+            const double gy = w * fma(-0.5, vs, fma(pvz, X, puy));
+            contrib = a.weights_only ? make_double2(w, w) : make_double2(gx, gy);
+            s0 += gx;
+            s1 += gy;
+            s2 = fma(X, gy, s2);
+          }
+        }
+        if (a.mode == 1 && WORK_CHK(a.bd.rec, slot, a.bd.wbuf, 19)) a.wbuf[slot] = contrib;
       }
-      if (a.mode == 1 && EIF_CHK(a.bd.rec, (long long)c * CHUNK + half * 32 + lane, a.bd.wbuf, 19))
-        a.wbuf[(size_t)c * CHUNK + half * 32 + lane] = contrib;
+      // sum_x, sum_y in lanes 0 and 16, the moment sum X f_y in lane 8, which takes Y sum_x off it
+      double v = warp_sum3(s0, s1, s2, lane);
+      const double sx = __shfl_sync(0xffffffffu, v, 0);
+      const int slot = lane == 0 ? 0 : (lane == 16 ? 1 : (lane == 8 ? 2 : -1));
+      if (slot >= 0 && WORK_CHK(a.bd.rec, 3LL * c + 2, a.bd.partial, 20)) {
+        if (slot == 2) v = fma(-Y, sx, v);
+        const double f = ldro<NC>(pd + (slot == 2 ? PD_QIM : PD_QM));
+        a.partial[3 * (size_t)c + slot] = a.mode == 0 ? v * f : v * (f * xscale);
+      }
     }
-    // sum_x, sum_y in lanes 0 and 16, the moment sum X f_y in lane 8, which takes Y sum_x off it
-    double v = warp_sum3(s0, s1, s2, lane);
-    const double sx = __shfl_sync(0xffffffffu, v, 0);
-    const int slot = lane == 0 ? 0 : (lane == 16 ? 1 : (lane == 8 ? 2 : -1));
-    if (slot >= 0 && EIF_CHK(a.bd.rec, 3LL * c + 2, a.bd.partial, 20)) {
-      if (slot == 2) v = fma(-Y, sx, v);
-      a.partial[3 * (size_t)c + slot] = v * (scale * ldro<NC>(pd + (slot == 2 ? PD_RPIM : PD_RPM)));
-    }
+    __syncwarp();
   }
 }
 
@@ -1453,6 +1561,7 @@ inline WorkArgs work_args(const eif_ctx *c, int mode, int cn) {
   w.pf = c->pf;
   w.pd = c->pd;
   w.tanh_tab = c->tanh_tab;
+  w.mid_tab = reinterpret_cast<const float2 *>(c->tanh_tab + TANH_N);
   w.tdesc = c->tdesc;
   w.coef = c->d_coef;
   w.rh_f = (float)(1. / w.h);

@@ -195,8 +195,7 @@ __device__ __forceinline__ void finish_particle(const SubDesc &d, int n, unsigne
 
 __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
   __shared__ unsigned act[SUB_MAX / 32];   // suspensions still iterating
-  __shared__ float2 slot_f[SUB_WARPS][CHUNK];
-  __shared__ double2 slot_d[SUB_WARPS][WORK_SLOTS];
+  __shared__ WorkSlots slot_d[SUB_WARPS];   // of the double-precision form, or the mixed form's cells
   __shared__ __align__(16) int bx[12];
   __shared__ __align__(16) float pf[PF_WORDS];
   __shared__ __align__(16) double pd[PD_WORDS];
@@ -323,7 +322,7 @@ __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
           const int r0 = (int)((long long)cnt * sl / d.ns), r1 = (int)((long long)cnt * (sl + 1) / d.ns);
           const OneParticle one{reinterpret_cast<const int4 *>(bx), pf, pd, p, c0, r1};
           if (d.mixed) {
-            ibm_work_f_tasks<false, true>(d.work, 0, r0 + wl, SUB_WARPS, slot_f[wl], &one);
+            ibm_work_f_tasks<false, true>(d.work, 0, r0 + wl, SUB_WARPS, reinterpret_cast<float2 *>(&slot_d[wl]), &one);
             if (sl == 0 && wl == SUB_WARPS - 2 && d.work.memo_mode == 2) memo_particle(d.work.memo, pf, bx, one.base, p);
           } else {
             ibm_work_tasks<false>(d.work, 0, r0 + wl, SUB_WARPS, slot_d[wl], &one);
