@@ -790,6 +790,9 @@ __device__ __forceinline__ double warp_sum3(double v0, double v1, double v2, int
 __device__ __noinline__ bool work_chk_fail(unsigned long long *rec, long long idx, long long bound, int tag) {
   return EIF_CHK(rec, idx, bound, tag);
 }
+__device__ __forceinline__ void prefetch_l1(const double *p) {
+  asm volatile("prefetch.global.L1 [%0];" : : "l"(p));
+}
 #define WORK_CHK(rec, idx, bound, tag) \
   ((unsigned long long)(idx) < (unsigned long long)(bound) || work_chk_fail((rec), (long long)(idx), (long long)(bound), (tag)))
 constexpr int WORK_ROWS = 4;
@@ -864,6 +867,12 @@ __device__ __noinline__ void ibm_work_tasks(const WorkArgs &a, int wmode, int fi
           // reference sign convention: +1 inside (auxiliary.c:36-38)
           const int side = !(Xf > olo && Xf < ohi) ? -1 : ((Xf >= ilo && Xf <= ihi) ? 1 : 0);
           const bool near = in && side == 0;
+          if (in) {
+            // the sums' velocities, needed some thousand cycles later
+            prefetch_l1(a.ux + t.j * ld + t.ib + at);
+            prefetch_l1(a.uy + t.j * ld + t.ib + at);
+            prefetch_l1(a.uy + (t.j + 1) * ld + t.ib + at);
+          }
           ws.th[q][at] = in ? (side > 0 ? 1. : (side < 0 ? -1. : 0.)) : 0.;
           const unsigned mask = __ballot_sync(0xffffffffu, near);
           if (near) ws.near[nnear + __popc(mask & ((1u << lane) - 1u))] = (unsigned char)at;
@@ -946,6 +955,8 @@ __device__ __noinline__ void ibm_work_tasks(const WorkArgs &a, int wmode, int fi
 #pragma unroll 1
       for (int half = 0; half < CHUNK / 32; half++) {
         const int at = half * 32 + lane, i = t.ib + at;
+        // nothing but the stored weights and contributions of a short row's second half
+        if (half > 0 && t.ib + 32 > t.ie && a.mode == 0 && wmode != 1) break;
         const long long slot = (long long)c * CHUNK + at;
         bool in = i <= t.ie;
         if (in) {
@@ -1451,10 +1462,8 @@ __device__ __forceinline__ double chunk_sum_warp(const double *partial, int c0, 
     s1 += partial[3 * (size_t)c + 1];
     s2 += partial[3 * (size_t)c + 2];
   }
-  s0 = eifd::warp_sum(s0);
-  s1 = eifd::warp_sum(s1);
-  s2 = eifd::warp_sum(s2);
-  return lane == 0 ? s0 : (lane == 1 ? s1 : s2);
+  // the sums are in lanes 0, 16 and 8
+  return __shfl_sync(0xffffffffu, warp_sum3(s0, s1, s2, lane), lane == 0 ? 0 : (lane == 1 ? 16 : 8));
 }
 
 // The same per-particle sums from the single-precision partials of the mixed form,

@@ -262,7 +262,9 @@ __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
     // units in order: the first by the CTA's number, the next ones as CTAs come free
     int next = blockIdx.x;
     for (;;) {
-      if (threadIdx.x == 0) {
+      // with a CTA for every unit a CTA keeps its unit as long as the set does not change
+      const bool kept = units <= G && !changed;
+      if (!kept && threadIdx.x == 0) {
         const int u = next;
         if (units > G) next = G + (int)atomicAdd(s.sync + 2 + m3, 1u);
         else next = units;
@@ -278,7 +280,7 @@ __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
         unit[1] = u - (lo > 0 ? stab[ST_WORDS * (lo - 1) + col] : (col == ST_SEND ? ncoll : 0)) +
                   (col == ST_CEND ? (1 << 30) : 0);
       }
-      __syncthreads();
+      if (!kept) __syncthreads();
       const int j = unit[0];
       if (j < 0) break;
       const bool coll = unit[1] >= (1 << 30);
@@ -461,7 +463,11 @@ int subiter_plan_create(eif_ctx *const *ctx, int n, SubiterPlan **out, std::stri
     p->np += ctx[j]->np;
   }
   for (int j = 0; j < n; j++) {
-    const int by_gpu = std::max(1, most / std::max(1, p->np));
+    // a CTA to an SM where that leaves a warp a task: a second one would share the FP64 pipe of
+    // the boxes (216 x 430 with 24 ellipses: boxes 6100 cycles with, 3700 without)
+    const int np = std::max(1, p->np), sms = ctx[0]->sms;
+    const int by_sm = (sms - (np + PAIR_WARPS - 1) / PAIR_WARPS) / np;
+    const int by_gpu = by_sm >= 1 && ctx[j]->max_tasks <= by_sm * SUB_WARPS ? by_sm : std::max(1, most / np);
     const int by_tasks = std::max(1, (ctx[j]->max_tasks + 3) / 4);
     p->ns.push_back(std::min(by_gpu, by_tasks));
     units += (long long)ctx[j]->np * p->ns[j] + (ctx[j]->np + PAIR_WARPS - 1) / PAIR_WARPS;
