@@ -118,7 +118,7 @@ struct eif_ctx {
   // second stream for particle-only work that runs beside the fluid kernels; the
   // launch functions use `stream`, which side_begin/side_end point at it
   cudaStream_t side = nullptr, main_stream = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_ibm = nullptr, ev_coll = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_ibm = nullptr, ev_bands = nullptr, ev_coll = nullptr;
   // eif_advance_pull: the step graphs record ev_fields once the last RK stage's
   // projection has written the fields; their copy to the host runs on copy_stream
   cudaEvent_t ev_fields = nullptr;
@@ -233,6 +233,7 @@ struct eif_ctx {
   // weights of the last indicator evaluation in a sub-iteration loop (mixed form), with
   // the particles' geometry words, boxes and first tasks (WeightMemo in ibm_device.cuh)
   // tasks of a stage start the memo did not serve: [0] count, then their numbers
+  bool memo_miss_zero = false;   // the box build's table kernel has cleared memo_miss[0]
   int *memo_miss = nullptr;
   float *memo_w = nullptr, *memo_pf = nullptr;
   int *memo_box = nullptr, *memo_off = nullptr, *memo_valid = nullptr;
@@ -369,6 +370,13 @@ int ibm_reserve(eif_ctx *c, size_t chunks);
 void ibm_free(eif_ctx *c);
 int launch_inertia(eif_ctx *c, int cn);
 int launch_exchange(eif_ctx *c);
+// the parts of launch_inertia(c, 0) and launch_exchange (np > 0), for two streams; the band
+// lists (launch_band_lists) come before the gather
+int launch_inertia_tasks(eif_ctx *c);
+int launch_inertia_sums(eif_ctx *c);
+int launch_exchange_tasks(eif_ctx *c);
+int launch_exchange_sums(eif_ctx *c);
+int launch_gather(eif_ctx *c);
 int launch_band_lists(eif_ctx *c);
 // transposed box evaluation of the discrete adjoint (ibm.cu): mode 0 the inertia
 // integrals at X (+ dX with use_increment), mode 1 the momentum exchange at X; bar

@@ -34,6 +34,22 @@
 
 namespace {
 
+// What the table kernels clear for the kernels after them (a clearing node of its own holds
+// the branch up for 4 us between two kernels): the bitmap that k_band_marks adds the boxes of
+// this build to (to which it adds them again when the lists are built twice from one build),
+// and the count of the tasks that the memo does not serve.
+struct TableClears {
+  unsigned *marks;   // or null: inside a sub-iteration loop, where no lists are built
+  int nmarks;
+  int *miss;         // or null: double precision
+  __device__ __forceinline__ void clear() const {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (miss && t == 0) *miss = 0;
+    if (marks)
+      for (int k = t; k < nmarks; k += gridDim.x * blockDim.x) marks[k] = 0u;
+  }
+};
+
 // Stand-alone kernels over the bodies of ibm_device.cuh. Inside the sub-iteration
 // loop of a step graph (iter set) the loop counter decides what runs: in the first
 // sub-iteration the increments are zero, the positions are X and the boxes and the
@@ -45,8 +61,9 @@ __global__ void __launch_bounds__(32) k_boxes(BoxArgs a) {
 
 __global__ void __launch_bounds__(TT_WARPS * 32) k_task_table_scan(const int *__restrict__ box, const int *__restrict__ cnt,
                                                                   int *__restrict__ off, int4 *__restrict__ tdesc, int np,
-                                                                  Bounds bd, int cap, const unsigned *__restrict__ iter) {
+                                                                  Bounds bd, int cap, const unsigned *__restrict__ iter, TableClears z) {
   if (iter && *iter == 0u) return;
+  z.clear();
   task_table_block(box, cnt, off, tdesc, np, bd, cap, blockIdx.x);
 }
 
@@ -112,7 +129,7 @@ __global__ void k_scan(const int *__restrict__ cnt, int *__restrict__ off, int n
   __syncthreads();
   for (int base = 0; base < np; base += 1024) {
     const int t = base + threadIdx.x;
-    const int v = (t < np && EIF_CHK(bd.rec, (cnt - off) + t, bd.off, 4)) ? cnt[t] : 0;
+    const int v = (t < np && EIF_CHK(bd.rec, (cnt - off) + 2 * np + t, bd.off, 4)) ? cnt[t] + cnt[np + t] + cnt[2 * np + t] : 0;
     s[threadIdx.x] = v;
     __syncthreads();
     for (int o = 1; o < 1024; o <<= 1) {
@@ -173,8 +190,9 @@ __global__ void __launch_bounds__(1024) k_task_bases(const double *__restrict__ 
 // load instead of a chain of dependent loads (owner, boxes, offsets). One warp
 // per particle.
 __global__ void k_task_table(const int *__restrict__ box, const int *__restrict__ off, int4 *__restrict__ tdesc,
-                             int np, Bounds bd, int cap, const unsigned *__restrict__ iter) {
+                             int np, Bounds bd, int cap, const unsigned *__restrict__ iter, TableClears z) {
   if (iter && *iter == 0u) return;
+  z.clear();
   const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (n >= np) return;
@@ -262,6 +280,7 @@ struct GatherArgs {
   void *dux, *duy;   // double (FP64 form) or float (mixed form) fields with the same pitch
   unsigned *flags;
   int np, itot, jtot, ld;
+  int halo;          // the halo rows and ghost columns too
   Bounds bd;
 };
 
@@ -329,8 +348,10 @@ __global__ void __launch_bounds__(GTHREADS, 6) k_gather(GatherArgs a) {
     }
     __syncthreads();
   }
-  // write the tile's interior cells (zero where no box covers); the halo rows and
-  // ghost columns are filled afterwards by k_ibm_halo from these cells
+  // write the tile's interior cells (zero where no box covers) and, with halo, their copies in
+  // the periodic halo rows (j = 0 <- jtot, j = jtot+1 <- 1) and the Neumann ghost columns
+  // (i = 0 <- 1, i = itot+1 <- itot, corners included), exchange.c:80-81 with the boundary
+  // update of the reference
   const int ld = a.ld;
 #pragma unroll
   for (int q = 0; q < NC; q++) {
@@ -340,33 +361,20 @@ __global__ void __launch_bounds__(GTHREADS, 6) k_gather(GatherArgs a) {
     if (!EIF_CHK(a.bd.rec, cidx, a.bd.field, 42)) continue;
     static_cast<Acc *>(a.dux)[cidx] = acc_x[q];
     static_cast<Acc *>(a.duy)[cidx] = acc_y[q];
+    if (a.halo && (i == 1 || i == a.itot || j == 1 || j == a.jtot)) {
+      for (int jj = 0; jj < 3; jj++) {
+        if ((jj == 1 && j != a.jtot) || (jj == 2 && j != 1)) continue;
+        const int row = (jj == 0 ? j : (jj == 1 ? 0 : a.jtot + 1)) * ld;
+        for (int ii = 0; ii < 3; ii++) {
+          if ((ii == 1 && i != 1) || (ii == 2 && i != a.itot)) continue;
+          const int col = ii == 0 ? i : (ii == 1 ? 0 : a.itot + 1);
+          if ((ii | jj) == 0 || !EIF_CHK(a.bd.rec, row + col, a.bd.field, 43)) continue;
+          static_cast<Acc *>(a.dux)[row + col] = acc_x[q];
+          static_cast<Acc *>(a.duy)[row + col] = acc_y[q];
+        }
+      }
+    }
   }
-}
-
-// Periodic halo rows (j = 0 <- jtot, j = jtot+1 <- 1) and Neumann ghost columns
-// (i = 0 <- 1, i = itot+1 <- itot, corners included) of the IBM field response,
-// exchange.c:80-81 with the boundary update of the reference. Every thread reads
-// one interior cell and writes one halo cell.
-template <typename T>
-__global__ void k_ibm_halo(T *__restrict__ dux, T *__restrict__ duy, int itot, int jtot, int ld) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nrow = itot + 2;
-  int dst, src;
-  if (t < 2 * nrow) {
-    const int i = t % nrow, top = t / nrow;
-    const int ic = i < 1 ? 1 : (i > itot ? itot : i);
-    dst = (top ? jtot + 1 : 0) * ld + i;
-    src = (top ? 1 : jtot) * ld + ic;
-  } else if (t < 2 * nrow + 2 * jtot) {
-    const int u = t - 2 * nrow;
-    const int j = 1 + u % jtot, right = u / jtot;
-    dst = j * ld + (right ? itot + 1 : 0);
-    src = j * ld + (right ? itot : 1);
-  } else {
-    return;
-  }
-  dux[dst] = dux[src];
-  duy[dst] = duy[src];
 }
 
 }  // namespace
@@ -418,9 +426,9 @@ int ibm_reserve(eif_ctx *c, size_t chunks) {
   c->chunk_cap = (int)chunks;
   c->wcap = chunks * CHUNK;
   EIF_CK(c, cudaMalloc((void **)&c->box, sizeof(int) * 12 * c->np));
-  EIF_CK(c, cudaMalloc((void **)&c->chunk_off, sizeof(int) * 2 * (c->np + 1)));
+  EIF_CK(c, cudaMalloc((void **)&c->chunk_off, sizeof(int) * (4 * (size_t)c->np + 1)));
   EIF_CK(c, cudaMalloc((void **)&c->task_base, sizeof(int) * c->np));
-  EIF_CK(c, cudaMalloc((void **)&c->partial, sizeof(double) * 3 * chunks));
+  EIF_CK(c, cudaMalloc((void **)&c->partial, sizeof(double) * 6 * chunks));
   EIF_CK(c, cudaMalloc((void **)&c->wbuf, sizeof(double2) * c->wcap));
   EIF_CK(c, cudaMalloc((void **)&c->wcache, sizeof(double) * c->wcap));
   if (c->cfg.precision == EIF_PREC_MIXED) EIF_CK(c, cudaMalloc((void **)&c->pf, sizeof(float) * PF_WORDS * c->np));
@@ -488,6 +496,9 @@ void ibm_free(eif_ctx *c) {
   c->chunk_cap = 0; c->wcap = 0;
 }
 
+// bitmap over the 3 np (particle, image) boxes, one row of words per band
+static int band_mark_words(const eif_ctx *c) { return (c->jtot + GTY - 1) / GTY * ((3 * c->np + 31) / 32); }
+
 static int launch_boxes(eif_ctx *c, bool use_increment) {
   // boxes at the positions X (no increment, or increments known to be zero) are
   // reused until the positions or the particle set change
@@ -500,25 +511,30 @@ static int launch_boxes(eif_ctx *c, bool use_increment) {
   b.iter = c->in_loop ? reinterpret_cast<const unsigned *>(c->d_inc + 1) : nullptr;
   int *cnt = b.nchunk;
   EIF_PROF(c, "ibm_boxes", c->np <= TT_MAX_NP ? 2 : 3);
-  EIF_CK(c, cudaMemsetAsync(cnt, 0, sizeof(int) * c->np, c->stream));
+  TableClears z;
+  z.marks = c->in_loop ? nullptr : c->band_marks;
+  z.nmarks = band_mark_words(c);
+  z.miss = c->memo_miss;
   k_boxes<<<dim3((c->np + 31) / 32, BOX_PARTS), 32, 0, c->stream>>>(b);
   EIF_LAUNCH_CK(c);
   if (c->np <= TT_MAX_NP) {
     k_task_table_scan<<<(c->np + TT_WARPS - 1) / TT_WARPS, TT_WARPS * 32, 0, c->stream>>>(
-        c->box, cnt, c->chunk_off, c->tdesc, c->np, bounds_of(c), c->chunk_cap, b.iter);
+        c->box, cnt, c->chunk_off, c->tdesc, c->np, bounds_of(c), c->chunk_cap, b.iter, z);
     EIF_LAUNCH_CK(c);
   } else {
     k_scan<<<1, 1024, 0, c->stream>>>(cnt, c->chunk_off, c->np, bounds_of(c), b.iter);
     EIF_LAUNCH_CK(c);
     k_task_table<<<(c->np * 32 + 255) / 256, 256, 0, c->stream>>>(c->box, c->chunk_off, c->tdesc, c->np,
-                                                                   bounds_of(c), c->chunk_cap, b.iter);
+                                                                   bounds_of(c), c->chunk_cap, b.iter, z);
     EIF_LAUNCH_CK(c);
   }
+  c->memo_miss_zero = !c->in_loop;
   c->boxes_x_valid = x_only;
   return EIF_OK;
 }
 
-static int launch_work(eif_ctx *c, int mode, int cn) {
+// store: the mixed form's evaluation that stores its weights in the memo (see launch_sums)
+static int launch_work(eif_ctx *c, int mode, int cn, bool *store) {
   WorkArgs w = work_args(c, mode, cn);
   const bool mixed = c->cfg.precision == EIF_PREC_MIXED;
   // weights at the positions X (inertia with zero increments, or the exchange)
@@ -561,7 +577,8 @@ static int launch_work(eif_ctx *c, int mode, int cn) {
     if (w.memo_mode == 1) {
       // the stage start: the memo-served tasks in the light kernel (sums-kernel
       // registers), then the full evaluation of the tasks it listed as not served
-      EIF_CK(c, cudaMemsetAsync(c->memo_miss, 0, sizeof(int), c->stream));
+      if (!c->memo_miss_zero) EIF_CK(c, cudaMemsetAsync(c->memo_miss, 0, sizeof(int), c->stream));
+      c->memo_miss_zero = false;
       WorkArgs wm = w, wf = w;
       wm.miss = c->memo_miss;
       wf.only = c->memo_miss;
@@ -587,17 +604,26 @@ static int launch_work(eif_ctx *c, int mode, int cn) {
     }
     EIF_LAUNCH_CK(c);
   }
+  *store = memo_store;
+  return EIF_OK;
+}
+
+// the particles' sums of the last evaluation of mode and cn
+static int launch_sums(eif_ctx *c, int mode, int cn, bool memo_store) {
+  const bool mixed = c->cfg.precision == EIF_PREC_MIXED;
+  const double *partial = partial_of(c, mode);
   const int f0 = mode == 0 ? EIF_P_IUX0 + cn : EIF_P_FUX;
   const int f1 = mode == 0 ? EIF_P_IUY0 + cn : EIF_P_FUY;
   const int f2 = mode == 0 ? EIF_P_IVZ0 + cn : EIF_P_TVZ;
   EIF_PROF(c, "ibm_reduce", 1);
   if (mixed) {
     k_chunk_reduce_f<<<(c->np * 32 + 255) / 256, 256, 0, c->stream>>>(
-        reinterpret_cast<const float *>(c->partial), c->chunk_off, c->P, c->pcap, c->np, f0, f1, f2, bounds_of(c),
-        memo_of(c), memo_store ? 1 : 0, c->in_loop ? w.iter : nullptr, c->pf, c->box);
+        reinterpret_cast<const float *>(partial), c->chunk_off, c->P, c->pcap, c->np, f0, f1, f2, bounds_of(c),
+        memo_of(c), memo_store ? 1 : 0, c->in_loop ? reinterpret_cast<const unsigned *>(c->d_inc + 1) : nullptr, c->pf,
+        c->box);
   } else {
-    k_chunk_reduce<<<(c->np * 32 + 255) / 256, 256, 0, c->stream>>>(c->partial, c->chunk_off, c->P, c->pcap, c->np,
-                                                                      f0, f1, f2, bounds_of(c));
+    k_chunk_reduce<<<(c->np * 32 + 255) / 256, 256, 0, c->stream>>>(partial, c->chunk_off, c->P, c->pcap, c->np, f0, f1,
+                                                                      f2, bounds_of(c));
   }
   EIF_LAUNCH_CK(c);
   return EIF_OK;
@@ -606,9 +632,24 @@ static int launch_work(eif_ctx *c, int mode, int cn) {
 int launch_inertia(eif_ctx *c, int cn) {
   if (c->np == 0) return EIF_OK;
   int rc = launch_boxes(c, true);
-  if (rc) return rc;
-  return launch_work(c, 0, cn);
+  bool store = false;
+  if (rc || (rc = launch_work(c, 0, cn, &store))) return rc;
+  return launch_sums(c, 0, cn, store);
 }
+
+int launch_inertia_tasks(eif_ctx *c) {
+  int rc = launch_boxes(c, true);
+  bool store = false;
+  return rc ? rc : launch_work(c, 0, 0, &store);
+}
+int launch_inertia_sums(eif_ctx *c) { return launch_sums(c, 0, 0, false); }
+
+int launch_exchange_tasks(eif_ctx *c) {
+  int rc = launch_boxes(c, false);
+  bool store = false;
+  return rc ? rc : launch_work(c, 1, 0, &store);
+}
+int launch_exchange_sums(eif_ctx *c) { return launch_sums(c, 1, 0, false); }
 
 static int band_lists_of_boxes(eif_ctx *c);
 
@@ -625,7 +666,6 @@ static int band_lists_of_boxes(eif_ctx *c) {
   const int nbands = (c->jtot + GTY - 1) / GTY;
   const int words = (3 * c->np + 31) / 32;
   EIF_PROF(c, "ibm_band_lists", 2);
-  EIF_CK(c, cudaMemsetAsync(c->band_marks, 0, sizeof(unsigned) * (size_t)nbands * words, c->stream));
   k_band_marks<<<(c->np + 127) / 128, 128, 0, c->stream>>>(c->box, c->chunk_off, c->np, c->jtot, c->band_marks,
                                                            words, c->edesc, bounds_of(c));
   EIF_LAUNCH_CK(c);
@@ -643,30 +683,27 @@ int launch_exchange(eif_ctx *c) {
     EIF_CK(c, cudaMemsetAsync(c->duy, 0, sizeof(double) * c->nfield, c->stream));
     return EIF_OK;
   }
-  int rc = launch_boxes(c, false);
-  if (rc) return rc;
-  rc = launch_work(c, 1, 0);
-  if (rc) return rc;
+  int rc;
+  if ((rc = launch_exchange_tasks(c)) || (rc = launch_exchange_sums(c))) return rc;
+  if (!(c->boxes_x_valid && c->bands_x_valid) && (rc = launch_band_lists(c))) return rc;
+  return launch_gather(c);
+}
+
+// the field response from the tasks' contributions and the band lists
+int launch_gather(eif_ctx *c) {
   GatherArgs g;
   g.edesc = c->edesc; g.wbuf = c->wbuf;
   g.dux = c->dux; g.duy = c->duy; g.flags = c->d_flags;
   g.np = c->np; g.itot = c->itot; g.jtot = c->jtot; g.ld = c->ld;
   g.bd = bounds_of(c);
   g.lists = c->band_lists; g.counts = c->band_counts; g.cap = c->band_cap;
-  if (!(c->boxes_x_valid && c->bands_x_valid) && (rc = launch_band_lists(c))) return rc;
+  g.halo = 1;
   dim3 grid((c->itot + GTX - 1) / GTX, (c->jtot + GTY - 1) / GTY);
-  EIF_PROF(c, "ibm_gather", 2);
-  const int nhalo = 2 * (c->itot + 2) + 2 * c->jtot;
+  EIF_PROF(c, "ibm_gather", 1);
   if (c->cfg.precision == EIF_PREC_MIXED) {
     k_gather<float2, float><<<grid, GTHREADS, 0, c->stream>>>(g);
-    EIF_LAUNCH_CK(c);
-    k_ibm_halo<float><<<(nhalo + 255) / 256, 256, 0, c->stream>>>(reinterpret_cast<float *>(c->dux),
-                                                                  reinterpret_cast<float *>(c->duy), c->itot,
-                                                                  c->jtot, c->ld);
   } else {
     k_gather<double2, double><<<grid, GTHREADS, 0, c->stream>>>(g);
-    EIF_LAUNCH_CK(c);
-    k_ibm_halo<double><<<(nhalo + 255) / 256, 256, 0, c->stream>>>(c->dux, c->duy, c->itot, c->jtot, c->ld);
   }
   EIF_LAUNCH_CK(c);
   return EIF_OK;
@@ -893,6 +930,7 @@ int launch_adj_pass(eif_ctx *c, const AdjPass &p) {
   GatherArgs g;
   g.edesc = c->edesc; g.wbuf = c->wbuf;
   g.dux = p.fx; g.duy = p.fy; g.flags = c->d_flags;
+  g.halo = 0;
   g.np = c->np; g.itot = c->itot; g.jtot = c->jtot; g.ld = c->ld;
   g.bd = bounds_of(c);
   g.lists = c->band_lists; g.counts = c->band_counts; g.cap = c->band_cap;

@@ -355,8 +355,10 @@ struct BoxArgs {
 // single-precision parameters. The double-precision work of one particle is a long
 // chain (divisions, sincos) and the FP64 pipe takes a warp instruction at a time, so
 // the work is split into eight parts run by different warps, each over 32
-// particles: parts 0-2 the boxes of images -1, 0, +1 (their task counts are added to
-// nchunk, zeroed before), parts 3-7 groups of parameters. One thread: particle n, part sub.
+// particles: parts 0-2 the boxes of images -1, 0, +1 (the task count of image q - 1 goes to
+// nchunk[q np + n]: a sum formed here would have to be cleared before, and the clearing node
+// ahead of this kernel held every stage up for 4 us), parts 3-7 groups of parameters. One
+// thread: particle n, part sub.
 constexpr int BOX_PARTS = 8;
 __device__ __forceinline__ void put_pair(float *p, double v) {
   const eifdf::DF t = eifdf::df_of(v);
@@ -480,7 +482,8 @@ __device__ __forceinline__ void box_part(const BoxArgs &a, int n, int sub) {
       df[PDF_RO2] = (mx + md) * (mx + md);
     }
   }
-  if (on && tasks && EIF_CHK(a.bd.rec, (a.nchunk - a.bd_off_base) + n, a.bd.off, 3)) atomicAdd(a.nchunk + n, tasks);
+  if (on && sub < 3 && EIF_CHK(a.bd.rec, (a.nchunk - a.bd_off_base) + sub * a.np + n, a.bd.off, 3))
+    a.nchunk[sub * a.np + n] = tasks;
 }
 
 __device__ __forceinline__ eifdf::DF get_pair(const float *p) { return eifdf::DF{p[0], p[1]}; }
@@ -611,7 +614,7 @@ __device__ __forceinline__ bool row_task(int4 bm, int4 b0, int4 bp, int r, RowTa
 // its own (a few thousand integers from L2), then each warp writes its particle's
 // offset and table entries. Replaces k_scan + k_task_table (one launch and one
 // single-block pass fewer on the path of every box build). One block of TT_WARPS
-// warps: particles block * TT_WARPS ...
+// warps: particles block * TT_WARPS ... cnt: the counts of the three images, np each.
 constexpr int TT_WARPS = 8;
 constexpr int TT_MAX_NP = 8192;
 __device__ __forceinline__ void task_table_block(const int *box, const int *cnt, int *off, int4 *tdesc, int np,
@@ -620,11 +623,11 @@ __device__ __forceinline__ void task_table_block(const int *box, const int *cnt,
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int n0 = block * TT_WARPS;
   int s = 0;
-  for (int q = threadIdx.x; q < n0; q += blockDim.x) s += cnt[q];
+  for (int q = threadIdx.x; q < n0; q += blockDim.x) s += cnt[q] + cnt[np + q] + cnt[2 * np + q];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   const int n = n0 + w;
-  const int my = n < np ? cnt[n] : 0;
+  const int my = n < np ? cnt[n] + cnt[np + n] + cnt[2 * np + n] : 0;
   if (lane == 0) {
     red[w] = s;
     wcnt[w] = my;
@@ -1519,7 +1522,7 @@ inline Bounds bounds_of(const eif_ctx *c) {
   Bounds b;
   b.P = (long long)EIF_NFIELDS * c->pcap;
   b.box = 12LL * c->np;
-  b.off = 2LL * (c->np + 1);
+  b.off = (c->np + 1) + 3LL * c->np;
   b.partial = 3LL * c->chunk_cap;
   b.wbuf = (long long)c->wcap;
   b.field = (long long)c->nfield;
@@ -1539,8 +1542,8 @@ inline WeightMemo memo_of(const eif_ctx *c) {
   return m;
 }
 
-// boxes of the particles at X (+ dX with use_increment); their task counts go to
-// nchunk = chunk_off + np + 1
+// boxes of the particles at X (+ dX with use_increment); the task counts of their images go
+// to nchunk = chunk_off + np + 1
 inline BoxArgs box_args(const eif_ctx *c, bool use_increment) {
   BoxArgs b;
   b.bd = bounds_of(c);
@@ -1557,13 +1560,17 @@ inline BoxArgs box_args(const eif_ctx *c, bool use_increment) {
   return b;
 }
 
+// the task sums of mode 0 or 1: arrays of their own, so that the inertia's are reduced beside
+// the exchange's evaluation (rk_stage_front)
+inline double *partial_of(const eif_ctx *c, int mode) { return c->partial + (mode == 0 ? 0 : 3 * (size_t)c->chunk_cap); }
+
 // task evaluations of mode 0 (inertia into the integrals cn) or 1 (exchange) over the
 // current velocity buffers; wmode 0, no loop counter, no counts
 inline WorkArgs work_args(const eif_ctx *c, int mode, int cn) {
   WorkArgs w;
   w.P = c->P; w.ux = c->ux[c->cur]; w.uy = c->uy[c->cur]; w.xc = c->xc; w.yc = c->yc; w.dt = c->d_scal;
   w.uxf = c->uxf[c->cur]; w.uyf = c->uyf[c->cur];
-  w.box = c->box; w.off = c->chunk_off; w.partial = c->partial; w.wbuf = reinterpret_cast<double2 *>(c->wbuf);
+  w.box = c->box; w.off = c->chunk_off; w.partial = partial_of(c, mode); w.wbuf = reinterpret_cast<double2 *>(c->wbuf);
   w.pcap = c->pcap; w.np = c->np; w.ld = c->ld; w.mode = mode; w.cn = cn;
   w.dx = c->dx; w.dy = c->dy; w.ly = c->ly; w.h = c->dx < c->dy ? c->dx : c->dy;
   w.bd = bounds_of(c);
