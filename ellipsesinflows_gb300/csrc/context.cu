@@ -108,11 +108,11 @@ int join(eif_ctx *c, cudaEvent_t ev) {
 
 }  // namespace
 
-// the part of an RK stage before the particle sub-iterations (src/main.c:14-35)
-int rk_stage_front(eif_ctx *c, int rk) {
+// the part of an RK stage before the particle sub-iterations (src/main.c:14-35); with_dt:
+// after the decision of dt (main.c:12)
+int rk_stage_front(eif_ctx *c, int rk, bool with_dt) {
   int rc;
   const bool ibm = c->np > 0;
-  if ((rc = launch_reset_increments(c))) return rc;
   if (ibm && overlap_on(c)) {
     // side: inertia at X (reads the current velocity buffer, which the predictor
     // does not write), the band lists, the inertia's sums and the collision forces at X
@@ -122,6 +122,7 @@ int rk_stage_front(eif_ctx *c, int rk) {
     // the next kernel's inputs are on it (64 x 128, 4 particles: 77 -> 55 us a stage).
     SideScope side(c);
     if ((rc = side.begin())) return rc;
+    if ((rc = launch_reset_increments(c))) return rc;
     if ((rc = launch_inertia_tasks(c))) return rc;
     if ((rc = side.mark(c->ev_ibm))) return rc;
     if ((rc = launch_band_lists(c))) return rc;
@@ -129,6 +130,8 @@ int rk_stage_front(eif_ctx *c, int rk) {
     if ((rc = launch_inertia_sums(c))) return rc;
     if ((rc = launch_collision(c, 0))) return rc;
     if ((rc = side.end(c->ev_coll))) return rc;
+    // dt: nothing on the side stream before the exchange's sums reads it
+    if (with_dt && (rc = launch_decide_dt(c))) return rc;
     if ((rc = launch_predictor(c, rk))) return rc;
     if ((rc = join(c, c->ev_ibm))) return rc;
     if ((rc = launch_exchange_tasks(c))) return rc;
@@ -141,6 +144,8 @@ int rk_stage_front(eif_ctx *c, int rk) {
     if ((rc = launch_correct(c, rk, ibm, true))) return rc;
     return join(c, c->ev_coll);
   }
+  if (with_dt && (rc = launch_decide_dt(c))) return rc;
+  if ((rc = launch_reset_increments(c))) return rc;
   if ((rc = launch_inertia(c, 0))) return rc;
   if ((rc = launch_predictor(c, rk))) return rc;
   if (ibm && (rc = launch_exchange(c))) return rc;
@@ -211,6 +216,17 @@ __global__ void k_records_out(const double *__restrict__ P, double *__restrict__
     const int k = (int)(t / EIF_NFIELDS), f = (int)(t - (size_t)k * EIF_NFIELDS);
     rec[t] = P[(size_t)f * pcap + k];
   }
+}
+
+// dt, flags and bounds record of a step into its page-locked slot, in one launch between the
+// steps' graphs
+__global__ void __launch_bounds__(32) k_step_record(const double *__restrict__ scal, const unsigned *__restrict__ flags,
+                                                    const unsigned long long *__restrict__ check,
+                                                    eif_ctx::StepSlot *__restrict__ out) {
+  const int t = threadIdx.x;
+  if (t < 4) out->scal[t] = scal[t];
+  else if (t < 8) out->check[t - 4] = check ? check[t - 4] : 0ull;
+  else if (t == 8) out->flags = *flags;
 }
 
 // device address of a page-locked host array, or null for pageable memory
@@ -838,14 +854,8 @@ int advance(eif_ctx *c, int nsteps, const FieldTargets *ft) {
       int rc = step_graph_launch(c, true);
       if (rc) return rc;
       eif_ctx::StepSlot &h = c->h_slots[s & 1];
-      EIF_CK(c, cudaMemcpyAsync(h.scal, c->d_scal, sizeof(double) * 4, cudaMemcpyDeviceToHost, c->stream));
-      EIF_CK(c, cudaMemcpyAsync(&h.flags, c->d_flags, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
-      if (c->d_check) {
-        EIF_CK(c, cudaMemcpyAsync(h.check, c->d_check, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost,
-                                  c->stream));
-      } else {
-        h.check[0] = 0ull;
-      }
+      eif_xfer::k_step_record<<<1, 32, 0, c->stream>>>(c->d_scal, c->d_flags, c->d_check, &h);
+      EIF_LAUNCH_CK(c);
       EIF_CK(c, cudaEventRecord(c->ev_step[s & 1], c->stream));
       if (ft && s == nsteps - 1) {
         // the fields are final once the graph has recorded ev_fields (after the last

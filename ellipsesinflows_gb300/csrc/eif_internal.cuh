@@ -325,7 +325,7 @@ int subiter_upload(SubiterPlan *p, std::string *err);
 // a stage front and the particle update; tape (optional): dX after sub-iteration m to
 // tape + 3 np m, and *contact = 1 where a collision force is not zero
 int launch_stage_kernel(eif_ctx *c, int rk, double *tape, int *contact);
-int rk_stage_front(eif_ctx *c, int rk);
+int rk_stage_front(eif_ctx *c, int rk, bool with_dt = false);
 int ibm_prepare(eif_ctx *c);
 void profile_free(eif_ctx *c);
 

@@ -668,39 +668,39 @@ __global__ void __launch_bounds__(CM_THREADS) k_dt_colmax(const double *__restri
   if (mx1) atomicMax(colmax + k0 + 2, mx1);
 }
 
-// single-precision products of dt used by the mixed-precision kernels, formed
-// once per time step instead of once per thread
-__device__ __forceinline__ void write_coef(double dt, float *coef) {
-  const double al[3] = {32. / 60., 25. / 60., 45. / 60.};
-  const double be[3] = {0. / 60., -17. / 60., -25. / 60.};
-  for (int rk = 0; rk < 3; rk++) {
-    coef[3 * rk + 0] = (float)(al[rk] * dt);
-    coef[3 * rk + 1] = (float)(be[rk] * dt);
-    coef[3 * rk + 2] = (float)((al[rk] + be[rk]) * dt);
-  }
-  coef[9] = (float)(1. / dt);
-  for (int rk = 0; rk < 3; rk++) {
-    const double gdt = (al[rk] + be[rk]) * dt;
-    const float hi = (float)gdt;
-    coef[20 + 2 * rk] = hi;
-    coef[21 + 2 * rk] = (float)(gdt - (double)hi);
-  }
-  for (int rk = 0; rk < 3; rk++) {
-    const double inv = 1. / ((al[rk] + be[rk]) * dt);
-    const float hi = (float)inv;
-    coef[12 + 2 * rk] = hi;
-    coef[13 + 2 * rk] = (float)(inv - (double)hi);
-  }
+// single-precision products of dt used by the mixed-precision kernels, formed once per time
+// step instead of once per thread. One warp; lane rk < 3 the products of its stage (a lone
+// warp's FP64 instruction takes 64 cycles and a division 650, for one lane or for three).
+__device__ __forceinline__ void write_coef(double dt, float *coef, int lane) {
+  if (lane >= 3) return;
+  const int rk = lane;
+  const double al = rk == 0 ? 32. / 60. : (rk == 1 ? 25. / 60. : 45. / 60.);
+  const double be = rk == 0 ? 0. / 60. : (rk == 1 ? -17. / 60. : -25. / 60.);
+  coef[3 * rk + 0] = (float)(al * dt);
+  coef[3 * rk + 1] = (float)(be * dt);
+  const double gdt = (al + be) * dt;
+  const float ghi = (float)gdt;
+  coef[3 * rk + 2] = ghi;
+  coef[20 + 2 * rk] = ghi;
+  coef[21 + 2 * rk] = (float)(gdt - (double)ghi);
+  const double inv = 1. / gdt;
+  const float hi = (float)inv;
+  coef[12 + 2 * rk] = hi;
+  coef[13 + 2 * rk] = (float)(inv - (double)hi);
+  if (lane == 0) coef[9] = (float)(1. / dt);
 }
 
-// dt from the maxima (decide_dt.c:25-80): one block.
-// dt limits of one slice of columns and particles (partial minima, one triple per
-// block), then the final combination: the divisions are spread over DT_BLOCKS SMs
+// dt from the maxima (decide_dt.c:25-80): limits of one slice of columns and particles
+// (partial minima, one triple per block; the divisions are spread over DT_BLOCKS SMs), then
+// the last block to finish combines them. As two launches, with the products of dt formed by
+// one lane, they took 9.0 us at 64 x 128; in one 6.5.
 constexpr int DT_BLOCKS = 32;
 
-__global__ void k_dt_partial(const unsigned long long *__restrict__ colmax, const unsigned long long *__restrict__ uymax,
+__global__ void k_dt(const unsigned long long *__restrict__ colmax, const unsigned long long *__restrict__ uymax,
                              const double *__restrict__ dxc, int itot, double dy, double lx, double dx_uniform,
-                             const double *__restrict__ P, int pcap, int np, double *__restrict__ part) {
+                             const double *__restrict__ P, int pcap, int np, double *__restrict__ part,
+                     unsigned long long *__restrict__ done, double Re, double sf_adv, double sf_dif, double sf_par,
+                     double *__restrict__ dt_out, float *__restrict__ coef) {
   const double small = 1.e-8;
   double dta = 5.e-2, dxmin = lx, dtp = DBL_MAX;
   const int stride = gridDim.x * blockDim.x;
@@ -709,12 +709,13 @@ __global__ void k_dt_partial(const unsigned long long *__restrict__ colmax, cons
     dta = fmin(dta, dxc[i] / vel);
     dxmin = fmin(dxmin, dxc[i]);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  // uy and the particles from the other end: not after a column's division in the same warp
+  if (blockIdx.x == gridDim.x / 2 && threadIdx.x == 0) {
     const double vel = fmax(__longlong_as_double((long long)uymax[0]), small);
     dta = fmin(dta, dy / vel);
   }
   const double delta = fmin(dx_uniform, dy);
-  for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < np; n += stride) {
+  for (int n = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x; n < np; n += stride) {
     const double a = P[EIF_P_A * pcap + n], b = P[EIF_P_B * pcap + n];
     const double r = fmax(a, b);
     const double vz = P[EIF_P_VZ * pcap + n];
@@ -731,30 +732,31 @@ __global__ void k_dt_partial(const unsigned long long *__restrict__ colmax, cons
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   if (l == 0) { s[0][w] = dta; s[1][w] = dxmin; s[2][w] = dtp; }
   __syncthreads();
+  if (threadIdx.x >= 32) return;
+  unsigned last = 0;
   if (threadIdx.x == 0) {
     const int nw = blockDim.x >> 5;
     for (int k = 1; k < nw; k++) { dta = fmin(dta, s[0][k]); dxmin = fmin(dxmin, s[1][k]); dtp = fmin(dtp, s[2][k]); }
     part[3 * blockIdx.x + 0] = dta;
     part[3 * blockIdx.x + 1] = dxmin;
     part[3 * blockIdx.x + 2] = dtp;
+    __threadfence();
+    last = atomicAdd(done, 1ull) == gridDim.x - 1;
   }
-}
-
-// param_decide_dt (decide_dt.c:11-81): minima of the partial limits, the safety
-// factors, dt and the single-precision dt products
-// one warp: every lane loads one block's partial limits (nparts <= 32), a shuffle
-// reduction forms the minima (exact, so independent of the order)
-__global__ void k_dt_final(const double *__restrict__ part, int nparts, double dy, double Re, double sf_adv,
-                           double sf_dif, double sf_par, double *__restrict__ dt_out, float *__restrict__ coef) {
-  const int l = threadIdx.x;
-  const int q = l < nparts ? l : 0;
-  double dta = part[3 * q], dxmin = part[3 * q + 1], dtp = part[3 * q + 2];
+  if (!__shfl_sync(0xffffffffu, last, 0)) return;
+  __threadfence();
+  // param_decide_dt (decide_dt.c:11-81): every lane loads one block's partial limits, a
+  // shuffle reduction forms the minima (exact, so independent of the order); then the safety
+  // factors, dt and its single-precision products
+  const int q = l < gridDim.x ? l : 0;
+  dta = __ldcg(part + 3 * q);
+  dxmin = __ldcg(part + 3 * q + 1);
+  dtp = __ldcg(part + 3 * q + 2);
   for (int o = 16; o > 0; o >>= 1) {
     dta = fmin(dta, __shfl_xor_sync(0xffffffffu, dta, o));
     dxmin = fmin(dxmin, __shfl_xor_sync(0xffffffffu, dxmin, o));
     dtp = fmin(dtp, __shfl_xor_sync(0xffffffffu, dtp, o));
   }
-  if (l != 0) return;
   dta *= sf_adv;
   double difx = 0.25 * Re * (dxmin * dxmin);
   double dify = 0.25 * Re * (dy * dy);
@@ -762,11 +764,13 @@ __global__ void k_dt_final(const double *__restrict__ part, int nparts, double d
   dify *= sf_dif;
   dtp *= sf_par;
   const double dt = fmin(fmin(dta, fmin(difx, dify)), dtp);
-  *dt_out = dt;
-  write_coef(dt, coef);
+  if (l == 0) *dt_out = dt;
+  write_coef(dt, coef, l);
 }
 
-__global__ void k_coef(const double *__restrict__ dt, float *__restrict__ coef) { write_coef(*dt, coef); }
+__global__ void __launch_bounds__(32) k_coef(const double *__restrict__ dt, float *__restrict__ coef) {
+  write_coef(*dt, coef, threadIdx.x);
+}
 
 // ---------------------------------------------------------------------------
 // check_divergence (logging.c:52-65): (UX(i+1) - UX(i)) / DXF(i) + (UY(j+1) - UY(j)) / dy
@@ -1102,20 +1106,19 @@ int launch_update_pressure(eif_ctx *c) { return launch_corr(c, -1, 0, 0, 1); }
 int launch_decide_dt(eif_ctx *c) {
   unsigned long long *colmax = reinterpret_cast<unsigned long long *>(c->qhat);  // scratch: itot+2 words
   unsigned long long *uymax = colmax + c->itot + 2;
-  EIF_PROF(c, "decide_dt", 3);
-  EIF_CK(c, cudaMemsetAsync(colmax, 0, sizeof(unsigned long long) * (c->itot + 3), c->stream));
+  unsigned long long *done = uymax + 1;
+  EIF_PROF(c, "decide_dt", 2);
+  EIF_CK(c, cudaMemsetAsync(colmax, 0, sizeof(unsigned long long) * (c->itot + 4), c->stream));
   const int gx = (c->itot / 2 + 1 + CM_THREADS - 1) / CM_THREADS;   // column pairs 0 .. itot/2
   const int gy = std::max(1, std::min(c->jtot, (c->sms * 8 + gx - 1) / gx));
   k_dt_colmax<<<dim3(gx, gy), CM_THREADS, 0, c->stream>>>(c->ux[c->cur], c->uy[c->cur], c->itot, c->jtot, c->ld,
                                                             colmax, uymax, c->d_flags);
   EIF_LAUNCH_CK(c);
-  double *part = reinterpret_cast<double *>(uymax + 1);   // scratch: 3 * DT_BLOCKS words
-  k_dt_partial<<<DT_BLOCKS, 64, 0, c->stream>>>(colmax, uymax, c->dxc, c->itot, c->dy, c->lx, c->dx, c->P, c->pcap,
-                                                c->np, part);
-  EIF_LAUNCH_CK(c);
+  double *part = reinterpret_cast<double *>(done + 1);   // scratch: 3 * DT_BLOCKS words
   static_assert(DT_BLOCKS <= 32, "one warp combines the dt partials");
-  k_dt_final<<<1, 32, 0, c->stream>>>(part, DT_BLOCKS, c->dy, c->cfg.Re, c->cfg.safefactors[0], c->cfg.safefactors[1],
-                                     c->cfg.safefactors[2], c->d_scal, c->d_coef);
+  k_dt<<<DT_BLOCKS, 64, 0, c->stream>>>(colmax, uymax, c->dxc, c->itot, c->dy, c->lx, c->dx, c->P, c->pcap, c->np, part,
+                                        done, c->cfg.Re, c->cfg.safefactors[0], c->cfg.safefactors[1],
+                                        c->cfg.safefactors[2], c->d_scal, c->d_coef);
   EIF_LAUNCH_CK(c);
   return EIF_OK;
 }
@@ -1249,7 +1252,7 @@ int launch_d2f_copy(eif_ctx *c, const double *in, float *out, size_t n) {
 
 namespace eif {
 int launch_coef(eif_ctx *c) {
-  k_coef<<<1, 1, 0, c->stream>>>(c->d_scal, c->d_coef);
+  k_coef<<<1, 32, 0, c->stream>>>(c->d_scal, c->d_coef);
   EIF_LAUNCH_CK(c);
   return EIF_OK;
 }

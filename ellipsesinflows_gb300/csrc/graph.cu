@@ -94,9 +94,7 @@ int capture_step_part(eif_ctx *c, cudaGraph_t g, const std::vector<cudaGraphNode
                                                 cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return check_cuda(c, e, "cudaStreamBeginCaptureToGraph");
   int rc;
-  if (part == 0) {
-    if (with_dt && (rc = launch_decide_dt(c))) return rc;
-  } else {
+  if (part > 0) {
     // after a sub-iteration loop: the increments are not zero and the boxes of the
     // loop's last positions are not those at X
     c->incr_zero = false;
@@ -107,7 +105,7 @@ int capture_step_part(eif_ctx *c, cudaGraph_t g, const std::vector<cudaGraphNode
   }
   if (part < 3) {
     c->reset_in_stage_kernel = particles_in_stage_kernel && part > 0;
-    rc = rk_stage_front(c, part);
+    rc = rk_stage_front(c, part, part == 0 && with_dt);
     c->reset_in_stage_kernel = false;
     if (rc) return rc;
   }
