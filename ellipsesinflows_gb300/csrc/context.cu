@@ -108,6 +108,8 @@ int join(eif_ctx *c, cudaEvent_t ev) {
 
 }  // namespace
 
+int join_collision(eif_ctx *c) { return join(c, c->ev_coll); }
+
 // the part of an RK stage before the particle sub-iterations (src/main.c:14-35); with_dt:
 // after the decision of dt (main.c:12)
 int rk_stage_front(eif_ctx *c, int rk, bool with_dt) {
@@ -163,8 +165,7 @@ int sub_iteration(eif_ctx *c, int rk) {
     if ((rc = side.begin())) return rc;
     if ((rc = launch_collision(c, 1))) return rc;
     if ((rc = side.end(c->ev_coll))) return rc;
-    if ((rc = launch_inertia(c, 1))) return rc;
-    if ((rc = join(c, c->ev_coll))) return rc;
+    return launch_inertia_increment(c, rk);
   } else {
     if ((rc = launch_inertia(c, 1))) return rc;
     if ((rc = launch_collision(c, 1))) return rc;

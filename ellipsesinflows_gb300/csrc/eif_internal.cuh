@@ -377,6 +377,11 @@ int launch_inertia_sums(eif_ctx *c);
 int launch_exchange_tasks(eif_ctx *c);
 int launch_exchange_sums(eif_ctx *c);
 int launch_gather(eif_ctx *c);
+// a sub-iteration beside the collision forces on the side stream (np > 0): inertia at X + dX, then
+// with the forces the increments, the residual and, in a loop, its condition
+int launch_inertia_increment(eif_ctx *c, int rk);
+// the current stream waits for the collision forces of the side stream
+int join_collision(eif_ctx *c);
 int launch_band_lists(eif_ctx *c);
 // transposed box evaluation of the discrete adjoint (ibm.cu): mode 0 the inertia
 // integrals at X (+ dX with use_increment), mode 1 the momentum exchange at X; bar

@@ -8,7 +8,7 @@
 // error flags. The kernels' bodies and their order are those of the host-driven path
 // (rk_stage), so both paths give bit-identical results. Contexts of many particles
 // (subiter_alone) have a conditional WHILE node per stage whose body is one
-// sub-iteration; the last block of k_increment sets its condition.
+// sub-iteration; the last block of k_sub_end sets its condition.
 //
 // The stage kernels swap the double-buffered velocity and source arrays, so the
 // buffers a step touches depend on the buffer indices at its start; one graph
@@ -120,7 +120,7 @@ int capture_step_part(eif_ctx *c, cudaGraph_t g, const std::vector<cudaGraphNode
 
 // The sub-iteration loop of RK stage rk of c as a conditional WHILE node after the
 // nodes deps (its counter reset before it); sinks = {the loop node}. The last block
-// of k_increment sets the loop condition on the device. Without particles one
+// of k_sub_end sets the loop condition on the device. Without particles one
 // sub-iteration is all there is: no loop.
 int capture_subiteration_loop(eif_ctx *c, cudaGraph_t g, const std::vector<cudaGraphNode_t> &deps, int rk,
                               std::vector<cudaGraphNode_t> *sinks) {

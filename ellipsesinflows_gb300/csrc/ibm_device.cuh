@@ -729,7 +729,6 @@ struct WorkArgs {
   void *wcache;
   int wmode;
   const unsigned *iter;
-  int gate;   // with iter (mixed form): 1 runs only in the first sub-iteration, 2 only afterwards
   int weights_only;   // exchange (double precision): the cell contributions are the weights (w, w)
   // box cells whose geometry is evaluated and, of those, the near cells that run the
   // normal-foot iteration, added to count[0] and count[1], and the tasks whose weights
@@ -1587,7 +1586,6 @@ inline WorkArgs work_args(const eif_ctx *c, int mode, int cn) {
   w.wcache = c->wcache;
   w.wmode = 0;
   w.iter = nullptr;
-  w.gate = 0;
   w.weights_only = c->ibm_weights_only ? 1 : 0;
   w.count = nullptr;
   w.memo = memo_of(c);

@@ -37,9 +37,7 @@ __global__ void k_reset(double *__restrict__ P, int pcap, int np) {
 // few FP64 lanes.
 __global__ void k_increment(double *__restrict__ P, int pcap, int np, double gamma, double Fr2,
                             double *__restrict__ scal, unsigned long long *__restrict__ res_bits,
-                            unsigned *__restrict__ counter, unsigned *__restrict__ arrivals,
-                            unsigned long long *__restrict__ total, cudaGraphConditionalHandle handle,
-                            int use_handle) {
+                            unsigned *__restrict__ arrivals, unsigned long long *__restrict__ total) {
   const double dt = scal[0];
   double res = 0.;
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < np; n += gridDim.x * blockDim.x)
@@ -63,12 +61,6 @@ __global__ void k_increment(double *__restrict__ P, int pcap, int np, double gam
     const double r = __longlong_as_double((long long)atomicExch(res_bits, 0ull));
     scal[1] = r;
     *total += 1ull;   // sub-iterations run (eif_counters)
-    // inside a step graph: the condition of the sub-iteration loop (main.c:40-48):
-    // continue while the residual is not below 1e-8 and at most 101 sub-iterations ran
-    if (use_handle) {
-      const unsigned count = ++*counter;
-      cudaGraphSetConditional(handle, (!(r < 1.e-8) && count <= 101u) ? 1u : 0u);
-    }
   }
 }
 
@@ -108,10 +100,9 @@ int launch_increment(eif_ctx *c, int rk) {
   EIF_PROF(c, "particle_increment", 1);
   // FP64-heavy per particle: small blocks spread the particles over many SMs
   const int blocks = std::max(1, std::min((c->np + 31) / 32, c->sms * 4));
-  unsigned *counter = reinterpret_cast<unsigned *>(c->d_inc + 1);   // low word: loop counter
+  // d_inc[1]: a loop's counter, then the arrivals
   k_increment<<<blocks, 32, 0, c->stream>>>(c->P, c->pcap, c->np, rk_coef(rk).gamma, Fr * Fr, c->d_scal, c->d_inc,
-                                             counter, counter + 1, c->d_inc + 2, c->loop_handle,
-                                             c->in_loop ? 1 : 0);
+                                             reinterpret_cast<unsigned *>(c->d_inc + 1) + 1, c->d_inc + 2);
   EIF_LAUNCH_CK(c);
   return EIF_OK;
 }
