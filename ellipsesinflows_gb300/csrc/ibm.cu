@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(256, 3) k_ibm_work(WorkArgs a) {
 }
 
 __global__ void __launch_bounds__(256, 3) k_ibm_work_f(WorkArgs a) {
-  __shared__ float2 slot_buf[8][CHUNK];
+  __shared__ WorkSlotsF slot_buf[8];
   ibm_work_f_tasks<true>(a, a.wmode, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
                          slot_buf[threadIdx.x >> 5]);
 }
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(256, 4) k_ibm_sum_f(WorkArgs a) {
 // full evaluation afterwards. One launch: a second one that finds that it is not its turn costs
 // each of some hundred sub-iterations of a step 3 us.
 __global__ void __launch_bounds__(256, 3) k_ibm_loop_f(WorkArgs a) {
-  __shared__ float2 slot_buf[8][CHUNK];
+  __shared__ WorkSlotsF slot_buf[8];
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
   if (*a.iter == 0u) {
     ibm_sum_f_tasks<true>(a, warp, warps, EIF_CHK(a.bd.rec, a.np, a.bd.off, 70) ? __ldg(a.off + a.np) : 0);

@@ -766,13 +766,14 @@ __device__ __forceinline__ int4 task_desc(const OneParticle &o, int r) {
 // Sums of three values over the warp, in 6 additions instead of 15: in each of the first
 // two steps the two halves of a group of lanes keep different values. The additions pair the
 // same lanes as warp_sum's. The sums are in lane 0 (v0), 16 (v1) and 8 (v2).
-__device__ __forceinline__ double warp_sum3(double v0, double v1, double v2, int lane) {
+template <typename T>
+__device__ __forceinline__ T warp_sum3(T v0, T v1, T v2, int lane) {
   const bool h16 = lane & 16, h8 = lane & 8;
-  const double o = __shfl_xor_sync(0xffffffffu, h16 ? v0 : v1, 16);
-  double v = (h16 ? v1 : v0) + o;
+  const T o = __shfl_xor_sync(0xffffffffu, h16 ? v0 : v1, 16);
+  T v = (h16 ? v1 : v0) + o;
   v2 += __shfl_xor_sync(0xffffffffu, v2, 16);
   // lanes 0-7, 16-23 go on with v, lanes 8-15, 24-31 with v2
-  const double q = __shfl_xor_sync(0xffffffffu, h8 ? v : v2, 8);
+  const T q = __shfl_xor_sync(0xffffffffu, h8 ? v : v2, 8);
   v = (h8 ? v2 : v) + q;
 #pragma unroll
   for (int d = 4; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
@@ -798,7 +799,7 @@ __device__ __forceinline__ void prefetch_l1(const double *p) {
 #define WORK_CHK(rec, idx, bound, tag) \
   ((unsigned long long)(idx) < (unsigned long long)(bound) || work_chk_fail((rec), (long long)(idx), (long long)(bound), (tag)))
 constexpr int WORK_ROWS = 4;
-struct WorkSlots {     // shared memory of a warp
+struct alignas(16) WorkSlots {     // shared memory of a warp (or a WorkSlotsF)
   double th[WORK_ROWS][CHUNK];        // weights; before pass 3 the feet (c, s) of its cells
   double px[WORK_ROWS], Y[WORK_ROWS];
   const double *pd[WORK_ROWS];
@@ -1052,190 +1053,226 @@ __device__ __forceinline__ void inertia_cell_f(float th, float X, float Y, float
   s2 = __fmaf_rn(__fmaf_rn(X, valy, __fmul_rn(-Y, valx)), rpim, s2);
 }
 
-// one warp per row task, single precision (see ibm_work_tasks); ONE: the tasks of one particle
+// One warp per row task, single precision, WORK_ROWS rows at a time as in ibm_work_tasks (ONE:
+// the tasks of one particle). Bound by instruction issue: the foot iteration of the near cells,
+// and what a row needs before it (descriptor, parameters, the chords' roots and divisions). One
+// lane prepares a row, four rows at once, instead of every lane the same row; the near cells of
+// the four rows, about 25 a row, are packed onto the lanes together. 2048 ellipses of 12 to 25
+// cells: 108 -> 95 us, 63-70 % of the issue slots; the persistent kernel of 12 suspensions 611 ->
+// 575 us a stage (24 ellipses alone, a row to a warp: 1 % slower). The products of x_, y_ are
+// written out with the roundings that every form of this body has had.
+struct RowF {
+  float4 ell;      // a, b, kex, key
+  float4 geo;      // cz, sz, Y, gx
+  float4 chords;   // row_chords' olo, ohi, ilo, ihi
+  float4 par;      // rpm, rpim, ux, uy
+  int4 cells;      // i0, first and last column, row
+  float vz;
+  int c;           // task number, or -1: skipped
+};
+struct WorkSlotsF {   // shared memory of a warp
+  float th[WORK_ROWS][CHUNK];              // weights
+  RowF row[WORK_ROWS];
+  unsigned char list[WORK_ROWS * CHUNK];   // row * CHUNK + cell of the near cells
+};
+static_assert(sizeof(WorkSlotsF) <= sizeof(WorkSlots) && alignof(WorkSlotsF) <= alignof(WorkSlots),
+              "the persistent kernel has one array for both");
 template <bool NC, bool ONE = false>
-__device__ __forceinline__ void ibm_work_f_tasks(const WorkArgs &a, int wmode, int first, int stride, float2 *slots,
+__device__ __forceinline__ void ibm_work_f_tasks(const WorkArgs &a, int wmode, int first, int stride, WorkSlotsF &ws,
                                                  const OneParticle *one = nullptr) {
   const int lane = threadIdx.x & 31;
   // all tasks, or (with a.only) the listed ones: task number c of list entry k
   const int total = ONE ? one->total
                         : (a.only ? (int)min((long long)ldro<NC>(a.only), (long long)(a.bd.partial / 3))
                                   : (EIF_CHK(a.bd.rec, a.np, a.bd.off, 50) ? ldro<NC>(a.off + a.np) : 0));
-  auto task_no = [&](int k) { return ONE ? one->base + k : (a.only ? ldro<NC>(a.only + 1 + k) : k); };
-  auto desc = [&](int k, int c) {
-    if constexpr (ONE) return task_desc(*one, k);
-    else return ldro<NC>(a.tdesc + c);
-  };
   const float rh = a.rh_f, dxf = a.dx_f, dyf = a.dy_f, dxdy = a.dxdy_f;
   const float rdtv = a.mode == 1 ? __ldg(a.coef + 9) : 0.f;
   const int ld = a.ld;
   float2 *wb = reinterpret_cast<float2 *>(a.wbuf);
   float *wcache = static_cast<float *>(a.wcache);
-  // the next task's table entry is loaded while the current task is processed
-  int4 nxt = make_int4(-1, 0, 0, 0);
-  if (first < total) {
-    const int cf = task_no(first);
-    if (EIF_CHK(a.bd.rec, cf, a.bd.partial / 3, 51)) nxt = desc(first, cf);
+  if (first >= total) return;
+  // the warp's tasks in groups of nearly the same size
+  int left = (total - first + stride - 1) / stride, rows = left;
+  if (left > WORK_ROWS) {
+    const int groups = (left + WORK_ROWS - 1) / WORK_ROWS;
+    rows = (left + groups - 1) / groups;
   }
-  for (int k = first; k < total; k += stride) {
-    const int c = task_no(k);
-    const int4 dsc = nxt;
-    if (k + stride < total) {
-      const int cn = task_no(k + stride);
-      if (EIF_CHK(a.bd.rec, cn, a.bd.partial / 3, 51)) nxt = desc(k + stride, cn);
+  // lane q: task number and descriptor of row q of the group from k0 on
+  auto fetch = [&](int k0, int &c, int4 &dsc) {
+    const int k = k0 + lane * stride;
+    c = -1;
+    dsc = make_int4(-1, 0, 0, 0);
+    if (lane < rows && k < total) {
+      c = ONE ? one->base + k : (a.only ? ldro<NC>(a.only + 1 + k) : k);
+      if (!EIF_CHK(a.bd.rec, c, a.bd.partial / 3, 51)) c = -1;
+      else if constexpr (ONE) dsc = task_desc(*one, k);
+      else dsc = ldro<NC>(a.tdesc + c);
     }
-    const int n = dsc.x;
-    if (!EIF_CHK(a.bd.rec, n, a.np, 52)) continue;
-    RowTask t;
-    const bool task = task_of(dsc, a.np, t);
-    const float4 *q4 = reinterpret_cast<const float4 *>(ONE ? one->pf : a.pf + (size_t)PF_WORDS * n);
-    const float4 qA = ldro<NC>(q4), qB = ldro<NC>(q4 + 1), qC = ldro<NC>(q4 + 2), qD = ldro<NC>(q4 + 3),
-                 qE = ldro<NC>(q4 + 4);
-    const float4 qF = ldro<NC>(q4 + 5), qG = ldro<NC>(q4 + 6);
-    EllF e;
-    e.a = qA.x; e.b = qA.y; e.cz = qA.z; e.sz = qA.w; e.kex = qB.x; e.key = qB.y;
-    const float rpm = qB.z, rpim = qB.w, pux = qC.x, puy = qC.y, pvz = qC.z, gx = qC.w;
-    const int i0 = __float_as_int(qD.x);
-    const int m = task ? t.img + 1 : 1;
-    // image row origin and fraction selected without a local array
-    const int j0i = __float_as_int(m == 0 ? qD.y : (m == 1 ? qD.z : qD.w));
-    const float gyi = m == 0 ? qE.x : (m == 1 ? qE.y : qE.z);
-    const int j = task ? t.j : 1;
-    const float Y = ((float)(j - j0i) - gyi) * dyf;
-    int rank[2];
-    float cX[2], th2[2];
-    bool cin[2];
-    unsigned near_mask[2];
-    // the cells of the task and their field values: loaded before the geometry, so that
-    // the loads are in flight while the weights are evaluated
-    float fuw[2], fue[2], fvs[2], fvn[2];
+  };
+  int nxt_c;
+  int4 nxt;
+  fetch(first, nxt_c, nxt);
+  // a row's field values
+  struct Vel {
+    float uw[CHUNK / 32], ue[CHUNK / 32], vs[CHUNK / 32], vn[CHUNK / 32];
+    bool in[CHUNK / 32];
+  };
+  auto load = [&](int q, Vel &v) {
+    const RowF &r = ws.row[q];
+    const int4 ce = r.cells;
+    const int j = ce.w;
 #pragma unroll
     for (int half = 0; half < CHUNK / 32; half++) {
-      const int i = (task ? t.ib : 1) + half * 32 + lane;
-      bool in = task && i <= t.ie;
+      const int i = ce.y + half * 32 + lane;
+      bool in = r.c >= 0 && i <= ce.z;
       if (in) {
         in = EIF_CHK(a.bd.rec, j * ld + i, a.bd.field, 54) && EIF_CHK(a.bd.rec, (j + 1) * ld + i, a.bd.field, 55) &&
              EIF_CHK(a.bd.rec, j * ld + (i - 1), a.bd.field, 56);
       }
-      cin[half] = in;
-      fuw[half] = fue[half] = fvs[half] = fvn[half] = 0.f;
+      v.in[half] = in;
+      v.uw[half] = v.ue[half] = v.vs[half] = v.vn[half] = 0.f;
       if (in) {
-        fuw[half] = __ldg(a.uxf + j * ld + (i - 1));
-        fue[half] = __ldg(a.uxf + j * ld + i);
-        fvs[half] = __ldg(a.uyf + j * ld + i);
-        fvn[half] = __ldg(a.uyf + (j + 1) * ld + i);
+        v.uw[half] = __ldg(a.uxf + j * ld + (i - 1));
+        v.ue[half] = __ldg(a.uxf + j * ld + i);
+        v.vs[half] = __ldg(a.uyf + j * ld + i);
+        v.vn[half] = __ldg(a.uyf + (j + 1) * ld + i);
       }
     }
-    // (the stage start's weights from the memo are taken by ibm_memo_f_tasks, which
-    // leaves this body only the tasks the memo did not serve)
-    if (wmode == 2) {
-      // weights of the same geometry from an earlier evaluation
+  };
+  for (int k0 = first; left > 0; k0 += rows * stride, left -= rows) {
+    const int nq = min(rows, left);
+    // the next rows' table entries are loaded while these are processed
+    int c = nxt_c;
+    const int4 dsc = nxt;
+    fetch(k0 + rows * stride, nxt_c, nxt);
+    if (lane < nq) {
+      const int n = dsc.x;
+      if (c >= 0 && !EIF_CHK(a.bd.rec, n, a.np, 52)) c = -1;
+      RowF &r = ws.row[lane];
+      r.c = c;
+      r.cells = make_int4(1, 1, 0, 1);
+      if (c >= 0) {
+        RowTask t;
+        const bool task = task_of(dsc, a.np, t);
+        const float4 *q4 = reinterpret_cast<const float4 *>(ONE ? one->pf : a.pf + (size_t)PF_WORDS * n);
+        const float4 qA = ldro<NC>(q4), qB = ldro<NC>(q4 + 1), qC = ldro<NC>(q4 + 2), qD = ldro<NC>(q4 + 3),
+                     qE = ldro<NC>(q4 + 4), qF = ldro<NC>(q4 + 5), qG = ldro<NC>(q4 + 6);
+        const int m = task ? t.img + 1 : 1;
+        // image row origin and fraction selected without a local array
+        const int j0i = __float_as_int(m == 0 ? qD.y : (m == 1 ? qD.z : qD.w));
+        const float gyi = m == 0 ? qE.x : (m == 1 ? qE.y : qE.z);
+        const int j = task ? t.j : 1;
+        const float Y = ((float)(j - j0i) - gyi) * dyf;
+        r.ell = make_float4(qA.x, qA.y, qB.x, qB.y);
+        r.geo = make_float4(qA.z, qA.w, Y, qC.w);
+        r.par = make_float4(qB.z, qB.w, qC.x, qC.y);
+        r.vz = qC.z;
+        r.cells = make_int4(__float_as_int(qD.x), task ? t.ib : 1, task ? t.ie : 0, j);
+        // far cells of the row (PF_AL .. PF_RO2: al, ka, de, so^2, si^2, ro^2)
+        float olo, ohi, ilo, ihi;
+        row_chords(qE.w, qF.x, qF.y, qF.z, qF.w, qG.x, Y, olo, ohi, ilo, ihi);
+        r.chords = make_float4(olo, ohi, ilo, ihi);
+      }
+    }
+    __syncwarp();
+    // the rows' field values are loaded a row ahead
+    Vel vel;
+    load(0, vel);
+    // pass 1: far cells settled, the near ones listed
+    int nnear = 0;
+#pragma unroll 1
+    for (int q = 0; q < nq; q++) {
+      const RowF &r = ws.row[q];
+      if (r.c < 0) continue;
+      const int4 ce = r.cells;
+      const float4 ch = r.chords;
+      const float gx = r.geo.w;
+      const int near0 = nnear;
 #pragma unroll
       for (int half = 0; half < CHUNK / 32; half++) {
-        const int i = (task ? t.ib : 1) + half * 32 + lane;
-        if (cin[half]) cin[half] = EIF_CHK(a.bd.rec, (long long)c * CHUNK + half * 32 + lane, 2 * a.bd.wbuf, 59);
-        cX[half] = ((float)(i - i0) - gx) * dxf;
-        th2[half] = cin[half] ? wcache[(size_t)c * CHUNK + half * 32 + lane] : 0.f;
+        const int at = half * 32 + lane, i = ce.y + at;
+        const bool in = i <= ce.z;
+        const float X = ((float)(i - ce.x) - gx) * dxf;
+        const int side = !(X > ch.x && X < ch.y) ? -1 : ((X >= ch.z && X <= ch.w) ? 1 : 0);
+        const bool near = in && side == 0;
+        ws.th[q][at] = in ? (float)side : 0.f;
+        const unsigned mask = __ballot_sync(0xffffffffu, near);
+        if (near) ws.list[nnear + __popc(mask & ((1u << lane) - 1u))] = (unsigned char)(q * CHUNK + at);
+        nnear += __popc(mask);
       }
-    } else {
-    // far cells of this row (PF_AL .. PF_RO2: al, ka, de, so^2, si^2, ro^2)
-    float olo, ohi, ilo, ihi;
-    row_chords(qE.w, qF.x, qF.y, qF.z, qF.w, qG.x, Y, olo, ohi, ilo, ihi);
-    // pass 1: cells of the row, far cells settled, body-frame offsets of the near ones
-#pragma unroll
-    for (int half = 0; half < CHUNK / 32; half++) {
-      const int i = (task ? t.ib : 1) + half * 32 + lane;
-      const bool in = cin[half];
-      bool near = false;
-      float x_ = 0.f, y_ = 0.f;
-      const float X = ((float)(i - i0) - gx) * dxf;
-      cX[half] = X;
-      th2[half] = 0.f;
-      if (in) {
-        const int side = !(X > olo && X < ohi) ? -1 : ((X >= ilo && X <= ihi) ? 1 : 0);
-        th2[half] = (float)side;
-        near = side == 0;
-        x_ = e.cz * X - e.sz * Y;
-        y_ = e.sz * X + e.cz * Y;
-      }
-      near_mask[half] = __ballot_sync(0xffffffffu, near);
-      rank[half] = (half ? __popc(near_mask[0]) : 0) + __popc(near_mask[half] & ((1u << lane) - 1u));
-      if (near) slots[rank[half]] = make_float2(x_, y_);
-    }
-    // pass 2: the near cells, packed onto consecutive lanes
-    const int nnear = __popc(near_mask[0]) + __popc(near_mask[1]);
-    if (a.count) {
-      const unsigned in0 = __ballot_sync(0xffffffffu, cin[0]), in1 = __ballot_sync(0xffffffffu, cin[1]);
-      if (lane == 0) {
-        atomicAdd(a.count, (unsigned long long)(__popc(in0) + __popc(in1)));
-        atomicAdd(a.count + 1, (unsigned long long)nnear);
+      if (a.count && lane == 0) {
+        atomicAdd(a.count, (unsigned long long)max(0, min(CHUNK, ce.z - ce.y + 1)));
+        atomicAdd(a.count + 1, (unsigned long long)(nnear - near0));
       }
     }
     __syncwarp();
+    // pass 2: the near cells, packed onto the lanes
     for (int k = lane; k < nnear; k += 32) {
-      const float2 o = slots[k];
-      slots[k].x = indicator_f(e, o.x, o.y, rh);
+      const int id = ws.list[k], q = id / CHUNK, at = id % CHUNK;
+      const RowF &r = ws.row[q];
+      const float4 el = r.ell, ge = r.geo;
+      EllF e;
+      e.a = el.x; e.b = el.y; e.kex = el.z; e.key = el.w; e.cz = ge.x; e.sz = ge.y;
+      const float X = ((float)(r.cells.y + at - r.cells.x) - ge.w) * dxf, Y = ge.z;
+      const float x_ = __fmaf_rn(e.cz, X, -__fmul_rn(e.sz, Y));
+      const float y_ = __fmaf_rn(e.sz, X, __fmul_rn(e.cz, Y));
+      ws.th[q][at] = indicator_f(e, x_, y_, rh);
     }
     __syncwarp();
+    // the sums
+#pragma unroll 1
+    for (int q = 0; q < nq; q++) {
+      const Vel v = vel;
+      if (q + 1 < nq) load(q + 1, vel);
+      const RowF &r = ws.row[q];
+      const int c = r.c;
+      if (c < 0) continue;
+      const float4 par = r.par;
+      const float Y = r.geo.z, gx = r.geo.w, pvz = r.vz;
+      const int at0 = r.cells.y - r.cells.x;
+      float sacc0 = 0.f, sacc1 = 0.f, sacc2 = 0.f;
 #pragma unroll
-    for (int half = 0; half < CHUNK / 32; half++)
-      if ((near_mask[half] >> lane) & 1u) th2[half] = slots[rank[half]].x;
-    __syncwarp();
-    if (a.memo_mode == 2) {
-#pragma unroll
-      for (int half = 0; half < CHUNK / 32; half++)
-        if (EIF_CHK(a.bd.rec, (long long)c * CHUNK + half * 32 + lane, a.bd.wbuf, 61))
-          a.memo.w[(size_t)c * CHUNK + half * 32 + lane] = th2[half];
-    }
-    }
-    if (wmode == 1) {
-#pragma unroll
-      for (int half = 0; half < CHUNK / 32; half++)
-        if (EIF_CHK(a.bd.rec, (long long)c * CHUNK + half * 32 + lane, 2 * a.bd.wbuf, 60))
-          wcache[(size_t)c * CHUNK + half * 32 + lane] = th2[half];
-    }
-    float sacc0 = 0.f, sacc1 = 0.f, sacc2 = 0.f;
-#pragma unroll
-    for (int half = 0; half < CHUNK / 32; half++) {
-      float2 contrib = make_float2(0.f, 0.f);
-      // cells of weight exactly zero (inertia: far outside; exchange: any far cell) are skipped
-      const float th_ = th2[half];
-      const bool live = a.mode == 0 ? th_ != -1.f : fabsf(th_) != 1.f;
-      if (cin[half] && live) {
-        const float X = cX[half], th = th_;
-        const float uxs = fuw[half] + fue[half];
-        const float uys = fvs[half] + fvn[half];
-        if (a.mode == 0) {
-          inertia_cell_f(th, X, Y, uxs, uys, dxdy, rpm, rpim, sacc0, sacc1, sacc2);
-        } else {
-          const float w = 1.f - th * th;
-          const float uxp = pux - pvz * Y;
-          const float uyp = puy + pvz * X;
-          const float gxv = w * (uxp - 0.5f * uxs);   // fx * dt
-          const float gyv = w * (uyp - 0.5f * uys);   // fy * dt
-          contrib = make_float2(gxv, gyv);
-          const float Fx = gxv * rdtv * dxdy, Fy = gyv * rdtv * dxdy;
-          sacc0 -= Fx * rpm;
-          sacc1 -= Fy * rpm;
-          sacc2 += (Y * Fx - X * Fy) * rpim;
+      for (int half = 0; half < CHUNK / 32; half++) {
+        const int at = half * 32 + lane;
+        float2 contrib = make_float2(0.f, 0.f);
+        const float th = ws.th[q][at];
+        // (the stage start's weights from the memo are taken by ibm_memo_f_tasks, which
+        // leaves this body only the tasks the memo did not serve)
+        if (a.memo_mode == 2 && EIF_CHK(a.bd.rec, (long long)c * CHUNK + at, a.bd.wbuf, 61))
+          a.memo.w[(size_t)c * CHUNK + at] = th;
+        if (wmode == 1 && EIF_CHK(a.bd.rec, (long long)c * CHUNK + at, 2 * a.bd.wbuf, 60))
+          wcache[(size_t)c * CHUNK + at] = th;
+        // cells of weight exactly zero (inertia: far outside; exchange: any far cell) are skipped
+        const bool live = a.mode == 0 ? th != -1.f : fabsf(th) != 1.f;
+        if (v.in[half] && live) {
+          const float X = ((float)(at0 + at) - gx) * dxf;
+          const float uxs = v.uw[half] + v.ue[half];
+          const float uys = v.vs[half] + v.vn[half];
+          if (a.mode == 0) {
+            inertia_cell_f(th, X, Y, uxs, uys, dxdy, par.x, par.y, sacc0, sacc1, sacc2);
+          } else {
+            const float w = 1.f - th * th;
+            const float uxp = par.z - pvz * Y;
+            const float uyp = par.w + pvz * X;
+            const float gxv = w * (uxp - 0.5f * uxs);   // fx * dt
+            const float gyv = w * (uyp - 0.5f * uys);   // fy * dt
+            contrib = make_float2(gxv, gyv);
+            const float Fx = gxv * rdtv * dxdy, Fy = gyv * rdtv * dxdy;
+            sacc0 -= Fx * par.x;
+            sacc1 -= Fy * par.x;
+            sacc2 += (Y * Fx - X * Fy) * par.y;
+          }
         }
+        if (a.mode == 1 && EIF_CHK(a.bd.rec, (long long)c * CHUNK + at, 2 * a.bd.wbuf, 57))
+          wb[(size_t)c * CHUNK + at] = contrib;
       }
-      if (a.mode == 1 && EIF_CHK(a.bd.rec, (long long)c * CHUNK + half * 32 + lane, 2 * a.bd.wbuf, 57))
-        wb[(size_t)c * CHUNK + half * 32 + lane] = contrib;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      sacc0 += __shfl_xor_sync(0xffffffffu, sacc0, o);
-      sacc1 += __shfl_xor_sync(0xffffffffu, sacc1, o);
-      sacc2 += __shfl_xor_sync(0xffffffffu, sacc2, o);
-    }
-    if (lane == 0 && EIF_CHK(a.bd.rec, 3LL * c + 2, a.bd.partial, 58)) {
       // single-precision partial sums, reduced per particle by k_chunk_reduce_f
-      float *pf3 = reinterpret_cast<float *>(a.partial);
-      pf3[3 * (size_t)c + 0] = sacc0;
-      pf3[3 * (size_t)c + 1] = sacc1;
-      pf3[3 * (size_t)c + 2] = sacc2;
+      const float sum = warp_sum3(sacc0, sacc1, sacc2, lane);
+      const int slot = lane == 0 ? 0 : (lane == 16 ? 1 : (lane == 8 ? 2 : -1));
+      if (slot >= 0 && EIF_CHK(a.bd.rec, 3LL * c + 2, a.bd.partial, 58))
+        reinterpret_cast<float *>(a.partial)[3 * (size_t)c + slot] = sum;
     }
+    __syncwarp();
   }
 }
 

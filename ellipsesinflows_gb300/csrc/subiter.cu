@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(SUB_THREADS, 2) k_subiterations(StageArgs s) {
           const int r0 = (int)((long long)cnt * sl / d.ns), r1 = (int)((long long)cnt * (sl + 1) / d.ns);
           const OneParticle one{reinterpret_cast<const int4 *>(bx), pf, pd, p, c0, r1};
           if (d.mixed) {
-            ibm_work_f_tasks<false, true>(d.work, 0, r0 + wl, SUB_WARPS, reinterpret_cast<float2 *>(&slot_d[wl]), &one);
+            ibm_work_f_tasks<false, true>(d.work, 0, r0 + wl, SUB_WARPS, reinterpret_cast<WorkSlotsF &>(slot_d[wl]), &one);
             if (sl == 0 && wl == SUB_WARPS - 2 && d.work.memo_mode == 2) memo_particle(d.work.memo, pf, bx, one.base, p);
           } else {
             ibm_work_tasks<false>(d.work, 0, r0 + wl, SUB_WARPS, slot_d[wl], &one);
