@@ -1053,14 +1053,34 @@ __device__ __forceinline__ void inertia_cell_f(float th, float X, float Y, float
   s2 = __fmaf_rn(__fmaf_rn(X, valy, __fmul_rn(-Y, valx)), rpim, s2);
 }
 
+// The bounds of a row's accesses, checked once for the row: cells ib - 1 .. ie of rows j and
+// j + 1, and the CHUNK slots of task c in a buffer of n. (A check of every cell's was two
+// compares and a divergence point each: 95 us of a full evaluation with 2048 ellipses, by the
+// row 88.)
+__device__ __forceinline__ bool row_cells_in(const Bounds &bd, const RowTask &t, int ld, int tag) {
+  return EIF_CHK(bd.rec, (long long)t.j * ld + t.ib - 1, bd.field, tag) &&
+         EIF_CHK(bd.rec, (long long)(t.j + 1) * ld + t.ie, bd.field, tag + 1);
+}
+__device__ __forceinline__ bool row_slots_in(const Bounds &bd, long long c, long long n, int tag) {
+  return EIF_CHK(bd.rec, c * CHUNK, n, tag) && EIF_CHK(bd.rec, c * CHUNK + CHUNK - 1, n, tag);
+}
+
 // One warp per row task, single precision, WORK_ROWS rows at a time as in ibm_work_tasks (ONE:
 // the tasks of one particle). Bound by instruction issue: the foot iteration of the near cells,
 // and what a row needs before it (descriptor, parameters, the chords' roots and divisions). One
 // lane prepares a row, four rows at once, instead of every lane the same row; the near cells of
 // the four rows, about 25 a row, are packed onto the lanes together. 2048 ellipses of 12 to 25
-// cells: 108 -> 95 us, 63-70 % of the issue slots; the persistent kernel of 12 suspensions 611 ->
-// 575 us a stage (24 ellipses alone, a row to a warp: 1 % slower). The products of x_, y_ are
+// cells: 108 -> 95 us (88 with the bounds checked by the row), 63-70 % of the issue slots; the
+// persistent kernel of 12 suspensions 611 -> 575 us a stage (24 ellipses alone, a row to a warp:
+// 1 % slower). The products of x_, y_ are
 // written out with the roundings that every form of this body has had.
+// single-precision partial sums of task c, reduced per particle by k_chunk_reduce_f
+__device__ __forceinline__ void store_sums_f(const WorkArgs &a, int c, float s0, float s1, float s2, int lane, int tag) {
+  const float sum = warp_sum3(s0, s1, s2, lane);
+  const int slot = lane == 0 ? 0 : (lane == 16 ? 1 : (lane == 8 ? 2 : -1));
+  if (slot >= 0 && EIF_CHK(a.bd.rec, 3LL * c + 2, a.bd.partial, tag))
+    reinterpret_cast<float *>(a.partial)[3 * (size_t)c + slot] = sum;
+}
 struct RowF {
   float4 ell;      // a, b, kex, key
   float4 geo;      // cz, sz, Y, gx
@@ -1124,11 +1144,7 @@ __device__ __forceinline__ void ibm_work_f_tasks(const WorkArgs &a, int wmode, i
 #pragma unroll
     for (int half = 0; half < CHUNK / 32; half++) {
       const int i = ce.y + half * 32 + lane;
-      bool in = r.c >= 0 && i <= ce.z;
-      if (in) {
-        in = EIF_CHK(a.bd.rec, j * ld + i, a.bd.field, 54) && EIF_CHK(a.bd.rec, (j + 1) * ld + i, a.bd.field, 55) &&
-             EIF_CHK(a.bd.rec, j * ld + (i - 1), a.bd.field, 56);
-      }
+      const bool in = r.c >= 0 && i <= ce.z;
       v.in[half] = in;
       v.uw[half] = v.ue[half] = v.vs[half] = v.vn[half] = 0.f;
       if (in) {
@@ -1147,13 +1163,13 @@ __device__ __forceinline__ void ibm_work_f_tasks(const WorkArgs &a, int wmode, i
     fetch(k0 + rows * stride, nxt_c, nxt);
     if (lane < nq) {
       const int n = dsc.x;
-      if (c >= 0 && !EIF_CHK(a.bd.rec, n, a.np, 52)) c = -1;
+      if (c >= 0 && !(EIF_CHK(a.bd.rec, n, a.np, 52) && row_slots_in(a.bd, c, a.bd.wbuf, 60))) c = -1;
       RowF &r = ws.row[lane];
       r.c = c;
       r.cells = make_int4(1, 1, 0, 1);
       if (c >= 0) {
         RowTask t;
-        const bool task = task_of(dsc, a.np, t);
+        const bool task = task_of(dsc, a.np, t) && (t.ib > t.ie || row_cells_in(a.bd, t, ld, 54));
         const float4 *q4 = reinterpret_cast<const float4 *>(ONE ? one->pf : a.pf + (size_t)PF_WORDS * n);
         const float4 qA = ldro<NC>(q4), qB = ldro<NC>(q4 + 1), qC = ldro<NC>(q4 + 2), qD = ldro<NC>(q4 + 3),
                      qE = ldro<NC>(q4 + 4), qF = ldro<NC>(q4 + 5), qG = ldro<NC>(q4 + 6);
@@ -1238,10 +1254,8 @@ __device__ __forceinline__ void ibm_work_f_tasks(const WorkArgs &a, int wmode, i
         const float th = ws.th[q][at];
         // (the stage start's weights from the memo are taken by ibm_memo_f_tasks, which
         // leaves this body only the tasks the memo did not serve)
-        if (a.memo_mode == 2 && EIF_CHK(a.bd.rec, (long long)c * CHUNK + at, a.bd.wbuf, 61))
-          a.memo.w[(size_t)c * CHUNK + at] = th;
-        if (wmode == 1 && EIF_CHK(a.bd.rec, (long long)c * CHUNK + at, 2 * a.bd.wbuf, 60))
-          wcache[(size_t)c * CHUNK + at] = th;
+        if (a.memo_mode == 2) a.memo.w[(size_t)c * CHUNK + at] = th;
+        if (wmode == 1) wcache[(size_t)c * CHUNK + at] = th;
         // cells of weight exactly zero (inertia: far outside; exchange: any far cell) are skipped
         const bool live = a.mode == 0 ? th != -1.f : fabsf(th) != 1.f;
         if (v.in[half] && live) {
@@ -1263,14 +1277,9 @@ __device__ __forceinline__ void ibm_work_f_tasks(const WorkArgs &a, int wmode, i
             sacc2 += (Y * Fx - X * Fy) * par.y;
           }
         }
-        if (a.mode == 1 && EIF_CHK(a.bd.rec, (long long)c * CHUNK + at, 2 * a.bd.wbuf, 57))
-          wb[(size_t)c * CHUNK + at] = contrib;
+        if (a.mode == 1) wb[(size_t)c * CHUNK + at] = contrib;
       }
-      // single-precision partial sums, reduced per particle by k_chunk_reduce_f
-      const float sum = warp_sum3(sacc0, sacc1, sacc2, lane);
-      const int slot = lane == 0 ? 0 : (lane == 16 ? 1 : (lane == 8 ? 2 : -1));
-      if (slot >= 0 && EIF_CHK(a.bd.rec, 3LL * c + 2, a.bd.partial, 58))
-        reinterpret_cast<float *>(a.partial)[3 * (size_t)c + slot] = sum;
+      store_sums_f(a, c, sacc0, sacc1, sacc2, lane, 58);
     }
     __syncwarp();
   }
@@ -1315,7 +1324,7 @@ __device__ __forceinline__ void ibm_memo_f_tasks(const WorkArgs &a, int first, i
     if (a.count && lane == 0) atomicAdd(a.count + 2, 1ull);
     const long long src = (long long)c + (ldro<NC>(a.memo.off + n) - ldro<NC>(a.off + n));
     RowTask t;
-    const bool task = task_of(dsc, a.np, t);
+    const bool task = task_of(dsc, a.np, t) && (t.ib > t.ie || row_cells_in(a.bd, t, ld, 94));
     const float4 *q4 = reinterpret_cast<const float4 *>(a.pf + (size_t)PF_WORDS * n);
     const float4 qB = ldro<NC>(q4 + 1), qC = ldro<NC>(q4 + 2), qD = ldro<NC>(q4 + 3), qE = ldro<NC>(q4 + 4);
     const float rpm = qB.z, rpim = qB.w, gx = qC.w;
@@ -1330,11 +1339,7 @@ __device__ __forceinline__ void ibm_memo_f_tasks(const WorkArgs &a, int first, i
 #pragma unroll
     for (int half = 0; half < CHUNK / 32; half++) {
       const int i = (task ? t.ib : 1) + half * 32 + lane;
-      bool in = task && i <= t.ie;
-      if (in) {
-        in = EIF_CHK(a.bd.rec, j * ld + i, a.bd.field, 94) && EIF_CHK(a.bd.rec, (j + 1) * ld + i, a.bd.field, 95) &&
-             EIF_CHK(a.bd.rec, j * ld + (i - 1), a.bd.field, 96);
-      }
+      const bool in = task && i <= t.ie;
       fuw[half] = fue[half] = fvs[half] = fvn[half] = 0.f;
       if (in) {
         fuw[half] = __ldg(a.uxf + j * ld + (i - 1));
@@ -1342,15 +1347,16 @@ __device__ __forceinline__ void ibm_memo_f_tasks(const WorkArgs &a, int first, i
         fvs[half] = __ldg(a.uyf + j * ld + i);
         fvn[half] = __ldg(a.uyf + (j + 1) * ld + i);
       }
-      if (in) in = EIF_CHK(a.bd.rec, src * CHUNK + half * 32 + lane, a.bd.wbuf, 97);
       cin[half] = in;
       cX[half] = ((float)(i - i0) - gx) * dxf;
-      th2[half] = in ? a.memo.w[(size_t)src * CHUNK + half * 32 + lane] : 0.f;
     }
+    // (after the field loads, which do not wait for the offsets)
+    if (!row_slots_in(a.bd, c, a.bd.wbuf, 98) || !row_slots_in(a.bd, src, a.bd.wbuf, 97)) continue;
 #pragma unroll
     for (int half = 0; half < CHUNK / 32; half++)
-      if (EIF_CHK(a.bd.rec, (long long)c * CHUNK + half * 32 + lane, 2 * a.bd.wbuf, 98))
-        wcache[(size_t)c * CHUNK + half * 32 + lane] = th2[half];
+      th2[half] = cin[half] ? a.memo.w[(size_t)src * CHUNK + half * 32 + lane] : 0.f;
+#pragma unroll
+    for (int half = 0; half < CHUNK / 32; half++) wcache[(size_t)c * CHUNK + half * 32 + lane] = th2[half];
     float sacc0 = 0.f, sacc1 = 0.f, sacc2 = 0.f;
 #pragma unroll
     for (int half = 0; half < CHUNK / 32; half++) {
@@ -1361,18 +1367,7 @@ __device__ __forceinline__ void ibm_memo_f_tasks(const WorkArgs &a, int first, i
         inertia_cell_f(th_, cX[half], Y, uxs, uys, dxdy, rpm, rpim, sacc0, sacc1, sacc2);
       }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      sacc0 += __shfl_xor_sync(0xffffffffu, sacc0, o);
-      sacc1 += __shfl_xor_sync(0xffffffffu, sacc1, o);
-      sacc2 += __shfl_xor_sync(0xffffffffu, sacc2, o);
-    }
-    if (lane == 0 && EIF_CHK(a.bd.rec, 3LL * c + 2, a.bd.partial, 99)) {
-      float *pf3 = reinterpret_cast<float *>(a.partial);
-      pf3[3 * (size_t)c + 0] = sacc0;
-      pf3[3 * (size_t)c + 1] = sacc1;
-      pf3[3 * (size_t)c + 2] = sacc2;
-    }
+    store_sums_f(a, c, sacc0, sacc1, sacc2, lane, 99);
   }
 }
 
@@ -1410,9 +1405,9 @@ __device__ __forceinline__ void ibm_sum_f_tasks(const WorkArgs &a, int first, in
       nth1 = wcache[(size_t)cn * CHUNK + 32 + lane];
     }
     const int n = dsc.x;
-    if (!EIF_CHK(a.bd.rec, n, a.np, 72)) continue;
+    if (!EIF_CHK(a.bd.rec, n, a.np, 72) || !row_slots_in(a.bd, c, 2 * a.bd.wbuf, 78)) continue;
     RowTask t;
-    const bool task = task_of(dsc, a.np, t);
+    const bool task = task_of(dsc, a.np, t) && (t.ib > t.ie || row_cells_in(a.bd, t, ld, 74));
     const float4 *q4 = reinterpret_cast<const float4 *>(a.pf + (size_t)PF_WORDS * n);
     const float4 qB = ldro<NC>(q4 + 1), qC = ldro<NC>(q4 + 2), qD = ldro<NC>(q4 + 3), qE = ldro<NC>(q4 + 4);
     const float rpm = qB.z, rpim = qB.w, pux = qC.x, puy = qC.y, pvz = qC.z, gx = qC.w;
@@ -1430,11 +1425,7 @@ __device__ __forceinline__ void ibm_sum_f_tasks(const WorkArgs &a, int first, in
 #pragma unroll
     for (int half = 0; half < CHUNK / 32; half++) {
       const int i = (task ? t.ib : 1) + half * 32 + lane;
-      bool in = task && i <= t.ie;
-      if (in) {
-        in = EIF_CHK(a.bd.rec, j * ld + i, a.bd.field, 74) && EIF_CHK(a.bd.rec, (j + 1) * ld + i, a.bd.field, 75) &&
-             EIF_CHK(a.bd.rec, j * ld + (i - 1), a.bd.field, 76);
-      }
+      const bool in = task && i <= t.ie;
       const float th = in ? th_pre[half] : 0.f;
       thv[half] = th;
       // cells of weight exactly zero (inertia: far outside; exchange: any far cell) are skipped
@@ -1473,21 +1464,9 @@ __device__ __forceinline__ void ibm_sum_f_tasks(const WorkArgs &a, int first, in
           sacc2 += (Y * Fx - X * Fy) * rpim;
         }
       }
-      if (a.mode == 1 && EIF_CHK(a.bd.rec, slot, 2 * a.bd.wbuf, 78)) wb[slot] = contrib;
+      if (a.mode == 1) wb[slot] = contrib;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      sacc0 += __shfl_xor_sync(0xffffffffu, sacc0, o);
-      sacc1 += __shfl_xor_sync(0xffffffffu, sacc1, o);
-      sacc2 += __shfl_xor_sync(0xffffffffu, sacc2, o);
-    }
-    if (lane == 0 && EIF_CHK(a.bd.rec, 3LL * c + 2, a.bd.partial, 79)) {
-      // single-precision partial sums, reduced per particle by k_chunk_reduce_f
-      float *pf3 = reinterpret_cast<float *>(a.partial);
-      pf3[3 * (size_t)c + 0] = sacc0;
-      pf3[3 * (size_t)c + 1] = sacc1;
-      pf3[3 * (size_t)c + 2] = sacc2;
-    }
+    store_sums_f(a, c, sacc0, sacc1, sacc2, lane, 79);
   }
 }
 
