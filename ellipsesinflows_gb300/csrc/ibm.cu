@@ -372,7 +372,6 @@ struct GatherArgs {
   void *dux, *duy;   // double (FP64 form) or float (mixed form) fields with the same pitch
   unsigned *flags;
   int np, itot, jtot, ld;
-  int halo;          // the halo rows and ghost columns too
   Bounds bd;
 };
 
@@ -440,10 +439,8 @@ __global__ void __launch_bounds__(GTHREADS, 6) k_gather(GatherArgs a) {
     }
     __syncthreads();
   }
-  // write the tile's interior cells (zero where no box covers) and, with halo, their copies in
-  // the periodic halo rows (j = 0 <- jtot, j = jtot+1 <- 1) and the Neumann ghost columns
-  // (i = 0 <- 1, i = itot+1 <- itot, corners included), exchange.c:80-81 with the boundary
-  // update of the reference
+  // write the tile's interior cells (zero where no box covers); the halo rows and
+  // ghost columns are filled afterwards by k_ibm_halo from these cells
   const int ld = a.ld;
 #pragma unroll
   for (int q = 0; q < NC; q++) {
@@ -453,20 +450,33 @@ __global__ void __launch_bounds__(GTHREADS, 6) k_gather(GatherArgs a) {
     if (!EIF_CHK(a.bd.rec, cidx, a.bd.field, 42)) continue;
     static_cast<Acc *>(a.dux)[cidx] = acc_x[q];
     static_cast<Acc *>(a.duy)[cidx] = acc_y[q];
-    if (a.halo && (i == 1 || i == a.itot || j == 1 || j == a.jtot)) {
-      for (int jj = 0; jj < 3; jj++) {
-        if ((jj == 1 && j != a.jtot) || (jj == 2 && j != 1)) continue;
-        const int row = (jj == 0 ? j : (jj == 1 ? 0 : a.jtot + 1)) * ld;
-        for (int ii = 0; ii < 3; ii++) {
-          if ((ii == 1 && i != 1) || (ii == 2 && i != a.itot)) continue;
-          const int col = ii == 0 ? i : (ii == 1 ? 0 : a.itot + 1);
-          if ((ii | jj) == 0 || !EIF_CHK(a.bd.rec, row + col, a.bd.field, 43)) continue;
-          static_cast<Acc *>(a.dux)[row + col] = acc_x[q];
-          static_cast<Acc *>(a.duy)[row + col] = acc_y[q];
-        }
-      }
-    }
   }
+}
+
+// Periodic halo rows (j = 0 <- jtot, j = jtot+1 <- 1) and Neumann ghost columns
+// (i = 0 <- 1, i = itot+1 <- itot, corners included) of the IBM field response,
+// exchange.c:80-81 with the boundary update of the reference. Every thread reads
+// one interior cell and writes one halo cell.
+template <typename T>
+__global__ void k_ibm_halo(T *__restrict__ dux, T *__restrict__ duy, int itot, int jtot, int ld) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nrow = itot + 2;
+  int dst, src;
+  if (t < 2 * nrow) {
+    const int i = t % nrow, top = t / nrow;
+    const int ic = i < 1 ? 1 : (i > itot ? itot : i);
+    dst = (top ? jtot + 1 : 0) * ld + i;
+    src = (top ? 1 : jtot) * ld + ic;
+  } else if (t < 2 * nrow + 2 * jtot) {
+    const int u = t - 2 * nrow;
+    const int j = 1 + u % jtot, right = u / jtot;
+    dst = j * ld + (right ? itot + 1 : 0);
+    src = j * ld + (right ? itot : 1);
+  } else {
+    return;
+  }
+  dux[dst] = dux[src];
+  duy[dst] = duy[src];
 }
 
 }  // namespace
@@ -808,13 +818,19 @@ int launch_gather(eif_ctx *c) {
   g.np = c->np; g.itot = c->itot; g.jtot = c->jtot; g.ld = c->ld;
   g.bd = bounds_of(c);
   g.lists = c->band_lists; g.counts = c->band_counts; g.cap = c->band_cap;
-  g.halo = 1;
   dim3 grid((c->itot + GTX - 1) / GTX, (c->jtot + GTY - 1) / GTY);
-  EIF_PROF(c, "ibm_gather", 1);
+  EIF_PROF(c, "ibm_gather", 2);
+  const int nhalo = 2 * (c->itot + 2) + 2 * c->jtot;
   if (c->cfg.precision == EIF_PREC_MIXED) {
     k_gather<float2, float><<<grid, GTHREADS, 0, c->stream>>>(g);
+    EIF_LAUNCH_CK(c);
+    k_ibm_halo<float><<<(nhalo + 255) / 256, 256, 0, c->stream>>>(reinterpret_cast<float *>(c->dux),
+                                                                  reinterpret_cast<float *>(c->duy), c->itot,
+                                                                  c->jtot, c->ld);
   } else {
     k_gather<double2, double><<<grid, GTHREADS, 0, c->stream>>>(g);
+    EIF_LAUNCH_CK(c);
+    k_ibm_halo<double><<<(nhalo + 255) / 256, 256, 0, c->stream>>>(c->dux, c->duy, c->itot, c->jtot, c->ld);
   }
   EIF_LAUNCH_CK(c);
   return EIF_OK;
@@ -1041,7 +1057,6 @@ int launch_adj_pass(eif_ctx *c, const AdjPass &p) {
   GatherArgs g;
   g.edesc = c->edesc; g.wbuf = c->wbuf;
   g.dux = p.fx; g.duy = p.fy; g.flags = c->d_flags;
-  g.halo = 0;
   g.np = c->np; g.itot = c->itot; g.jtot = c->jtot; g.ld = c->ld;
   g.bd = bounds_of(c);
   g.lists = c->band_lists; g.counts = c->band_counts; g.cap = c->band_cap;
