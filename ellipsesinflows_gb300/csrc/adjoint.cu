@@ -53,7 +53,7 @@ struct Adjoint {
   double *gcx = nullptr, *gcy = nullptr;   // cell cotangents of the field response (cell layout)
   // particle cotangents (3 x np each): position, velocity, carried increment, force,
   // inertia at X, inertia of one sub-iteration; box-pass output (6 x np) and scratch
-  double *xb = nullptr, *vpb = nullptr, *dub = nullptr, *fb = nullptr, *i0b = nullptr, *i1b = nullptr;
+  double *xb = nullptr, *vpb = nullptr, *fb = nullptr, *i0b = nullptr, *i1b = nullptr;
   double *pout = nullptr, *part = nullptr;
   int part_cap = 0;
   // indicator geometry of the box cells at X, shared by the three transposed evaluations
@@ -341,13 +341,6 @@ __global__ void k_adj_dxsave(const double *__restrict__ P, int pcap, int np, dou
   dst[np + n] = P[EIF_P_DY * pcap + n];
   dst[2 * np + n] = P[EIF_P_DAZ * pcap + n];
 }
-__global__ void k_adj_dxload(double *__restrict__ P, int pcap, int np, const double *__restrict__ src) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= np) return;
-  P[EIF_P_DX * pcap + n] = src[n];
-  P[EIF_P_DY * pcap + n] = src[np + n];
-  P[EIF_P_DAZ * pcap + n] = src[2 * np + n];
-}
 // any non-zero collision force or torque of this stage (increment.c:24-36)
 __global__ void k_adj_contact(const double *__restrict__ P, int pcap, int np, int *__restrict__ flag) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
@@ -358,36 +351,46 @@ __global__ void k_adj_contact(const double *__restrict__ P, int pcap, int np, in
 }
 // reverse of U' = U + dU_K, X' = X + dX_K, dX_K = g dt (U + dU_K / 2):
 // dUbar = Ubar' + (g dt / 2) Xbar', Ubar = Ubar' + g dt Xbar', Xbar = Xbar'
-__global__ void k_adj_stage_init(int np, double gdt, const double *__restrict__ xb, double *__restrict__ vpb,
-                                 double *__restrict__ dub, double *__restrict__ fb, double *__restrict__ i0b) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * np) return;
-  dub[t] = vpb[t] + 0.5 * gdt * xb[t];
-  vpb[t] += gdt * xb[t];
-  fb[t] = 0.;
-  i0b[t] = 0.;
-}
 // reverse of dU_{m+1} = dt F + I1_m - I0
-__global__ void k_adj_iter_pre(int np, double dt, const double *__restrict__ dub, double *__restrict__ fb,
-                               double *__restrict__ i0b, double *__restrict__ i1b) {
+// Between the passes of two sub-iterations in reverse, one component of a particle per thread:
+// what the pass of sub-iteration m + 1 gave (k_adj_iter_end's sum and, as m + 1 > 0, the
+// velocities), or for the last one (first) the start of the stage; then the
+// cotangents and the increments of the pass of sub-iteration m. One launch: the backward sweep
+// of a small grid is as long as its launches (4 us each, 256 x 512 with 8 ellipses).
+__device__ __forceinline__ int increment_field(int k) { return k == 0 ? EIF_P_DX : (k == 1 ? EIF_P_DY : EIF_P_DAZ); }
+__global__ void k_adj_iter(int np, int first, double dt, double gdt, const double *__restrict__ pout,
+                           double *__restrict__ xb, double *__restrict__ vpb, double *__restrict__ fb,
+                           double *__restrict__ i0b, double *__restrict__ i1b, double *__restrict__ P, int pcap,
+                           const double *__restrict__ dx) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 3 * np) return;
-  fb[t] += dt * dub[t];
-  i0b[t] -= dub[t];
-  i1b[t] = dub[t];
-}
-// reverse of I1_m = Inert(X + dX_m) in the particle state: the position cotangent z
-// goes to X, and for m >= 1 through dX_m = g dt (U + dU_m / 2) to U and dU_m
-__global__ void k_adj_iter_post(int np, double gdt, const double *__restrict__ pout, double *__restrict__ xb,
-                                double *__restrict__ vpb, double *__restrict__ dub, int more) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * np) return;
-  const double z = pout[t];
-  xb[t] += z;
-  if (more) {
+  double dub, f, i0;
+  if (first) {
+    const double x = xb[t], v = vpb[t];
+    dub = v + 0.5 * gdt * x;
+    vpb[t] = v + gdt * x;
+    f = 0.;
+    i0 = 0.;
+  } else {
+    const double z = pout[t];
+    xb[t] += z;
     vpb[t] += gdt * z;
-    dub[t] = 0.5 * gdt * z;
+    dub = 0.5 * gdt * z;
+    f = fb[t];
+    i0 = i0b[t];
   }
+  fb[t] = f + dt * dub;
+  i0b[t] = i0 - dub;
+  i1b[t] = dub;
+  P[increment_field(t / np) * pcap + t % np] = dx[t];
+}
+// after the pass of the first sub-iteration, whose increments (dx) are zero
+__global__ void k_adj_iter_end(int np, const double *__restrict__ pout, double *__restrict__ xb, double *__restrict__ P,
+                               int pcap, const double *__restrict__ dx) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 3 * np) return;
+  xb[t] += pout[t];
+  P[increment_field(t / np) * pcap + t % np] = dx[t];
 }
 __global__ void k_adj_part_add(int np, const double *__restrict__ pout, double *__restrict__ xb,
                                double *__restrict__ vpb, int with_velocity) {
@@ -414,7 +417,7 @@ void adj_free(eif_ctx *c) {
     for (double *p : *v)
       if (p) cudaFree(p);
   for (double *p : {a->ub, a->vb, a->pb, a->abx, a->aby, a->tu, a->tv, a->rhs, a->w, a->fcx, a->fcy, a->gcx, a->gcy, a->xb, a->vpb,
-                    a->dub, a->fb, a->i0b, a->i1b, a->pout, a->part, a->wall_rows, a->wall, a->pbackup, a->geom})
+                    a->fb, a->i0b, a->i1b, a->pout, a->part, a->wall_rows, a->wall, a->pbackup, a->geom})
     if (p) cudaFree(p);
   if (a->d_contact) cudaFree(a->d_contact);
   delete a;
@@ -571,7 +574,7 @@ int eif_adjoint_begin(eif_ctx *c, int max_steps, int mode) {
     EIF_CK(c, cudaMalloc((void **)p, bytes));
   }
   const int n3 = std::max(1, 3 * np);
-  for (double **p : {&a->xb, &a->vpb, &a->dub, &a->fb, &a->i0b, &a->i1b})
+  for (double **p : {&a->xb, &a->vpb, &a->fb, &a->i0b, &a->i1b})
     EIF_CK(c, cudaMalloc((void **)p, sizeof(double) * n3));
   EIF_CK(c, cudaMalloc((void **)&a->pout, sizeof(double) * 2 * n3));
   EIF_CK(c, cudaMalloc((void **)&a->wall_rows, sizeof(double) * 2 * c->jtot));
@@ -598,7 +601,7 @@ int adj_clear(eif_ctx *c) {
   int rc;
   for (double *p : {a->ub, a->vb, a->pb, a->abx, a->aby, a->tu, a->tv, a->rhs, a->w, a->fcx, a->fcy, a->gcx, a->gcy})
     EIF_CK(c, cudaMemsetAsync(p, 0, bytes, c->stream));
-  for (double *p : {a->xb, a->vpb, a->dub, a->fb, a->i0b, a->i1b})
+  for (double *p : {a->xb, a->vpb, a->fb, a->i0b, a->i1b})
     EIF_CK(c, cudaMemsetAsync(p, 0, sizeof(double) * n3, c->stream));
   EIF_CK(c, cudaMemsetAsync(a->wall_rows, 0, sizeof(double) * 2 * c->jtot, c->stream));
   EIF_CK(c, cudaMemsetAsync(a->wall, 0, sizeof(double) * 2, c->stream));
@@ -821,16 +824,14 @@ int eif_adjoint_backward(eif_ctx *c) {
       c->boxes_x_valid = false;
       c->weights_x_valid = false;
       c->bands_x_valid = false;
-      k_adj_stage_init<<<pblocks(3 * np), 128, 0, c->stream>>>(np, gdt, a->xb, a->vpb, a->dub, a->fb, a->i0b);
-      EIF_LAUNCH_CK(c);
       pass.mode = 0;
       pass.ux = rk < 2 ? a->tape_u[slot + 1] : a->tape_out_u[s];
       pass.uy = rk < 2 ? a->tape_v[slot + 1] : a->tape_out_v[s];
       pass.bar = a->i1b;
       for (int m = a->tape_k[slot] - 1; m >= 0; m--) {
-        k_adj_iter_pre<<<pblocks(3 * np), 128, 0, c->stream>>>(np, dt, a->dub, a->fb, a->i0b, a->i1b);
-        EIF_LAUNCH_CK(c);
-        k_adj_dxload<<<pblocks(np), 128, 0, c->stream>>>(c->P, c->pcap, np, a->tape_dx[slot] + (size_t)3 * np * m);
+        k_adj_iter<<<pblocks(3 * np), 128, 0, c->stream>>>(np, m == a->tape_k[slot] - 1, dt, gdt, a->pout, a->xb, a->vpb,
+                                                           a->fb, a->i0b, a->i1b, c->P, c->pcap,
+                                                           a->tape_dx[slot] + (size_t)3 * np * m);
         EIF_LAUNCH_CK(c);
         pass.use_increment = m > 0;
         pass.geo = m == 0 ? 1 : 0;   // the pass at X keeps the geometry for the two below
@@ -838,10 +839,8 @@ int eif_adjoint_backward(eif_ctx *c) {
         if ((rc = launch_adj_pass(c, pass))) return rc;
         k_adj_avgT_add<<<G, B, 0, c->stream>>>(a->fcx, a->fcy, a->ub, a->vb, c->itot, c->jtot, c->ld);
         EIF_LAUNCH_CK(c);
-        k_adj_iter_post<<<pblocks(3 * np), 128, 0, c->stream>>>(np, gdt, a->pout, a->xb, a->vpb, a->dub, m > 0);
-        EIF_LAUNCH_CK(c);
       }
-      k_adj_dxload<<<pblocks(np), 128, 0, c->stream>>>(c->P, c->pcap, np, a->tape_dx[slot]);   // dX_0 = 0
+      k_adj_iter_end<<<pblocks(3 * np), 128, 0, c->stream>>>(np, a->pout, a->xb, c->P, c->pcap, a->tape_dx[slot]);   // dX_0 = 0
       EIF_LAUNCH_CK(c);
       // the boxes of the last pass (m = 0) are those at X, kept for the passes below
     }

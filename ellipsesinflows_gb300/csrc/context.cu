@@ -121,7 +121,7 @@ int rk_stage_front(eif_ctx *c, int rk, bool with_dt) {
     // (particle fields only), the exchange's sums; main: predictor, then what waits for the
     // inertia's weights: exchange, gather (after the lists), Poisson, projection. The path
     // boxes, inertia, exchange, gather, ... is the longer one of the smaller grids, and only
-    // the next kernel's inputs are on it (64 x 128, 4 particles: 77 -> 57 us a stage).
+    // the next kernel's inputs are on it (64 x 128, one ellipse: 77 -> 57 us a stage).
     SideScope side(c);
     if ((rc = side.begin())) return rc;
     if ((rc = launch_reset_increments(c))) return rc;
