@@ -521,6 +521,34 @@ int ibm_task_bases(eif_ctx *c) {
   return EIF_OK;
 }
 
+// tanh_tab's values, then tanh_mid's (float pairs), formed once in the process: long double
+// functions are software on some hosts (1.4 ms for the 2100 of them), so the exponentials are
+// products with a constant step, restarted every 16 (an error of some 2^-60 at most).
+static const std::vector<double2> &tanh_tables() {
+  static const std::vector<double2> tab = [] {
+    std::vector<double2> t(TANH_N + (MID_N + 1) / 2);
+    auto exps = [](int n, long double z0, int steps, auto put) {   // put(k, exp(-2 (z0 + k / steps)))
+      const long double step = expl(-2.L / steps);
+      long double e = 0.L;
+      for (int k = 0; k < n; k++) {
+        e = k % 16 == 0 ? expl(-2.L * (z0 + (long double)k / steps)) : e * step;
+        put(k, e);
+      }
+    };
+    exps(TANH_N, 0.L, TANH_STEPS, [&](int k, long double e) {
+      const long double d = 1.L + e;
+      t[k] = make_double2((double)((1.L - e) / d), (double)(4.L * e / (d * d)));
+    });
+    float2 *mid = reinterpret_cast<float2 *>(t.data() + TANH_N);
+    exps(MID_N, MID_Z0, MID_STEPS, [&](int k, long double e) {
+      const float hi = (float)(2.L * e);
+      mid[k] = make_float2(hi, (float)(2.L * e - (long double)hi));
+    });
+    return t;
+  }();
+  return tab;
+}
+
 int ibm_reserve(eif_ctx *c, size_t chunks) {
   // called after a particle push that changed the particle set: size the task and scratch buffers
   ibm_free(c);
@@ -536,18 +564,7 @@ int ibm_reserve(eif_ctx *c, size_t chunks) {
   if (c->cfg.precision == EIF_PREC_MIXED) EIF_CK(c, cudaMalloc((void **)&c->pf, sizeof(float) * PF_WORDS * c->np));
   else EIF_CK(c, cudaMalloc((void **)&c->pd, sizeof(double) * PD_WORDS * c->np));
   if (c->cfg.precision != EIF_PREC_MIXED && !c->tanh_tab) {
-    // tanh_tab's values, then tanh_mid's (float pairs)
-    std::vector<double2> tab(TANH_N + (MID_N + 1) / 2);
-    for (int k = 0; k < TANH_N; k++) {
-      const long double z = (long double)k / TANH_STEPS, ch = coshl(z);
-      tab[k] = make_double2((double)tanhl(z), (double)(1.L / (ch * ch)));
-    }
-    float2 *mid = reinterpret_cast<float2 *>(tab.data() + TANH_N);
-    for (int k = 0; k < MID_N; k++) {
-      const long double x = 2.L * expl(-2.L * (MID_Z0 + (long double)k / MID_STEPS));
-      const float hi = (float)x;
-      mid[k] = make_float2(hi, (float)(x - (long double)hi));
-    }
+    const std::vector<double2> &tab = tanh_tables();
     EIF_CK(c, cudaMalloc((void **)&c->tanh_tab, sizeof(double2) * tab.size()));
     EIF_CK(c, cudaMemcpy(c->tanh_tab, tab.data(), sizeof(double2) * tab.size(), cudaMemcpyHostToDevice));
   }
