@@ -662,7 +662,6 @@ int eif_adjoint_forward(eif_ctx *c, int record) {
     if (graph) {
       // a step that is not recorded: the graph of eif_integrate
       if ((rc = tune_tiles(c)) || (rc = step_graph_launch(c, false))) return rc;
-      c->incr_zero = false;
     }
     for (int rk = 0; !graph && rk < 3; rk++)
       if ((rc = coupled_stage(c, rk, record ? 3 * s + rk : -1))) return rc;

@@ -320,6 +320,7 @@ int eif_batch_advance(eif_batch *b, int nsteps) {
     for (size_t i = 0; i < b->ctx.size(); i++) {
       b->ctx[i]->cur = g->cur1[i];
       b->ctx[i]->scur = g->scur1[i];
+      eif::step_graph_ran(b->ctx[i]);
     }
     const int n = (int)b->ctx.size();
     k_pack_scalars<<<(n + 63) / 64, 64, 0, b->stream>>>(b->d_src, b->d_pack, n);

@@ -797,7 +797,6 @@ int eif_integrate(eif_ctx *c, int *substeps) {
   if (c->use_graphs && !c->sync_debug && !c->prof.enabled) {
     // the three stages in one graph, as eif_advance runs them
     if (int rc = step_graph_launch(c, false)) return rc;
-    c->incr_zero = false;
     EIF_CK(c, cudaMemcpyAsync(c->h_flags + 1, c->d_sub, sizeof(unsigned) * 3, cudaMemcpyDeviceToHost, c->stream));
     if (int rc = sync_scalars(c)) return rc;
     for (int rk = 0; substeps && rk < 3; rk++) substeps[rk] = c->np > 0 ? (int)c->h_flags[1 + rk] : 1;

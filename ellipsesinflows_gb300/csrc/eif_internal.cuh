@@ -292,6 +292,7 @@ void touch_pages(void *p, size_t bytes);
 // ---- step graphs (graph.cu) ----
 // one step as a graph: all of it, or without the dt decision
 int step_graph_launch(eif_ctx *c, bool with_dt);
+void step_graph_ran(eif_ctx *c);   // after every launch of a graph that holds a step of c
 void graphs_free(eif_ctx *c);
 struct SubiterPlan;
 // plan: where set and the context is subiter_alone, the sub-iteration loops are stage kernels

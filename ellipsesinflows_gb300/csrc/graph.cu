@@ -264,6 +264,17 @@ void graphs_free(eif_ctx *c) {
   c->stage_plan = nullptr;
 }
 
+// A launch of a captured step moves the particles and leaves the increments of its last
+// stage, without the launch functions that keep the host's record of what the buffers hold:
+// nothing formed before it is valid after it.
+void step_graph_ran(eif_ctx *c) {
+  c->boxes_x_valid = false;
+  c->weights_x_valid = false;
+  c->bands_x_valid = false;
+  c->incr_zero = false;
+  c->memo_miss_zero = false;
+}
+
 int step_graph_launch(eif_ctx *c, bool with_dt) {
   auto &graphs = with_dt ? c->graphs : c->igraphs;
   eif_ctx::StepGraph *sg = nullptr;
@@ -284,6 +295,7 @@ int step_graph_launch(eif_ctx *c, bool with_dt) {
   EIF_CK(c, cudaGraphLaunch(sg->exec, c->stream));
   c->cur = sg->cur1;
   c->scur = sg->scur1;
+  step_graph_ran(c);
   return EIF_OK;
 }
 
