@@ -157,15 +157,18 @@ int rk_stage_front(eif_ctx *c, int rk, bool with_dt) {
 }
 
 // one particle sub-iteration (src/main.c:36-39): inertia at X + dX and the
-// collision forces (independent, the latter on the side stream), then increments
+// collision forces (independent, the latter on the side stream), then increments. The body of
+// a loop node always ends with k_sub_end, which sets the loop's condition: also in a batch's
+// graph while its member is profiled, without the side stream.
 int sub_iteration(eif_ctx *c, int rk) {
   int rc;
-  if (c->np > 0 && overlap_on(c)) {
+  const bool beside = overlap_on(c);
+  if (c->np > 0 && (beside || c->in_loop)) {
     SideScope side(c);
-    if ((rc = side.begin())) return rc;
+    if (beside && (rc = side.begin())) return rc;
     if ((rc = launch_collision(c, 1))) return rc;
     if ((rc = side.end(c->ev_coll))) return rc;
-    return launch_inertia_increment(c, rk);
+    return launch_inertia_increment(c, rk, beside);
   } else {
     if ((rc = launch_inertia(c, 1))) return rc;
     if ((rc = launch_collision(c, 1))) return rc;

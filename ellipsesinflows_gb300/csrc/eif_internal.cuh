@@ -378,9 +378,9 @@ int launch_inertia_sums(eif_ctx *c);
 int launch_exchange_tasks(eif_ctx *c);
 int launch_exchange_sums(eif_ctx *c);
 int launch_gather(eif_ctx *c);
-// a sub-iteration beside the collision forces on the side stream (np > 0): inertia at X + dX, then
-// with the forces the increments, the residual and, in a loop, its condition
-int launch_inertia_increment(eif_ctx *c, int rk);
+// a sub-iteration after its collision forces, or beside those on the side stream (np > 0): inertia
+// at X + dX, then with the forces the increments, the residual and, in a loop, its condition
+int launch_inertia_increment(eif_ctx *c, int rk, bool beside);
 // the current stream waits for the collision forces of the side stream
 int join_collision(eif_ctx *c);
 int launch_band_lists(eif_ctx *c);

@@ -757,11 +757,11 @@ int launch_inertia_tasks(eif_ctx *c) {
 }
 int launch_inertia_sums(eif_ctx *c) { return launch_sums(c, 0, 0, false); }
 
-int launch_inertia_increment(eif_ctx *c, int rk) {
+int launch_inertia_increment(eif_ctx *c, int rk, bool beside) {
   int rc = launch_boxes(c, true);
   bool store = false;
   if (rc || (rc = launch_work(c, 0, 1, &store))) return rc;
-  if ((rc = join_collision(c))) return rc;
+  if (beside && (rc = join_collision(c))) return rc;
   c->incr_zero = false;
   EndArgs a;
   a.P = c->P; a.scal = c->d_scal; a.partial = partial_of(c, 0);

@@ -95,6 +95,8 @@ int launch_reset_increments(eif_ctx *c) {
 }
 
 int launch_increment(eif_ctx *c, int rk) {
+  // k_increment sets no loop condition: in a loop node it would never end
+  if (c->in_loop) return fail(c, EIF_ERR_STATE, "a sub-iteration loop ends with launch_inertia_increment");
   c->incr_zero = false;
   const double Fr = c->cfg.Fr;
   EIF_PROF(c, "particle_increment", 1);
