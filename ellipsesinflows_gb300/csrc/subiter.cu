@@ -567,8 +567,11 @@ int subiter_add_stage(SubiterPlan *p, int rk, cudaGraph_t g, const std::vector<c
   return e == cudaSuccess ? EIF_OK : plan_fail(err, "cudaGraphKernelNodeSetAttribute (cooperative)", e);
 }
 
+// The kernels that read the descriptors run on streams that do not wait for the null stream, and a
+// copy from pageable memory may return before it has reached the device: it is waited for here.
 int subiter_upload(SubiterPlan *p, std::string *err) {
-  const cudaError_t e = cudaMemcpy(p->d_desc, p->h.data(), sizeof(SubDesc) * p->h.size(), cudaMemcpyHostToDevice);
+  cudaError_t e = cudaMemcpy(p->d_desc, p->h.data(), sizeof(SubDesc) * p->h.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   return e == cudaSuccess ? EIF_OK : plan_fail(err, "cudaMemcpy (stage descriptors)", e);
 }
 
