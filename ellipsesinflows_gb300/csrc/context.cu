@@ -432,7 +432,7 @@ int ensure_pcap(eif_ctx *c, int n) {
   c->P = nullptr;
   const int cap = n > 0 ? n : 1;
   EIF_CK(c, cudaMalloc((void **)&c->P, sizeof(double) * EIF_NFIELDS * (size_t)cap));
-  EIF_CK(c, cudaMemset(c->P, 0, sizeof(double) * EIF_NFIELDS * (size_t)cap));
+  EIF_CK(c, cudaMemsetAsync(c->P, 0, sizeof(double) * EIF_NFIELDS * (size_t)cap, c->stream));
   c->pcap = cap;
   return EIF_OK;
 }
@@ -661,8 +661,10 @@ int eif_push_particles(eif_ctx *c, int n, const double *rec) {
     std::vector<double> soa((size_t)EIF_NFIELDS * c->pcap, 0.);
     for (int f = 0; f < EIF_NFIELDS; f++)
       for (int k = 0; k < n; k++) soa[(size_t)f * c->pcap + k] = rec[(size_t)k * EIF_NFIELDS + f];
+    // on the context's stream: its kernels do not wait for copies on the null stream, which
+    // may return before pageable data is on the device, and the next one reads the radii
+    EIF_CK(c, cudaMemcpyAsync(c->P, soa.data(), sizeof(double) * soa.size(), cudaMemcpyHostToDevice, c->stream));
     EIF_CK(c, cudaStreamSynchronize(c->stream));
-    EIF_CK(c, cudaMemcpy(c->P, soa.data(), sizeof(double) * soa.size(), cudaMemcpyHostToDevice));
   }
   c->np = n;
   c->max_tasks = (int)std::min<size_t>(most, 1u << 30);

@@ -3,7 +3,7 @@ that do not wait for the null stream."""
 import numpy as np
 import pytest
 
-from ellipsesinflows_gb300 import Simulation, cases
+from ellipsesinflows_gb300 import PREC_FP64, PREC_MIXED, F, Simulation, cases
 
 pytestmark = pytest.mark.gpu
 
@@ -28,4 +28,32 @@ def test_descriptors_of_new_stage_kernels(gpu_lib, monkeypatch):
     s = Simulation(some[0].config())
     for k in range(16):
         for a, b in zip(step(s, some[k % 2]), want[k % 2]):
+            assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("prec", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
+def test_radii_of_pageable_records(prec, gpu_lib):
+    """The radii pushed from pageable memory decide where a particle's sums are kept in the
+    stage kernel. The same particles in two orders have the same total, so the buffers and
+    graphs are kept between these pushes; every step is that of a fresh context."""
+    case = cases.poiseuille(itot=96, jtot=192, n=8, a=0.05, b=0.03, seed=6)
+    rec = case.particles
+    size = np.linspace(0.5, 1.0, len(rec))
+    orders = []
+    for scale in (size, size[::-1]):
+        r = rec.copy()
+        r[:, F["a"]] *= scale
+        r[:, F["b"]] *= scale
+        orders.append(r)
+
+    def step(s, r):
+        s.push_fluid(*case.fluid())
+        s.push_particles(r)
+        s.advance(1)
+        return [np.array(a) for a in s.pull_fluid()[:3]] + [np.array(s.pull_particles())]
+
+    want = [step(Simulation(case.config(precision=prec)), r) for r in orders]
+    s = Simulation(case.config(precision=prec))
+    for k in range(16):
+        for a, b in zip(step(s, orders[k % 2]), want[k % 2]):
             assert np.array_equal(a, b)
