@@ -201,7 +201,7 @@ int finish_step(eif_batch *b, int s) {
     int rc = EIF_OK;
     if (w[4] != 0ull) {
       cudaStreamSynchronize(b->stream);
-      cudaMemset(c->d_check, 0, sizeof(unsigned long long) * 4);
+      cudaMemsetAsync(c->d_check, 0, sizeof(unsigned long long) * 4, b->stream);
       rc = eif::fail(c, EIF_ERR_CUDA, "bounds guard %llu: index %llu outside [0, %llu)", w[5], w[6], w[7]);
     } else if (w[8] != 0ull) {
       cudaStreamSynchronize(b->stream);
@@ -244,7 +244,8 @@ int eif_batch_create(eif_ctx *const *ctxs, int n, eif_batch **out) {
             cudaEventCreateWithFlags(&b->ev_step[0], cudaEventDisableTiming) == cudaSuccess &&
             cudaEventCreateWithFlags(&b->ev_step[1], cudaEventDisableTiming) == cudaSuccess &&
             cudaMalloc((void **)&b->d_src, sizeof(void *) * src.size()) == cudaSuccess &&
-            cudaMemcpy(b->d_src, src.data(), sizeof(void *) * src.size(), cudaMemcpyHostToDevice) == cudaSuccess &&
+            cudaMemcpyAsync(b->d_src, src.data(), sizeof(void *) * src.size(), cudaMemcpyHostToDevice, b->stream) == cudaSuccess &&
+            cudaStreamSynchronize(b->stream) == cudaSuccess &&
             cudaMalloc((void **)&b->d_pack, sizeof(unsigned long long) * PACK_WORDS * n) == cudaSuccess &&
             cudaMallocHost((void **)&b->h_pack[0], sizeof(unsigned long long) * PACK_WORDS * n) == cudaSuccess &&
             cudaMallocHost((void **)&b->h_pack[1], sizeof(unsigned long long) * PACK_WORDS * n) == cudaSuccess;

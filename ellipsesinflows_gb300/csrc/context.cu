@@ -535,6 +535,8 @@ int eif_create(const eif_config_t *cfg, eif_ctx **out) {
   if ((rc = predictor_prepare(c))) return rc;
   rc = ensure_pcap(c, 1);
   if (rc) return rc;
+  // the copies and clears above are on the null stream, which the context's streams do not wait for
+  EIF_CK(c, cudaStreamSynchronize(nullptr));
   rc = launch_boundaries(c);
   if (rc) return rc;
   EIF_CK(c, cudaStreamSynchronize(c->stream));

@@ -566,7 +566,7 @@ int ibm_reserve(eif_ctx *c, size_t chunks) {
   if (c->cfg.precision != EIF_PREC_MIXED && !c->tanh_tab) {
     const std::vector<double2> &tab = tanh_tables();
     EIF_CK(c, cudaMalloc((void **)&c->tanh_tab, sizeof(double2) * tab.size()));
-    EIF_CK(c, cudaMemcpy(c->tanh_tab, tab.data(), sizeof(double2) * tab.size(), cudaMemcpyHostToDevice));
+    EIF_CK(c, cudaMemcpyAsync(c->tanh_tab, tab.data(), sizeof(double2) * tab.size(), cudaMemcpyHostToDevice, c->stream));
   }
   EIF_CK(c, cudaMalloc((void **)&c->tdesc, sizeof(int4) * (size_t)chunks));
   const int nbands = (c->jtot + GTY - 1) / GTY;
@@ -581,7 +581,7 @@ int ibm_reserve(eif_ctx *c, size_t chunks) {
     EIF_CK(c, cudaMalloc((void **)&c->memo_box, sizeof(int) * 12 * c->np));
     EIF_CK(c, cudaMalloc((void **)&c->memo_off, sizeof(int) * c->np));
     EIF_CK(c, cudaMalloc((void **)&c->memo_valid, sizeof(int)));
-    EIF_CK(c, cudaMemset(c->memo_valid, 0, sizeof(int)));
+    EIF_CK(c, cudaMemsetAsync(c->memo_valid, 0, sizeof(int), c->stream));
     EIF_CK(c, cudaMalloc((void **)&c->memo_miss, sizeof(int) * ((size_t)chunks + 1)));
   }
   return EIF_OK;

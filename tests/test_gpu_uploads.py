@@ -57,3 +57,23 @@ def test_radii_of_pageable_records(prec, gpu_lib):
     for k in range(16):
         for a, b in zip(step(s, orders[k % 2]), want[k % 2]):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("prec", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
+def test_tables_of_new_buffers(prec, gpu_lib):
+    """A new context, and a push of another particle count, upload tables that the first stage
+    call reads at once: always the same field response."""
+    case = cases.poiseuille(itot=96, jtot=192, n=8, a=0.05, b=0.03, seed=6)
+    case.particles[:, F["vz"]] = 1.0
+    first = None
+    for _ in range(8):
+        with Simulation(case.config(precision=prec)) as s:
+            for n in (8, 3, 8):
+                s.push_fluid(*case.fluid())
+                s.push_particles(case.particles[:n])
+                s.dt = 1.0e-3
+                s.exchange_momentum()
+            got = [np.array(a) for a in s.pull_ibm_fields()]
+        first = first or got
+        for a, b in zip(got, first):
+            assert np.array_equal(a, b) and np.abs(a).max() > 0.0
