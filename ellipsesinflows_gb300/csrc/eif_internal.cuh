@@ -228,7 +228,7 @@ struct eif_ctx {
   int chunk_cap;                // capacity of partial in chunks
   float *pf;                    // per-particle single-precision parameters (mixed form)
   double *pd = nullptr;         // per-particle parameters of the indicator (double-precision form)
-  double2 *tanh_tab = nullptr;  // tanh and sech^2 at multiples of 1/16 (double-precision form)
+  double2 *tanh_tab = nullptr;  // tables of the indicator's tanh (double-precision form)
   int4 *tdesc;                  // task table: particle, row, columns and image of every chunk
   // weights of the last indicator evaluation in a sub-iteration loop (mixed form), with
   // the particles' geometry words, boxes and first tasks (WeightMemo in ibm_device.cuh)

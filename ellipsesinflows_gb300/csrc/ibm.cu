@@ -521,12 +521,13 @@ int ibm_task_bases(eif_ctx *c) {
   return EIF_OK;
 }
 
-// tanh_tab's values, then tanh_mid's (float pairs), formed once in the process: long double
+// tanh_tab's values (tanh rounded to double and 1 minus its square, then where tanh has that
+// value), then tanh_mid's (float pairs), formed once in the process: long double
 // functions are software on some hosts (1.4 ms for the 2100 of them), so the exponentials are
 // products with a constant step, restarted every 16 (an error of some 2^-60 at most).
 static const std::vector<double2> &tanh_tables() {
   static const std::vector<double2> tab = [] {
-    std::vector<double2> t(TANH_N + (MID_N + 1) / 2);
+    std::vector<double2> t(2 * TANH_N + (MID_N + 1) / 2);
     auto exps = [](int n, long double z0, int steps, auto put) {   // put(k, exp(-2 (z0 + k / steps)))
       const long double step = expl(-2.L / steps);
       long double e = 0.L;
@@ -536,10 +537,12 @@ static const std::vector<double2> &tanh_tables() {
       }
     };
     exps(TANH_N, 0.L, TANH_STEPS, [&](int k, long double e) {
-      const long double d = 1.L + e;
-      t[k] = make_double2((double)((1.L - e) / d), (double)(4.L * e / (d * d)));
+      // below 1, the place of which is infinite
+      const double th = std::min((double)((1.L - e) / (1.L + e)), 1. - 0.5 * DBL_EPSILON);
+      t[2 * k] = make_double2(th, (double)((1.L - th) * (1.L + th)));
+      t[2 * k + 1] = make_double2((double)(0.5L * logl((1.L + th) / (1.L - th))), 0.);
     });
-    float2 *mid = reinterpret_cast<float2 *>(t.data() + TANH_N);
+    float2 *mid = reinterpret_cast<float2 *>(t.data() + 2 * TANH_N);
     exps(MID_N, MID_Z0, MID_STEPS, [&](int k, long double e) {
       const float hi = (float)(2.L * e);
       mid[k] = make_float2(hi, (float)(2.L * e - (long double)hi));

@@ -179,18 +179,20 @@ __device__ __forceinline__ bool foot_d(double a, double b, float abf, float c0, 
   return false;
 }
 
-// tanh(z) for z >= 0 from the values at multiples of 1/16 (tab: tanh and sech^2 there, up to
-// TANH_TOP) by the addition theorem, tanh(z_k + d) = T + S t / (1 + T t), t = tanh(d) from
+// tanh(z) for z >= 0 from its values near the multiples of 1/16 (tab, up to TANH_TOP) by the
+// addition theorem, tanh(z_k + d) = T + S t / (1 + T t), t = tanh(d) from
 // its Taylor series (|d| <= 1/32: the first term left out is 3e-19); the quotient from a
-// single-precision reciprocal and one third-order step. 15 FP64 instructions; absolute
-// error about 1e-16.
+// single-precision reciprocal and one third-order step. The table's T is tanh(k/16) rounded to
+// double, z_k the place where tanh has that very value (near k/16; beyond z = 16 up to 1 away,
+// where S is below 1e-13), so that the rounding of T does not add to the result's own: with
+// z_k = k/16 the largest error at z = 4 to 6 was 1.1e-16, now half of that. 15 FP64 instructions.
 constexpr int TANH_STEPS = 16, TANH_TOP = 20, TANH_N = TANH_STEPS * TANH_TOP + 1;
 __device__ __forceinline__ double tanh_tab(double z, const double2 *__restrict__ tab) {
   const float zf = eifd::d2f(z);
   if (!(zf < (float)TANH_TOP)) return z > 0. ? 1. : z;   // a NaN stays one
-  const float kf = rintf(zf * (float)TANH_STEPS);
-  const double2 ts = __ldg(tab + (int)kf);
-  const double d = z - eifd::f2d(kf * (1.f / TANH_STEPS));
+  const int k = (int)rintf(zf * (float)TANH_STEPS);
+  const double2 ts = __ldg(tab + 2 * k);   // T, S; the next entry's first is z_k
+  const double d = z - __ldg(&tab[2 * k + 1].x);
   const double u = d * d;
   const double p = fma(u, fma(u, fma(u, 62. / 2835., -17. / 315.), 2. / 15.), -1. / 3.);
   const double t = fma(d * u, p, d);
@@ -235,15 +237,18 @@ __device__ __forceinline__ double indicator_d(double a, double b, float abf, flo
   return __double2hiint(dist) < 0 ? th : -th;
 }
 
-// Cells whose tanh(BETA D) the FP32 pipe gives to the last bit of the double: with z = |BETA D|,
+// Cells whose tanh(BETA D) the FP32 pipe gives as well as the FP64 pipe: with z = |BETA D|,
 // tanh z = 1 - x, x = 2 / (exp(2 z) + 1), and an error dz of the distance changes it by
-// 4 exp(-2 z) dz.
-// foot_f's foot (once its Newton step is below 1e-3) and the distance and x in double-float
-// arithmetic (dist_mid, good to 1e-13 rms and 2e-12 at A = 48, in proportion to A; tanh_mid) leave
-// less than 1e-17 rms at z >= 6 + A / 400 for every major semi-axis A (in the same barred units).
-// Only the cells within three of the interface are left to the FP64 pipe, a pass of 32 of them
-// being as long as 3000 instructions of the FP32 pipe.
-__device__ __forceinline__ float z_mid(float A) { return fmaf(0.0025f, A, 6.f); }
+// 4 exp(-2 z) dz. foot_f's foot (once its Newton step is below 1e-3) and the distance in
+// double-float arithmetic (dist_mid, good to 1e-13 rms and 2e-12 at A = 48, in proportion to the
+// major semi-axis A in the same barred units) then leave less than 1e-17, and tanh_mid rounds x
+// once. The line at z = 6.5 + A / 100 is where nothing is seen of dz: against extended precision
+// the weights 1 - tanh^2 there are off by 6.4e-17 rms (at most 1.13e-16), as with every cell in
+// double precision (6.4e-17, 1.11e-16), for ellipses of 3 to 128 cells and ratios to 20; with
+// the line at 6 + A / 400 at most 1.26e-16, and 1.5 % faster (2048 x 4096, 2048 ellipses).
+// Only the cells within about three and a half of the interface are left to the FP64 pipe, a pass
+// of 32 of them being as long as 3000 instructions of the FP32 pipe.
+__device__ __forceinline__ float z_mid(float A) { return fmaf(0.01f, A, 6.5f); }
 // (1 - m 2^-53) with the sign of -dist; the doubles below 1 are 2^-53 apart
 __device__ __forceinline__ double tanh_of(long long m, float dist) {
   const long long b = 0x3ff0000000000000ll - m;
@@ -279,21 +284,30 @@ __device__ __forceinline__ DF dist_mid(DF a, DF b, float abf, float c, float s, 
   const DF d = df_mulf(nw, y0);
   return eifdf::fast_sum(d.hi, d.lo + fmaf(d.hi, 0.5f * e, corr));
 }
-// tanh z of z = |d| from 2 exp(-2 z) at multiples of 1 / MID_STEPS (tab, from MID_Z0 up)
+// tanh z of z = |d| from 2 exp(-2 z) at multiples of 1 / MID_STEPS (tab, from MID_Z0 up), within
+// 0.52 of the doubles' spacing below 1 at z = 6 and 0.51 from 6.5 on (half of it is the rounding)
 constexpr int MID_STEPS = 128, MID_Z0 = 6, MID_Z1 = 20, MID_N = (MID_Z1 - MID_Z0) * MID_STEPS + 1;
 __device__ __forceinline__ double tanh_mid(DF d, const float2 *__restrict__ tab) {
   const float zh = fmaxf(fminf(fabsf(d.hi), (float)MID_Z1), (float)MID_Z0), zl = d.hi < 0.f ? -d.lo : d.lo;
   const float kf = rintf((zh - (float)MID_Z0) * (float)MID_STEPS);
   const float2 E = __ldg(tab + (int)kf);
-  // exp(-2 (z - z_k)) = (1 + y + q)(1 + yl); x = E (1 - E / 2 + E^2 / 4)
+  // e = exp(-2 (z - z_k)) = (1 + y + y^2 / 2 + r)(1 + yl) with y exact. At z = 6 the spacing of
+  // the doubles is 2^-37 of x, so that what is above 2^-25 of E is summed as pairs: E, E y,
+  // E y^2 / 2 and then the square in x = E e - (E e)^2 / 2 + (E e)^3 / 4
   const float y = -2.f * (zh - fmaf(kf, 1.f / MID_STEPS, (float)MID_Z0)), yl = -2.f * zl;
-  const float q = y * y * fmaf(y, fmaf(y, 1.f / 24.f, 1.f / 6.f), 0.5f);
-  const float p = E.x * y;
-  const DF m = eifdf::fast_sum(E.x, p);
-  const float l0 = m.lo + (fmaf(E.x, y, -p) + fmaf(E.x, q + fmaf(yl, y, yl), fmaf(E.y, y, E.y))), x = m.hi + l0;
-  const float lo = l0 - 0.5f * x * x * fmaf(-0.5f, x, 1.f);
+  const float h = 0.5f * y, q = h * y, s = y + q;
+  const float r = q * y * fmaf(y, fmaf(y, 1.f / 60.f, 1.f / 12.f), 1.f / 3.f) + fmaf(h, y, -q);
+  const float p1 = E.x * y, p2 = E.x * q;
+  const DF e1 = eifdf::fast_sum(E.x, p1), e2 = eifdf::fast_sum(e1.hi, p2);
+  const float el = (e1.lo + e2.lo) +
+                   ((fmaf(E.x, y, -p1) + fmaf(E.x, q, -p2)) + fmaf(E.x, fmaf(yl, s, yl) + r, fmaf(E.y, s, E.y)));
+  const float eh = 0.5f * e2.hi, t = eh * e2.hi;
+  const DF m = eifdf::fast_sum(e2.hi, -t);
+  const float lo = m.lo + (el - (fmaf(eh, e2.hi, -t) + e2.hi * (el - 0.5f * t)));
+  // in units of the doubles' spacing, rounded once
   constexpr float U = 9007199254740992.f;   // 2^53
-  return tanh_of(__float2ll_rn(m.hi * U) + __float2ll_rn(lo * U), d.hi);
+  const float mu = m.hi * U, mr = rintf(mu);
+  return tanh_of(__float2ll_rn(mr) + __float2int_rn(fmaf(lo, U, mu - mr)), d.hi);
 }
 
 // Cells far from the interface. With rho = sqrt((x/a)^2 + (y/b)^2) (the gauge of
@@ -1592,7 +1606,7 @@ inline WorkArgs work_args(const eif_ctx *c, int mode, int cn) {
   w.pf = c->pf;
   w.pd = c->pd;
   w.tanh_tab = c->tanh_tab;
-  w.mid_tab = reinterpret_cast<const float2 *>(c->tanh_tab + TANH_N);
+  w.mid_tab = reinterpret_cast<const float2 *>(c->tanh_tab + 2 * TANH_N);
   w.tdesc = c->tdesc;
   w.coef = c->d_coef;
   w.rh_f = (float)(1. / w.h);
