@@ -189,6 +189,7 @@ struct eif_ctx {
   // tile heights (rows per block of 32 columns), threads per block of the block Thomas
   struct Tiles {
     int pred = 8, corr = 8, tdm = 128;
+    bool pred_set = false;   // pred is the tuner's or EIF_TILES's
     bool pred_copy = true;   // mixed predictor: tiles staged by tensor copies where available
     bool tuned = false;
   } tiles;
@@ -344,6 +345,8 @@ int launch_check(eif_ctx *c, const char *file, int line);
 int launch_boundaries(eif_ctx *c);
 int launch_bc_p_like(eif_ctx *c, double *a);
 int launch_predictor(eif_ctx *c, int rk);
+int predictor_rows(const eif_ctx *c);
+long predictor_warps(const eif_ctx *c, int rows);
 int launch_update_momentum_field(eif_ctx *c);
 int launch_correct(eif_ctx *c, int rk, bool with_ibm, bool with_pressure);
 int launch_update_pressure(eif_ctx *c);

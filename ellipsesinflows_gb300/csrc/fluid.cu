@@ -87,7 +87,9 @@ struct PredArgs {
 // cycles), so what two cells share is formed once: lane l forms the terms of the face (ux: the
 // cell centre) to the west of its column i, those of the east come from lane l + 1 (lane 31 has
 // no column of its own), and the rows are walked upwards with the terms of the south face
-// kept. Constant factors are folded into one weight per term. 43 FP64 instructions per cell
+// kept. Constant factors are folded into one weight per term; the two sums of products are
+// rounded as written, so that every TY gives the same bits (one row per warp, where both
+// products are formed beside their sum, was fused otherwise). 43 FP64 instructions per cell
 // instead of about 90 with every term formed at both its cells: 2048 x 4096 1263 -> 716 us.
 constexpr int PCOLS = 31, PWARPS = 4;
 template <int TY>
@@ -130,7 +132,7 @@ __global__ void __launch_bounds__(32 * PWARPS) k_predictor(PredArgs a) {
     const double Fn = vn - v0, Rn = (v0 + vn) * Fn;
     if (face) {
       double A = fma(wxm, P, wxp * Pe);
-      A = fma(hx, Qs + Qn, A);
+      A = fma(hx, __dadd_rn(Qs, Qn), A);
       A = fma(kx, De - D, A);
       A = fma(ky, En - Es, A);
       a.sxa[cx] = A;
@@ -141,7 +143,7 @@ __global__ void __launch_bounds__(32 * PWARPS) k_predictor(PredArgs a) {
     }
     if (own) {
       double A = fma(wym, H, fma(wyp, He, a.ext));
-      A = fma(hy, Rs + Rn, A);
+      A = fma(hy, __dadd_rn(Rs, Rn), A);
       A = fma(kv, Ge - G, A);
       A = fma(ky, Fn - Fs, A);
       a.sya[cy] = A;
@@ -1012,6 +1014,21 @@ static int launch_predictor_mixed(eif_ctx *c, int rk) {
   return EIF_OK;
 }
 
+// Warps of the double-precision predictor at so many rows per warp
+long predictor_warps(const eif_ctx *c, int rows) { return (long)((c->itot + PCOLS - 1) / PCOLS) * ((c->jtot + rows - 1) / rows); }
+
+// Rows per tile (mixed form) or per warp (double-precision form) that the predictor runs: what
+// the tuner timed fastest or EIF_TILES fixes. Before the tuner has run, or without it, the default;
+// in the double-precision form fewer where it gives less than eight warps per SM: the walk is then
+// a chain of loads and FP64 latencies (64 x 128: 13.1 us at 4 rows, 8.5 at 1), which costs more
+// than the south terms formed again.
+int predictor_rows(const eif_ctx *c) {
+  int rows = c->tiles.pred;
+  if (c->cfg.precision == EIF_PREC_FP64 && !c->tiles.pred_set)
+    while (rows > 1 && predictor_warps(c, rows) < 8L * c->sms) rows /= 2;
+  return rows;
+}
+
 int launch_predictor(eif_ctx *c, int rk) {
   const RK k = rk_coef(rk);
   // the explicit term of the previous stage becomes srcB (update_velocity.c:26,110)
@@ -1036,12 +1053,7 @@ int launch_predictor(eif_ctx *c, int rk) {
   a.ext = c->cfg.extfrcy;
   a.itot = c->itot; a.jtot = c->jtot; a.ld = c->ld;
   EIF_PROF(c, "predictor", 1);
-  // the tuner's rows per warp, fewer where the grid gives less than eight warps per SM: the walk
-  // is then a chain of loads and FP64 latencies (96 x 192: 10.0 us at 4 rows, 6.7 at 1), which
-  // costs more than the south terms formed again
-  int rows = c->tiles.pred;
-  const long strips = (c->itot + PCOLS - 1) / PCOLS;
-  while (rows > 1 && strips * ((c->jtot + rows - 1) / rows) < 8L * c->sms) rows /= 2;
+  const int rows = predictor_rows(c);
   if (rows == 1) launch_predictor_rows<1>(a, c->stream);
   else if (rows == 2) launch_predictor_rows<2>(a, c->stream);
   else if (rows == 4) launch_predictor_rows<4>(a, c->stream);

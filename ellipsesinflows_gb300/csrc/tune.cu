@@ -1,7 +1,8 @@
 // Tile-shape tuner. The stencil kernels (predictor, projection) process tiles of 32
 // columns by TY rows, and the block-Thomas kernel one wavenumber column per thread;
 // none of these shapes changes a result, only the speed (occupancy, the halo overhead
-// of the staged mixed-precision predictor, the L2 reuse of neighbouring rows). For a
+// of the staged mixed-precision predictor, the L2 reuse of neighbouring rows). The
+// double-precision predictor walks its rows a warp each, 31 columns wide. For a
 // grid size and precision the tuner times every candidate on scratch copies of the
 // fields the kernels write and keeps the fastest; the choice is cached for the
 // process, so contexts of the same size (a batch of suspensions) are timed once.
@@ -57,6 +58,7 @@ int tune_tiles(eif_ctx *c) {
     if (std::sscanf(fx, "%d,%d,%d", &a, &b, &t) != 3 || !rows_ok(a) || !rows_ok(b) || (t != 64 && t != 128 && t != 256))
       return fail(c, EIF_ERR_ARG, "EIF_TILES must be rows,rows,threads with rows 4|8|16 and threads 64|128|256");
     c->tiles.pred = a;
+    c->tiles.pred_set = true;
     c->tiles.corr = b;
     c->tiles.tdm = t;
     return EIF_OK;
@@ -115,12 +117,17 @@ int tune_tiles(eif_ctx *c) {
     }
     const bool ibm = c->np > 0;
     const int tys[3] = {4, 8, 16};
+    // the double-precision predictor also with one or two rows per warp, where four leave fewer than
+    // 16 warps per SM (fastest up to 216 x 430; 256 x 512: 21.0 us at 2, 19.5 at 4)
+    std::vector<int> rows(tys, tys + 3);
+    if (!mixed && predictor_warps(c, 4) < 16L * c->sms) rows.insert(rows.begin(), {1, 2});
+    c->tiles.pred_set = true;
     float best = 1e30f;
     int pick = c->tiles.pred;
     bool pick_copy = c->tiles.pred_copy;
     // the mixed predictor with tensor-copy staging and the plain one, each tile height
     for (int copy = 0; copy < (mixed ? 2 : 1); copy++) {
-      for (int ty : tys) {
+      for (int ty : rows) {
         c->tiles.pred = ty;
         c->tiles.pred_copy = copy == 1;
         float ms = 0.f;
@@ -173,7 +180,7 @@ int tune_tiles(eif_ctx *c) {
 
 extern "C" int eif_tiles(eif_ctx *c, int *tiles) {
   if (!c || !tiles) return EIF_ERR_ARG;
-  tiles[0] = c->tiles.pred;
+  tiles[0] = eif::predictor_rows(c);
   tiles[1] = c->tiles.corr;
   tiles[2] = c->tiles.tdm;
   tiles[3] = (c->tiles.tuned ? 1 : 0) | (c->tiles.pred_copy && c->pred_tma_ctas[1] > 0 ? 2 : 0) |

@@ -172,8 +172,10 @@ int eif_snapshot_wait(eif_ctx *ctx, double *ux, double *uy, double *p, int n, do
  * candidates (tiles of 32 columns by 4, 8 or 16 rows for the predictor and the
  * projection; 64, 128 or 256 threads per block of the block Thomas) once per grid
  * size and precision, before the first eif_integrate / eif_advance / batch capture,
- * and keeps the fastest. The shapes do not change any result. EIF_TUNE=0 in the
- * environment keeps the defaults (8, 8, 128). In the mixed form the predictor runs either
+ * and keeps the fastest. In the double-precision form the predictor's rows are those a
+ * warp walks, and on small grids also 1 or 2. The shapes do not change any result.
+ * EIF_TUNE=0 in the environment keeps the defaults (8, 8, 128; fewer rows of the
+ * double-precision predictor on small grids), EIF_TILES=p,c,t fixes them. In the mixed form the predictor runs either
  * with its tiles staged by bulk tensor copies (double-buffered, TMA) or with plain loads,
  * whichever the tuner timed faster (EIF_NO_TMA=1 at context creation: plain loads only).
  * tiles[4]: predictor rows, projection rows, Thomas threads, flags (bit 0: tuned, bit 1:
