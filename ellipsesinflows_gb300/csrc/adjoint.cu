@@ -658,6 +658,7 @@ int eif_adjoint_forward(eif_ctx *c, int record) {
     }
   } else {
     if (record) EIF_CK(c, cudaMemsetAsync(a->d_contact, 0, sizeof(int), c->stream));
+    if (record && stage_kernels(c) && (rc = stage_kernel_prepare(c))) return rc;
     const bool graph = !record && c->use_graphs && !c->sync_debug && !c->prof.enabled;
     if (graph) {
       // a step that is not recorded: the graph of eif_integrate

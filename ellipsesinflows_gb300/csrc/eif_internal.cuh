@@ -181,6 +181,7 @@ struct eif_ctx {
   } graphs[2], igraphs[2];              // of eif_advance; of eif_integrate (without the dt decision)
   // stage kernels launched one by one (adjoint.cu), for the buffers of generation stage_gen
   eif::SubiterPlan *stage_plan = nullptr;
+  bool stage_off = false;               // the stage kernel is not to be had: loops of kernels
   unsigned stage_gen = 0;
   unsigned *d_sub = nullptr;            // sub-iterations of the stages of a step
   bool use_graphs = true;
@@ -323,7 +324,10 @@ int subiter_add_reset(SubiterPlan *p, cudaGraph_t g, cudaGraphNode_t *node, std:
 int subiter_add_stage(SubiterPlan *p, int rk, cudaGraph_t g, const std::vector<cudaGraphNode_t> &deps,
                       cudaGraphNode_t *node, std::string *err);
 int subiter_upload(SubiterPlan *p, std::string *err);
-// the stage kernel of RK stage rk on c's stream (np > 0, subiter_alone): the sub-iterations after
+// the plan for launch_stage_kernel (subiter_alone); where there can be none, subiter_alone is false
+// afterwards
+int stage_kernel_prepare(eif_ctx *c);
+// the stage kernel of RK stage rk on c's stream (np > 0, prepared): the sub-iterations after
 // a stage front and the particle update; tape (optional): dX after sub-iteration m to
 // tape + 3 np m, and *contact = 1 where a collision force is not zero
 int launch_stage_kernel(eif_ctx *c, int rk, double *tape, int *contact);

@@ -181,7 +181,7 @@ int capture_step(eif_ctx *c, cudaGraph_t g, int *cur1, int *scur1, SubiterPlan *
   int rc = step_capture_begin(c);
   if (rc) return rc;
   const int cur0 = c->cur, scur0 = c->scur;
-  const bool stage_kernels = plan && subiter_alone(c);
+  bool stage_kernels = plan && subiter_alone(c);
   SubiterPlan *p = nullptr;
   std::string err;
   std::vector<cudaGraphNode_t> tail;
@@ -191,10 +191,12 @@ int capture_step(eif_ctx *c, cudaGraph_t g, int *cur1, int *scur1, SubiterPlan *
     step_capture_end(c, cur0, scur0);
     return stage ? fail(c, code, "stage kernel: %s", err.c_str()) : code;
   };
-  if (stage_kernels) {
-    if ((rc = subiter_plan_create(&c, 1, &p, &err)) || (rc = subiter_add_reset(p, g, &reset, &err)))
-      return failed(rc, true);
+  if (stage_kernels && subiter_plan_create(&c, 1, &p, &err)) {
+    cudaGetLastError();
+    c->stage_off = true;
+    stage_kernels = false;
   }
+  if (stage_kernels && (rc = subiter_add_reset(p, g, &reset, &err))) return failed(rc, true);
   for (int part = 0; part < 4; part++) {
     if ((rc = capture_step_part(c, g, tail, part, &tail, stage_kernels, true, with_dt))) return failed(rc, false);
     if (part == 3) break;
@@ -234,6 +236,11 @@ int build(eif_ctx *c, eif_ctx::StepGraph &sg, bool with_dt) {
   if (e != cudaSuccess) {
     cudaGraphDestroy(g);
     subiter_plan_destroy(plan);
+    if (plan && e == cudaErrorCooperativeLaunchTooLarge) {
+      cudaGetLastError();
+      c->stage_off = true;
+      return build(c, sg, with_dt);
+    }
     return check_cuda(c, e, "cudaGraphInstantiate");
   }
   sg.graph = g;
@@ -292,7 +299,16 @@ int step_graph_launch(eif_ctx *c, bool with_dt) {
     int rc = build(c, *sg, with_dt);
     if (rc) return rc;
   }
-  EIF_CK(c, cudaGraphLaunch(sg->exec, c->stream));
+  const cudaError_t e = cudaGraphLaunch(sg->exec, c->stream);
+  if (e == cudaErrorCooperativeLaunchTooLarge && sg->plan) {
+    // fewer resident CTAs than the occupancy query gave (another limit on the SMs): nothing ran
+    cudaGetLastError();
+    c->stage_off = true;
+    free_graphs(c->graphs);
+    free_graphs(c->igraphs);
+    return step_graph_launch(c, with_dt);
+  }
+  if (e != cudaSuccess) return check_cuda(c, e, "cudaGraphLaunch");
   c->cur = sg->cur1;
   c->scur = sg->scur1;
   step_graph_ran(c);
