@@ -1,6 +1,7 @@
 // C ABI of include/eif.h: context lifetime, state transfer, stage entry points
 // and the time-step orchestration of integrate (src/main.c:13-55).
 #include "eif_internal.cuh"
+#include "host_pages.h"
 #include <cstdio>
 #include <cstdarg>
 #include <cstring>
@@ -55,9 +56,7 @@ void touch_pages(void *p, size_t bytes) {
     return;
   }
   if (at.type != cudaMemoryTypeUnregistered) return;
-  volatile char *q = static_cast<volatile char *>(p);
-  for (size_t k = 0; k < bytes; k += 4096) q[k] = 0;
-  if (bytes) q[bytes - 1] = 0;
+  fault_in_pages(p, bytes);
 }
 
 // Particle-only work beside the fluid kernels. The kernels of a stage and their
