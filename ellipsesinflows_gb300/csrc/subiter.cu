@@ -409,11 +409,15 @@ struct SubiterPlan {
 
 bool subiter_joinable(const eif_ctx *c) { return c->np <= TT_MAX_NP; }
 
-// One suspension's loops in stage kernels: while every unit has a CTA of its own. With more, a
-// loop of kernels is faster: the stand-alone indicator has 24 warps on an SM and no
-// CTA-wide steps, the stage kernel 16 (registers of the fits). 768 x 1536 with 512 ellipses, 177
-// sub-iterations: 15.2 ms against 18.5; 2048 x 4096 with 2048: 54 against 83 (mixed form); with
-// 128 at 512 x 1024 11.3 against 10.8, with 24 at 216 x 430 8.4 against 7.2.
+// One suspension's loops in stage kernels: while every unit has a CTA of its own, np + np / 8 of
+// them on two CTAs an SM, so up to 270 particles on 152 SMs. There the loop of kernels takes 1.05
+// to 1.75 times as long; as soon as some CTAs have a second unit, a sub-iteration of the stage
+// kernel takes two units' time, while the stand-alone indicator has 24 warps on an SM (16 here, for
+// the registers of the fits) and no CTA-wide steps. Passes of some steps, loop over stage kernel:
+//   256 x 512, 16 / 160 ellipses   double precision 1.34 / 1.17, mixed 1.75 / 1.37
+//   512 x 1024, 270 / 340          1.17 / 0.94 (4.81 and 4.11 ms / 5.50 and 5.83), 1.18 / 0.99
+//   768 x 1536, 270 / 320 / 640    1.10 / 0.90 / 0.97, 1.15 / 0.99 / 0.80
+//   1024 x 2048, 256 / 320 / 768   1.06 / 0.91 / 0.98, 1.16 / 0.97 / 0.85
 bool subiter_alone(const eif_ctx *c) {
   return c->np > 0 && !c->stage_off && c->np + (c->np + PAIR_WARPS - 1) / PAIR_WARPS <= 2 * c->sms;
 }
