@@ -349,14 +349,14 @@ __global__ void k_adj_contact(const double *__restrict__ P, int pcap, int np, in
   for (int f = EIF_P_CFX0; f <= EIF_P_CTZ1; f++) any |= P[f * pcap + n] != 0.;
   if (any) *flag = 1;
 }
-// reverse of U' = U + dU_K, X' = X + dX_K, dX_K = g dt (U + dU_K / 2):
-// dUbar = Ubar' + (g dt / 2) Xbar', Ubar = Ubar' + g dt Xbar', Xbar = Xbar'
-// reverse of dU_{m+1} = dt F + I1_m - I0
-// Between the passes of two sub-iterations in reverse, one component of a particle per thread:
-// what the pass of sub-iteration m + 1 gave (k_adj_iter_end's sum and, as m + 1 > 0, the
-// velocities), or for the last one (first) the start of the stage; then the
-// cotangents and the increments of the pass of sub-iteration m. One launch: the backward sweep
-// of a small grid is as long as its launches (4 us each, 256 x 512 with 8 ellipses).
+// Between the passes of two sub-iterations in reverse, one component of a particle per thread.
+// First what the pass of sub-iteration m + 1 gave, the reverse of I1 = Inert(X + dX) with dX = g dt
+// (U + dU / 2): its position cotangent z goes to X (k_adj_iter_end's sum) and, as m + 1 > 0, to U
+// and dU. For the last sub-iteration (first) instead the start of the stage, the reverse of U' =
+// U + dU_K, X' = X + dX_K: dUbar = Ubar' + (g dt / 2) Xbar', Ubar = Ubar' + g dt Xbar', Xbar =
+// Xbar'. Then the reverse of dU_{m+1} = dt F + I1_m - I0, and the increments of the pass of
+// sub-iteration m. One launch: the backward sweep of a small grid is as long as its launches (4 us
+// each, 256 x 512 with 8 ellipses).
 __device__ __forceinline__ int increment_field(int k) { return k == 0 ? EIF_P_DX : (k == 1 ? EIF_P_DY : EIF_P_DAZ); }
 __global__ void k_adj_iter(int np, int first, double dt, double gdt, const double *__restrict__ pout,
                            double *__restrict__ xb, double *__restrict__ vpb, double *__restrict__ fb,

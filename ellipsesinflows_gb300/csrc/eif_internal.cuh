@@ -213,7 +213,7 @@ struct eif_ctx {
   bool weights_x_valid = false; // wcache holds the indicator weights of those boxes
   void *wcache = nullptr;       // indicator weight per IBM task slot (wcap entries)
   bool in_loop = false;                      // capturing the body of a sub-iteration loop
-  bool reset_in_stage_kernel = false;        // batch capture: the stage kernel resets the increments
+  bool reset_in_stage_kernel = false;        // capture with stage kernels: they reset the increments
   cudaGraphConditionalHandle loop_handle = 0;
   int ibm_ctas_per_sm[3] = {0, 0, 0};  // resident CTAs per SM of the IBM work kernels (FP64, mixed, mixed cached)
   unsigned *band_marks = nullptr;  // per band of 8 rows: bitmap over the 3*np (particle, image) boxes
@@ -232,11 +232,11 @@ struct eif_ctx {
   double *pd = nullptr;         // per-particle parameters of the indicator (double-precision form)
   double2 *tanh_tab = nullptr;  // tables of the indicator's tanh (double-precision form)
   int4 *tdesc;                  // task table: particle, row, columns and image of every chunk
+  // tasks of a stage start the memo did not serve: [0] count, then their numbers
+  int *memo_miss = nullptr;
+  bool memo_miss_zero = false;   // the box build's table kernel has cleared memo_miss[0]
   // weights of the last indicator evaluation in a sub-iteration loop (mixed form), with
   // the particles' geometry words, boxes and first tasks (WeightMemo in ibm_device.cuh)
-  // tasks of a stage start the memo did not serve: [0] count, then their numbers
-  bool memo_miss_zero = false;   // the box build's table kernel has cleared memo_miss[0]
-  int *memo_miss = nullptr;
   float *memo_w = nullptr, *memo_pf = nullptr;
   int *memo_box = nullptr, *memo_off = nullptr, *memo_valid = nullptr;
   bool memo_on = true;          // false: EIF_NO_MEMO set, every evaluation computes

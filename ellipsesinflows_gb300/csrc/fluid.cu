@@ -699,8 +699,8 @@ __device__ __forceinline__ void write_coef(double dt, float *coef, int lane) {
 constexpr int DT_BLOCKS = 32;
 
 __global__ void k_dt(const unsigned long long *__restrict__ colmax, const unsigned long long *__restrict__ uymax,
-                             const double *__restrict__ dxc, int itot, double dy, double lx, double dx_uniform,
-                             const double *__restrict__ P, int pcap, int np, double *__restrict__ part,
+                     const double *__restrict__ dxc, int itot, double dy, double lx, double dx_uniform,
+                     const double *__restrict__ P, int pcap, int np, double *__restrict__ part,
                      unsigned long long *__restrict__ done, double Re, double sf_adv, double sf_dif, double sf_par,
                      double *__restrict__ dt_out, float *__restrict__ coef) {
   const double small = 1.e-8;

@@ -895,8 +895,8 @@ struct AdjWorkArgs {
   double *geom;             // geo 1/2: per task slot th, gwx, gwy (3 x slots, by component)
   long long nslot;
   int geo;
-  int pcap, np, ld, mode, use_increment;
-  double dx, dy, ly, h;
+  int pcap, np, ld, mode;
+  double dx, dy, ly;
   Bounds bd;
 };
 
@@ -1064,8 +1064,8 @@ int launch_adj_pass(eif_ctx *c, const AdjPass &p) {
   w.geom = p.geom;
   w.nslot = (long long)c->wcap;
   w.geo = p.geom ? p.geo : 0;
-  w.pcap = c->pcap; w.np = c->np; w.ld = c->ld; w.mode = p.mode; w.use_increment = p.use_increment ? 1 : 0;
-  w.dx = c->dx; w.dy = c->dy; w.ly = c->ly; w.h = std::min(c->dx, c->dy);
+  w.pcap = c->pcap; w.np = c->np; w.ld = c->ld; w.mode = p.mode;
+  w.dx = c->dx; w.dy = c->dy; w.ly = c->ly;
   w.bd = bounds_of(c);
   const int blocks = std::max(1, std::min(c->sms * 8, (c->chunk_cap * 32 + 255) / 256));
   k_ibm_adj<<<blocks, 256, 0, c->stream>>>(w);

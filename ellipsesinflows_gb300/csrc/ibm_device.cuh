@@ -1,5 +1,5 @@
 // Device code of the immersed-boundary evaluations shared by the stand-alone
-// kernels (ibm.cu) and the batch's per-stage sub-iteration kernel (subiter.cu):
+// kernels (ibm.cu) and the persistent stage kernel (subiter.cu):
 // geometry helpers, the per-particle boxes, the task table and the per-task and
 // per-particle bodies of the volume integrals and the momentum exchange.
 //
@@ -1079,15 +1079,6 @@ __device__ __forceinline__ bool row_slots_in(const Bounds &bd, long long c, long
   return EIF_CHK(bd.rec, c * CHUNK, n, tag) && EIF_CHK(bd.rec, c * CHUNK + CHUNK - 1, n, tag);
 }
 
-// One warp per row task, single precision, WORK_ROWS rows at a time as in ibm_work_tasks (ONE:
-// the tasks of one particle). Bound by instruction issue: the foot iteration of the near cells,
-// and what a row needs before it (descriptor, parameters, the chords' roots and divisions). One
-// lane prepares a row, four rows at once, instead of every lane the same row; the near cells of
-// the four rows, about 25 a row, are packed onto the lanes together. 2048 ellipses of 12 to 25
-// cells: 108 -> 95 us (88 with the bounds checked by the row), 63-70 % of the issue slots; the
-// persistent kernel of 12 suspensions 611 -> 575 us a stage (24 ellipses alone, a row to a warp:
-// 1 % slower). The products of x_, y_ are
-// written out with the roundings that every form of this body has had.
 // single-precision partial sums of task c, reduced per particle by k_chunk_reduce_f
 __device__ __forceinline__ void store_sums_f(const WorkArgs &a, int c, float s0, float s1, float s2, int lane, int tag) {
   const float sum = warp_sum3(s0, s1, s2, lane);
@@ -1111,6 +1102,15 @@ struct WorkSlotsF {   // shared memory of a warp
 };
 static_assert(sizeof(WorkSlotsF) <= sizeof(WorkSlots) && alignof(WorkSlotsF) <= alignof(WorkSlots),
               "the persistent kernel has one array for both");
+// One warp per row task, single precision, WORK_ROWS rows at a time as in ibm_work_tasks (ONE:
+// the tasks of one particle). Bound by instruction issue: the foot iteration of the near cells,
+// and what a row needs before it (descriptor, parameters, the chords' roots and divisions). One
+// lane prepares a row, four rows at once, instead of every lane the same row; the near cells of
+// the four rows, about 25 a row, are packed onto the lanes together. 2048 ellipses of 12 to 25
+// cells: 108 -> 95 us (88 with the bounds checked by the row), 63-70 % of the issue slots; the
+// persistent kernel of 12 suspensions 611 -> 575 us a stage (24 ellipses alone, a row to a warp:
+// 1 % slower). The products of x_, y_ are written out with the roundings that every form of this
+// body has had.
 template <bool NC, bool ONE = false>
 __device__ __forceinline__ void ibm_work_f_tasks(const WorkArgs &a, int wmode, int first, int stride, WorkSlotsF &ws,
                                                  const OneParticle *one = nullptr) {

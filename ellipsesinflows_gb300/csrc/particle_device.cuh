@@ -1,6 +1,5 @@
 // Device code of the collision forces and the Crank-Nicolson increments, shared by
-// the stand-alone kernels (particles.cu) and the batch's per-stage sub-iteration
-// kernel (subiter.cu).
+// the stand-alone kernels (particles.cu) and the persistent stage kernel (subiter.cu).
 //
 // Reference functions restated here (NaokiHori/EllipsesInFlows):
 //   compute_evolute, find_equivalent_circle(s)   src/suspensions/collision.c:75-154

@@ -86,7 +86,7 @@ int launch_collision(eif_ctx *c, int cn) {
 
 int launch_reset_increments(eif_ctx *c) {
   c->incr_zero = true;
-  // in a batch graph the stage kernel before this front has reset the increments
+  // in a graph with stage kernels the one before this front has reset the increments
   if (c->np == 0 || c->reset_in_stage_kernel) return EIF_OK;
   EIF_PROF(c, "particle_reset", 1);
   k_reset<<<(c->np + 127) / 128, 128, 0, c->stream>>>(c->P, c->pcap, c->np);
