@@ -117,10 +117,18 @@ int tune_tiles(eif_ctx *c) {
     }
     const bool ibm = c->np > 0;
     const int tys[3] = {4, 8, 16};
-    // the double-precision predictor also with one or two rows per warp, where four leave fewer than
-    // 16 warps per SM (fastest up to 216 x 430; 256 x 512: 21.0 us at 2, 19.5 at 4)
+    // The double-precision predictor: the rows that leave 7.5 warps per SM or more, one and two
+    // where four leave fewer than 16, and one where no other does. It is timed alone, but runs beside
+    // the inertia in a step, where fewer warps tell: 512 x 1024 with 16 rows (7.2 warps) 55.2 us
+    // alone and with 8 rows 56.6, but 5.88 and 5.71 ms for a pass of four steps; 256 x 512 with 4
+    // rows (7.6) 19.5 us and with 2 rows 21.0, and the same passes.
     std::vector<int> rows(tys, tys + 3);
-    if (!mixed && predictor_warps(c, 4) < 16L * c->sms) rows.insert(rows.begin(), {1, 2});
+    if (!mixed) {
+      rows.clear();
+      for (int r : {1, 2, 4, 8, 16})
+        if ((r > 2 || predictor_warps(c, 4) < 16L * c->sms) && 2 * predictor_warps(c, r) >= 15L * c->sms) rows.push_back(r);
+      if (rows.empty()) rows.push_back(1);
+    }
     c->tiles.pred_set = true;
     float best = 1e30f;
     int pick = c->tiles.pred;
