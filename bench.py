@@ -69,13 +69,13 @@ HBM_BYTES = {
 # unchanged (otherwise null, marked stale)
 # (the DCT entries are the mean of the two passes' launches)
 _KPROF = "profiles/kernels_suspension_2048x4096_mixed.md"
-_FLUID_SHA = "2afdd44547a4d7470dac4d752b3dbe6f0c52ab4e"
-_POISSON_SHA = "7b859e57013264f78a70fa51d00e837ea3f919cd"
+_FLUID_SHA = "14b884fb460422dc2863d3c16327e3ac00734e13"
+_POISSON_SHA = "62f82ddc5b4c6d41231f7e91da0dca04d35e6523"
 NCU_TRAFFIC = {
     ("mixed", 2048, 4096): {
-        "predictor": (494.9e6, "fluid.cu", _FLUID_SHA, _KPROF),
-        "correct": (552.2e6, "fluid.cu", _FLUID_SHA, _KPROF),
-        "poisson_dct2": (195.5e6, "poisson.cu", _POISSON_SHA, _KPROF),
+        "predictor": (494.7e6, "fluid.cu", _FLUID_SHA, _KPROF),
+        "correct": (548.7e6, "fluid.cu", _FLUID_SHA, _KPROF),
+        "poisson_dct2": (194.2e6, "poisson.cu", _POISSON_SHA, _KPROF),
         "poisson_dct3": (33.7e6, "poisson.cu", _POISSON_SHA, _KPROF),
     },
 }
@@ -94,9 +94,9 @@ FP32_TFLOPS_MEASURED = 69.9
 
 # FP32 flops (FFMA counted twice, FADD and FMUL once) of the mixed-form indicator kernel
 # per normal-foot evaluation (all of the launch's flops, the far-cell tests and sums
-# included, over its evaluations): 9.03e8 flops in the captured launch of k_ibm_work_f
+# included, over its evaluations): 6.66e8 flops in the captured launch of k_ibm_work_f
 # over the 2.86e6 evaluations that launch counts at this workload (value, source)
-INDICATOR_FLOPS_PER_EVAL = (316, "ncu capture of k_ibm_work_f, " + "profiles/kernels_suspension_2048x4096_mixed.md")
+INDICATOR_FLOPS_PER_EVAL = (233, "ncu capture of k_ibm_work_f, " + "profiles/kernels_suspension_2048x4096_mixed.md")
 
 
 def parse():
