@@ -803,6 +803,13 @@ int eif_adjoint_backward(eif_ctx *c) {
       a->geom_cap = adj_slot_cap(c);
       EIF_CK(c, cudaMalloc((void **)&a->geom, sizeof(double) * 3 * a->geom_cap));
     }
+    // a larger particle set pushed and taken back since begin leaves the records' pitch larger
+    if (c->pcap > a->pcap) {
+      cudaFree(a->pbackup);
+      a->pbackup = nullptr;
+      a->pcap = c->pcap;
+      EIF_CK(c, cudaMalloc((void **)&a->pbackup, sizeof(double) * EIF_NFIELDS * a->pcap));
+    }
     EIF_CK(c, cudaMemcpyAsync(a->pbackup, c->P, sizeof(double) * EIF_NFIELDS * c->pcap, cudaMemcpyDeviceToDevice,
                               c->stream));
   }
